@@ -107,6 +107,137 @@ gemv_rows_kernel(const uint8_t* __restrict__ W, int64_t row_bytes, int64_t rows,
   }
 }
 
+// Three rows of activations and more.  The kernel above reads every activation from L1 once per weight row: with eight of them a
+// warp moves 16 bytes of activations per byte of BF16 weights, and the load path, not HBM, sets the time (32000 x 2048 BF16,
+// eight rows: 158 us for 131 MB).  Here a warp works on R weight rows, the CTA's warps share a tile of the activations in shared
+// memory, and each value read from it serves R rows.  Activations of two rows lie side by side in the tile, so that one
+// fma.rn.f32x2 carries two sums.  A sum is formed as above: per lane in ascending columns, then the shuffles; a row's result
+// is the same alone and in a batch.  Bound: the FMA pipe and the shared-memory reads, which four weight rows per warp balance.
+// Measured, 32000 x 2048 BF16: 3 / 8 / 16 rows 62 / 144 / 287 -> 37 / 49 / 92 us; 4096 x 4104 F32, 7 rows 59 -> 25 us.
+// RUNS (batches of more than 32 rows): a lane's sum is closed every 512 columns (256 up to 2048 columns) and added to the row's, which keeps the rounding
+// error below that of the staged kernel, which served such batches at 8 rows per pass (14336 x 4096 F16, 100 rows: 2234 us).
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+  return v;
+}
+__device__ __forceinline__ void fma2(unsigned long long& s, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s) : "l"(a), "l"(b));
+}
+template <int T> struct WideTile { static constexpr int SLOTS = T / 2 * 4 * 32; };  // 16-byte slots: (pair of rows, two columns, lane)
+template <int DT, int T, int R, bool RUNS>
+__global__ void __launch_bounds__(ROW_WARPS * 32, R * T * (DT == DT_F32 || RUNS ? 2 : 1) >= 64 ? 1 : 2)
+gemv_rows_wide_kernel(const uint8_t* __restrict__ W, int64_t row_bytes, int64_t rows, int64_t cols, const float* __restrict__ X,
+                      float* __restrict__ Y, int tokens) {
+  constexpr int NP = T / 2, FILL = (NP * 64 + ROW_WARPS * 32 - 1) / (ROW_WARPS * 32);  // float4 pairs of a tile per thread
+  __shared__ __align__(16) uint4 tile[2][WideTile<T>::SLOTS];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int64_t row0 = (int64_t)blockIdx.x * (ROW_WARPS * R) + (tid >> 5) * R;
+  const uint8_t* wr[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) wr[r] = W + (row0 + r < rows ? row0 + r : rows - 1) * row_bytes;
+  unsigned long long acc[R][NP], sum[RUNS ? R : 1][RUNS ? NP : 1];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      acc[r][p] = 0ull;
+      if (RUNS) sum[r][p] = 0ull;
+    }
+
+  float4 xa[FILL], xb[FILL];
+  auto load_x = [&](int64_t c0) {  // four columns of two activation rows per piece; rows and columns beyond the end are zeros
+#pragma unroll
+    for (int f = 0; f < FILL; ++f) {
+      const int piece = f * ROW_WARPS * 32 + tid, p = piece >> 6;
+      const int64_t c = c0 + 4 * (piece & 63);
+      xa[f] = xb[f] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (piece < NP * 64 && c < cols) {
+        if (2 * p < tokens) xa[f] = __ldg((const float4*)(X + (int64_t)(2 * p) * cols + c));
+        if (2 * p + 1 < tokens) xb[f] = __ldg((const float4*)(X + (int64_t)(2 * p + 1) * cols + c));
+      }
+    }
+  };
+  auto store_x = [&](int buf) {
+#pragma unroll
+    for (int f = 0; f < FILL; ++f) {
+      const int piece = f * ROW_WARPS * 32 + tid, p = piece >> 6, q = piece & 63;
+      if (piece >= NP * 64) break;
+      float4* at = (float4*)&tile[buf][(p * 4 + 2 * (q & 1)) * 32 + (q >> 1)];
+      at[0] = make_float4(xa[f].x, xb[f].x, xa[f].y, xb[f].y);
+      at[32] = make_float4(xa[f].z, xb[f].z, xa[f].w, xb[f].w);
+    }
+  };
+  Raw8<DT> raw[2][R];
+  auto load_w = [&](int64_t c, Raw8<DT> (&to)[R]) {
+    if (c < cols) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) fetch8<DT>(wr[r], c, to[r]);
+    }
+  };
+  load_w(8 * lane, raw[0]);
+  load_x(0);
+  store_x(0);
+  __syncthreads();
+  auto step = [&](int64_t c0, int buf, Raw8<DT> (&now)[R], Raw8<DT> (&next)[R]) {
+    load_w(c0 + 256 + 8 * lane, next);
+    load_x(c0 + 256);
+    if (c0 + 8 * lane < cols) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {  // four columns at a time
+        unsigned long long w2[R][4];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          float w[8];
+          widen8<DT>(now[r], w);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) w2[r][k] = pack2(w[4 * h + k], w[4 * h + k]);
+        }
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+          const ulonglong2 u = *(const ulonglong2*)&tile[buf][(p * 4 + 2 * h) * 32 + lane];
+          const ulonglong2 v = *(const ulonglong2*)&tile[buf][(p * 4 + 2 * h + 1) * 32 + lane];
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            fma2(acc[r][p], w2[r][0], u.x); fma2(acc[r][p], w2[r][1], u.y);
+            fma2(acc[r][p], w2[r][2], v.x); fma2(acc[r][p], w2[r][3], v.y);
+          }
+        }
+      }
+    }
+    store_x(buf ^ 1);
+    __syncthreads();
+  };
+  auto close_run = [&] {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum[RUNS ? r : 0][RUNS ? p : 0]) : "l"(acc[r][p]));
+        acc[r][p] = 0ull;
+      }
+  };
+  for (int64_t c0 = 0; c0 < cols; c0 += 512) {
+    step(c0, 0, raw[0], raw[1]);
+    if (RUNS && cols <= 2048) close_run();
+    if (c0 + 256 < cols) step(c0 + 256, 1, raw[1], raw[0]);
+    if (RUNS) close_run();
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const unsigned long long v = RUNS ? sum[RUNS ? r : 0][RUNS ? p : 0] : acc[r][p];
+      float a = __uint_as_float((uint32_t)v), b = __uint_as_float((uint32_t)(v >> 32));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) { a += __shfl_xor_sync(~0u, a, o); b += __shfl_xor_sync(~0u, b, o); }
+      if (lane == 0 && row0 + r < rows) {
+        if (2 * p < tokens) Y[(int64_t)(2 * p) * rows + row0 + r] = a;
+        if (2 * p + 1 < tokens) Y[(int64_t)(2 * p + 1) * rows + row0 + r] = b;
+      }
+    }
+}
+
 // Rows i and n + i of a stacked gate | up matrix by one warp, which then has both factors of result i: half the pieces in
 // flight per row, two rows at a time.
 template <int DT, int MT>
@@ -183,12 +314,23 @@ cudaError_t launch_rows(const MatView& m, const float* x, float* y, int tokens, 
   return cudaGetLastError();
 }
 
+template <int DT, int T, int R, bool RUNS = false>
+cudaError_t launch_rows_wide(const MatView& m, const float* x, float* y, int tokens, cudaStream_t stream) {
+  gemv_rows_wide_kernel<DT, T, R, RUNS><<<(unsigned)((m.rows + ROW_WARPS * R - 1) / (ROW_WARPS * R)), ROW_WARPS * 32, 0, stream>>>(
+      m.w, m.row_bytes, m.rows, m.cols, x, y, tokens);
+  return cudaGetLastError();
+}
+
 template <int DT>
-cudaError_t launch_rows_mt(const MatView& m, const float* x, float* y, int tokens, cudaStream_t stream, int sm_count) {
+cudaError_t launch_rows_mt(const MatView& m, const float* x, float* y, int tokens, bool runs, cudaStream_t stream, int sm_count) {
+  if (runs) return launch_rows_wide<DT, 8, 4, true>(m, x, y, tokens, stream);
   if (tokens == 1) return launch_rows<DT, 1>(m, x, y, tokens, stream, sm_count);
   if (tokens == 2) return launch_rows<DT, 2>(m, x, y, tokens, stream, sm_count);
-  if (tokens <= 4) return launch_rows<DT, 4>(m, x, y, tokens, stream, sm_count);
-  return launch_rows<DT, 8>(m, x, y, tokens, stream, sm_count);
+  // four weight rows per warp, two where they would leave SMs without a block
+  const bool few = m.rows < (int64_t)sm_count * 2 * ROW_WARPS * 4;
+  if (tokens <= 4) return few ? launch_rows_wide<DT, 4, 2>(m, x, y, tokens, stream) : launch_rows_wide<DT, 4, 4>(m, x, y, tokens, stream);
+  if (tokens <= 8) return few ? launch_rows_wide<DT, 8, 2>(m, x, y, tokens, stream) : launch_rows_wide<DT, 8, 4>(m, x, y, tokens, stream);
+  return few ? launch_rows_wide<DT, 16, 2>(m, x, y, tokens, stream) : launch_rows_wide<DT, 16, 4>(m, x, y, tokens, stream);
 }
 
 }  // namespace
@@ -209,14 +351,16 @@ bool gemv_rows_supported(const MatView& m) {
 
 cudaError_t launch_gemv_rows(const MatView& m, const float* x, float* y, int64_t tokens, cudaStream_t stream, int sm_count,
                              uint64_t* launches) {
-  for (int64_t t0 = 0; t0 < tokens; t0 += 8) {
-    const int nt = (int)(tokens - t0 < 8 ? tokens - t0 : 8);
+  const bool runs = tokens > 32;
+  const int64_t pass = runs ? 8 : 16;
+  for (int64_t t0 = 0; t0 < tokens; t0 += pass) {
+    const int nt = (int)(tokens - t0 < pass ? tokens - t0 : pass);
     const float* xp = x + t0 * m.cols;
     float* yp = y + t0 * m.rows;
     cudaError_t e;
-    if (m.dtype == DT_F32) e = launch_rows_mt<DT_F32>(m, xp, yp, nt, stream, sm_count);
-    else if (m.dtype == DT_F16) e = launch_rows_mt<DT_F16>(m, xp, yp, nt, stream, sm_count);
-    else e = launch_rows_mt<DT_BF16>(m, xp, yp, nt, stream, sm_count);
+    if (m.dtype == DT_F32) e = launch_rows_mt<DT_F32>(m, xp, yp, nt, runs, stream, sm_count);
+    else if (m.dtype == DT_F16) e = launch_rows_mt<DT_F16>(m, xp, yp, nt, runs, stream, sm_count);
+    else e = launch_rows_mt<DT_BF16>(m, xp, yp, nt, runs, stream, sm_count);
     if (e != cudaSuccess) return e;
     if (launches) ++*launches;
   }

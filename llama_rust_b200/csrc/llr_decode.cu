@@ -158,16 +158,24 @@ __device__ __forceinline__ void rope_in_place(float* vecs, int n_vec, int hd, in
   }
 }
 
+// The rows of a batch that a block of an attention kernel works on: runs [first, first + n) of at most 64 rows of ONE sequence at
+// consecutive positions, n << 16 | first.
+constexpr int MAX_TILES = 512;
+struct RowTiles {
+  int n;
+  uint32_t run[MAX_TILES];
+  __device__ __forceinline__ int begin(int z) const { return (int)(run[z] & 0xffff); }
+  __device__ __forceinline__ int end(int z) const { return begin(z) + (int)(run[z] >> 16); }
+};
+
 // grid (kv head, position slice, token): one row per block, K and V straight from the paged cache (decode steps).
 // With k_new / v_new (a single decode token) the kernel also does what rope_store_kernel does for that token: q is
 // rotated as it is loaded, and the block whose slice holds the token's position rotates the new key, writes it and
 // the new value into the cache and then reads them back like any other position: one launch less per layer.
-__global__ void __launch_bounds__(ATT_THREADS)
-attention_partial_kernel(const float* __restrict__ q, KvView kv, float* __restrict__ part, RowMap rows, int layer, int chunk,
-                         WalkShape w, const float* __restrict__ k_new, const float* __restrict__ v_new) {
-  pdl_enter();
+__device__ __forceinline__ void attention_partial_row(const float* __restrict__ q, const KvView& kv, float* __restrict__ part, const RowMap& rows, int t, int layer,
+                                                      int chunk, const WalkShape& w, const float* __restrict__ k_new, const float* __restrict__ v_new) {
   extern __shared__ float sm[];  // q[gqa][hd] | scores[gqa][chunk] or sums[P][gqa][hd]
-  const int hkv = blockIdx.x, split = blockIdx.y, t = blockIdx.z;
+  const int hkv = blockIdx.x, split = blockIdx.y;
   const int hd = w.head_dim, gqa = w.n_head / w.n_head_kv;
   const int seq = row_position(rows, t) + 1;  // positions this row attends to
   const int sid = row_sequence(rows, t);
@@ -197,6 +205,19 @@ attention_partial_kernel(const float* __restrict__ q, KvView kv, float* __restri
   __syncthreads();
   float* out = part + (((int64_t)t * w.n_head_kv + hkv) * n_split + split) * gqa * (hd + 2);
   attend_slice<ATT_THREADS>(KvGlobal{kv, sid, layer, hkv, w.n_head_kv, hd, 1.0f / sqrtf((float)hd)}, sq, sc, out, s0, s1, chunk, hd, hd, gqa);
+}
+__global__ void __launch_bounds__(ATT_THREADS)
+attention_partial_kernel(const float* __restrict__ q, KvView kv, float* __restrict__ part, RowMap rows, int layer, int chunk,
+                         WalkShape w, const float* __restrict__ k_new, const float* __restrict__ v_new) {
+  pdl_enter();
+  attention_partial_row(q, kv, part, rows, blockIdx.z, layer, chunk, w, k_new, v_new);
+}
+// the listed rows of a batch, one per blockIdx.z
+__global__ void __launch_bounds__(ATT_THREADS)
+attention_rows_kernel(const float* __restrict__ q, KvView kv, float* __restrict__ part, RowMap rows, int layer, int chunk, WalkShape w,
+                      const __grid_constant__ RowTiles tiles) {
+  pdl_enter();
+  attention_partial_row(q, kv, part, rows, tiles.begin(blockIdx.z), layer, chunk, w, nullptr, nullptr);
 }
 
 // The same slice of one row done by ONE warp, every elementary sum formed in the order attend_slice forms it (a
@@ -296,13 +317,14 @@ __device__ __forceinline__ void attend_slice_warp(const KV& src, const float* sq
     }
 }
 
-// grid (kv head, position slice, group of ATT_ROWS rows): the rows of a prompt chunk share the slice's key and value
-// rows, which the block stages in shared memory once per run of rows of one sequence; each warp then takes rows of
-// its own, with no block-wide barrier between rows.
+// grid (kv head, position slice, run of up to ATT_ROWS rows of one sequence): the rows share the slice's key and value rows,
+// which the block stages in shared memory once; each warp then takes rows of its own, with no block-wide barrier between rows.
+// (A block that took the next sixteen rows of a ragged batch, whatever their sequences, staged a slice per sequence one after
+// the other: 24 rows of 24 sequences 129 us.)
 template <int GQA, int P>
 __global__ void __launch_bounds__(ATT_THREADS, 3)
 attention_tile_kernel(const float* __restrict__ q, KvView kv, float* __restrict__ part, RowMap rows, int layer, int chunk,
-                      WalkShape w, int tokens) {
+                      WalkShape w, const __grid_constant__ RowTiles tiles) {
   pdl_enter();
   extern __shared__ float sm[];  // k tile [chunk][hd] | v tile [chunk][hd] | per warp: q[gqa][hd], scores[gqa][chunk]
   constexpr int hd = ATT_THREADS / P, gqa = GQA;
@@ -316,41 +338,28 @@ attention_tile_kernel(const float* __restrict__ q, KvView kv, float* __restrict_
   float* sc = vt + chunk * hd + nw * gqa * hd + warp * gqa * chunk;
   // the last rows first: in a prompt chunk they attend to the most slices, the blocks of the first rows (which leave at once for
   // the slices beyond them) then fill the tail
-  const int t_begin = ((int)gridDim.z - 1 - (int)blockIdx.z) * ATT_ROWS, t_end = min(tokens, t_begin + ATT_ROWS);
-  // sequence and position of the group's rows, fetched in one go (the runs below are found in shared memory)
-  __shared__ int s_seq[ATT_ROWS], s_pos[ATT_ROWS];
-  if (threadIdx.x < ATT_ROWS && t_begin + (int)threadIdx.x < t_end) {
-    s_seq[threadIdx.x] = row_sequence(rows, t_begin + threadIdx.x);
-    s_pos[threadIdx.x] = row_position(rows, t_begin + threadIdx.x);
+  const int t_begin = tiles.begin((int)gridDim.z - 1 - (int)blockIdx.z), t_end = tiles.end((int)gridDim.z - 1 - (int)blockIdx.z);
+  const int sid = row_sequence(rows, t_begin), p0 = row_position(rows, t_begin);
+  // positions [s0, s0 + need) lie in blocks the sequence owns: a row's position is below its reserved length
+  const int need = min(p0 + t_end - t_begin, s0 + chunk) - s0;
+  if (need <= 0) return;
+  constexpr int vec = hd / 4;
+  for (int idx = threadIdx.x; idx < need * vec; idx += ATT_THREADS) {
+    const int p = idx / vec, c = idx % vec;
+    const int64_t off = kv_offset(kv, sid, layer, hkv, s0 + p, w.n_head_kv, hd);
+    ((float4*)(kt + p * hd))[c] = ((const float4*)(kv.k + off))[c];
+    ((float4*)(vt + p * hd))[c] = ((const float4*)(kv.v + off))[c];
   }
   __syncthreads();
-  for (int t = t_begin; t < t_end;) {  // runs of rows of one sequence; everything here is block-uniform
-    const int sid = s_seq[t - t_begin];
-    int u = t, need = 0;
-    for (; u < t_end && s_seq[u - t_begin] == sid; ++u) need = max(need, min(s_pos[u - t_begin] + 1, s0 + chunk) - s0);
-    if (need > 0) {
-      // positions [s0, s0 + need) lie in blocks the sequence owns: a row's position is below its reserved length
-      __syncthreads();  // the previous run's readers are done with the tile
-      constexpr int vec = hd / 4;
-      for (int idx = threadIdx.x; idx < need * vec; idx += ATT_THREADS) {
-        const int p = idx / vec, c = idx % vec;
-        const int64_t off = kv_offset(kv, sid, layer, hkv, s0 + p, w.n_head_kv, hd);
-        ((float4*)(kt + p * hd))[c] = ((const float4*)(kv.k + off))[c];
-        ((float4*)(vt + p * hd))[c] = ((const float4*)(kv.v + off))[c];
-      }
-      __syncthreads();
-      for (int r = t + warp; r < u; r += nw) {
-        const int seq = s_pos[r - t_begin] + 1;
-        if (s0 >= seq) continue;
-        const int s1 = min(seq, s0 + chunk);
-        for (int i = lane; i < gqa * hd; i += 32) sq[i] = q[((int64_t)r * w.n_head + hkv * gqa) * hd + i];
-        __syncwarp();
-        float* out = part + (((int64_t)r * w.n_head_kv + hkv) * n_split + split) * gqa * (hd + 2);
-        attend_slice_warp<GQA, P>(KvTile{kt, vt, s0, hd}, sq, sc, out, s0, s1, chunk);
-        __syncwarp();
-      }
-    }
-    t = u;
+  for (int r = t_begin + warp; r < t_end; r += nw) {
+    const int seq = p0 + r - t_begin + 1;
+    if (s0 >= seq) continue;
+    const int s1 = min(seq, s0 + chunk);
+    for (int i = lane; i < gqa * hd; i += 32) sq[i] = q[((int64_t)r * w.n_head + hkv * gqa) * hd + i];
+    __syncwarp();
+    float* out = part + (((int64_t)r * w.n_head_kv + hkv) * n_split + split) * gqa * (hd + 2);
+    attend_slice_warp<GQA, P>(KvTile{kt, vt, s0, hd}, sq, sc, out, s0, s1, chunk);
+    __syncwarp();
   }
 }
 
@@ -375,8 +384,8 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], u
 
 template <int GQA, int HD, int NT, int RT>
 __global__ void __launch_bounds__(32 * GQA * RT)
-attention_tile_mma_kernel(const float* __restrict__ q, KvView kv, float* __restrict__ part, RowMap rows, int layer, WalkShape w, int tokens,
-                          int n_split) {
+attention_tile_mma_kernel(const float* __restrict__ q, KvView kv, float* __restrict__ part, RowMap rows, int layer, WalkShape w,
+                          int n_split, const __grid_constant__ RowTiles tiles) {
   pdl_enter();
   // strides in 32-bit words (two binary16 each); + 4 words spreads the fragment reads of eight rows over all banks
   constexpr int CH = 8 * NT, KW = HD / 2 + 4, VW = CH / 2 + 4, QW = HD / 2 + 4, PW = CH / 2 + 4, NW = GQA * RT, NTHR = 32 * NW;
@@ -388,10 +397,10 @@ attention_tile_mma_kernel(const float* __restrict__ q, KvView kv, float* __restr
   uint32_t* pw = vt + HD * VW + NW * 16 * QW + warp * 16 * PW;
   const int hkv = blockIdx.x, head = warp % GQA;  // a warp: one query head of the group, sixteen of the block's 16 RT rows
   // the last rows first: they attend to the most positions, and the short blocks of the first rows then fill the tail
-  const int b_begin = ((int)gridDim.z - 1 - (int)blockIdx.z) * (16 * RT), b_rows = min(tokens - b_begin, 16 * RT);
+  const int b_begin = tiles.begin((int)gridDim.z - 1 - (int)blockIdx.z), b_end = tiles.end((int)gridDim.z - 1 - (int)blockIdx.z), b_rows = b_end - b_begin;
   const int last_pos = row_position(rows, b_begin) + b_rows - 1;  // of the block: the slices it walks
   if ((int)blockIdx.y * CH > last_pos) return;
-  const int t_begin = b_begin + 16 * (warp / GQA), n_rows = max(0, min(tokens - t_begin, 16));
+  const int t_begin = b_begin + 16 * (warp / GQA), n_rows = max(0, min(b_end - t_begin, 16));
   const int p0 = row_position(rows, b_begin) + 16 * (warp / GQA);  // row r of the warp stands at position p0 + r
   const int sid = row_sequence(rows, b_begin);
   constexpr int vec = HD / 4;
@@ -514,12 +523,22 @@ attention_tile_mma_kernel(const float* __restrict__ q, KvView kv, float* __restr
   }
 }
 
+// Rows whose records the tensor-core kernel left: at most eight groups of 64 rows and more in a batch of 512.
+struct RowRanges {
+  int n, lo[8], hi[8];
+  __device__ __forceinline__ bool has(int t) const {
+    for (int i = 0; i < n; ++i)
+      if (t >= lo[i] && t < hi[i]) return true;
+    return false;
+  }
+};
+
 // grid (query heads / 4, token), one warp per query head: merges the position slices (at most 32).  Lane sp turns
 // slice sp's maximum into the weight exp(m_slice - m); the denominator is the shuffle-tree sum of the weighted slice
 // sums; then every lane adds its dimensions over the slices in ascending order, the weights coming by shuffle.
 __global__ void __launch_bounds__(128)
 attention_combine_kernel(const float* __restrict__ part, float* __restrict__ out, RowMap rows, int chunk, WalkShape w, int heads_per_block,
-                         int max_records, int record_chunk) {
+                         int max_records, int record_chunk, const __grid_constant__ RowRanges mma_rows) {
   pdl_enter();
   // heads_per_block 4: one warp per head (many rows: fewer, fuller blocks); 1: the four warps share a head's
   // dimensions (a decode step has few blocks to fill the device with)
@@ -533,6 +552,7 @@ attention_combine_kernel(const float* __restrict__ part, float* __restrict__ out
   // chunk: positions per slice of the f32 kernels, which fixes the room a row's records take.  The tensor-core kernel
   // walks slices of record_chunk positions of its own and leaves one record per walked run of slices, at the first
   // max_records indices.
+  if (!mma_rows.has(t)) { max_records = 32; record_chunk = chunk; }
   const int n_split = (w.n_ctx + chunk - 1) / chunk, used = min(min(n_split, (seq + record_chunk - 1) / record_chunk), max_records);
   const float* base = part + ((int64_t)t * w.n_head_kv + hkv) * n_split * gqa * (hd + 2) + g * (hd + 2);
   const int64_t stride = (int64_t)gqa * (hd + 2);
@@ -740,41 +760,65 @@ size_t attention_scratch_floats(int tokens, const WalkShape& w) {
   return (size_t)tokens * w.n_head_kv * attention_splits(w) * (w.n_head / w.n_head_kv) * (w.head_dim + 2);
 }
 
-cudaError_t launch_attention(const float* q, const KvView& kv, float* out, float* scratch, const RowMap& rows, int tokens,
-                             int layer, const WalkShape& w, cudaStream_t s, uint64_t* launches, const float* k_new, const float* v_new,
-                             bool tensor_cores, bool one_sequence) {
-  if (tokens <= 0) return cudaSuccess;
-  const int gqa = w.n_head / w.n_head_kv;
+// shared memory of the per-row kernels, checked and allowed; 0: the shape is not served
+static cudaError_t attention_rows_smem(const WalkShape& w, size_t* out) {
+  const int gqa = w.n_head / w.n_head_kv, max_chunk = attention_chunk(w);
   if (gqa < 1 || gqa > ATT_MAX_GQA || w.n_head % w.n_head_kv != 0 || w.head_dim > ATT_THREADS) return cudaErrorInvalidValue;
-  const int splits = attention_splits(w);
-  const int max_chunk = attention_chunk(w);
   const size_t groups = ATT_THREADS / w.head_dim > 0 ? ATT_THREADS / w.head_dim : 1;
   const size_t score_floats = (size_t)gqa * max_chunk > groups * gqa * w.head_dim ? (size_t)gqa * max_chunk : groups * gqa * w.head_dim;
   const size_t smem = ((size_t)gqa * w.head_dim + score_floats + 32) * sizeof(float);
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
-  static PerDevice configured;  // largest size the kernel has been allowed on this device
+  static PerDevice configured;  // largest size the kernels have been allowed on this device
   std::atomic<int>& allowed = configured.here();
   if (smem > 48 * 1024 && (int)smem > allowed.load(std::memory_order_relaxed)) {
     cudaError_t e = cudaFuncSetAttribute(attention_partial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     allowed.store((int)smem, std::memory_order_relaxed);
   }
+  *out = smem;
+  return cudaSuccess;
+}
+
+cudaError_t launch_attention(const float* q, const KvView& kv, float* out, float* scratch, const RowMap& rows, int layer, const WalkShape& w, cudaStream_t s,
+                             uint64_t* launches, const float* k_new, const float* v_new) {
+  size_t smem = 0;
+  cudaError_t e = attention_rows_smem(w, &smem);
+  if (e != cudaSuccess) return e;
+  const int splits = attention_splits(w), chunk = attention_chunk(w);
   if (launches) *launches += 2;
-  cudaError_t e;
+  e = launch_walk(attention_partial_kernel, dim3(w.n_head_kv, splits, 1), dim3(ATT_THREADS), smem, s, q, kv, scratch, rows, layer, chunk, w, k_new, v_new);
+  if (e != cudaSuccess) return e;
+  return launch_walk(attention_combine_kernel, dim3(w.n_head, 1), dim3(128), 0, s, (const float*)scratch, out, rows, chunk, w, 1, splits, chunk, RowRanges{});
+}
+
+cudaError_t launch_attention_groups(const float* q, const KvView& kv, float* out, float* scratch, const RowMap& rows, int tokens, int layer, const WalkShape& w,
+                                    const AttentionGroup* groups, int n_groups, bool tensor_cores, cudaStream_t s, uint64_t* launches) {
+  if (tokens <= 0) return cudaSuccess;
+  if (tokens > MAX_TILES) return cudaErrorInvalidValue;
+  const int gqa = w.n_head_kv > 0 ? w.n_head / w.n_head_kv : 0;
+  size_t smem = 0;
+  cudaError_t e = attention_rows_smem(w, &smem);
+  if (e != cudaSuccess) return e;
+  const int splits = attention_splits(w);
+  const int max_chunk = attention_chunk(w);
+  const AttentionGroup all{0, tokens};
+  if (!groups) { groups = &all; n_groups = 1; }
   // prompt chunks: rows of a group share the slice's keys and values through a shared-memory tile
   const size_t tile_smem = (2 * (size_t)max_chunk * w.head_dim + (ATT_THREADS / 32) * ((size_t)gqa * w.head_dim + (size_t)gqa * max_chunk)) * sizeof(float);
-  void (*tile)(const float*, KvView, float*, RowMap, int, int, WalkShape, int) = nullptr;
+  void (*tile)(const float*, KvView, float*, RowMap, int, int, WalkShape, const RowTiles) = nullptr;
 #define LLR_TILE(G, PP) if (gqa == G && w.head_dim == ATT_THREADS / PP) tile = attention_tile_kernel<G, PP>;
   LLR_TILE(1, 1) LLR_TILE(2, 1) LLR_TILE(4, 1) LLR_TILE(1, 2) LLR_TILE(2, 2) LLR_TILE(4, 2) LLR_TILE(8, 2)
   LLR_TILE(1, 4) LLR_TILE(2, 4) LLR_TILE(4, 4) LLR_TILE(8, 4)
 #undef LLR_TILE
-  // a prompt chunk of one sequence at consecutive positions, when the caller allows 16-bit operands: tensor cores
-  void (*mma)(const float*, KvView, float*, RowMap, int, WalkShape, int, int) = nullptr;
+  if (max_chunk > ATT_TILE_CHUNK || tile_smem > 200 * 1024) tile = nullptr;
+  // groups long enough, when the caller allows 16-bit operands: tensor cores
+  void (*mma)(const float*, KvView, float*, RowMap, int, WalkShape, int, const RowTiles) = nullptr;
   size_t mma_smem = 0;
   int mma_rt = 1;
   // its slices are its own (64 positions; 32 when the context is short): the records it leaves do not depend on max_chunk
   const int mma_chunk = w.n_ctx > 1024 ? 64 : 32;
-  if (tensor_cores && (one_sequence || (!rows.row_pos && !rows.row_seq)) && tokens >= 64 && (w.head_dim == 64 || w.head_dim == 128)) {
+  if (tensor_cores && (w.head_dim == 64 || w.head_dim == 128)) {
 #define LLR_MMA(G, H, N) if (gqa == G && w.head_dim == H && mma_chunk == 8 * N) mma = attention_tile_mma_kernel<G, H, N, (G <= 4 ? 4 : 2)>;
     LLR_MMA(1, 64, 4) LLR_MMA(2, 64, 4) LLR_MMA(4, 64, 4) LLR_MMA(8, 64, 4) LLR_MMA(1, 64, 8) LLR_MMA(2, 64, 8) LLR_MMA(4, 64, 8) LLR_MMA(8, 64, 8)
     LLR_MMA(1, 128, 4) LLR_MMA(2, 128, 4) LLR_MMA(4, 128, 4) LLR_MMA(8, 128, 4) LLR_MMA(1, 128, 8) LLR_MMA(2, 128, 8) LLR_MMA(4, 128, 8) LLR_MMA(8, 128, 8)
@@ -782,32 +826,42 @@ cudaError_t launch_attention(const float* q, const KvView& kv, float* out, float
     mma_rt = gqa <= 4 ? 4 : 2;  // sixteen-row tiles per block
     mma_smem = ((size_t)mma_chunk * (w.head_dim / 2 + 4) + (size_t)w.head_dim * (mma_chunk / 2 + 4) +
                 (size_t)gqa * mma_rt * 16 * (w.head_dim / 2 + 4 + mma_chunk / 2 + 4)) * sizeof(uint32_t);
+    if (mma_smem > 200 * 1024) mma = nullptr;
   }
-  int max_records = splits, record_chunk = max_chunk;
-  if (mma && mma_smem <= 200 * 1024) {
-    const int mma_splits = (w.n_ctx + mma_chunk - 1) / mma_chunk;
-    max_records = std::min(std::min(mma_splits, splits), 4);
-    record_chunk = mma_chunk;
-    if (mma_smem > 48 * 1024) {
-      e = cudaFuncSetAttribute((const void*)mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mma_smem);
-      if (e != cudaSuccess) return e;
-    }
-    e = launch_walk(mma, dim3(w.n_head_kv, max_records, (tokens + 16 * mma_rt - 1) / (16 * mma_rt)), dim3(32 * gqa * mma_rt), mma_smem,
-                    s, q, kv, scratch, rows, layer, w, tokens, splits);
-  } else if (tile && tokens >= 4 && max_chunk <= ATT_TILE_CHUNK && tile_smem <= 200 * 1024) {
-    if (tile_smem > 48 * 1024) {
-      e = cudaFuncSetAttribute((const void*)tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem);
-      if (e != cudaSuccess) return e;
-    }
-    e = launch_walk(tile, dim3(w.n_head_kv, splits, (tokens + ATT_ROWS - 1) / ATT_ROWS), dim3(ATT_THREADS), tile_smem, s, q, kv, scratch,
-                    rows, layer, max_chunk, w, tokens);
-  } else {
-    e = launch_walk(attention_partial_kernel, dim3(w.n_head_kv, splits, tokens), dim3(ATT_THREADS), smem, s, q, kv, scratch, rows, layer,
-                    max_chunk, w, tokens == 1 ? k_new : (const float*)nullptr, tokens == 1 ? v_new : (const float*)nullptr);
+  // Every group goes to one of three kernels, one launch each: binary16 MMAs (64 rows and more), the tiled f32 kernel (four rows
+  // and more: below that a block of eight warps would have work for one to three), the f32 kernel of a block per row.
+  RowTiles big{}, tiled{}, single{};
+  RowRanges mma_rows{};
+  for (int g = 0; g < n_groups; ++g) {
+    const int first = groups[g].first, n = groups[g].rows;
+    const bool on_mma = mma && n >= 64 && mma_rows.n < 8;
+    RowTiles& to = on_mma ? big : tile && n >= 4 ? tiled : single;
+    const int per = on_mma ? 16 * mma_rt : tile && n >= 4 ? ATT_ROWS : 1;
+    for (int r = 0; r < n; r += per) to.run[to.n++] = (uint32_t)std::min(per, n - r) << 16 | (uint32_t)(first + r);
+    if (on_mma) { mma_rows.lo[mma_rows.n] = first; mma_rows.hi[mma_rows.n++] = first + n; }
   }
-  if (e != cudaSuccess) return e;
+  int max_records = splits;
+  if (big.n) {
+    if (launches) ++*launches;
+    max_records = std::min(std::min((w.n_ctx + mma_chunk - 1) / mma_chunk, splits), 4);
+    if (mma_smem > 48 * 1024 && (e = cudaFuncSetAttribute((const void*)mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mma_smem)) != cudaSuccess) return e;
+    e = launch_walk(mma, dim3(w.n_head_kv, max_records, big.n), dim3(32 * gqa * mma_rt), mma_smem, s, q, kv, scratch, rows, layer, w, splits, big);
+    if (e != cudaSuccess) return e;
+  }
+  if (tiled.n) {
+    if (launches) ++*launches;
+    if (tile_smem > 48 * 1024 && (e = cudaFuncSetAttribute((const void*)tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem)) != cudaSuccess) return e;
+    e = launch_walk(tile, dim3(w.n_head_kv, splits, tiled.n), dim3(ATT_THREADS), tile_smem, s, q, kv, scratch, rows, layer, max_chunk, w, tiled);
+    if (e != cudaSuccess) return e;
+  }
+  if (single.n) {
+    if (launches) ++*launches;
+    e = launch_walk(attention_rows_kernel, dim3(w.n_head_kv, splits, single.n), dim3(ATT_THREADS), smem, s, q, kv, scratch, rows, layer, max_chunk, w, single);
+    if (e != cudaSuccess) return e;
+  }
+  if (launches) ++*launches;
   return launch_walk(attention_combine_kernel, dim3(tokens >= 16 ? (w.n_head + 3) / 4 : w.n_head, tokens), dim3(128), 0, s, (const float*)scratch, out, rows,
-                     max_chunk, w, tokens >= 16 ? 4 : 1, max_records, record_chunk);
+                     max_chunk, w, tokens >= 16 ? 4 : 1, max_records, mma_chunk, mma_rows);
 }
 
 cudaError_t launch_swiglu(float* g, const float* u, int64_t n, cudaStream_t s, uint64_t* launches) {

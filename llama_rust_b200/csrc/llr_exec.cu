@@ -1631,7 +1631,7 @@ struct LayeredDecoder {
   float embd_scale = 1.f, eps = 0.f;
   bool norm_input = false;
   const llr_matrix *token_embd = nullptr, *pos_embd = nullptr;
-  size_t block_floats = 0, y_rows = 1, state_floats = 0;
+  size_t block_floats = 0, y_rows = 1, state_floats = 0, scratch_floats = 0;
   std::vector<double> freq;  // every distinct rotation, end to end
   float *proj = nullptr, *lat_q = nullptr, *lat_o = nullptr, *att = nullptr, *gu = nullptr, *act = nullptr, *y = nullptr, *scratch = nullptr, *state = nullptr,
         *prep = nullptr, *records = nullptr, *low = nullptr;  // low: what the mixers' own products leave
@@ -1702,6 +1702,7 @@ struct llr_session {
   };
   std::vector<std::unique_ptr<Moe>> moe;  // per layer, null: dense FFN
   std::vector<std::pair<size_t, size_t>> batch_groups;  // llr_session_batch: (first row, rows) of each group of the batch in flight
+  std::vector<size_t> batch_first;                      // and the position of its first row
   std::unique_ptr<LayeredDecoder> dec;  // a decoder described layer by layer (null: the Llama walk)
   bool has_moe = false, moe_select = false;  // moe_select: every routed layer can choose its experts' products on the device
   int* moe_sel = nullptr;     // one token's experts in ascending id (8 ints), then their router weights (8 floats)
@@ -1874,35 +1875,16 @@ cudaError_t session_layers(llr_session* s, const int* ids_dev, size_t n, const R
       if ((ce = session_matmul(e, W.attn_v, n, s->xn, s->v)) != cudaSuccess) break;
     }
     if (n == 1) {  // a decode token: rotation and cache store happen inside the attention kernel
-      if ((ce = launch_attention(s->q, kv, s->attn, s->att_scratch, rows, 1, (int)li, s->shape, st, L, s->k, s->v)) != cudaSuccess) break;
+      if ((ce = launch_attention(s->q, kv, s->attn, s->att_scratch, rows, (int)li, s->shape, st, L, s->k, s->v)) != cudaSuccess) break;
     } else {
       if ((ce = launch_rope_store(s->q, s->k, s->v, kv, rows, (int)n, (int)li, s->shape, st, L)) != cudaSuccess) break;
       // the automatic path takes the tensor cores for chunks of 64 rows and more of one sequence, as it does for the products
-      const bool tc = e->path == PATH_AUTO && n >= TC_MIN_TOKENS;
-      bool big_group = false;
-      if (tc && rows.row_seq)
-        for (const auto& gr : s->batch_groups) big_group = big_group || gr.second >= (size_t)TC_MIN_TOKENS;
-      if (big_group) {
-        // a ragged batch: every group of 64 rows and more on its own (tensor cores), the runs of smaller groups between them together
-        const size_t q_row = (size_t)c.n_head * c.head_dim, rec_row = attention_scratch_floats(1, s->shape);
-        auto part = [&](size_t t0, size_t len, bool one) {
-          return launch_attention(s->q + t0 * q_row, kv, s->attn + t0 * q_row, s->att_scratch + t0 * rec_row,
-                                  RowMap{nullptr, rows.row_pos + t0, rows.row_seq + t0}, (int)len, (int)li, s->shape, st, L, nullptr, nullptr, one, one);
-        };
-        size_t run0 = 0, at = 0;
-        for (const auto& gr : s->batch_groups) {
-          if (gr.second >= (size_t)TC_MIN_TOKENS) {
-            if (at > run0 && (ce = part(run0, at - run0, false)) != cudaSuccess) break;
-            if ((ce = part(gr.first, gr.second, true)) != cudaSuccess) break;
-            run0 = gr.first + gr.second;
-          }
-          at = gr.first + gr.second;
-        }
-        if (ce == cudaSuccess && at > run0) ce = part(run0, at - run0, false);
-        if (ce != cudaSuccess) break;
-      } else if ((ce = launch_attention(s->q, kv, s->attn, s->att_scratch, rows, (int)n, (int)li, s->shape, st, L, nullptr, nullptr, tc)) != cudaSuccess) {
+      const bool tc = e->path == PATH_AUTO;
+      std::vector<AttentionGroup> groups;
+      for (const auto& gr : s->batch_groups) groups.push_back(AttentionGroup{(int)gr.first, (int)gr.second});
+      if ((ce = launch_attention_groups(s->q, kv, s->attn, s->att_scratch, rows, (int)n, (int)li, s->shape, rows.row_seq ? groups.data() : nullptr,
+                                        rows.row_seq ? (int)groups.size() : 0, tc, st, L)) != cudaSuccess)
         break;
-      }
     }
     if ((ce = session_matmul(e, W.attn_output, n, s->attn, s->proj)) != cudaSuccess) break;
     if ((ce = launch_rmsnorm(s->x, s->proj, s->ffn_norm[li], s->xn, (int)n, (int)E, c.rms_eps, st, L)) != cudaSuccess) break;
@@ -2385,10 +2367,12 @@ static int session_batch(llr_session* s, size_t n_groups, const uint32_t* seq_id
   std::vector<int> ids(total), rpos(total), rseq(total), last(n_groups), row_of(rows ? total : 0);
   size_t r = 0;
   s->batch_groups.clear();
+  s->batch_first.clear();
   for (size_t oi = 0; oi < n_groups; ++oi) {
     const size_t g = order[oi], q = seq_ids[g];
     if ((rc = session_reserve(s, q, s->position[q] + counts[g]))) return rc;
     s->batch_groups.emplace_back(r, (size_t)counts[g]);
+    s->batch_first.push_back(s->position[q]);
     for (size_t i = 0; i < counts[g]; ++i, ++r) {
       ids[r] = tokens[first[g] + i];
       if (rows) row_of[first[g] + i] = (int)r;

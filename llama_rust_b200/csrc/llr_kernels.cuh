@@ -288,11 +288,15 @@ cudaError_t launch_rope_store(float* q, float* k, const float* v, const KvView& 
 // out[t][hq] = softmax(q[t][hq] . K[0..pos(t)] / sqrt(hd)) V over row t's own sequence, grouped-query heads; scratch holds
 // the partial results of the position splits (attention_scratch_floats)
 size_t attention_scratch_floats(int tokens, const WalkShape& w);
-cudaError_t launch_attention(const float* q, const KvView& kv, float* out, float* scratch, const RowMap& rows, int tokens,
-                             int layer, const WalkShape& w, cudaStream_t s, uint64_t* launches,
-                             const float* k_new = nullptr, const float* v_new = nullptr,  // k_new / v_new: one decode token whose rotation and cache store the attention kernel does itself
-                             bool tensor_cores = false,  // a prompt chunk of one sequence may run as binary16 MMAs with f32 accumulation (the tolerance of the 16-bit chunk GEMM)
-                             bool one_sequence = false);  // the caller vouches that the rows are one sequence at consecutive positions (rows given per row)
+// k_new / v_new: one decode token whose rotation and cache store the attention kernel does itself
+cudaError_t launch_attention(const float* q, const KvView& kv, float* out, float* scratch, const RowMap& rows, int layer,
+                             const WalkShape& w, cudaStream_t s, uint64_t* launches, const float* k_new, const float* v_new);
+// The same for the rows of a batch.  groups: runs of rows of one sequence at consecutive positions that make up the batch,
+// ascending (null: all rows are one); with tensor_cores those of 64 rows and more may run as binary16 MMAs with f32
+// accumulation (the tolerance of the 16-bit chunk GEMM).
+struct AttentionGroup { int first, rows; };
+cudaError_t launch_attention_groups(const float* q, const KvView& kv, float* out, float* scratch, const RowMap& rows, int tokens, int layer, const WalkShape& w,
+                                    const AttentionGroup* groups, int n_groups, bool tensor_cores, cudaStream_t s, uint64_t* launches);
 cudaError_t launch_swiglu(float* g, const float* u, int64_t n, cudaStream_t s, uint64_t* launches);
 cudaError_t launch_add(float* x, const float* y, int64_t n, cudaStream_t s, uint64_t* launches);
 // first index of the strict maximum of logits[0..n) -> *out_id (device; n == 0: no argmax), and *pos_dev += advance
@@ -402,7 +406,6 @@ cudaError_t launch_head_product(const void* w, int heads, int rows, int cols, co
                                 int64_t gate_ld, int tokens, cudaStream_t s, uint64_t* launches);
 cudaError_t launch_head_transpose(const void* w, int heads, int rows, int cols, void* out, cudaStream_t s, uint64_t* launches);
 // Attention over the visible keys.  q: row t at q + t * q_ld.  Results go where SpanOut says.
-// one_sequence: the rows are one sequence at consecutive positions; with tensor_cores such rows may run as binary16 MMAs.
 // A single decode token whose projection the attention kernel takes in itself (null proj: it is in the cache already):
 // the row's stacked q | k | v with launch_qkv_store's arguments, or (latent) its latent with the weights in k_norm.
 struct NewToken {
@@ -424,9 +427,12 @@ struct SpanOut {
 };
 size_t span_scratch_floats(const SpanShape& sh, int max_rows);
 bool span_supported(const SpanShape& sh);
-cudaError_t launch_span_attention(const float* q, int64_t q_ld, const SpanShape& sh, const LayerKv& kv, const RowMap& rows, int t0, int tokens,
-                                  const SpanOut& out, float* scratch, bool tensor_cores, bool one_sequence, const NewToken* nt, cudaStream_t s,
-                                  uint64_t* launches);
+// Rows [t0, t0 + rows) of a batch: one sequence at consecutive positions, from position `first` on (-1: the device knows it).
+// With tensor_cores, groups of BF16_TC_MIN_TOKENS rows and more run as binary16 MMAs, all of them in one launch as far as the
+// scratch holds their gathered keys; the rows of shorter groups share a launch of the f32 kernels.
+struct SpanGroup { int t0, rows, first; };
+cudaError_t launch_span_attention(const float* q, int64_t q_ld, const SpanShape& sh, const LayerKv& kv, const RowMap& rows, const SpanGroup* groups, int n_groups,
+                                  const SpanOut& out, float* scratch, size_t scratch_floats, bool tensor_cores, const NewToken* nt, cudaStream_t s, uint64_t* launches);
 // x[t] += y[t] / rms(y[t]) * w, y given as `slices` partial sums `slice_stride` floats apart; x16 (may be null): the new x
 cudaError_t launch_norm_add(float* x, const float* y, int slices, int64_t slice_stride, const float* w, float eps, void* x16, int tokens, int n,
                             cudaStream_t s, uint64_t* launches);

@@ -219,23 +219,14 @@ struct LayeredPass {
     nt.q_norm = M.q_norm;
     nt.k_norm = latent ? M.kv_norm : M.k_norm;
     nt.rot = rotation(M);
-    auto attend = [&](size_t t0, size_t len, bool one) {
-      return launch_span_attention(q, q_ld, M.span, kv, rows, (int)t0, (int)len, so, D.scratch, tc && len >= (size_t)BF16_TC_MIN_TOKENS, one, &nt, st, lc);
-    };
-    ce = cudaSuccess;
     if (!rows.row_seq) {
-      ce = attend(0, n, true);
-    } else {  // a ragged batch: groups long enough for the tensor cores on their own, the runs of shorter ones together
-      size_t run = 0, at = 0;
-      for (const auto& g : s->batch_groups) {
-        if (ce == cudaSuccess && tc && g.second >= (size_t)BF16_TC_MIN_TOKENS) {
-          if (g.first > run) ce = attend(run, g.first - run, false);
-          if (ce == cudaSuccess) ce = attend(g.first, g.second, true);
-          run = g.first + g.second;
-        }
-        at = g.first + g.second;
-      }
-      if (ce == cudaSuccess && at > run) ce = attend(run, at - run, false);
+      const SpanGroup all{0, N, -1};
+      ce = launch_span_attention(q, q_ld, M.span, kv, rows, &all, 1, so, D.scratch, D.scratch_floats, tc, &nt, st, lc);
+    } else {
+      std::vector<SpanGroup> ragged;
+      for (size_t g = 0; g < s->batch_groups.size(); ++g)
+        ragged.push_back(SpanGroup{(int)s->batch_groups[g].first, (int)s->batch_groups[g].second, (int)s->batch_first[g]});
+      ce = launch_span_attention(q, q_ld, M.span, kv, rows, ragged.data(), (int)ragged.size(), so, D.scratch, D.scratch_floats, tc, &nt, st, lc);
     }
     if (ce != cudaSuccess || !latent) return ce;
     // results out of the latent space, times the head gate
@@ -645,6 +636,7 @@ int layered_create(llr_exec* e, const llr_decoder_model* m, size_t n_seq, size_t
   alloc(&s->logits, s->logits_rows * V); alloc(&s->last_x, s->logits_rows * E); alloc(&s->arg_part, 512);
   alloc(&s->cache_k, s->n_blocks * D->block_floats + 64);
   alloc(&D->proj, B * in_rows); alloc(&D->att, B * heads); alloc(&D->scratch, scratch);
+  D->scratch_floats = scratch;
   if (lat) { alloc(&D->lat_q, B * lat); alloc(&D->lat_o, B * lat); }
   if (ff) { alloc(&D->gu, B * 2 * ff); alloc(&D->act, B * ff); }
   if (D->state_floats) { alloc(&D->state, n_seq * D->state_floats); alloc(&D->low, B * low + 8); ialloc(&D->group_first, n_seq + 1); }

@@ -359,6 +359,18 @@ __device__ __forceinline__ int span_step(int n) { return max(32, (n + 31) / 32);
 // Query heads of a kv head that share a block: eight, four where a head's query and value rows are long.
 inline __host__ __device__ int span_heads(const SpanShape& sh) { return sh.dk + sh.dv > 512 ? ATT_MAX_GQA / 2 : ATT_MAX_GQA; }
 
+// The rows of a launch of the f32 kernels: the runs [start[i], start[i] + at[i + 1] - at[i]) of the batch, row z of the launch being
+// row z - at[i] of its run.
+struct SpanRuns {
+  int n;
+  int start[64], at[65];
+  __device__ __forceinline__ int row(int z) const {
+    int i = 0;
+    while (i + 1 < n && z >= at[i + 1]) ++i;
+    return start[i] + z - at[i];
+  }
+};
+
 // grid (kv head x group of span_heads query heads, slice of the visible keys, row)
 // With nt (a single decode token) the kernel also does what the store kernels do for that token: the query is biased and
 // normed as it is loaded, and the blocks whose slice holds the token's own position write its key and value (or its
@@ -366,15 +378,15 @@ inline __host__ __device__ int span_heads(const SpanShape& sh) { return sh.dk + 
 static_assert(PROJ_THREADS == ATT_THREADS, "the sums over a projection are formed in one order");
 template <int MAX_VALUE>
 __global__ void __launch_bounds__(ATT_THREADS)
-span_partial_kernel(const float* __restrict__ q, int64_t q_ld, SpanShape sh, LayerKv kv, RowMap rows, int t0, int chunk, float* __restrict__ part,
-                    NewToken nt) {
+span_partial_kernel(const float* __restrict__ q, int64_t q_ld, SpanShape sh, LayerKv kv, RowMap rows, const __grid_constant__ SpanRuns runs, int chunk,
+                    float* __restrict__ part, NewToken nt) {
   pdl_enter();
   __shared__ float red[2][32];
   extern __shared__ int2 smw[];  // pages [chunk] | q [heads][dk] | scores [heads][chunk] or sums [P][heads][dv]
   float* sm = (float*)(smw + chunk);
   const int gq = sh.n_head / sh.n_kv, per = span_heads(sh), groups = (gq + per - 1) / per;
   const int head = blockIdx.x / groups, g0 = (blockIdx.x % groups) * per, heads = min(per, gq - g0);
-  const int t = t0 + blockIdx.z, split = blockIdx.y, n_split = (int)gridDim.y, h0 = head * gq + g0;
+  const int t = runs.row(blockIdx.z), split = blockIdx.y, n_split = (int)gridDim.y, h0 = head * gq + g0;
   const int pos = row_position(rows, t);
   const Span span = span_of(pos, sh.window, sh.keep_first);
   const int step = span_step(span.n), s0 = split * step, s1 = min(span.n, s0 + step);
@@ -412,9 +424,9 @@ span_partial_kernel(const float* __restrict__ q, int64_t q_ld, SpanShape sh, Lay
 
 // grid (query head, row, 128 dimensions): merges a head's slices (at most 32) and the sink, applies the gate
 __global__ void __launch_bounds__(128)
-span_combine_kernel(const float* __restrict__ part, SpanShape sh, RowMap rows, int t0, int n_split, SpanOut so) {
+span_combine_kernel(const float* __restrict__ part, SpanShape sh, RowMap rows, const __grid_constant__ SpanRuns runs, int n_split, SpanOut so) {
   pdl_enter();
-  const int lane = threadIdx.x & 31, h = blockIdx.x, t = t0 + blockIdx.y;
+  const int lane = threadIdx.x & 31, h = blockIdx.x, t = runs.row(blockIdx.y);
   const int gq = sh.n_head / sh.n_kv, per = span_heads(sh), groups = (gq + per - 1) / per;
   const int bx = (h / gq) * groups + (h % gq) / per, g = (h % gq) % per;
   const int seen = span_of(row_position(rows, t), sh.window, sh.keep_first).n, step = span_step(seen), used = (seen + step - 1) / step;
@@ -518,13 +530,31 @@ __device__ __forceinline__ GroupKeys group_keys(int first, int rows, int window,
   return GroupKeys{lo, nk, nk + first + rows - lo};
 }
 
-// one warp per key row: grid (keys / 8, kv head)
+// The groups of one launch: group i has the rows [t0, t0 + rows), blocks [keys_at[i], keys_at[i + 1]) of the gather and
+// [tiles_at[i], tiles_at[i + 1]) of the attention, and its gathered rows k_off / v_off halves into the scratch.  A group alone
+// fills a few SMs (a prompt of 24 rows: eight blocks), and a ragged batch has dozens: with a launch each, 24 groups of 30 rows
+// took 16 x (5 + 30) us per layer one after the other.
+constexpr int SPAN_GROUPS = 64;
+struct SpanBatch {
+  int n;
+  int t0[SPAN_GROUPS], rows[SPAN_GROUPS], keys_at[SPAN_GROUPS + 1], tiles_at[SPAN_GROUPS + 1];
+  int64_t k_off[SPAN_GROUPS], v_off[SPAN_GROUPS];
+};
+__device__ __forceinline__ int span_group(const int* at, int n, int block) {
+  int i = 0;
+  while (i + 1 < n && block >= at[i + 1]) ++i;
+  return i;
+}
+
+// one warp per key row: grid (keys / 8 of all groups, kv head)
 __global__ void __launch_bounds__(256)
-span_gather_kernel(SpanShape sh, LayerKv kv, RowMap rows, int t0, int tokens, int kr, int vr, __half* __restrict__ k16, __half* __restrict__ v16) {
+span_gather_kernel(SpanShape sh, LayerKv kv, RowMap rows, const __grid_constant__ SpanBatch b, int kr, int vr, __half* __restrict__ scratch) {
   pdl_enter();
-  const GroupKeys gk = group_keys(row_position(rows, t0), tokens, sh.window, sh.keep_first);
-  const int m = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, head = blockIdx.y, seq = row_sequence(rows, t0);
+  const int gi = span_group(b.keys_at, b.n, blockIdx.x), t0 = b.t0[gi];
+  const GroupKeys gk = group_keys(row_position(rows, t0), b.rows[gi], sh.window, sh.keep_first);
+  const int m = (blockIdx.x - b.keys_at[gi]) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, head = blockIdx.y, seq = row_sequence(rows, t0);
   if (m >= gk.n) return;
+  __half *k16 = scratch + b.k_off[gi], *v16 = scratch + b.v_off[gi];
   auto put = [&](const float* src, int d, __half* dst, int w) {
     for (int i = 4 * lane; i < w; i += 128) {
       const float4 v = i < d ? *(const float4*)(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);  // d is a multiple of four
@@ -538,9 +568,11 @@ span_gather_kernel(SpanShape sh, LayerKv kv, RowMap rows, int t0, int tokens, in
 
 template <int ND, int NS>
 __global__ void __launch_bounds__(128 * NS)
-span_mma_kernel(const float* __restrict__ q, int64_t q_ld, SpanShape sh, const __half* __restrict__ k16, const __half* __restrict__ v16, bool shared_kv,
-                RowMap rows, int t0, int tokens, SpanOut so) {
+span_mma_kernel(const float* __restrict__ q, int64_t q_ld, SpanShape sh, const __half* __restrict__ scratch, bool shared_kv, RowMap rows,
+                const __grid_constant__ SpanBatch b, SpanOut so) {
   pdl_enter();
+  const int gi = span_group(b.tiles_at, b.n, blockIdx.x), t0 = b.t0[gi], tokens = b.rows[gi];
+  const __half *k16 = scratch + b.k_off[gi], *v16 = scratch + b.v_off[gi];
   constexpr int THR = 128 * NS, NT = CH / 8 / NS;  // score tiles of eight keys per warp
   static_assert(NT % 2 == 0, "keys are loaded sixteen at a time");
   extern __shared__ __align__(16) unsigned char raw[];
@@ -553,7 +585,7 @@ span_mma_kernel(const float* __restrict__ q, int64_t q_ld, SpanShape sh, const _
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
   const int rw = warp & 3, ns = warp >> 2;  // rows 16 rw .., key and value share ns
   // the last rows first: in a window that is still filling they see the most keys
-  const int head = blockIdx.y, gq = sh.n_head / sh.n_kv, pairs = tokens * gq, pair0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * 64;
+  const int head = blockIdx.y, gq = sh.n_head / sh.n_kv, pairs = tokens * gq, pair0 = (b.tiles_at[gi + 1] - 1 - (int)blockIdx.x) * 64;
   const int p_first = row_position(rows, t0);
   const GroupKeys gk = group_keys(p_first, tokens, sh.window, sh.keep_first);
   const int pa = p_first + pair0 / gq, pb = p_first + min(pairs - 1, pair0 + 63) / gq;  // positions of the tile's rows
@@ -920,9 +952,14 @@ int span_rows_per_pass(const SpanShape& sh) { return (int)std::min<size_t>(512, 
 int span_group_keys(const SpanShape& sh, int rows) {
   return sh.window > 0 ? (int)std::min<int64_t>(sh.n_ctx, (int64_t)sh.window + sh.keep_first + rows) : sh.n_ctx;
 }
+int group_key_count(const SpanShape& sh, const SpanGroup& g) {
+  if (g.first < 0) return span_group_keys(sh, g.rows);
+  const int lo = sh.window > 0 ? std::max(0, g.first - sh.window + 1) : 0;  // as group_keys
+  return std::min(sh.keep_first, lo) + g.first + g.rows - lo;
+}
 constexpr size_t MMA_SMEM_LIMIT = 222 * 1024;
 
-typedef void (*MmaKernel)(const float*, int64_t, SpanShape, const __half*, const __half*, bool, RowMap, int, int, SpanOut);
+typedef void (*MmaKernel)(const float*, int64_t, SpanShape, const __half*, bool, RowMap, const SpanBatch, SpanOut);
 // the smallest instantiation that covers the value dimensions
 MmaKernel mma_kernel(int dv, int* nd, int* ns) {
 #define LLR_SPAN(N, S) if (dv <= 8 * N * S) { *nd = N; *ns = S; return span_mma_kernel<N, S>; }
@@ -1009,51 +1046,87 @@ size_t span_scratch_floats(const SpanShape& sh, int max_rows) {
   return std::max((size_t)span_rows_per_pass(sh) * span_row_floats(sh), gathered);
 }
 
-cudaError_t launch_span_attention(const float* q, int64_t q_ld, const SpanShape& sh, const LayerKv& kv, const RowMap& rows, int t0, int tokens,
-                                  const SpanOut& out, float* scratch, bool tensor_cores, bool one_sequence, const NewToken* nt, cudaStream_t s,
-                                  uint64_t* launches) {
-  if (tokens <= 0) return cudaSuccess;
+cudaError_t launch_span_attention(const float* q, int64_t q_ld, const SpanShape& sh, const LayerKv& kv, const RowMap& rows, const SpanGroup* groups, int n_groups,
+                                  const SpanOut& out, float* scratch, size_t scratch_floats, bool tensor_cores, const NewToken* nt, cudaStream_t s, uint64_t* launches) {
   if (!span_supported(sh)) return cudaErrorInvalidValue;
   const int gq = sh.n_head / sh.n_kv;
-  if (tensor_cores && one_sequence && sh.dk % 8 == 0 && sh.dv % 8 == 0 && out.ld % 2 == 0 && ((uintptr_t)out.out & 7) == 0 && ((uintptr_t)out.out16 & 3) == 0 &&
-      (!out.gate || out.head_gate || (out.gate_ld % 2 == 0 && ((uintptr_t)out.gate & 7) == 0))) {
-    int nd = 0, ns = 0;
-    MmaKernel kern = mma_kernel(sh.dv, &nd, &ns);
-    const bool shared = kv.k == kv.v;
-    const MmaLayout L = mma_layout(sh.dk, sh.dv, nd, ns, shared);
-    const size_t smem = kern ? mma_smem(L, ns) : 0;
-    if (kern && smem <= MMA_SMEM_LIMIT) {
-      if (smem > 40 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-      }
-      if (launches) *launches += 2;
-      const int keys = span_group_keys(sh, tokens);
-      __half* k16 = (__half*)scratch;
-      __half* v16 = shared ? k16 : k16 + (size_t)sh.n_kv * keys * L.kr;
-      cudaError_t e = launch_walk(span_gather_kernel, dim3((keys + 7) / 8, sh.n_kv), dim3(256), 0, s, sh, kv, rows, t0, tokens, L.kr, L.vr, k16, v16);
-      if (e != cudaSuccess) return e;
-      return launch_walk(kern, dim3((unsigned)(((int64_t)tokens * gq + 63) / 64), sh.n_kv), dim3(128 * ns), smem, s, q, q_ld, sh, (const __half*)k16,
-                         (const __half*)v16, shared, rows, t0, tokens, out);
-    }
+  int nd = 0, ns = 0;
+  const bool shared = kv.k == kv.v;
+  MmaKernel mma = nullptr;
+  if (tensor_cores && sh.dk % 8 == 0 && sh.dv % 8 == 0 && out.ld % 2 == 0 && ((uintptr_t)out.out & 7) == 0 && ((uintptr_t)out.out16 & 3) == 0 &&
+      (!out.gate || out.head_gate || (out.gate_ld % 2 == 0 && ((uintptr_t)out.gate & 7) == 0)))
+    mma = mma_kernel(sh.dv, &nd, &ns);
+  MmaLayout L{};
+  size_t mma_bytes = 0;
+  if (mma) {
+    L = mma_layout(sh.dk, sh.dv, nd, ns, shared);
+    mma_bytes = mma_smem(L, ns);
+    if (mma_bytes > MMA_SMEM_LIMIT) mma = nullptr;
   }
-  const int groups = (gq + span_heads(sh) - 1) / span_heads(sh), chunk = span_chunk(sh), splits = span_splits(sh), per = span_rows_per_pass(sh);
+  if (mma && mma_bytes > 40 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute((const void*)mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mma_bytes);
+    if (e != cudaSuccess) return e;
+  }
+  const int head_groups = (gq + span_heads(sh) - 1) / span_heads(sh), chunk = span_chunk(sh), splits = span_splits(sh), per = span_rows_per_pass(sh);
   const size_t smem = span_smem(sh);
   auto kern = sh.dv <= ATT_THREADS ? span_partial_kernel<ATT_THREADS> : sh.dv <= 2 * ATT_THREADS ? span_partial_kernel<2 * ATT_THREADS> : span_partial_kernel<MAX_VALUE>;
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  for (int r = 0; r < tokens; r += per) {
-    const int n = std::min(per, tokens - r);
+
+  // groups that are long enough for the tensor cores, as many per launch as the scratch holds the gathered keys of
+  SpanBatch b{};
+  size_t used = 0;  // halves of the scratch
+  auto run_batch = [&] {
+    if (b.n == 0) return cudaSuccess;
     if (launches) *launches += 2;
-    cudaError_t e = launch_walk(kern, dim3(sh.n_kv * groups, splits, n), dim3(ATT_THREADS), smem, s, q, q_ld, sh, kv, rows, t0 + r, chunk, scratch,
-                                nt && tokens == 1 ? *nt : NewToken{});
+    cudaError_t e = launch_walk(span_gather_kernel, dim3(b.keys_at[b.n], sh.n_kv), dim3(256), 0, s, sh, kv, rows, b, L.kr, L.vr, (__half*)scratch);
+    if (e == cudaSuccess) e = launch_walk(mma, dim3(b.tiles_at[b.n], sh.n_kv), dim3(128 * ns), mma_bytes, s, q, q_ld, sh, (const __half*)scratch, shared, rows, b, out);
+    b.n = 0;
+    used = 0;
+    return e;
+  };
+  // the rows of the others, as many runs and rows per launch as the lists and the scratch hold
+  SpanRuns runs{};
+  bool configured = smem <= 48 * 1024;
+  auto run_rows = [&] {
+    if (runs.n == 0) return cudaSuccess;
+    cudaError_t e = cudaSuccess;
+    if (!configured) e = cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    configured = true;
     if (e != cudaSuccess) return e;
-    e = launch_walk(span_combine_kernel, dim3(sh.n_head, n, (sh.dv + 127) / 128), dim3(128), 0, s, (const float*)scratch, sh, rows, t0 + r, splits, out);
-    if (e != cudaSuccess) return e;
+    if (launches) *launches += 2;
+    const int n = runs.at[runs.n];
+    const bool fresh = nt && n == 1 && n_groups == 1 && groups[0].rows == 1;
+    e = launch_walk(kern, dim3(sh.n_kv * head_groups, splits, n), dim3(ATT_THREADS), smem, s, q, q_ld, sh, kv, rows, runs, chunk, scratch, fresh ? *nt : NewToken{});
+    if (e == cudaSuccess) e = launch_walk(span_combine_kernel, dim3(sh.n_head, n, (sh.dv + 127) / 128), dim3(128), 0, s, (const float*)scratch, sh, rows, runs, splits, out);
+    runs.n = 0;
+    return e;
+  };
+  cudaError_t e = cudaSuccess;
+  for (int g = 0; g < n_groups && e == cudaSuccess; ++g) {
+    if (!mma || groups[g].rows < BF16_TC_MIN_TOKENS) continue;
+    const int keys = group_key_count(sh, groups[g]);
+    const size_t need = (size_t)sh.n_kv * keys * (L.kr + L.vr);
+    if (b.n == SPAN_GROUPS || (b.n > 0 && used + need > 2 * scratch_floats)) e = run_batch();
+    const int i = b.n++;
+    b.t0[i] = groups[g].t0;
+    b.rows[i] = groups[g].rows;
+    b.k_off[i] = (int64_t)used;
+    b.v_off[i] = b.k_off[i] + (shared ? 0 : (int64_t)sh.n_kv * keys * L.kr);
+    b.keys_at[i + 1] = b.keys_at[i] + (keys + 7) / 8;
+    b.tiles_at[i + 1] = b.tiles_at[i] + (int)(((int64_t)groups[g].rows * gq + 63) / 64);
+    used += need;
   }
-  return cudaSuccess;
+  if (e == cudaSuccess) e = run_batch();
+  for (int g = 0; g < n_groups && e == cudaSuccess; ++g) {
+    if (mma && groups[g].rows >= BF16_TC_MIN_TOKENS) continue;
+    for (int r = 0; r < groups[g].rows && e == cudaSuccess;) {
+      if (runs.n == 64 || (runs.n > 0 && runs.at[runs.n] == per)) e = run_rows();
+      const int n = std::min(groups[g].rows - r, per - (runs.n ? runs.at[runs.n] : 0)), i = runs.n++;
+      runs.start[i] = groups[g].t0 + r;
+      runs.at[i + 1] = runs.at[i] + n;
+      r += n;
+    }
+  }
+  return e == cudaSuccess ? run_rows() : e;
 }
 
 cudaError_t launch_norm_add(float* x, const float* y, int slices, int64_t slice_stride, const float* w, float eps, void* x16, int tokens, int n,

@@ -1,7 +1,10 @@
-"""Products of a few dozen activation rows."""
+"""Batches of many rows and of many sequences: products of a few dozen activation rows, ragged batches whose groups share the
+attention launches."""
 import numpy as np
 import pytest
 
+import nagolix_models as nm
+import nagolix_plain as plain
 from helpers import ALL
 
 pytestmark = pytest.mark.gpu
@@ -41,3 +44,77 @@ def test_rows_of_unpacked_formats_alone_and_in_a_batch(ex, name, rows, cols):
     for n in (33, 40):
         assert np.all(np.abs(_product(ex, m, x[:n]) - exact[:n]) <= 2.0 ** -24 * (cols + 3) * size[:n]), n
     m.free()
+
+
+@pytest.mark.parametrize("lens", [[1 + i * 7 % 13 for i in range(70)],      # more runs of short groups than one list holds
+                                  [15, 16, 17, 1, 64, 2, 16, 40, 31, 1, 3, 100]])
+def test_many_groups_in_one_batch(ex, tmp_path, lens):
+    """f32: the bits of every sequence alone; the serving path: the plain logits."""
+    from llama_rust_b200 import models
+    cfg, buckets = nm.MODELS["mix"]
+    for path in (nm.F32, nm.AUTO):
+        w = nm.weights(cfg, 21, buckets, nm.SHARP[path])
+        ex.set_path(path)
+        s = models.load(ex, nm.write(tmp_path / f"m{path}", cfg, w), n_seq=len(lens), n_ctx=160)
+        toks = [nm.tokens(n, cfg, 100 + i) for i, n in enumerate(lens)]
+        together = s.forward(list(enumerate(toks)), [list(range(n)) for n in lens])
+        s.reset()
+        at = 0
+        for i, t in enumerate(toks):
+            mine = together[at:at + len(t)]
+            at += len(t)
+            if path == nm.F32 and i % 5 == 0:
+                assert _same_bits(mine, s.forward([(0, t)], [list(range(len(t)))])), i
+                s.reset()
+            elif path == nm.AUTO:
+                assert nm.error(mine, plain.forward(cfg, w, t)).max() <= nm.TOLERANCE[path], i
+        s.free()
+    ex.set_path(0)
+
+
+def test_groups_whose_keys_do_not_fit_one_launch(ex, tmp_path):
+    """Twelve groups that each see hundreds of cached keys: the gathered keys of all exceed the scratch, which holds those of one
+    group of the longest kind, so the groups go in several launches."""
+    from llama_rust_b200 import models
+    cfg, buckets = nm.MODELS["wide window"]
+    w = nm.weights(cfg, 22, buckets, nm.SHARP[nm.AUTO])
+    ex.set_path(nm.AUTO)
+    s = models.load(ex, nm.write(tmp_path / "m", cfg, w), n_seq=12, n_ctx=400)
+    toks = [nm.tokens(300 + 17 + q, cfg, 200 + q) for q in range(12)]
+    s.forward([(q, t[:300]) for q, t in enumerate(toks)], [[] for _ in toks])
+    got = s.forward([(q, t[300:]) for q, t in enumerate(toks)], [list(range(17 + q)) for q in range(12)])
+    at = 0
+    for q in (0, 5, 11):
+        at = sum(17 + i for i in range(q))
+        assert nm.error(got[at:at + 17 + q], plain.forward(cfg, w, toks[q])[300:]).max() <= nm.TOLERANCE[nm.AUTO], q
+    s.free()
+
+
+def test_llama_batch_of_every_kind_of_group(ex):
+    """Groups for the three attention kernels of the Llama walk in one batch (a block per row, tiles of one sequence, binary16
+    MMAs) with F32 weights: short groups have the bits they have alone, long ones agree with f32 attention."""
+    import llama_walk as lw
+    from llama_rust_b200 import Session
+    cfg = dict(n_layer=2, n_embd=256, n_head=4, n_head_kv=2, head_dim=64, n_ff=256, n_vocab=300)
+    rng = np.random.default_rng(72)
+    tl = lw.tensor_list(cfg)
+    mats = [ex.upload(ALL["F32"], r, c, (rng.standard_normal(r * c) / np.sqrt(c)).astype(np.float32).view(np.uint8)) for _, _, r, c in tl]
+    embd = ex.upload(ALL["F32"], 300, 256, rng.standard_normal(300 * 256).astype(np.float32).view(np.uint8))
+    names = ("attn_q", "attn_k", "attn_v", "attn_output", "ffn_gate", "ffn_up", "ffn_down")
+    layers = [dict(zip(names, mats[7 * i:7 * i + 7])) for i in range(2)]
+    lens = [1, 1, 2, 3, 4, 15, 16, 17, 33, 63, 64, 65, 1, 130]
+    toks = [lw.prompt_ids(n, 300, n + i) for i, n in enumerate(lens)]
+    logits = {}
+    for path in (3, 0):
+        ex.set_path(path)
+        s = Session(ex, dict(cfg, n_ctx=512), embd, layers, output=mats[14], n_seq=len(lens))
+        logits[path] = s.batch(list(enumerate(toks)), want_logits=True)[1]
+        if path == 3:
+            s.reset()
+            for q, t in enumerate(toks):
+                assert _same_bits(s.batch([(q, t)], want_logits=True)[1][0], logits[3][q]), lens[q]
+        s.free()
+    ex.set_path(0)
+    for q, n in enumerate(lens):
+        err, size = np.abs(logits[0][q] - logits[3][q]).max(), np.abs(logits[3][q]).max()
+        assert err <= 1e-3 * size if n >= 64 else err <= 1e-5 * size, n

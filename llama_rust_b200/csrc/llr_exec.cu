@@ -144,6 +144,7 @@ struct llr_exec {
   float* dev_y = nullptr; size_t dev_y_cap = 0;
   float* dev_moe = nullptr; size_t dev_moe_cap = 0;  // workspace of the routed-expert layer
   uint8_t* dev_s = nullptr; size_t dev_s_cap = 0;  // kernel scratch (bf16 activations of the tensor-core GEMM)
+  uint8_t* dev_q = nullptr; size_t dev_q_cap = 0;  // kernel scratch (digits of the integer GEMM), this executor's stream only
   // residency
   std::list<CacheEntry> cache;  // front = least recently used
   bool limit_resolved = false;
@@ -299,10 +300,20 @@ MatView view_of(const llr_matrix* m) {
   return MatView{m->dev, m->dtype, m->rows, m->cols, m->row_bytes, m->f16_ok};
 }
 
-// scratch for the tensor-core GEMM; growing frees the old buffer, which synchronizes the device
-cudaError_t ensure_scratch(llr_exec* e, const llr_matrix* m, size_t tokens, void** out) {
+// scratch for the tensor-core GEMM; growing frees the old buffer, which synchronizes the device.
+// The integer GEMM has a buffer of its own, and does without where that is not safe or not to be had (the decode kernel then runs,
+// with the same results): on a stream of the caller's, whose work may overlap other work of this executor; under capture, since a
+// replay would outlive the buffer; when memory is short.
+cudaError_t ensure_scratch(llr_exec* e, const llr_matrix* m, size_t tokens, cudaStream_t stream, void** out) {
   *out = nullptr;
   const MatView v = view_of(m);
+  if (matmul_wants_i8(v, (int64_t)tokens, e->path)) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (stream != e->stream || cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return cudaSuccess;
+    if (grow_device(&e->dev_q, &e->dev_q_cap, gemm_i8_scratch_bytes(v, (int64_t)tokens)) == cudaSuccess) *out = e->dev_q;
+    else cudaGetLastError();
+    return cudaSuccess;
+  }
   if (!matmul_wants_tc(v, (int64_t)tokens, e->path)) return cudaSuccess;
   cudaError_t ce = grow_device(&e->dev_s, &e->dev_s_cap, matmul_scratch_bytes(v, (int64_t)tokens));
   if (ce == cudaSuccess) *out = e->dev_s;
@@ -383,7 +394,7 @@ int run_host(llr_exec* e, const llr_matrix* m, size_t tokens, const float* x, fl
     y_alias = e->pin_y_alias;
   }
   void* scratch = nullptr;
-  if ((ce = ensure_scratch(e, m, tokens, &scratch)) != cudaSuccess) return fail_cuda(e, ce, "kernel scratch");
+  if ((ce = ensure_scratch(e, m, tokens, e->stream, &scratch)) != cudaSuccess) return fail_cuda(e, ce, "kernel scratch");
   if ((ce = cudaMemcpyAsync(e->dev_x, src, nx * sizeof(float), cudaMemcpyHostToDevice, e->stream)) != cudaSuccess)
     return fail_cuda(e, ce, "activation upload");
   const MatView v = view_of(m);
@@ -438,6 +449,9 @@ bool matmul_wants_tc(const MatView& m, int64_t tokens, int path) {
   if (path != PATH_TC && !(path == PATH_AUTO && tokens >= TC_MIN_TOKENS)) return false;
   return gemm_tc_supported(m, tokens) || bf16_chunk(m, tokens);
 }
+bool matmul_wants_i8(const MatView& m, int64_t tokens, int path) {
+  return (path == PATH_AUTO || path == PATH_MMA || path == PATH_TC) && !matmul_wants_tc(m, tokens, path) && gemm_i8_supported(m, tokens);
+}
 size_t matmul_scratch_bytes(const MatView& m, int64_t tokens) {
   return bf16_chunk(m, tokens) ? ((size_t)tokens * m.cols * 2 + 255) / 256 * 256 : gemm_tc_scratch_bytes(m, tokens);
 }
@@ -456,6 +470,7 @@ cudaError_t launch_matmul(const MatView& m, const float* x, float* y, int64_t to
   }
   if (scratch && err_flag && x_aligned && matmul_wants_tc(m, tokens, path) && gemm_tc_supported(m, tokens))
     return launch_gemm_tc(m, x, y, tokens, scratch, gemm_tc_scratch_bytes(m, tokens), stream, err_flag, launches);
+  if (scratch && err_flag && x_aligned && matmul_wants_i8(m, tokens, path)) return launch_gemm_i8(m, x, y, tokens, scratch, stream, err_flag, launches);
   if (path == PATH_TC) path = PATH_AUTO;
   if ((path == PATH_AUTO || path == PATH_MMA) && x_aligned && err_flag && gemv_mma_supported(m))
     return launch_gemv_mma(m, x, y, tokens, stream, sm_count, err_flag, launches);
@@ -556,6 +571,7 @@ int llr_exec_destroy(llr_exec* e) {
   if (e->dev_x) cudaFree(e->dev_x);
   if (e->dev_y) cudaFree(e->dev_y);
   if (e->dev_s) cudaFree(e->dev_s);
+  if (e->dev_q) cudaFree(e->dev_q);
   if (e->dev_moe) cudaFree(e->dev_moe);
   if (e->err_pinned) cudaFreeHost((void*)e->err_pinned);
   if (e->done_count) cudaFree(e->done_count);
@@ -815,7 +831,7 @@ int llr_matmul_device(llr_exec* e, const llr_matrix* m, size_t tokens, const flo
   DeviceGuard guard(e->device);
   cudaStream_t s = stream ? (cudaStream_t)stream : e->stream;
   void* scratch = nullptr;
-  cudaError_t ce = ensure_scratch(e, m, tokens, &scratch);
+  cudaError_t ce = ensure_scratch(e, m, tokens, s, &scratch);
   if (ce != cudaSuccess) return fail_cuda(e, ce, "kernel scratch");
   ce = launch_matmul(view_of(m), x_dev, y_dev, (int64_t)tokens, s, e->path, e->sm_count, e->err_flag,
                      scratch, &e->ctr.launches);
@@ -868,7 +884,7 @@ cudaError_t matmul_dev(llr_exec* e, const llr_matrix* m, size_t tokens, const fl
   void* scratch = nullptr;
   const int saved = e->path;
   e->path = path;
-  cudaError_t ce = ensure_scratch(e, m, tokens, &scratch);
+  cudaError_t ce = ensure_scratch(e, m, tokens, e->stream, &scratch);
   if (ce == cudaSuccess)
     ce = launch_matmul(view_of(m), x, y, (int64_t)tokens, e->stream, path, e->sm_count, e->err_flag, scratch,
                        &e->ctr.launches);
@@ -959,8 +975,8 @@ cudaError_t moe_run_experts(llr_exec* e, const llr_moe_layer* L, const MoeShape&
     for (size_t ex = 0; ex < n_exp; ++ex)
       if (S.local[ex] && (size_t)(first_row[ex + 1] - first_row[ex]) > most) { most = (size_t)(first_row[ex + 1] - first_row[ex]); busiest = ex; }
     void* unused = nullptr;
-    if (most > 0 && ((ce = ensure_scratch(e, L->down[busiest], most, &unused)) != cudaSuccess ||
-                     (ce = ensure_scratch(e, L->gate[busiest], most, &unused)) != cudaSuccess))
+    if (most > 0 && ((ce = ensure_scratch(e, L->down[busiest], most, e->stream, &unused)) != cudaSuccess ||
+                     (ce = ensure_scratch(e, L->gate[busiest], most, e->stream, &unused)) != cudaSuccess))
       return ce;
     if (most == 0) return cudaSuccess;  // nothing routed to a resident expert
   }
@@ -1746,7 +1762,7 @@ void session_orphan(llr_session* s) {
 
 cudaError_t session_matmul(llr_exec* e, const llr_matrix* m, size_t tokens, const float* x, float* y) {
   void* scratch = nullptr;
-  cudaError_t ce = ensure_scratch(e, m, tokens, &scratch);
+  cudaError_t ce = ensure_scratch(e, m, tokens, e->stream, &scratch);
   if (ce != cudaSuccess) return ce;
   return launch_matmul(view_of(m), x, y, (int64_t)tokens, e->stream, e->path, e->sm_count, e->err_flag, scratch, &e->ctr.launches);
 }

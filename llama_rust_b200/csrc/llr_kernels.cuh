@@ -45,11 +45,13 @@ constexpr int64_t TC_MIN_TOKENS = 64;  // from here on AUTO prefers the bf16 tcg
 // y[t*rows + r] = sum_c W[r,c] * x[t*cols + c] for t < tokens.  Any shape the
 // entry points accept.  `launches` is incremented by the kernels launched.
 // `err_flag` is a device int that kernels with bounded waits set to non-zero when a wait ran out.
-// `scratch` (matmul_scratch_bytes, or null) lets the tensor-core GEMM stage 16-bit activations.
+// `scratch` lets the tensor-core GEMM stage 16-bit activations (matmul_wants_tc: matmul_scratch_bytes) or the integer GEMM its
+// digits (matmul_wants_i8: gemm_i8_scratch_bytes); null: other kernels run.
 cudaError_t launch_matmul(const MatView& m, const float* x, float* y, int64_t tokens,
                           cudaStream_t stream, int path, int sm_count, int* err_flag,
                           void* scratch, uint64_t* launches);
 bool matmul_wants_tc(const MatView& m, int64_t tokens, int path);
+bool matmul_wants_i8(const MatView& m, int64_t tokens, int path);
 size_t matmul_scratch_bytes(const MatView& m, int64_t tokens);  // for launch_matmul when matmul_wants_tc
 
 // Always-available reference kernel: one warp per row, byte loads, any alignment.
@@ -76,6 +78,14 @@ cudaError_t launch_gemv_rows_glu(const MatView& m, const float* x, float* out, c
 bool gemv_mma_supported(const MatView& m);
 cudaError_t launch_gemv_mma(const MatView& m, const float* x, float* y, int64_t tokens,
                             cudaStream_t stream, int sm_count, int* err_flag, uint64_t* launches);
+// The same products, bit for bit, for more activation rows and the K-quants: tcgen05 integer MMAs (llr_gemm_i8.cu).  Below
+// I8_MIN_TOKENS a pass of eight rows and a narrower one are as fast (Q4_K 14336 x 4096: 9 rows 30 us against 37, 16 rows 41
+// against 37; 4096 x 4096: 16 against 15, 23 against 16).  scratch: gemm_i8_scratch_bytes of the caller's, used until the
+// launched work has finished.
+constexpr int64_t I8_MIN_TOKENS = 13, I8_MAX_TOKENS = 4096;
+bool gemm_i8_supported(const MatView& m, int64_t tokens);
+size_t gemm_i8_scratch_bytes(const MatView& m, int64_t tokens);
+cudaError_t launch_gemm_i8(const MatView& m, const float* x, float* y, int64_t tokens, void* scratch, cudaStream_t stream, int* err_flag, uint64_t* launches);
 // Result delivery to the host by the kernel itself (host-pointer calls with at most 8 activation
 // rows): the reducer also stores each finished value at y + y_delta bytes, a device alias of
 // mapped pinned host memory, and the CTA that finishes last stores `ticket` into *done (mapped

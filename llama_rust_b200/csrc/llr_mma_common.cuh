@@ -655,6 +655,48 @@ __device__ __forceinline__ void row_inv_rms(const XSrc& s, int cols, int tokens,
   asm volatile("bar.sync 1, %0;" ::"n"(NWARP * 32) : "memory");
 }
 
+// Eight values per lane of one 256-column block of an activation row -> its four digit planes (pk[p]: this lane's eight bytes of
+// plane p), the sum of the 32-column group the lane belongs to (equal in its four lanes) and the block's 2^-e.
+__device__ __forceinline__ void split_block(const float (&v)[8], uint32_t (&pk)[4][2], float& sum, float& scale) {
+  // Largest magnitude of the block as a bit pattern: for non-negative floats the unsigned order of
+  // the bits is the numeric order, infinities and NaNs sort above every finite value, and one
+  // redux.sync replaces a five-step shuffle reduction on the latency-critical start of a phase.
+  uint32_t mb = 0;
+  sum = 0.f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) { mb = max(mb, __float_as_uint(v[j]) & 0x7fffffffu); sum += v[j]; }
+  mb = __reduce_max_sync(~0u, mb);
+  const bool bad = mb >= 0x7f800000u;  // a non-finite activation anywhere in the block
+  sum += __shfl_xor_sync(~0u, sum, 1);
+  sum += __shfl_xor_sync(~0u, sum, 2);
+  const int be = (int)(mb >> 23);
+  float s = 0.f, sinv = 0.f;  // an all-zero (or denormal) block contributes nothing
+  if (be != 0 && !bad) {
+    int e = 29 - (be - 127);
+    e = e > 126 ? 126 : e;
+    s = __uint_as_float((uint32_t)(e + 127) << 23);
+    sinv = __uint_as_float((uint32_t)(127 - e) << 23);
+  }
+  // digits of a value = bytes of (X + 0x80808080) ^ 0x80808080; a 4 x 4 byte transpose (eight
+  // byte permutes) turns four values into one word per digit plane
+#pragma unroll
+  for (int hq = 0; hq < 2; ++hq) {
+    uint32_t D[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int xi = bad ? 0 : __float2int_rn(v[4 * hq + j] * s);
+      D[j] = ((uint32_t)xi + 0x80808080u) ^ 0x80808080u;
+    }
+    const uint32_t t0 = __byte_perm(D[0], D[1], 0x5140), t1 = __byte_perm(D[2], D[3], 0x5140);
+    const uint32_t t2 = __byte_perm(D[0], D[1], 0x7362), t3 = __byte_perm(D[2], D[3], 0x7362);
+    pk[0][hq] = __byte_perm(t0, t1, 0x5410);
+    pk[1][hq] = __byte_perm(t0, t1, 0x7632);
+    pk[2][hq] = __byte_perm(t2, t3, 0x5410);
+    pk[3][hq] = __byte_perm(t2, t3, 0x7632);
+  }
+  scale = bad ? __uint_as_float(0x7fc00000u) : sinv;  // a non-finite activation makes the whole output row of that token NaN
+}
+
 // Activations of one span (nblk256 blocks of 256 columns starting at column col0, `tokens`
 // activation rows) -> four int8 digit planes per activation row, the f32 sums of x per 32
 // columns (Q4_K mins) and 2^-e per block.  Plain loads are L2-coherent and kept in L2 (policy
@@ -701,50 +743,15 @@ __device__ __forceinline__ void split_activations(const XSrc& src, int cols, int
         for (int j = 0; j < 8; ++j) v[j] = __fmul_rn(v[j], r);
       }
     }
-    // Largest magnitude of the block as a bit pattern: for non-negative floats the unsigned order of
-    // the bits is the numeric order, infinities and NaNs sort above every finite value, and one
-    // redux.sync replaces a five-step shuffle reduction on the latency-critical start of a phase.
-    uint32_t mb = 0;
-    float sum = 0.f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) { mb = max(mb, __float_as_uint(v[j]) & 0x7fffffffu); sum += v[j]; }
-    mb = __reduce_max_sync(~0u, mb);
-    const bool bad = mb >= 0x7f800000u;  // a non-finite activation anywhere in the block
-    sum += __shfl_xor_sync(~0u, sum, 1);
-    sum += __shfl_xor_sync(~0u, sum, 2);
-    const int be = (int)(mb >> 23);
-    float s = 0.f, sinv = 0.f;  // an all-zero (or denormal) block contributes nothing
-    if (be != 0 && !bad) {
-      int e = 29 - (be - 127);
-      e = e > 126 ? 126 : e;
-      s = __uint_as_float((uint32_t)(e + 127) << 23);
-      sinv = __uint_as_float((uint32_t)(127 - e) << 23);
-    }
-    // digits of a value = bytes of (X + 0x80808080) ^ 0x80808080; a 4 x 4 byte transpose (eight
-    // byte permutes) turns four values into one word per digit plane
     uint32_t pk[4][2];
-#pragma unroll
-    for (int hq = 0; hq < 2; ++hq) {
-      uint32_t D[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int xi = bad ? 0 : __float2int_rn(v[4 * hq + j] * s);
-        D[j] = ((uint32_t)xi + 0x80808080u) ^ 0x80808080u;
-      }
-      const uint32_t t0 = __byte_perm(D[0], D[1], 0x5140), t1 = __byte_perm(D[2], D[3], 0x5140);
-      const uint32_t t2 = __byte_perm(D[0], D[1], 0x7362), t3 = __byte_perm(D[2], D[3], 0x7362);
-      pk[0][hq] = __byte_perm(t0, t1, 0x5410);
-      pk[1][hq] = __byte_perm(t0, t1, 0x7632);
-      pk[2][hq] = __byte_perm(t2, t3, 0x5410);
-      pk[3][hq] = __byte_perm(t2, t3, 0x7632);
-    }
+    float sum, scale;
+    split_block(v, pk, sum, scale);
     const int nt = tok >> 1, plane0 = (tok & 1) * 4;
 #pragma unroll
     for (int p = 0; p < 4; ++p)
       *(uint2*)(dig + (size_t)(nt * 8 + plane0 + p) * Sp<MT>::DS + b * 256 + 8 * lane) = make_uint2(pk[p][0], pk[p][1]);
     if ((lane & 3) == 0) sxf[tok * (Sp<MT>::SPAN / 32) + b * 8 + (lane >> 2)] = sum;
-    // a non-finite activation makes the whole output row of that token NaN
-    if (lane == 0) xsi[tok * (Sp<MT>::SPAN / 256) + b] = bad ? __uint_as_float(0x7fc00000u) : sinv;
+    if (lane == 0) xsi[tok * (Sp<MT>::SPAN / 256) + b] = scale;
    }
   }
 }

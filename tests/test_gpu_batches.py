@@ -46,6 +46,66 @@ def test_rows_of_unpacked_formats_alone_and_in_a_batch(ex, name, rows, cols):
     m.free()
 
 
+# one block; the last rows of a tile; parts of 4096 columns that end in single blocks, in pairs and singles; units spread over CTAs; many tiles
+@pytest.mark.parametrize("name,rows,cols", [("Q4_K", 1, 256), ("Q4_K", 127, 2304), ("Q4_K", 130, 4096 + 256), ("Q4_K", 257, 2 * 4096 + 9 * 256),
+                                            ("Q4_K", 9600, 768), ("Q5_K", 64, 256), ("Q5_K", 129, 6400), ("Q5_K", 5000, 1024),
+                                            ("Q6_K", 3, 2048), ("Q6_K", 129, 4096), ("Q6_K", 260, 3 * 2048), ("Q6_K", 6000, 2048)])
+def test_rows_of_k_quants_alone_and_in_a_batch(ex, name, rows, cols):
+    """A row's bits do not depend on its batch: eight rows go through the decode kernel, more through the integer GEMM (whose sums are
+    the same integers).  Rows of zeros, of tiny and of huge values, of one sign, and one with an infinity among them."""
+    from llama_rust_b200 import synth
+    m = ex.synth(ALL[name], rows, cols, 7)
+    x = synth.activations(100 * cols, 8).reshape(100, cols).copy()
+    x[1] = 0
+    x[2] *= 1e-30
+    x[3] *= 1e30
+    x[4] = 1
+    x[5, ::3] *= 1e4
+    x[6] = np.abs(x[6])
+    x[23, cols // 2] = np.inf
+    ex.set_path(3)
+    alone = np.concatenate([_product(ex, m, x[t:t + 8]) for t in range(0, 100, 8)])
+    finite = np.arange(100) != 23
+    assert np.isnan(alone[23]).all() and np.isfinite(alone[finite]).all()
+    for path, counts in ((0, (12, 13, 16, 17, 24, 25, 32, 33, 48, 49, 63)), (3, (64, 100))):
+        ex.set_path(path)
+        for n in counts:
+            y = _product(ex, m, x[:n])
+            assert _same_bits(y[finite[:n]], alone[:n][finite[:n]]) and np.isnan(y[23:24]).all(), n
+    ex.set_path(0)
+    m.free()
+
+
+def test_products_on_other_streams_keep_their_bits(ex):
+    """The integer GEMM's workspace belongs to the executor's stream: on streams of the caller's, also while one is captured, the
+    decode kernel makes the same products."""
+    import torch
+    from llama_rust_b200 import synth
+    ex.set_path(0)
+    m = ex.synth(ALL["Q4_K"], 640, 1024, 9)
+    x = torch.from_numpy(synth.activations(20 * 1024, 10)).cuda()
+    want = torch.empty(20 * 640, device="cuda")
+    ex.matmul_device(m, 20, x.data_ptr(), want.data_ptr())
+    ex.synchronize()
+    side = torch.cuda.Stream()
+    got = torch.empty_like(want)
+    ex.matmul_device(m, 20, x.data_ptr(), got.data_ptr(), side.cuda_stream)
+    side.synchronize()
+    assert torch.equal(got, want)
+    graph = torch.cuda.CUDAGraph()
+    got.zero_()
+    with torch.cuda.graph(graph, stream=side):
+        ex.matmul_device(m, 20, x.data_ptr(), got.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    big = ex.synth(ALL["Q4_K"], 256, 4096, 9)
+    _product(ex, big, np.ones((63, 4096), np.float32))  # a larger workspace between capture and replay
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    del graph
+    m.free()
+    big.free()
+
+
 @pytest.mark.parametrize("lens", [[1 + i * 7 % 13 for i in range(70)],      # more runs of short groups than one list holds
                                   [15, 16, 17, 1, 64, 2, 16, 40, 31, 1, 3, 100]])
 def test_many_groups_in_one_batch(ex, tmp_path, lens):

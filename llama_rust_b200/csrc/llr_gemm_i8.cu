@@ -16,21 +16,27 @@
 //
 // A CTA owns 128 weight rows, TB activation rows and a range of units.  A unit is what one warp of the decode kernel owns of
 // 4096 columns: blocks w and w + 8.  Its result is one float per (row, activation row); the floats of the eight units of a
-// part are added in order, then the parts.  Twenty warps:
-//   * eight dequantize: packed bytes (TMA ring) -> low | high bytes in tensor memory (A operand), 64 columns a step;
+// part are added in order, then the parts.  28 warps:
+//   * sixteen dequantize: packed bytes (TMA ring) -> low | high bytes in tensor memory (A operand, stages of 128 columns); each
+//     decodes 64 columns of 32 weight rows of every block before it waits for a free stage, since the ring holds one to three
+//     blocks and its round trip is what the MMAs would otherwise wait for;
 //   * eight drain: accumulators of a finished unit -> floats, the mins, the sums over units, and the stores; two warps share
-//     the 32 tensor-memory lanes (weight rows) of a quarter, half of the activation rows each;
-//   * one copies packed weights, one digit tiles and the blocks' sums and scales, one issues the MMAs.
+//     the 32 tensor-memory lanes (weight rows) of a quarter, half of the activation rows each, and fetch the next activation row's
+//     accumulators while they work on one;
+//   * one copies packed weights, one digit tiles and the blocks' sums and scales, two issue the MMAs.
+// (Eight dequantizing warps, one issuing warp that waited for every 64 columns: 44 us instead of 34 for 24 rows of Q4_K
+// 14336 x 4096, 37 instead of 30 for 16 rows.)
 // Both blocks of a unit have accumulators of their own (2 x 2 x 4 TB columns of tensor memory), the rest holds the A ring.
 // Few row tiles: the units are spread over several CTAs (grid z), each unit's floats go to memory and a second kernel adds
 // them in the same order.
-// Measured, passes of the decode kernel -> this: 24 rows Q4_K 14336 x 4096 62 -> 44 us, 4096 x 4096 34 -> 18, 1024 x 4096
-// 28 -> 12; Q6_K 4096 x 14336 124 -> 58; 63 rows Q4_K 4096 x 4096 90 -> 43.
+// Measured, passes of the decode kernel -> this: 24 rows Q4_K 14336 x 4096 62 -> 34 us, 4096 x 4096 34 -> 15, 1024 x 4096
+// 28 -> 10; Q6_K 4096 x 14336 124 -> 47, 32000 x 4096 138 -> 71; 48 rows Q4_K 4096 x 4096 68 -> 23.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "llr_formats.cuh"
 #include "llr_kernels.cuh"
@@ -42,15 +48,19 @@ namespace llr {
 namespace {
 using namespace umma;
 
-constexpr int DQ = 8, DR = 8;  // dequantizing and draining warps
-constexpr int W_PACKED = DQ + DR, W_DIG = W_PACKED + 1, W_MMA = W_DIG + 1, THREADS = 32 * (W_MMA + 2);
+constexpr int DQ = 16, DR = 8;  // dequantizing and draining warps
+// Registers per thread: the drain keeps two activation rows' accumulators in flight, the others need few.  All warpgroups give or
+// take at their start; the sum is what the block was launched with (28 warps x 72).
+constexpr int REG_DQ = 64, REG_DR = 104, REG_REST = 40;
+static_assert(4 * REG_DQ + 2 * REG_DR + REG_REST <= 7 * 72, "register split");
+constexpr int W_PACKED = DQ + DR, W_DIG = W_PACKED + 1, W_MMA = W_DIG + 1, THREADS = 32 * (W_MMA + 2);  // two MMA warps
 constexpr int PART_BLOCKS = 16, PART_UNITS = 8;  // of 4096 columns
 constexpr int AUX = 48;  // bytes per (block, activation row): eight sums of 32 columns, 2^-e, padding
 
 template <int DT, int TB> struct ILay {
   static constexpr int N = 4 * TB;             // digit planes of TB activation rows
   static constexpr int ACC = 2 * 2 * N;        // accumulator columns: (low, high) of a unit's two blocks
-  static constexpr int A_COLS = 32;            // 64 weight columns: (low, high) x 2 sub-blocks x 8 words
+  static constexpr int A_COLS = 64;            // 128 weight columns: 4 sub-blocks x (low, high) x 8 words
   static constexpr int NA = (512 - ACC) / A_COLS;
   static constexpr int IMG = N * 256;          // digits of one block, as the MMA reads them
   static constexpr int REC = IMG + TB * AUX;   // a block's record in memory
@@ -61,7 +71,7 @@ template <int DT, int TB> struct ILay {
   static constexpr int FIT = (SMEM_LIMIT - FIXED - P) / P_STAGE, NPK = FIT > 6 ? 6 : FIT;
   static constexpr int BAR = (P + NPK * P_STAGE + 64 + 15) / 16 * 16;
   static constexpr int TOTAL = BAR + 512 + 1024;
-  static_assert(NA >= 4 && NA % 4 == 0 && NPK >= 2 && P % 128 == 0 && IMG % 1024 == 0 && REC % 16 == 0, "rings");
+  static_assert(NA >= 2 && NA % 2 == 0 && NPK >= 2 && P % 128 == 0 && IMG % 1024 == 0 && REC % 16 == 0, "rings");
   static_assert((2 * NA + 2 * NB + 2 * NX + 2 * NPK + 2) * 8 + 8 <= 512 && TOTAL <= SMEM_LIMIT, "shared memory");
 };
 
@@ -102,24 +112,21 @@ __device__ __forceinline__ void split_bytes(uint32_t p02, uint32_t p13, uint32_t
   hi = __byte_perm(p02, p13, 0x7351);
 }
 
-// 64 columns (sub-blocks 2G, 2G + 1) of the row at prow: o[0..7] low bytes of the first, o[8..15] its high bytes, then the second.
+// Sub-block 2 G + S (32 columns) of the row at prow: o[0..7] low bytes, o[8..15] high bytes.
 // Q4_K: 16 scale code, Q5_K: scale code, Q6_K: 4 scale (code - 32), the multiples that the decode kernel sums too.
-template <int DT>
-__device__ __forceinline__ void decode64(uint32_t prow, int lead, int G, uint32_t (&o)[32]) {
+template <int DT, int S>
+__device__ __forceinline__ void decode32(uint32_t prow, int lead, int G, uint32_t (&o)[16]) {
   if constexpr (DT == DT_Q6_K) {
+    uint32_t c[8];
+    float d;
+    int sc[2];
+    q6k_codes(prow, lead, 2 * G + S, c, d, sc[0], sc[1]);
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      uint32_t c[8];
-      float d;
-      int sc[2];
-      q6k_codes(prow, lead, 2 * G + s, c, d, sc[0], sc[1]);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        // both halves of 4 scale (code - 32) + 32768 lie in [16384, 49152]; flipping the top bit takes the 32768 off again
-        const uint32_t k = 4u * (uint32_t)sc[i >> 2], bias = 0x80008000u - 32u * k * 0x10001u;
-        split_bytes((c[i] & 0x00ff00ffu) * k + bias, ((c[i] >> 8) & 0x00ff00ffu) * k + bias, o[16 * s + i], o[16 * s + 8 + i]);
-        o[16 * s + 8 + i] ^= 0x80808080u;
-      }
+    for (int i = 0; i < 8; ++i) {
+      // both halves of 4 scale (code - 32) + 32768 lie in [16384, 49152]; flipping the top bit takes the 32768 off again
+      const uint32_t k = 4u * (uint32_t)sc[i >> 2], bias = 0x80008000u - 32u * k * 0x10001u;
+      split_bytes((c[i] & 0x00ff00ffu) * k + bias, ((c[i] >> 8) & 0x00ff00ffu) * k + bias, o[i], o[8 + i]);
+      o[8 + i] ^= 0x80808080u;
     }
   } else {
     constexpr bool K5 = DT == DT_Q5_K;
@@ -127,25 +134,20 @@ __device__ __forceinline__ void decode64(uint32_t prow, int lead, int G, uint32_
     lds_chunks<1>(prow, h);
     lds_chunks<2>(prow + (K5 ? 48 : 16) + 32 * G, q);
     const uint32_t sc = G < 2 ? h[1] & 0x3f3f3f3fu : (h[3] & 0x0f0f0f0fu) | ((h[1] >> 2) & 0x30303030u);
-    const uint32_t s0 = (sc >> (16 * (G & 1))) & 255u, s1 = (sc >> (16 * (G & 1) + 8)) & 255u;
+    const uint32_t s = (sc >> (16 * (G & 1) + 8 * S)) & 255u;
     if constexpr (K5) {
       uint32_t f[8];
       lds_chunks<2>(prow + 16, f);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const uint32_t fb = f[i] >> (2 * G);
-        const uint32_t a = (q[i] & 0x0f0f0f0fu) | ((fb & 0x01010101u) << 4), b = ((q[i] >> 4) & 0x0f0f0f0fu) | ((fb & 0x02020202u) << 3);
-        split_bytes((a & 0x00ff00ffu) * s0, ((a >> 8) & 0x00ff00ffu) * s0, o[i], o[8 + i]);
-        split_bytes((b & 0x00ff00ffu) * s1, ((b >> 8) & 0x00ff00ffu) * s1, o[16 + i], o[24 + i]);
+        const uint32_t a = ((q[i] >> (4 * S)) & 0x0f0f0f0fu) | (((f[i] >> (2 * G + S)) & 0x01010101u) << 4);
+        split_bytes((a & 0x00ff00ffu) * s, ((a >> 8) & 0x00ff00ffu) * s, o[i], o[8 + i]);
       }
     } else {
-      const uint32_t s16 = 16u * s0;
+      constexpr uint32_t M = S ? 0x00f000f0u : 0x000f000fu;
+      const uint32_t k = S ? s : 16u * s;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const uint32_t t = q[i] >> 8;
-        split_bytes((q[i] & 0x000f000fu) * s16, (t & 0x000f000fu) * s16, o[i], o[8 + i]);
-        split_bytes((q[i] & 0x00f000f0u) * s1, (t & 0x00f000f0u) * s1, o[16 + i], o[24 + i]);
-      }
+      for (int i = 0; i < 8; ++i) split_bytes((q[i] & M) * k, ((q[i] >> 8) & M) * k, o[i], o[8 + i]);
     }
   }
 }
@@ -170,9 +172,43 @@ __device__ __forceinline__ void read_head(uint32_t prow, int lead, Head<DT>& H) 
   }
 }
 
-__device__ __forceinline__ void tmem_ld8(uint32_t addr, int (&v)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(addr) : "memory");
+// four digit sums of one activation row
+__device__ __forceinline__ void tmem_ld4(uint32_t addr, int (&v)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&o)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               ::"r"(addr), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]), "r"(o[8]), "r"(o[9]), "r"(o[10]),
+                 "r"(o[11]), "r"(o[12]), "r"(o[13]), "r"(o[14]), "r"(o[15]) : "memory");
+}
+
+// One activation row of a finished unit of NBK blocks; its sums and scale lie at xa[k] + off
+template <int DT, int NBK>
+__device__ __forceinline__ float join(const int (&v)[NBK][2][4], const Head<DT> (&H)[2], const uint32_t (&xa)[2], uint32_t off) {
+  constexpr float W0 = DT == DT_Q4_K ? 0.0625f : DT == DT_Q6_K ? 0.25f : 1.f;  // weights of the digits: 256^p, and 1/16 or 1/4 for the codes' multiples
+  const pair w01 = pack2(W0, W0 * 256.f), w23 = pack2(W0 * 65536.f, W0 * 16777216.f);
+  pair s01 = 0, s23 = 0, m01 = 0, m23 = 0;
+#pragma unroll
+  for (int k = 0; k < NBK; ++k) {
+    float xs;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(xs) : "r"(xa[k] + off + 32));
+    const float m = __fmul_rn(H[k].d, xs);
+    const pair mm = pack2(m, m);  // times the weight as the decode kernel does it: the scales of tiny activations round there
+    const int* l = v[k][0];
+    const int* h = v[k][1];
+    s01 = fma2(pack2((float)(l[0] + 256 * h[0]), (float)(l[1] + 256 * h[1])), mul2(mm, w01), s01);
+    s23 = fma2(pack2((float)(l[2] + 256 * h[2]), (float)(l[3] + 256 * h[3])), mul2(mm, w23), s23);
+    if constexpr (DT != DT_Q6_K) {
+      pair c[4];
+      asm volatile("ld.shared.v2.u64 {%0,%1}, [%2];" : "=l"(c[0]), "=l"(c[1]) : "r"(xa[k] + off));
+      asm volatile("ld.shared.v2.u64 {%0,%1}, [%2];" : "=l"(c[2]), "=l"(c[3]) : "r"(xa[k] + off + 16));
+      m01 = fma2(H[k].m[0], c[0], fma2(H[k].m[2], c[2], m01));
+      m23 = fma2(H[k].m[1], c[1], fma2(H[k].m[3], c[3], m23));
+    }
+  }
+  float r = __fadd_rn(__fadd_rn(low2(s01), high2(s01)), __fadd_rn(low2(s23), high2(s23)));
+  if constexpr (DT != DT_Q6_K) r = __fsub_rn(r, __fadd_rn(__fadd_rn(low2(m01), high2(m01)), __fadd_rn(low2(m23), high2(m23))));
+  return r;
 }
 
 struct Args {
@@ -205,11 +241,11 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap wmap, const Args P, int* __re
 
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (tid == 0) {
-    for (int s = 0; s < NA; ++s) { bar_init(&full_a[s], 4); bar_init(&empty_a[s], 1); }
-    for (int s = 0; s < NB; ++s) { bar_init(&full_b[s], 1); bar_init(&empty_b[s], 1); }
+    for (int s = 0; s < NA; ++s) { bar_init(&full_a[s], 8); bar_init(&empty_a[s], 2); }
+    for (int s = 0; s < NB; ++s) { bar_init(&full_b[s], 1); bar_init(&empty_b[s], 2); }
     for (int s = 0; s < NX; ++s) { bar_init(&full_x[s], 1); bar_init(&empty_x[s], DR); }
     for (int s = 0; s < NPK; ++s) { bar_init(&pk_full[s], 1); bar_init(&pk_empty[s], DQ + DR); }
-    bar_init(acc_full, 1);
+    bar_init(acc_full, 2);
     bar_init(acc_empty, DR);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -230,49 +266,39 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap wmap, const Args P, int* __re
   };
 
   if (warp < DQ) {
-    // ------------------------------------------------------------ dequantization: groups gh and gh + 2 of every block
-    const int q = warp & 3, gh = warp >> 2;
+    // ------------------------------------------------------------ dequantization: columns 64 G .. 64 G + 63 of every block
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REG_DQ));
+    const int q = warp & 3, G = warp >> 2;
     const uint32_t a_dst = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)L::ACC;
     int n = 0;
     for (int u = u_begin; u < u_end; ++u) {
       int first;
       const int nb = unit_blocks(u, P.blocks, first);
       for (int k = 0; k < nb; ++k, ++n) {
-        const int b = first + PART_UNITS * k, lead = DT == DT_Q6_K ? (b * RB) & 15 : 0;
+        const int b = first + PART_UNITS * k, lead = DT == DT_Q6_K ? (b * RB) & 15 : 0, st = 2 * n + (G >> 1);
         wait(pk_full, n, NPK);
-        const uint32_t prow = s32(smem + L::P) + (uint32_t)((n % NPK) * L::P_STAGE + (32 * q + lane) * PITCH);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          uint32_t o[32];
-          decode64<DT>(prow, lead, gh + 2 * i, o);
-          if (i == 1) {
-            __syncwarp();
-            if (lane == 0) bar_arrive(&pk_empty[n % NPK]);
-          }
-          const int st = 4 * n + gh + 2 * i;
-          wait_free(empty_a, st, NA);
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          asm volatile(
-              "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-              "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-              ::"r"(a_dst + (uint32_t)(st % NA * L::A_COLS)), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]),
-                "r"(o[8]), "r"(o[9]), "r"(o[10]), "r"(o[11]), "r"(o[12]), "r"(o[13]), "r"(o[14]), "r"(o[15]), "r"(o[16]), "r"(o[17]), "r"(o[18]),
-                "r"(o[19]), "r"(o[20]), "r"(o[21]), "r"(o[22]), "r"(o[23]), "r"(o[24]), "r"(o[25]), "r"(o[26]), "r"(o[27]), "r"(o[28]), "r"(o[29]),
-                "r"(o[30]), "r"(o[31]) : "memory");
-          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) bar_arrive(&full_a[st % NA]);
-        }
+        const uint32_t prow = s32(smem + L::P) + (uint32_t)((n % NPK) * L::P_STAGE + (32 * q + lane) * PITCH), dst = a_dst + (uint32_t)(st % NA * L::A_COLS + 32 * (G & 1));
+        uint32_t o[2][16];  // decoded before a stage is free: what follows, up to the MMA, is the latency that the short ring has to cover
+        decode32<DT, 0>(prow, lead, G, o[0]);
+        decode32<DT, 1>(prow, lead, G, o[1]);
+        __syncwarp();
+        if (lane == 0) bar_arrive(&pk_empty[n % NPK]);
+        wait_free(empty_a, st, NA);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tmem_st16(dst, o[0]);
+        tmem_st16(dst + 16, o[1]);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) bar_arrive(&full_a[st % NA]);
       }
     }
   } else if (warp < DQ + DR) {
     // -------------------------------------------------------------------------------------------------------- drain
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REG_DR));
     constexpr int TW = TB / 2;  // activation rows of this warp
     const int q = warp & 3, half = (warp - DQ) >> 2, row = row0 + 32 * q + lane;
     const uint32_t acc = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(4 * TW * half);
-    constexpr float W0 = DT == DT_Q4_K ? 0.0625f : DT == DT_Q6_K ? 0.25f : 1.f;  // weights of the digits: 256^p, and 1/16 or 1/4 for the codes' multiples
-    const pair w01 = pack2(W0, W0 * 256.f), w23 = pack2(W0 * 65536.f, W0 * 16777216.f);
     const bool split = gridDim.z > 1;
     float sum[TW], carry[TW];
 #pragma unroll
@@ -283,6 +309,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap wmap, const Args P, int* __re
       int first;
       const int nb = unit_blocks(u, P.blocks, first);
       Head<DT> H[2];
+      uint32_t xa[2];
 #pragma unroll
       for (int k = 0; k < 2; ++k)
         if (k < nb) {
@@ -291,56 +318,37 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap wmap, const Args P, int* __re
           read_head<DT>(s32(smem + L::P) + (uint32_t)((n + k) % NPK * L::P_STAGE + (32 * q + lane) * PITCH), DT == DT_Q6_K ? (b * RB) & 15 : 0, H[k]);
           __syncwarp();
           if (lane == 0) bar_arrive(&pk_empty[(n + k) % NPK]);
+          wait(full_x, n + k, NX);
+          xa[k] = s32(smem + L::X) + (uint32_t)(((n + k) % NX * TB + half * TW) * AUX);
         }
-      wait(full_x, n, NX);
-      if (nb == 2) wait(full_x, n + 1, NX);
-      const uint32_t x0 = s32(smem + L::X) + (uint32_t)(n % NX * TB * AUX + half * TW * AUX), x1 = s32(smem + L::X) + (uint32_t)((n + 1) % NX * TB * AUX + half * TW * AUX);
       wait(acc_full, u - u_begin, 1);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      auto unit = [&](auto NBK_) {
+        constexpr int NBK = decltype(NBK_)::value;
+        int v[2][NBK][2][4];
+        auto fetch = [&](int t, int (&d)[NBK][2][4]) {
 #pragma unroll
-      for (int t0 = 0; t0 < TW; t0 += 2) {
-        int lo[2][8], hi[2][8];
-        tmem_ld8(acc + (uint32_t)(4 * t0), lo[0]);
-        tmem_ld8(acc + (uint32_t)(N + 4 * t0), hi[0]);
-        if (nb == 2) {
-          tmem_ld8(acc + (uint32_t)(2 * N + 4 * t0), lo[1]);
-          tmem_ld8(acc + (uint32_t)(3 * N + 4 * t0), hi[1]);
-        }
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          for (int k = 0; k < NBK; ++k) {
+            tmem_ld4(acc + (uint32_t)(2 * N * k + 4 * t), d[k][0]);
+            tmem_ld4(acc + (uint32_t)(2 * N * k + N + 4 * t), d[k][1]);
+          }
+        };
+        fetch(0, v[0]);
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int t = t0 + j;
-          pair s01 = 0, s23 = 0, m01 = 0, m23 = 0;
-#pragma unroll
-          for (int k = 0; k < 2; ++k)
-            if (k < nb) {
-              const uint32_t xa = (k ? x1 : x0) + (uint32_t)(t * AUX);
-              float xs;
-              asm volatile("ld.shared.f32 %0, [%1];" : "=f"(xs) : "r"(xa + 32));
-              const float m = __fmul_rn(H[k].d, xs);
-              const pair mm = pack2(m, m);  // times the weight as the decode kernel does it: the scales of tiny activations round there
-              const int* l = lo[k] + 4 * j;
-              const int* h = hi[k] + 4 * j;
-              s01 = fma2(pack2((float)(l[0] + 256 * h[0]), (float)(l[1] + 256 * h[1])), mul2(mm, w01), s01);
-              s23 = fma2(pack2((float)(l[2] + 256 * h[2]), (float)(l[3] + 256 * h[3])), mul2(mm, w23), s23);
-              if constexpr (DT != DT_Q6_K) {
-                pair c[4];
-                asm volatile("ld.shared.v2.u64 {%0,%1}, [%2];" : "=l"(c[0]), "=l"(c[1]) : "r"(xa));
-                asm volatile("ld.shared.v2.u64 {%0,%1}, [%2];" : "=l"(c[2]), "=l"(c[3]) : "r"(xa + 16));
-                m01 = fma2(H[k].m[0], c[0], fma2(H[k].m[2], c[2], m01));
-                m23 = fma2(H[k].m[1], c[1], fma2(H[k].m[3], c[3], m23));
-              }
-            }
-          float v = __fadd_rn(__fadd_rn(low2(s01), high2(s01)), __fadd_rn(low2(s23), high2(s23)));
-          if constexpr (DT != DT_Q6_K) v = __fsub_rn(v, __fadd_rn(__fadd_rn(low2(m01), high2(m01)), __fadd_rn(low2(m23), high2(m23))));
+        for (int t = 0; t < TW; ++t) {
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (t + 1 < TW) fetch(t + 1, v[(t + 1) & 1]);
+          const float r = join<DT, NBK>(v[t & 1], H, xa, (uint32_t)(t * AUX));
           if (split) {
             const int tok = tok0 + TW * half + t;
-            if (row < P.rows && tok < P.tokens) P.y[((int64_t)u * P.tokens + tok) * P.rows + row] = v;
+            if (row < P.rows && tok < P.tokens) P.y[((int64_t)u * P.tokens + tok) * P.rows + row] = r;
           } else {
-            sum[t] = __fadd_rn(sum[t], v);
+            sum[t] = __fadd_rn(sum[t], r);
           }
         }
-      }
+      };
+      if (nb == 2) unit(std::integral_constant<int, 2>{});
+      else unit(std::integral_constant<int, 1>{});
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) {
@@ -365,7 +373,9 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap wmap, const Args P, int* __re
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  } else if (warp == W_PACKED) {
+  } else {
+   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REG_REST));
+   if (warp == W_PACKED) {
     if (lane == 0) {
       int n = 0;
       for (int u = u_begin; u < u_end; ++u) {
@@ -382,7 +392,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap wmap, const Args P, int* __re
         }
       }
     }
-  } else if (warp == W_DIG) {
+   } else if (warp == W_DIG) {
     if (lane == 0) {
       asm volatile("griddepcontrol.wait;" ::: "memory");  // the records are the kernel before's output
       int n = 0;
@@ -403,9 +413,13 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap wmap, const Args P, int* __re
         }
       }
     }
-  } else if (warp == W_MMA) {
-    // converged loop, one elected lane issues: addresses and descriptors stay in uniform registers
+   } else {
+    // Two warps issue, one the low bytes' MMAs and one the high bytes' (accumulators of their own): a stage's wait, its MMAs and its
+    // commit take one warp longer than the tensor pipe needs for them.  Converged loops, one elected lane issues: addresses and
+    // descriptors stay in uniform registers.
+    const int high = warp - W_MMA;
     const uint32_t td = __shfl_sync(0xffffffffu, tmem, 0), sb = __shfl_sync(0xffffffffu, s32(smem + L::B), 0);
+    const uint32_t idesc = high ? desc_i8<N, true>() : desc_i8<N, false>();
     int n = 0;
     for (int u = u_begin; u < u_end; ++u) {
       int first;
@@ -413,23 +427,22 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap wmap, const Args P, int* __re
       wait_free(acc_empty, u - u_begin, 1);
       for (int k = 0; k < nb; ++k, ++n) {
         wait(full_b, n, NB);
-        for (int G = 0; G < 4; ++G) {
-          const int st = 4 * n + G;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int st = 2 * n + h;
           wait(full_a, st, NA);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           if (elect_one()) {
-            const uint32_t ta = td + (uint32_t)(L::ACC + st % NA * L::A_COLS), acc = td + (uint32_t)(2 * N * k);
-            const uint64_t db = smem_desc_u(sb + (uint32_t)(n % NB * L::IMG + (G >> 1) * (N * 128))) + (uint64_t)(4 * (G & 1));
+            const uint32_t ta = td + (uint32_t)(L::ACC + st % NA * L::A_COLS + 8 * high), acc = td + (uint32_t)(2 * N * k + N * high);
+            const uint64_t db = smem_desc_u(sb + (uint32_t)(n % NB * L::IMG + h * (N * 128)));
 #pragma unroll
-            for (int s = 0; s < 2; ++s) {
-              const uint32_t more = G + s ? 1u : 0u;
+            for (int s = 0; s < 4; ++s) {
+              const uint32_t more = h + s ? 1u : 0u;
               asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p; }"
-                           ::"r"(acc), "r"(ta + 16 * s), "l"(db + 2 * s), "r"(desc_i8<N, false>()), "r"(more) : "memory");
-              asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p; }"
-                           ::"r"(acc + N), "r"(ta + 16 * s + 8), "l"(db + 2 * s), "r"(desc_i8<N, true>()), "r"(more) : "memory");
+                           ::"r"(acc), "r"(ta + 16 * s), "l"(db + 2 * s), "r"(idesc), "r"(more) : "memory");
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(&empty_a[st % NA])) : "memory");
-            if (G == 3) {
+            if (h == 1) {
               asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(&empty_b[n % NB])) : "memory");
               if (k == nb - 1) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(acc_full)) : "memory");
             }
@@ -438,6 +451,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap wmap, const Args P, int* __re
         }
       }
     }
+   }
   }
   __syncthreads();
   if (warp == W_MMA) {

@@ -79,8 +79,8 @@ bool gemv_mma_supported(const MatView& m);
 cudaError_t launch_gemv_mma(const MatView& m, const float* x, float* y, int64_t tokens,
                             cudaStream_t stream, int sm_count, int* err_flag, uint64_t* launches);
 // The same products, bit for bit, for more activation rows and the K-quants: tcgen05 integer MMAs (llr_gemm_i8.cu).  Below
-// I8_MIN_TOKENS a pass of eight rows and a narrower one are as fast (Q4_K 14336 x 4096: 9 rows 30 us against 37, 16 rows 41
-// against 37; 4096 x 4096: 16 against 15, 23 against 16).  scratch: gemm_i8_scratch_bytes of the caller's, used until the
+// I8_MIN_TOKENS a pass of eight rows and a narrower one are as fast (Q4_K 14336 x 4096: 9 rows 30 us against 30, 13 rows 40
+// against 30; 4096 x 4096: 16 against 14, 21 against 14).  scratch: gemm_i8_scratch_bytes of the caller's, used until the
 // launched work has finished.
 constexpr int64_t I8_MIN_TOKENS = 13, I8_MAX_TOKENS = 4096;
 bool gemm_i8_supported(const MatView& m, int64_t tokens);

@@ -12,11 +12,12 @@
 // With `glu` W stacks gate | up (2 rows rows) and the results are gated units: a tile then holds as many gate rows
 // as up rows, so that a thread of the epilogue has both factors of each result.
 //
-// One CTA computes a tile of 128 activation rows x bn <= BN weight rows: the activation rows are the MMA's M dimension (one
+// One CTA computes a tile of 128 or 256 activation rows x bn <= BN weight rows: the activation rows are the MMA's M dimension (one
 // tensor-memory lane each), so that a thread of the epilogue holds consecutive results of one activation row and stores
-// them as vectors.  Six warps: four read the accumulators, one issues the TMA loads, one the MMAs.  Two CTAs fit an SM
-// at BN <= 128 (96 KB of stages, 128 columns of tensor memory each), so one tile's epilogue overlaps another's loads.
-// bn is the width, a multiple of sixteen, for which the grid's waves over the SMs cost least.  A K range may be cut into slices (gridDim.z): slice s leaves its partial sums at y + s * slice_stride and the reader
+// them as vectors.  One warp issues the TMA loads, one the MMAs, four read the accumulators, eight where a CTA has the SM to itself.
+// Two CTAs fit an SM at BN <= 128 (96 KB of stages, 128 columns of tensor memory each), so one tile's epilogue overlaps another's
+// loads.  Wide tiles are bound by what the SMs draw from L2, so 256 activation rows share a stage's weights where that saves waves
+// (tile_shape).  A K range may be cut into slices (gridDim.z): slice s leaves its partial sums at y + s * slice_stride and the reader
 // adds them in slice order.  Every wait is bounded.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -31,17 +32,18 @@
 namespace llr {
 namespace {
 
-constexpr int BM = 128;  // activation rows per CTA = UMMA M
+constexpr int BM = 128;  // activation rows per MMA = UMMA M
 constexpr int BK = 64;   // columns per stage: one 128-byte swizzle row
-constexpr int THREADS = 6 * 32, W_TMA = 4, W_MMA = 5;
 constexpr int SPIN = 1 << 24;
 
-template <int BN> struct Lay {
-  static constexpr int A_STAGE = BM * 128, B_STAGE = BN * 128, STAGE = A_STAGE + B_STAGE;
-  static constexpr int NS = BN == 256 ? 4 : BN == 128 ? 3 : 4;  // 192, 96, 96 KB
+// RT: tiles of BM activation rows per CTA
+template <int BN, int RT> struct Lay {
+  static constexpr int A_STAGE = RT * BM * 128, B_STAGE = BN * 128, STAGE = A_STAGE + B_STAGE;
+  static constexpr int NS = RT == 2 ? 3 : BN == 256 ? 4 : BN == 128 ? 3 : 4;  // 192, 192, 96, 96 KB
+  static constexpr int EPI = BN == 256 ? 8 : 4, W_TMA = EPI, W_MMA = EPI + 1, THREADS = (EPI + 2) * 32;  // epilogue warps first
   static constexpr int BAR = NS * STAGE;
   static constexpr int TOTAL = 1024 /*alignment*/ + NS * STAGE + 256;
-  static constexpr int TMEM_COLS = BN;
+  static constexpr int TMEM_COLS = RT * BN;
 };
 
 __device__ __forceinline__ uint32_t s32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -96,11 +98,11 @@ __device__ __forceinline__ void load32(uint32_t taddr, uint32_t (&v)[32]) {
       : "r"(taddr) : "memory");
 }
 
-template <int BN, bool GLU>
-__global__ void __launch_bounds__(THREADS)
+template <int BN, int RT, bool GLU>
+__global__ void __launch_bounds__(Lay<BN, RT>::THREADS)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const Args a, int* __restrict__ err) {
-  using L = Lay<BN>;
-  constexpr int NS = L::NS;
+  using L = Lay<BN, RT>;
+  constexpr int NS = L::NS, W_TMA = L::W_TMA, W_MMA = L::W_MMA;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full = (uint64_t*)(smem + L::BAR);
@@ -110,7 +112,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int bn = a.bn, width = GLU ? bn / 2 : bn;  // results per activation row of the tile
   // token tiles run fastest: the CTAs that share weight rows run at the same time, and the weights are read from HBM once
-  const int row0 = blockIdx.y * width, tok0 = blockIdx.x * BM;
+  const int row0 = blockIdx.y * width, tok0 = blockIdx.x * (RT * BM);
   const int z = (int)blockIdx.z / a.slices, slice = (int)blockIdx.z % a.slices;
   const int per = (a.nk + a.slices - 1) / a.slices, k0 = slice * per, k1 = min(a.nk, k0 + per);  // never empty: the launcher sees to it
 
@@ -158,8 +160,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
 #pragma unroll
         for (int kk = 0; kk < BK / 16; ++kk) {
           const uint32_t acc = (k > k0 || kk > 0) ? 1u : 0u;
-          asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }"
-                       ::"r"(td), "l"(da + 2 * kk), "l"(db + 2 * kk), "r"(idesc), "r"(acc) : "memory");
+#pragma unroll
+          for (int r = 0; r < RT; ++r)
+            asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }"
+                         ::"r"(td + (uint32_t)(r * BN)), "l"(da + (uint64_t)(r * BM * 128 / 16 + 2 * kk)), "l"(db + 2 * kk), "r"(idesc), "r"(acc) : "memory");
         }
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(&empty[s])) : "memory");
       }
@@ -171,7 +175,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
   } else {
     if (!bar_wait(done, 0)) { ok = false; report_error(err, 5); }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int t = tok0 + 32 * warp + lane;
+    // warps 4.. read the second tile of activation rows, or every other run of columns of the only one
+    const int r = RT == 2 ? warp >> 2 : 0, t = tok0 + BM * r + 32 * (warp & 3) + lane;
+    constexpr int C_STEP = RT == 1 ? 8 * L::EPI : 32;
     const int n_live = min(width, a.rows - row0);
     const int64_t off = (int64_t)t * a.y_ld + (int64_t)z * a.rows + row0;
     float* y = a.y ? a.y + slice * a.slice_stride + off : nullptr;
@@ -180,9 +186,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
     if (a.gate && t < a.tokens) gate = 1.0f / (1.0f + expf(-a.gate[(int64_t)t * a.gate_ld + z]));
     const bool vec = ((a.y_ld | a.rows) & 7) == 0;  // every run of eight results starts on a 16-byte boundary in either format
 #pragma unroll 1
-    for (int c0 = 0; c0 < n_live; c0 += 32) {
+    for (int c0 = RT == 1 ? 32 * (warp >> 2) : 0; c0 < n_live; c0 += C_STEP) {
       uint32_t v[32], u[32];
-      const uint32_t taddr = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0;
+      const uint32_t taddr = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(r * BN + c0);
       load32(taddr, v);
       if constexpr (GLU) load32(taddr + (uint32_t)width, u);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -238,39 +244,44 @@ bool encode_rows(CUtensorMap* map, const void* base, int64_t cols, int64_t rows,
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN, bool GLU>
+template <int BN, int RT, bool GLU>
 cudaError_t launch_tiles(const Bf16Product& p, const Args& a, cudaStream_t stream, int* err) {
   CUtensorMap xmap, wmap;
   const int width = GLU ? a.bn / 2 : a.bn;  // rows of one box of W
-  if (!encode_rows(&xmap, p.x16, p.x_cols, p.tokens, p.x_ld, BM) || !encode_rows(&wmap, p.w, p.cols, (int64_t)p.rows * (GLU ? 2 : p.batch), p.cols, width))
+  if (!encode_rows(&xmap, p.x16, p.x_cols, p.tokens, p.x_ld, RT * BM) || !encode_rows(&wmap, p.w, p.cols, (int64_t)p.rows * (GLU ? 2 : p.batch), p.cols, width))
     return cudaErrorInvalidValue;
-  constexpr int smem = Lay<BN>::TOTAL;
+  constexpr int smem = Lay<BN, RT>::TOTAL;
   static PerDevice ready;
   std::atomic<int>& slot = ready.here();
   if (slot.load(std::memory_order_relaxed) == 0) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, RT, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     slot.store(1, std::memory_order_relaxed);
   }
-  const dim3 grid((unsigned)((p.tokens + BM - 1) / BM), (unsigned)((p.rows + width - 1) / width), (unsigned)(p.batch * a.slices));
+  const dim3 grid((unsigned)((p.tokens + RT * BM - 1) / (RT * BM)), (unsigned)((p.rows + width - 1) / width), (unsigned)(p.batch * a.slices));
   if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidValue;
-  gemm_bf16_kernel<BN, GLU><<<grid, THREADS, smem, stream>>>(xmap, wmap, a, err);
+  gemm_bf16_kernel<BN, RT, GLU><<<grid, Lay<BN, RT>::THREADS, smem, stream>>>(xmap, wmap, a, err);
   return cudaGetLastError();
 }
 
 constexpr int SMS = 148;
-int tiles_of(int tokens, int rows, int batch, int bn) { return ((tokens + BM - 1) / BM) * ((rows + bn - 1) / bn) * batch; }
-// Width of a tile: with many tiles the one of 160 .. 256 (a multiple of `step`, so that both halves of a gated tile are
-// whole eight-row groups) whose waves over the SMs cost least, where a wave costs as much as its columns and WAVE_COST
-// more (measured: it hardly depends on the width); otherwise 128 or 64.
-constexpr int WAVE_COST = 450;
-int tile_width(int tokens, int rows, int batch, int step = 16) {
-  if (tiles_of(tokens, rows, batch, 256) < 132) return rows > 64 ? 128 : 64;
-  int best = 256, cost = 1 << 30;
-  for (int bn = 256; bn >= 160; bn -= step) {
-    const int c = (tiles_of(tokens, rows, batch, bn) + SMS - 1) / SMS * (bn + WAVE_COST);
-    if (c < cost) { cost = c; best = bn; }
-  }
+int tiles_of(int tokens, int rows, int batch, int bn, int rt = 1) { return ((tokens + rt * BM - 1) / (rt * BM)) * ((rows + bn - 1) / bn) * batch; }
+// Shape of a tile.  Few tiles: 128 or 64 weight rows.  Many: 160 .. 256 weight rows (a multiple of `step`, so that both halves of a
+// gated tile are whole eight-row groups) and one or two tiles of 128 activation rows, for which the waves over the SMs cost least.
+// What a wave costs was measured at 4096 columns, 512 activation rows: 27 / 31 / 33 us with 160 / 224 / 256 weight rows, 43 / 54 /
+// 58 us with two tiles of activation rows.  The stages come from L2 at about 50 bytes a cycle and SM, which is what bounds a
+// wave; the second tile of activation rows uses a stage's weights again.  28672 x 4096: 126 -> 111 us, 16384 x 2048: 54 -> 44,
+// 10240 x 4096: 64 -> 54, and with the wide tile from 120 tiles on (132 before) 8192 x 4096: 43 -> 39.
+struct Tile { int bn, rt; };
+Tile tile_shape(int tokens, int rows, int batch, int step = 16) {
+  if (tiles_of(tokens, rows, batch, 256) < 120) return {rows > 64 ? 128 : 64, 1};
+  Tile best{256, 1};
+  int cost = 1 << 30;
+  for (int rt = 1; rt <= 2; ++rt)
+    for (int bn = 256; bn >= 160; bn -= step) {
+      const int c = (tiles_of(tokens, rows, batch, bn, rt) + SMS - 1) / SMS * (rt == 1 ? 5 * bn + 1410 : 12 * bn + 1640);
+      if (c < cost) { cost = c; best = {bn, rt}; }
+    }
   return best;
 }
 
@@ -283,7 +294,7 @@ bool gemm_bf16_supported(const void* w, int64_t rows, int64_t cols) {
 // K slices of a product without heads: as many as keep the grid within one wave of two CTAs per SM, every slice at
 // least 512 columns long
 int gemm_bf16_slices(int tokens, int rows, int cols) {
-  const int bn = tile_width(tokens, rows, 1);
+  const int bn = tile_shape(tokens, rows, 1).bn;
   if (bn > 128) return 1;
   const int tiles = tiles_of(tokens, rows, 1, bn), nk = (cols + BK - 1) / BK;
   int s = 1;
@@ -307,12 +318,16 @@ cudaError_t launch_gemm_bf16(const Bf16Product& p, cudaStream_t stream, int* err
   if (launches) ++*launches;
   if (p.glu) {
     a.glu = *p.glu;
-    a.bn = std::max(tile_width(p.tokens, 2 * p.rows, 1, 32), 128);
-    return a.bn > 128 ? launch_tiles<256, true>(p, a, stream, err) : launch_tiles<128, true>(p, a, stream, err);
+    const Tile tile = tile_shape(p.tokens, 2 * p.rows, 1, 32);
+    a.bn = std::max(tile.bn, 128);
+    return tile.rt == 2 ? launch_tiles<256, 2, true>(p, a, stream, err) : a.bn > 128 ? launch_tiles<256, 1, true>(p, a, stream, err)
+                                                                                     : launch_tiles<128, 1, true>(p, a, stream, err);
   }
-  a.bn = tile_width(p.tokens, p.rows, p.batch);
-  if (a.bn > 128) return launch_tiles<256, false>(p, a, stream, err);
-  return a.bn == 128 ? launch_tiles<128, false>(p, a, stream, err) : launch_tiles<64, false>(p, a, stream, err);
+  const Tile tile = tile_shape(p.tokens, p.rows, p.batch);
+  a.bn = tile.bn;
+  if (tile.rt == 2) return launch_tiles<256, 2, false>(p, a, stream, err);
+  if (a.bn > 128) return launch_tiles<256, 1, false>(p, a, stream, err);
+  return a.bn == 128 ? launch_tiles<128, 1, false>(p, a, stream, err) : launch_tiles<64, 1, false>(p, a, stream, err);
 }
 
 }  // namespace llr

@@ -46,6 +46,36 @@ def test_rows_of_unpacked_formats_alone_and_in_a_batch(ex, name, rows, cols):
     m.free()
 
 
+# tiles of 256 activation rows: whole ones and not, with rows that are and are not stored as vectors
+@pytest.mark.parametrize("rows,cols,tokens", [(16400, 264, 257), (16390, 128, 300), (16384, 192, 489), (16384, 64, 512)])
+def test_wide_tiles_of_bf16_products(ex, rows, cols, tokens):
+    """Products of bfloat16 values are exact in f32; every sum of `cols` of them, in whatever order, stays within cols ulps of the
+    sum of their sizes (the tensor cores cut where f32 rounds, twice its unit)."""
+    import torch
+    from llama_rust_b200 import synth
+    ex.set_path(0)
+    m = ex.synth(ALL["BF16"], rows, cols, 5)
+    x = synth.activations(tokens * cols, 6).reshape(tokens, cols)
+    w = torch.from_numpy(ex.dequant_rows(m)).cuda().double()
+    xb = torch.from_numpy(x).cuda().bfloat16().double()
+    err = (torch.from_numpy(_product(ex, m, x)).cuda().double() - xb @ w.T).abs()
+    assert bool((err <= 2.0 ** -23 * (cols + 3) * (xb.abs() @ w.abs().T)).all())
+    m.free()
+
+
+def test_wide_tiles_of_gated_units(ex, tmp_path):
+    """A feed-forward layer whose gate | up product takes tiles of 256 activation rows, against the plain model."""
+    from llama_rust_b200 import models
+    cfg = nm.config(80, 120, [nm.attention(2, 1, 24, 24, 9, 2, 20)], 8200, limit=0.8)
+    w = nm.weights(cfg, 23, 8, nm.SHARP[nm.AUTO])
+    ex.set_path(nm.AUTO)
+    s = models.load(ex, nm.write(tmp_path / "m", cfg, w), n_seq=1, n_ctx=300)
+    t = nm.tokens(300, cfg, 24)
+    got = s.forward([(0, t)], [list(range(300))])
+    assert nm.error(got, plain.forward(cfg, w, t)).max() <= nm.TOLERANCE[nm.AUTO]
+    s.free()
+
+
 # one block; the last rows of a tile; parts of 4096 columns that end in single blocks, in pairs and singles; units spread over CTAs; many tiles
 @pytest.mark.parametrize("name,rows,cols", [("Q4_K", 1, 256), ("Q4_K", 127, 2304), ("Q4_K", 130, 4096 + 256), ("Q4_K", 257, 2 * 4096 + 9 * 256),
                                             ("Q4_K", 9600, 768), ("Q5_K", 64, 256), ("Q5_K", 129, 6400), ("Q5_K", 5000, 1024),

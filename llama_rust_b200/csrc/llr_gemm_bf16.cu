@@ -116,6 +116,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
   const int z = (int)blockIdx.z / a.slices, slice = (int)blockIdx.z % a.slices;
   const int per = (a.nk + a.slices - 1) / a.slices, k0 = slice * per, k1 = min(a.nk, k0 + per);  // never empty: the launcher sees to it
 
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0) {
     for (int s = 0; s < NS; ++s) { bar_init(&full[s], 1); bar_init(&empty[s], 1); }
     bar_init(done, 1);
@@ -133,16 +134,26 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
 
   if (warp == W_TMA) {
     const uint32_t base = __shfl_sync(0xffffffffu, s32(smem), 0);
+    auto load_w = [&](int k, int s) {
+      bar_expect(&full[s], (uint32_t)(L::A_STAGE + bn * 128));  // boxes are always complete: what lies outside the matrices is filled with zeros
+      asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                   ::"r"(base + (uint32_t)(s * L::STAGE + L::A_STAGE)), "l"(&wmap), "r"(k * BK), "r"(z * a.rows + row0), "r"(s32(&full[s])) : "memory");
+      if constexpr (GLU)
+        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                     ::"r"(base + (uint32_t)(s * L::STAGE + L::A_STAGE + width * 128)), "l"(&wmap), "r"(k * BK), "r"(a.rows + row0), "r"(s32(&full[s])) : "memory");
+    };
+    // the first stages' weights are on their way while the kernel before this one still runs; its results are waited for
+    const int ahead = min(NS, k1 - k0);
+    for (int s = 0; s < ahead; ++s) {
+      if (elect_one()) load_w(k0 + s, s);
+      __syncwarp();
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     for (int k = k0; k < k1; ++k) {
       const int s = (k - k0) % NS;
       if (ok && !bar_wait(&empty[s], (uint32_t)((((k - k0) / NS) & 1) ^ 1))) { ok = false; report_error(err, 5); }
       if (ok && elect_one()) {
-        bar_expect(&full[s], (uint32_t)(L::A_STAGE + bn * 128));  // boxes are always complete: what lies outside the matrices is filled with zeros
-        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                     ::"r"(base + (uint32_t)(s * L::STAGE + L::A_STAGE)), "l"(&wmap), "r"(k * BK), "r"(z * a.rows + row0), "r"(s32(&full[s])) : "memory");
-        if constexpr (GLU)
-          asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                       ::"r"(base + (uint32_t)(s * L::STAGE + L::A_STAGE + width * 128)), "l"(&wmap), "r"(k * BK), "r"(a.rows + row0), "r"(s32(&full[s])) : "memory");
+        if (k - k0 >= ahead) load_w(k, s);
         asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                      ::"r"(base + (uint32_t)(s * L::STAGE)), "l"(&xmap), "r"(z * a.xk + k * BK), "r"(tok0), "r"(s32(&full[s])) : "memory");
       }
@@ -173,6 +184,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(done)) : "memory");
     __syncwarp();
   } else {
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // gates; results may still be read by an earlier kernel
     if (!bar_wait(done, 0)) { ok = false; report_error(err, 5); }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // warps 4.. read the second tile of activation rows, or every other run of columns of the only one
@@ -260,8 +272,7 @@ cudaError_t launch_tiles(const Bf16Product& p, const Args& a, cudaStream_t strea
   }
   const dim3 grid((unsigned)((p.tokens + RT * BM - 1) / (RT * BM)), (unsigned)((p.rows + width - 1) / width), (unsigned)(p.batch * a.slices));
   if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidValue;
-  gemm_bf16_kernel<BN, RT, GLU><<<grid, Lay<BN, RT>::THREADS, smem, stream>>>(xmap, wmap, a, err);
-  return cudaGetLastError();
+  return launch_overlapped(gemm_bf16_kernel<BN, RT, GLU>, grid, Lay<BN, RT>::THREADS, smem, stream, xmap, wmap, a, err);
 }
 
 constexpr int SMS = 148;

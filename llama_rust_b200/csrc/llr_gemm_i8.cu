@@ -511,21 +511,6 @@ add_units_kernel(const float* __restrict__ part, float* __restrict__ y, int64_t 
   }
 }
 
-template <class... KArgs, class... Args_>
-cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t stream, Args_... args) {
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
-}
-
 // Activation rows per tile: as few tiles as 24 rows each allow, the rows spread evenly over them
 int tile_rows(int64_t tokens) {
   const int64_t tiles = (tokens + 23) / 24, per = (tokens + tiles - 1) / tiles;
@@ -557,7 +542,7 @@ cudaError_t launch_tb(const MatView& m, const CUtensorMap& wmap, const Args& a, 
     slot.store(1, std::memory_order_relaxed);
   }
   const dim3 grid((unsigned)((m.rows + BM - 1) / BM), (unsigned)((a.tokens + TB - 1) / TB), (unsigned)slices);
-  return launch_pdl(kern, grid, THREADS, smem, stream, wmap, a, err);
+  return launch_overlapped(kern, grid, THREADS, smem, stream, wmap, a, err);
 }
 template <int DT>
 cudaError_t launch_dt(const MatView& m, const Args& a, int tb, int slices, cudaStream_t stream, int* err) {
@@ -588,7 +573,7 @@ cudaError_t launch_gemm_i8(const MatView& m, const float* x, float* y, int64_t t
   const int tb = tile_rows(tokens), tiles = (int)((tokens + tb - 1) / tb), blocks = (int)(m.cols / MACRO), slices = unit_slices(m, tokens);
   uint8_t* rec = (uint8_t*)scratch;
   float* part = (float*)(rec + (record_bytes(m, tokens) + 255) / 256 * 256);
-  cudaError_t e = launch_pdl(digit_records_kernel, dim3((unsigned)blocks, (unsigned)((tiles * tb + 7) / 8)), 256, 0, stream, x, rec, (int)m.cols, (int)tokens, tb,
+  cudaError_t e = launch_overlapped(digit_records_kernel, dim3((unsigned)blocks, (unsigned)((tiles * tb + 7) / 8)), 256, 0, stream, x, rec, (int)m.cols, (int)tokens, tb,
                              tiles * tb);
   if (e != cudaSuccess) return e;
   const Args a{rec, slices > 1 ? part : y, (int)m.rows, blocks, (int)tokens};
@@ -599,7 +584,7 @@ cudaError_t launch_gemm_i8(const MatView& m, const float* x, float* y, int64_t t
   if (slices > 1) {
     const int64_t n = tokens * m.rows;
     const int64_t grid = std::min<int64_t>((n + 255) / 256, 148 * 8);
-    e = launch_pdl(add_units_kernel, dim3((unsigned)grid), 256, 0, stream, (const float*)part, y, n, units_of(blocks));
+    e = launch_overlapped(add_units_kernel, dim3((unsigned)grid), 256, 0, stream, (const float*)part, y, n, units_of(blocks));
     if (e == cudaSuccess && launches) ++*launches;
   }
   return e;

@@ -689,6 +689,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int rows, int cols, int tokens,
                const __grid_constant__ CUtensorMap xmap, const float* __restrict__ xscale, float* __restrict__ Y,
                int* __restrict__ err) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // split-K: gridDim.z CTAs share a tile's K range; slice z writes its partial sums to Y + z * tokens * rows
   // (with one slice Y is the result itself), and a second kernel adds the slices in order
   const int per = cols / MACRO / (int)gridDim.z;
@@ -698,6 +699,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int rows, int cols, int
 
 __global__ void add_slices_kernel(const float* __restrict__ part, float* __restrict__ y, int64_t n, int slices) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < n; i += (int64_t)gridDim.x * blockDim.x * 4) {
     float4 acc = *(const float4*)(part + i);
     for (int z = 1; z < slices; ++z) {  // ascending slice order: the result does not depend on scheduling
@@ -867,19 +869,10 @@ cudaError_t launch_bn(const MatView& m, const CUtensorMap& wmap, const CUtensorM
     if (e != cudaSuccess) return e;
     slot.store(1, std::memory_order_relaxed);
   }
-  // Programmatic dependent launch: the packed-weight pipeline and the dequantization start while the
-  // conversion kernel before it is still running; what depends on that kernel waits inside.
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((m.rows + BM - 1) / BM), (unsigned)((tokens + BN - 1) / BN), (unsigned)splits);
-  cfg.blockDim = dim3(TC_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, wmap, (int)m.rows, (int)m.cols, tokens, xmap, xscale, y, err);
+  // The packed-weight pipeline and the dequantization start while the conversion kernel before it is still running; what depends
+  // on that kernel waits inside.
+  const dim3 grid((unsigned)((m.rows + BM - 1) / BM), (unsigned)((tokens + BN - 1) / BN), (unsigned)splits);
+  return launch_overlapped(kern, grid, TC_THREADS, smem, stream, wmap, (int)m.rows, (int)m.cols, tokens, xmap, xscale, y, err);
 }
 
 template <int DT, bool F16>
@@ -971,24 +964,14 @@ bool weight_bound_allows_f16(unsigned int bound_bits) {
 
 cudaError_t launch_gemm_tc(const MatView& m, const float* x, float* y, int64_t tokens, void* scratch, size_t scratch_bytes,
                            cudaStream_t stream, int* err_flag, uint64_t* launches) {
-  const int64_t n = tokens * m.cols;
   const bool f16 = m.f16_ok == 1;
   float* xscale = (float*)((char*)scratch + tc_x16_bytes(m, tokens));
   float* part = (float*)((char*)xscale + tc_scale_bytes(tokens));
   int splits = gemm_tc_splits(m, tokens);
   if (scratch_bytes < gemm_tc_scratch_bytes(m, tokens)) splits = 1;  // a fixed-size staging area may not hold the slices
   if (((uintptr_t)y & 15) != 0 || (tokens * m.rows) % 4 != 0) splits = 1;  // the slice adder works on aligned float4
-  if (f16) {
-    to_f16_rows_kernel<<<(unsigned)tokens, 256, 0, stream>>>(x, (__half*)scratch, xscale, (int)m.cols);
-  } else {
-    int64_t blocks = (n / 4 + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    if (blocks < 1) blocks = 1;
-    to_bf16_kernel<<<(unsigned)blocks, 256, 0, stream>>>(x, (__nv_bfloat16*)scratch, n);
-  }
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = tc_convert_activations(x, tokens, (int)m.cols, f16, scratch, xscale, stream, launches);
   if (e != cudaSuccess) return e;
-  if (launches) ++*launches;
   float* dst = splits > 1 ? part : y;
 #define LLR_TC(D) (f16 ? launch_dt<D, true>(m, scratch, xscale, dst, (int)tokens, splits, stream, err_flag) \
                        : launch_dt<D, false>(m, scratch, nullptr, dst, (int)tokens, splits, stream, err_flag))
@@ -1010,8 +993,7 @@ cudaError_t launch_gemm_tc(const MatView& m, const float* x, float* y, int64_t t
     const int64_t ny = tokens * m.rows;
     int64_t blocks = (ny / 4 + 255) / 256;
     if (blocks > 148 * 8) blocks = 148 * 8;
-    add_slices_kernel<<<(unsigned)blocks, 256, 0, stream>>>(part, y, ny, splits);
-    e = cudaGetLastError();
+    e = launch_overlapped(add_slices_kernel, dim3((unsigned)blocks), 256, 0, stream, part, y, ny, splits);
     if (e == cudaSuccess && launches) ++*launches;
   }
   return e;
@@ -1092,17 +1074,13 @@ size_t gemm_tc_group_desc_bytes(int n_groups) { return (size_t)n_groups * sizeof
 
 cudaError_t tc_convert_activations(const float* x, int64_t n_rows, int cols, bool f16, void* out16, float* xscale,
                                    cudaStream_t stream, uint64_t* launches) {
-  if (f16) {
-    to_f16_rows_kernel<<<(unsigned)n_rows, 256, 0, stream>>>(x, (__half*)out16, xscale, cols);
-  } else {
-    const int64_t n = n_rows * cols;
-    int64_t blocks = (n / 4 + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    if (blocks < 1) blocks = 1;
-    to_bf16_kernel<<<(unsigned)blocks, 256, 0, stream>>>(x, (__nv_bfloat16*)out16, n);
-  }
   if (launches) ++*launches;
-  return cudaGetLastError();
+  if (f16) return launch_overlapped(to_f16_rows_kernel, dim3((unsigned)n_rows), 256, 0, stream, x, (__half*)out16, xscale, cols);
+  const int64_t n = n_rows * cols;
+  int64_t blocks = (n / 4 + 255) / 256;
+  if (blocks > 148 * 16) blocks = 148 * 16;
+  if (blocks < 1) blocks = 1;
+  return launch_overlapped(to_bf16_kernel, dim3((unsigned)blocks), 256, 0, stream, x, (__nv_bfloat16*)out16, n);
 }
 
 cudaError_t tc_convert_expert_rows(const float* x, const int* src_row, int64_t n_rows, int cols, bool f16,

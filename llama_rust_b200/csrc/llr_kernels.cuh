@@ -29,6 +29,23 @@ struct PerDevice {
 // after synchronizing, with no copy on the path.
 #ifdef __CUDACC__
 __device__ __forceinline__ void report_error(int* err, int code) { *(volatile int*)err = code; }
+
+// A launch that may be placed on the SMs while its predecessor in the stream still runs (programmatic stream serialization).  The
+// kernel waits (griddepcontrol.wait) before it touches anything but weights.
+template <class... P, class... A>
+cudaError_t launch_overlapped(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
 #endif
 
 struct MatView {

@@ -56,7 +56,11 @@ constexpr int ATT_MAX_GQA = 8;
 // sc: [max(gqa * max_chunk, P * gqa * dv)] floats of shared memory, P = max(1, ATT_THREADS / dv); out: the slice's record
 // of this row, per query head dv sums, the maximum, the sum of exponentials.
 // Ends with the block's threads past their last read of sq and sc only after the caller's next __syncthreads().
-template <int ATT_MAX_VALUE, typename KV>  // ATT_MAX_VALUE: the longest value row, a multiple of ATT_THREADS
+// k(s) and v(s) are cheap (the cache's pages have been looked up before): every thread works its addresses out, and those of
+// positions past the slice are the last position's, so that no load hangs on a branch.  With a page lookup and two divisions per
+// position, loads under their own branches and eight heads' worth of predicated arithmetic for four, a slice of 32 positions took
+// 14 us, most of it in loads one after the other.
+template <int ATT_MAX_VALUE, int G, typename KV>  // ATT_MAX_VALUE: the longest value row, a multiple of ATT_THREADS; G: the most heads, gqa <= G
 __device__ __forceinline__ void attend_slice(const KV& src, const float* sq, float* sc, float* out, int s0, int s1, int max_chunk,
                                              int dk, int dv, int gqa) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = ATT_THREADS / 32;
@@ -65,14 +69,14 @@ __device__ __forceinline__ void attend_slice(const KV& src, const float* sq, flo
   // by arithmetic.  Each position's sum is formed exactly as if it were alone: columns in ascending order per lane.
   constexpr int SP = 4;
   for (int sbase = s0 + warp; sbase < s1; sbase += nw * SP) {
-    float acc[SP][ATT_MAX_GQA];
+    float acc[SP][G];
     const float* krow[SP];
 #pragma unroll
     for (int j = 0; j < SP; ++j) {
       const int sj = sbase + j * nw;
-      krow[j] = sj < s1 ? src.k(sj) : nullptr;
+      krow[j] = src.k(min(sj, s1 - 1));
 #pragma unroll
-      for (int g = 0; g < ATT_MAX_GQA; ++g) acc[j][g] = 0.f;
+      for (int g = 0; g < G; ++g) acc[j][g] = 0.f;
     }
     for (int i0 = 0; i0 < dk; i0 += 128) {
       float kvv[SP][4];
@@ -81,16 +85,16 @@ __device__ __forceinline__ void attend_slice(const KV& src, const float* sq, flo
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const int i = i0 + lane + 32 * u;
-          kvv[j][u] = (krow[j] && i < dk) ? krow[j][i] : 0.f;
+          kvv[j][u] = i < dk ? krow[j][i] : 0.f;
         }
 #pragma unroll
       for (int j = 0; j < SP; ++j)
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const int i = i0 + lane + 32 * u;
-          if (krow[j] && i < dk) {
+          if (i < dk) {
 #pragma unroll
-            for (int g = 0; g < ATT_MAX_GQA; ++g)
+            for (int g = 0; g < G; ++g)
               if (g < gqa) acc[j][g] = fmaf(sq[g * dk + i], kvv[j][u], acc[j][g]);
           }
         }
@@ -100,7 +104,7 @@ __device__ __forceinline__ void attend_slice(const KV& src, const float* sq, flo
       const int sj = sbase + j * nw;
       if (sj < s1) {  // warp-uniform
 #pragma unroll
-        for (int g = 0; g < ATT_MAX_GQA; ++g)
+        for (int g = 0; g < G; ++g)
           if (g < gqa) {
             const float d = warp_sum(acc[j][g]);
             if (lane == 0) sc[g * max_chunk + (sj - s0)] = src.score(g, sj, d);
@@ -130,11 +134,11 @@ __device__ __forceinline__ void attend_slice(const KV& src, const float* sq, flo
   const int P = ATT_THREADS / dv > 0 ? ATT_THREADS / dv : 1;
   const int i = P > 1 || dv == ATT_THREADS ? threadIdx.x % dv : threadIdx.x, grp = P > 1 || dv == ATT_THREADS ? threadIdx.x / dv : 0;
   constexpr int ND = ATT_MAX_VALUE / ATT_THREADS;  // dimensions a thread may own
-  float acc[ND][ATT_MAX_GQA];
+  float acc[ND][G];
 #pragma unroll
   for (int n = 0; n < ND; ++n)
 #pragma unroll
-    for (int g = 0; g < ATT_MAX_GQA; ++g) acc[n][g] = 0.f;
+    for (int g = 0; g < G; ++g) acc[n][g] = 0.f;
   if (grp < P) {
     // runs of eight positions go to the groups in turn: the split does not depend on the KV block size.  The eight
     // value rows of a run are fetched before the first is used; the sums are formed in ascending position order.
@@ -142,15 +146,15 @@ __device__ __forceinline__ void attend_slice(const KV& src, const float* sq, flo
       float vv[ND][8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const float* vrow = sb + j < s1 ? src.v(sb + j) : nullptr;
+        const float* vrow = src.v(min(sb + j, s1 - 1));
 #pragma unroll
-        for (int n = 0; n < ND; ++n) vv[n][j] = vrow && i + n * ATT_THREADS < dv ? vrow[i + n * ATT_THREADS] : 0.f;
+        for (int n = 0; n < ND; ++n) vv[n][j] = i + n * ATT_THREADS < dv ? vrow[i + n * ATT_THREADS] : 0.f;
       }
 #pragma unroll
       for (int j = 0; j < 8; ++j)
         if (sb + j < s1) {
 #pragma unroll
-          for (int g = 0; g < ATT_MAX_GQA; ++g)
+          for (int g = 0; g < G; ++g)
             if (g < gqa) {
               const float e = sc[g * max_chunk + (sb + j - s0)];
 #pragma unroll
@@ -165,7 +169,7 @@ __device__ __forceinline__ void attend_slice(const KV& src, const float* sq, flo
   for (int n = 0; n < ND; ++n)
     if (grp < P && i + n * ATT_THREADS < dv)
 #pragma unroll
-      for (int g = 0; g < ATT_MAX_GQA; ++g)
+      for (int g = 0; g < G; ++g)
         if (g < gqa) vsum[(grp * gqa + g) * dv + i + n * ATT_THREADS] = acc[n][g];
   __syncthreads();
   for (int idx = threadIdx.x; idx < gqa * dv; idx += ATT_THREADS) {

@@ -20,9 +20,16 @@ namespace llr {
 namespace {
 
 // first float of the head vector of (sequence, layer, kv head, position) in a paged cache
-__device__ __forceinline__ int64_t kv_offset(const KvView& kv, int seq, int layer, int head, int pos, int n_head_kv, int hd) {
+// A row of the cache is the slot'th of hd floats.  Decode attention looks the slots of a slice up once; they fit 32 bits where
+// hd >= 16 (2^32 rows of 64 bytes are more than the device holds), and shared memory in slices of up to SLOT_CHUNK positions.
+constexpr int SLOT_CHUNK = 2048;
+__host__ __device__ inline int slot_words(int chunk, int hd) { return chunk <= SLOT_CHUNK && hd >= 16 ? chunk : 0; }
+__device__ __forceinline__ int64_t kv_slot(const KvView& kv, int seq, int layer, int head, int pos, int n_head_kv) {
   const int b = kv.table[(int64_t)seq * kv.max_blocks + pos / kv.block_tokens];
-  return ((((int64_t)b * kv.n_layer + layer) * n_head_kv + head) * kv.block_tokens + pos % kv.block_tokens) * hd;
+  return (((int64_t)b * kv.n_layer + layer) * n_head_kv + head) * kv.block_tokens + pos % kv.block_tokens;
+}
+__device__ __forceinline__ int64_t kv_offset(const KvView& kv, int seq, int layer, int head, int pos, int n_head_kv, int hd) {
+  return kv_slot(kv, seq, layer, head, pos, n_head_kv) * hd;
 }
 
 // one block per activation row; a row of up to 4096 values stays in registers between the two passes
@@ -131,8 +138,11 @@ struct KvGlobal {
   const KvView& kv;
   int sid, layer, hkv, n_head_kv, hd;
   float scale;
-  __device__ __forceinline__ const float* k(int s) const { return kv.k + kv_offset(kv, sid, layer, hkv, s, n_head_kv, hd); }
-  __device__ __forceinline__ const float* v(int s) const { return kv.v + kv_offset(kv, sid, layer, hkv, s, n_head_kv, hd); }
+  const uint32_t* slots;  // of positions s0, s0 + 1, ... (shared memory), or null
+  int s0;
+  __device__ __forceinline__ int64_t at(int s) const { return (slots ? (int64_t)slots[s - s0] : kv_slot(kv, sid, layer, hkv, s, n_head_kv)) * hd; }
+  __device__ __forceinline__ const float* k(int s) const { return kv.k + at(s); }
+  __device__ __forceinline__ const float* v(int s) const { return kv.v + at(s); }
   __device__ __forceinline__ float score(int, int, float dot) const { return __fmul_rn(dot, scale); }
 };
 struct KvTile {
@@ -172,9 +182,10 @@ struct RowTiles {
 // With k_new / v_new (a single decode token) the kernel also does what rope_store_kernel does for that token: q is
 // rotated as it is loaded, and the block whose slice holds the token's position rotates the new key, writes it and
 // the new value into the cache and then reads them back like any other position: one launch less per layer.
+template <int G>
 __device__ __forceinline__ void attention_partial_row(const float* __restrict__ q, const KvView& kv, float* __restrict__ part, const RowMap& rows, int t, int layer,
                                                       int chunk, const WalkShape& w, const float* __restrict__ k_new, const float* __restrict__ v_new) {
-  extern __shared__ float sm[];  // q[gqa][hd] | scores[gqa][chunk] or sums[P][gqa][hd]
+  extern __shared__ float sm[];  // slots[slot_words] | q[gqa][hd] | scores[gqa][chunk] or sums[P][gqa][hd]
   const int hkv = blockIdx.x, split = blockIdx.y;
   const int hd = w.head_dim, gqa = w.n_head / w.n_head_kv;
   const int seq = row_position(rows, t) + 1;  // positions this row attends to
@@ -182,8 +193,11 @@ __device__ __forceinline__ void attention_partial_row(const float* __restrict__ 
   const int n_split = (int)gridDim.y;
   const int s0 = split * chunk, s1 = min(seq, s0 + chunk);
   if (s0 >= seq) return;  // this row's sequence ends before the slice
-  float* sq = sm;
+  uint32_t* slots = slot_words(chunk, hd) ? (uint32_t*)sm : nullptr;
+  float* sq = sm + slot_words(chunk, hd);
   float* sc = sq + gqa * hd;
+  if (slots)
+    for (int i = threadIdx.x; i < s1 - s0; i += ATT_THREADS) slots[i] = (uint32_t)kv_slot(kv, sid, layer, hkv, s0 + i, w.n_head_kv);
   for (int i = threadIdx.x; i < gqa * hd; i += ATT_THREADS)
     sq[i] = q[((int64_t)t * w.n_head + hkv * gqa) * hd + i];
   if (k_new) {
@@ -204,20 +218,22 @@ __device__ __forceinline__ void attention_partial_row(const float* __restrict__ 
   }
   __syncthreads();
   float* out = part + (((int64_t)t * w.n_head_kv + hkv) * n_split + split) * gqa * (hd + 2);
-  attend_slice<ATT_THREADS>(KvGlobal{kv, sid, layer, hkv, w.n_head_kv, hd, 1.0f / sqrtf((float)hd)}, sq, sc, out, s0, s1, chunk, hd, hd, gqa);
+  attend_slice<ATT_THREADS, G>(KvGlobal{kv, sid, layer, hkv, w.n_head_kv, hd, 1.0f / sqrtf((float)hd), slots, s0}, sq, sc, out, s0, s1, chunk, hd, hd, gqa);
 }
+template <int G>
 __global__ void __launch_bounds__(ATT_THREADS)
 attention_partial_kernel(const float* __restrict__ q, KvView kv, float* __restrict__ part, RowMap rows, int layer, int chunk,
                          WalkShape w, const float* __restrict__ k_new, const float* __restrict__ v_new) {
   pdl_enter();
-  attention_partial_row(q, kv, part, rows, blockIdx.z, layer, chunk, w, k_new, v_new);
+  attention_partial_row<G>(q, kv, part, rows, blockIdx.z, layer, chunk, w, k_new, v_new);
 }
 // the listed rows of a batch, one per blockIdx.z
+template <int G>
 __global__ void __launch_bounds__(ATT_THREADS)
 attention_rows_kernel(const float* __restrict__ q, KvView kv, float* __restrict__ part, RowMap rows, int layer, int chunk, WalkShape w,
                       const __grid_constant__ RowTiles tiles) {
   pdl_enter();
-  attention_partial_row(q, kv, part, rows, tiles.begin(blockIdx.z), layer, chunk, w, nullptr, nullptr);
+  attention_partial_row<G>(q, kv, part, rows, tiles.begin(blockIdx.z), layer, chunk, w, nullptr, nullptr);
 }
 
 // The same slice of one row done by ONE warp, every elementary sum formed in the order attend_slice forms it (a
@@ -760,34 +776,46 @@ size_t attention_scratch_floats(int tokens, const WalkShape& w) {
   return (size_t)tokens * w.n_head_kv * attention_splits(w) * (w.n_head / w.n_head_kv) * (w.head_dim + 2);
 }
 
-// shared memory of the per-row kernels, checked and allowed; 0: the shape is not served
-static cudaError_t attention_rows_smem(const WalkShape& w, size_t* out) {
+// The per-row kernels for the heads per group of a shape (the smallest of 1, 2, 4, 8 that holds them) and their shared memory,
+// checked and allowed
+struct RowKernels {
+  void (*partial)(const float*, KvView, float*, RowMap, int, int, WalkShape, const float*, const float*);
+  void (*rows)(const float*, KvView, float*, RowMap, int, int, WalkShape, const RowTiles);
+  size_t smem;
+};
+template <int G>
+static cudaError_t allow_rows(RowKernels* k) {
+  k->partial = attention_partial_kernel<G>;
+  k->rows = attention_rows_kernel<G>;
+  static PerDevice configured;  // per instantiation: the largest size the kernels have been allowed on this device
+  std::atomic<int>& allowed = configured.here();
+  if (k->smem > 48 * 1024 && (int)k->smem > allowed.load(std::memory_order_relaxed)) {
+    cudaError_t e = cudaFuncSetAttribute(k->partial, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k->smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k->rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k->smem);
+    if (e != cudaSuccess) return e;
+    allowed.store((int)k->smem, std::memory_order_relaxed);
+  }
+  return cudaSuccess;
+}
+static cudaError_t attention_row_kernels(const WalkShape& w, RowKernels* k) {
   const int gqa = w.n_head / w.n_head_kv, max_chunk = attention_chunk(w);
   if (gqa < 1 || gqa > ATT_MAX_GQA || w.n_head % w.n_head_kv != 0 || w.head_dim > ATT_THREADS) return cudaErrorInvalidValue;
   const size_t groups = ATT_THREADS / w.head_dim > 0 ? ATT_THREADS / w.head_dim : 1;
   const size_t score_floats = (size_t)gqa * max_chunk > groups * gqa * w.head_dim ? (size_t)gqa * max_chunk : groups * gqa * w.head_dim;
-  const size_t smem = ((size_t)gqa * w.head_dim + score_floats + 32) * sizeof(float);
-  if (smem > 200 * 1024) return cudaErrorInvalidValue;
-  static PerDevice configured;  // largest size the kernels have been allowed on this device
-  std::atomic<int>& allowed = configured.here();
-  if (smem > 48 * 1024 && (int)smem > allowed.load(std::memory_order_relaxed)) {
-    cudaError_t e = cudaFuncSetAttribute(attention_partial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    allowed.store((int)smem, std::memory_order_relaxed);
-  }
-  *out = smem;
-  return cudaSuccess;
+  const size_t floats = (size_t)gqa * w.head_dim + score_floats + 32;
+  if (floats * sizeof(float) > 200 * 1024) return cudaErrorInvalidValue;
+  k->smem = (floats + (size_t)slot_words(max_chunk, w.head_dim)) * sizeof(float);
+  return gqa == 1 ? allow_rows<1>(k) : gqa == 2 ? allow_rows<2>(k) : gqa <= 4 ? allow_rows<4>(k) : allow_rows<8>(k);
 }
 
 cudaError_t launch_attention(const float* q, const KvView& kv, float* out, float* scratch, const RowMap& rows, int layer, const WalkShape& w, cudaStream_t s,
                              uint64_t* launches, const float* k_new, const float* v_new) {
-  size_t smem = 0;
-  cudaError_t e = attention_rows_smem(w, &smem);
+  RowKernels row;
+  cudaError_t e = attention_row_kernels(w, &row);
   if (e != cudaSuccess) return e;
   const int splits = attention_splits(w), chunk = attention_chunk(w);
   if (launches) *launches += 2;
-  e = launch_walk(attention_partial_kernel, dim3(w.n_head_kv, splits, 1), dim3(ATT_THREADS), smem, s, q, kv, scratch, rows, layer, chunk, w, k_new, v_new);
+  e = launch_walk(row.partial, dim3(w.n_head_kv, splits, 1), dim3(ATT_THREADS), row.smem, s, q, kv, scratch, rows, layer, chunk, w, k_new, v_new);
   if (e != cudaSuccess) return e;
   return launch_walk(attention_combine_kernel, dim3(w.n_head, 1), dim3(128), 0, s, (const float*)scratch, out, rows, chunk, w, 1, splits, chunk, RowRanges{});
 }
@@ -797,8 +825,8 @@ cudaError_t launch_attention_groups(const float* q, const KvView& kv, float* out
   if (tokens <= 0) return cudaSuccess;
   if (tokens > MAX_TILES) return cudaErrorInvalidValue;
   const int gqa = w.n_head_kv > 0 ? w.n_head / w.n_head_kv : 0;
-  size_t smem = 0;
-  cudaError_t e = attention_rows_smem(w, &smem);
+  RowKernels row;
+  cudaError_t e = attention_row_kernels(w, &row);
   if (e != cudaSuccess) return e;
   const int splits = attention_splits(w);
   const int max_chunk = attention_chunk(w);
@@ -856,7 +884,7 @@ cudaError_t launch_attention_groups(const float* q, const KvView& kv, float* out
   }
   if (single.n) {
     if (launches) ++*launches;
-    e = launch_walk(attention_rows_kernel, dim3(w.n_head_kv, splits, single.n), dim3(ATT_THREADS), smem, s, q, kv, scratch, rows, layer, max_chunk, w, single);
+    e = launch_walk(row.rows, dim3(w.n_head_kv, splits, single.n), dim3(ATT_THREADS), row.smem, s, q, kv, scratch, rows, layer, max_chunk, w, single);
     if (e != cudaSuccess) return e;
   }
   if (launches) ++*launches;

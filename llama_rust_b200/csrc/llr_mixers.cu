@@ -376,7 +376,7 @@ struct SpanRuns {
 // normed as it is loaded, and the blocks whose slice holds the token's own position write its key and value (or its
 // latent) into the cache and read them back like any other; blocks that share a kv head write the same values.
 static_assert(PROJ_THREADS == ATT_THREADS, "the sums over a projection are formed in one order");
-template <int MAX_VALUE>
+template <int MAX_VALUE, int G>  // G: the most query heads of a block
 __global__ void __launch_bounds__(ATT_THREADS)
 span_partial_kernel(const float* __restrict__ q, int64_t q_ld, SpanShape sh, LayerKv kv, RowMap rows, const __grid_constant__ SpanRuns runs, int chunk,
                     float* __restrict__ part, NewToken nt) {
@@ -419,7 +419,7 @@ span_partial_kernel(const float* __restrict__ q, int64_t q_ld, SpanShape sh, Lay
   __syncthreads();
   // records: [row of the pass][query head][slice][dv + 2]; a group's heads follow each other n_split records apart
   float* rec = part + (((int64_t)blockIdx.z * sh.n_kv * groups + blockIdx.x) * n_split + split) * per * (sh.dv + 2);
-  attend_slice<MAX_VALUE>(KvSpan{kv, sh, smw, span, s0, head, pos, h0}, sq, sc, rec, s0, s1, chunk, sh.dk, sh.dv, heads);
+  attend_slice<MAX_VALUE, G>(KvSpan{kv, sh, smw, span, s0, head, pos, h0}, sq, sc, rec, s0, s1, chunk, sh.dk, sh.dv, heads);
 }
 
 // grid (query head, row, 128 dimensions): merges a head's slices (at most 32) and the sink, applies the gate
@@ -1069,7 +1069,10 @@ cudaError_t launch_span_attention(const float* q, int64_t q_ld, const SpanShape&
   }
   const int head_groups = (gq + span_heads(sh) - 1) / span_heads(sh), chunk = span_chunk(sh), splits = span_splits(sh), per = span_rows_per_pass(sh);
   const size_t smem = span_smem(sh);
-  auto kern = sh.dv <= ATT_THREADS ? span_partial_kernel<ATT_THREADS> : sh.dv <= 2 * ATT_THREADS ? span_partial_kernel<2 * ATT_THREADS> : span_partial_kernel<MAX_VALUE>;
+  const int most = std::min(gq, span_heads(sh));  // query heads of a block
+#define LLR_SPAN(G) (sh.dv <= ATT_THREADS ? span_partial_kernel<ATT_THREADS, G> : sh.dv <= 2 * ATT_THREADS ? span_partial_kernel<2 * ATT_THREADS, G> : span_partial_kernel<MAX_VALUE, G>)
+  auto kern = most <= 2 ? LLR_SPAN(2) : most <= 4 ? LLR_SPAN(4) : LLR_SPAN(8);
+#undef LLR_SPAN
 
   // groups that are long enough for the tensor cores, as many per launch as the scratch holds the gathered keys of
   SpanBatch b{};

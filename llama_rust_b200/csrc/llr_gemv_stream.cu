@@ -788,6 +788,8 @@ bool gemv_mma_supported(const MatView& m) {
   return true;
 }
 
+// Kernels of 1, 2, 4, 6 and 8 activation rows: an n-tile holds two rows, and five or six rows in the kernel of eight would spend a
+// quarter of its MMAs and scale arithmetic on padding (14336 x 4096 Q4_K, 6 rows: 19.5 us there, 17.2 here).
 static cudaError_t launch_passes(const MatView& m, const float* x, float* y, int64_t tokens, cudaStream_t stream,
                                  int sm_count, int* err, uint64_t* launches, const HostOut* ho) {
   for (int64_t t0 = 0; t0 < tokens; t0 += 8) {
@@ -799,6 +801,7 @@ static cudaError_t launch_passes(const MatView& m, const float* x, float* y, int
     (nt == 1 ? launch_single<1, D>(m, xp, yp, nt, stream, sm_count, err, ho)                  \
      : nt == 2 ? launch_single<2, D>(m, xp, yp, nt, stream, sm_count, err, ho)                \
      : nt <= 4 ? launch_single<4, D>(m, xp, yp, nt, stream, sm_count, err, ho)                \
+     : nt <= 6 ? launch_single<6, D>(m, xp, yp, nt, stream, sm_count, err, ho)                \
                : launch_single<8, D>(m, xp, yp, nt, stream, sm_count, err, ho))
     if (m.dtype == DT_Q4_K) e = LLR_LAUNCH_DT(DT_Q4_K);
     else if (m.dtype == DT_Q6_K) e = LLR_LAUNCH_DT(DT_Q6_K);
@@ -1076,6 +1079,7 @@ cudaError_t program_create(const std::vector<ProgEntry>& entries_in, const std::
   if (mt == 1) e = LLR_PREP(1);
   else if (mt == 2) e = LLR_PREP(2);
   else if (mt <= 4) e = LLR_PREP(4);
+  else if (mt <= 6) e = LLR_PREP(6);
   else e = LLR_PREP(8);
 #undef LLR_PREP
   if (e == cudaSuccess && !sharded && tagged_bytes > 0) {
@@ -1156,6 +1160,7 @@ cudaError_t program_run(Program* p, cudaStream_t stream, int* err_flag, int poll
   if (mt == 1) e = LLR_RUN(1);
   else if (mt == 2) e = LLR_RUN(2);
   else if (mt <= 4) e = LLR_RUN(4);
+  else if (mt <= 6) e = LLR_RUN(6);
   else e = LLR_RUN(8);
 #undef LLR_RUN
   if (e == cudaSuccess && launches) ++*launches;

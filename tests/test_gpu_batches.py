@@ -97,7 +97,7 @@ def test_rows_of_k_quants_alone_and_in_a_batch(ex, name, rows, cols):
     alone = np.concatenate([_product(ex, m, x[t:t + 8]) for t in range(0, 100, 8)])
     finite = np.arange(100) != 23
     assert np.isnan(alone[23]).all() and np.isfinite(alone[finite]).all()
-    for path, counts in ((0, (12, 13, 16, 17, 24, 25, 32, 33, 48, 49, 63)), (3, (64, 100))):
+    for path, counts in ((0, (5, 6, 12, 13, 16, 17, 24, 25, 32, 33, 48, 49, 63)), (3, (64, 100))):
         ex.set_path(path)
         for n in counts:
             y = _product(ex, m, x[:n])

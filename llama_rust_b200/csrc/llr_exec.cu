@@ -452,13 +452,21 @@ bool matmul_wants_tc(const MatView& m, int64_t tokens, int path) {
 bool matmul_wants_i8(const MatView& m, int64_t tokens, int path) {
   return (path == PATH_AUTO || path == PATH_MMA || path == PATH_TC) && !matmul_wants_tc(m, tokens, path) && gemm_i8_supported(m, tokens);
 }
+// Both products stage their activations (16-bit rows and scales, or digit records) alike: the layout hangs on rows, columns and operand
+// format alone, not on the weight rows.
+bool matmul_stages_alike(const MatView& a, const MatView& b, int64_t tokens, int path) {
+  if (a.cols != b.cols) return false;
+  if (matmul_wants_i8(a, tokens, path)) return matmul_wants_i8(b, tokens, path);
+  return matmul_wants_tc(a, tokens, path) && matmul_wants_tc(b, tokens, path) && gemm_tc_supported(a, tokens) && gemm_tc_supported(b, tokens) &&
+         (a.f16_ok == 1) == (b.f16_ok == 1);
+}
 size_t matmul_scratch_bytes(const MatView& m, int64_t tokens) {
   return bf16_chunk(m, tokens) ? ((size_t)tokens * m.cols * 2 + 255) / 256 * 256 : gemm_tc_scratch_bytes(m, tokens);
 }
 
 cudaError_t launch_matmul(const MatView& m, const float* x, float* y, int64_t tokens,
                           cudaStream_t stream, int path, int sm_count, int* err_flag,
-                          void* scratch, uint64_t* launches) {
+                          void* scratch, uint64_t* launches, bool x_staged) {
   const bool x_aligned = ((uintptr_t)x & 15) == 0 && (m.cols % 4 == 0);
   if (scratch && err_flag && x_aligned && ((uintptr_t)y & 15) == 0 && matmul_wants_tc(m, tokens, path) && bf16_chunk(m, tokens)) {
     const cudaError_t ce = tc_convert_activations(x, tokens, (int)m.cols, false, scratch, nullptr, stream, launches);
@@ -469,8 +477,8 @@ cudaError_t launch_matmul(const MatView& m, const float* x, float* y, int64_t to
     return launch_gemm_bf16(p, stream, err_flag, launches);
   }
   if (scratch && err_flag && x_aligned && matmul_wants_tc(m, tokens, path) && gemm_tc_supported(m, tokens))
-    return launch_gemm_tc(m, x, y, tokens, scratch, gemm_tc_scratch_bytes(m, tokens), stream, err_flag, launches);
-  if (scratch && err_flag && x_aligned && matmul_wants_i8(m, tokens, path)) return launch_gemm_i8(m, x, y, tokens, scratch, stream, err_flag, launches);
+    return launch_gemm_tc(m, x, y, tokens, scratch, gemm_tc_scratch_bytes(m, tokens), stream, err_flag, launches, x_staged);
+  if (scratch && err_flag && x_aligned && matmul_wants_i8(m, tokens, path)) return launch_gemm_i8(m, x, y, tokens, scratch, stream, err_flag, launches, x_staged);
   if (path == PATH_TC) path = PATH_AUTO;
   if ((path == PATH_AUTO || path == PATH_MMA) && x_aligned && err_flag && gemv_mma_supported(m))
     return launch_gemv_mma(m, x, y, tokens, stream, sm_count, err_flag, launches);
@@ -1760,11 +1768,15 @@ void session_orphan(llr_session* s) {
   s->owner = nullptr;
 }
 
-cudaError_t session_matmul(llr_exec* e, const llr_matrix* m, size_t tokens, const float* x, float* y) {
+// before: the matrix of the product launched just before on the same x, or null; its staged activations are used again where they
+// still lie in the same buffer (q, k, v and gate, up read the same rows: three of a layer's seven conversions, 4 us each at 512 rows)
+cudaError_t session_matmul(llr_exec* e, const llr_matrix* m, size_t tokens, const float* x, float* y, const llr_matrix* before = nullptr) {
+  const void *const s_was = e->dev_s, *const q_was = e->dev_q;
   void* scratch = nullptr;
   cudaError_t ce = ensure_scratch(e, m, tokens, e->stream, &scratch);
   if (ce != cudaSuccess) return ce;
-  return launch_matmul(view_of(m), x, y, (int64_t)tokens, e->stream, e->path, e->sm_count, e->err_flag, scratch, &e->ctr.launches);
+  const bool staged = before && scratch && (scratch == s_was || scratch == q_was) && matmul_stages_alike(view_of(before), view_of(m), (int64_t)tokens, e->path);
+  return launch_matmul(view_of(m), x, y, (int64_t)tokens, e->stream, e->path, e->sm_count, e->err_flag, scratch, &e->ctr.launches, staged);
 }
 
 KvView session_kv(const llr_session* s) {
@@ -1887,8 +1899,8 @@ cudaError_t session_layers(llr_session* s, const int* ids_dev, size_t n, const R
       if ((ce = program_run(s->qkv_prog[li], st, e->err_flag, e->poll_limit, L)) != cudaSuccess) break;
     } else {
       if ((ce = session_matmul(e, W.attn_q, n, s->xn, s->q)) != cudaSuccess) break;
-      if ((ce = session_matmul(e, W.attn_k, n, s->xn, s->k)) != cudaSuccess) break;
-      if ((ce = session_matmul(e, W.attn_v, n, s->xn, s->v)) != cudaSuccess) break;
+      if ((ce = session_matmul(e, W.attn_k, n, s->xn, s->k, W.attn_q)) != cudaSuccess) break;
+      if ((ce = session_matmul(e, W.attn_v, n, s->xn, s->v, W.attn_k)) != cudaSuccess) break;
     }
     if (n == 1) {  // a decode token: rotation and cache store happen inside the attention kernel
       if ((ce = launch_attention(s->q, kv, s->attn, s->att_scratch, rows, (int)li, s->shape, st, L, s->k, s->v)) != cudaSuccess) break;
@@ -1913,7 +1925,7 @@ cudaError_t session_layers(llr_session* s, const int* ids_dev, size_t n, const R
       if ((ce = program_run(s->gateup_prog[li], st, e->err_flag, e->poll_limit, L)) != cudaSuccess) break;
     } else {
       if ((ce = session_matmul(e, W.ffn_gate, n, s->xn, s->gate)) != cudaSuccess) break;
-      if ((ce = session_matmul(e, W.ffn_up, n, s->xn, s->up)) != cudaSuccess) break;
+      if ((ce = session_matmul(e, W.ffn_up, n, s->xn, s->up, W.ffn_gate)) != cudaSuccess) break;
     }
     if ((ce = launch_swiglu(s->gate, s->up, (int64_t)(n * FF), st, L)) != cudaSuccess) break;
     if ((ce = session_matmul(e, W.ffn_down, n, s->gate, s->proj)) != cudaSuccess) break;

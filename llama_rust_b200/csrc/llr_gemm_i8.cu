@@ -569,18 +569,22 @@ size_t gemm_i8_scratch_bytes(const MatView& m, int64_t tokens) {
   return (record_bytes(m, tokens) + 255) / 256 * 256 + (s > 1 ? (size_t)units_of((int)(m.cols / MACRO)) * (size_t)tokens * (size_t)m.rows * 4 : 0);
 }
 
-cudaError_t launch_gemm_i8(const MatView& m, const float* x, float* y, int64_t tokens, void* scratch, cudaStream_t stream, int* err, uint64_t* launches) {
+cudaError_t launch_gemm_i8(const MatView& m, const float* x, float* y, int64_t tokens, void* scratch, cudaStream_t stream, int* err, uint64_t* launches, bool x_staged) {
   const int tb = tile_rows(tokens), tiles = (int)((tokens + tb - 1) / tb), blocks = (int)(m.cols / MACRO), slices = unit_slices(m, tokens);
   uint8_t* rec = (uint8_t*)scratch;
   float* part = (float*)(rec + (record_bytes(m, tokens) + 255) / 256 * 256);
-  cudaError_t e = launch_overlapped(digit_records_kernel, dim3((unsigned)blocks, (unsigned)((tiles * tb + 7) / 8)), 256, 0, stream, x, rec, (int)m.cols, (int)tokens, tb,
-                             tiles * tb);
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
+  if (!x_staged) {
+    e = launch_overlapped(digit_records_kernel, dim3((unsigned)blocks, (unsigned)((tiles * tb + 7) / 8)), 256, 0, stream, x, rec, (int)m.cols, (int)tokens, tb,
+                          tiles * tb);
+    if (e != cudaSuccess) return e;
+    if (launches) ++*launches;
+  }
   const Args a{rec, slices > 1 ? part : y, (int)m.rows, blocks, (int)tokens};
   e = m.dtype == DT_Q4_K ? launch_dt<DT_Q4_K>(m, a, tb, slices, stream, err) : m.dtype == DT_Q5_K ? launch_dt<DT_Q5_K>(m, a, tb, slices, stream, err)
                                                                              : launch_dt<DT_Q6_K>(m, a, tb, slices, stream, err);
   if (e != cudaSuccess) return e;
-  if (launches) *launches += 2;
+  if (launches) ++*launches;
   if (slices > 1) {
     const int64_t n = tokens * m.rows;
     const int64_t grid = std::min<int64_t>((n + 255) / 256, 148 * 8);

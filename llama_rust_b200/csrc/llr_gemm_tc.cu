@@ -963,14 +963,14 @@ bool weight_bound_allows_f16(unsigned int bound_bits) {
 }
 
 cudaError_t launch_gemm_tc(const MatView& m, const float* x, float* y, int64_t tokens, void* scratch, size_t scratch_bytes,
-                           cudaStream_t stream, int* err_flag, uint64_t* launches) {
+                           cudaStream_t stream, int* err_flag, uint64_t* launches, bool x_staged) {
   const bool f16 = m.f16_ok == 1;
   float* xscale = (float*)((char*)scratch + tc_x16_bytes(m, tokens));
   float* part = (float*)((char*)xscale + tc_scale_bytes(tokens));
   int splits = gemm_tc_splits(m, tokens);
   if (scratch_bytes < gemm_tc_scratch_bytes(m, tokens)) splits = 1;  // a fixed-size staging area may not hold the slices
   if (((uintptr_t)y & 15) != 0 || (tokens * m.rows) % 4 != 0) splits = 1;  // the slice adder works on aligned float4
-  cudaError_t e = tc_convert_activations(x, tokens, (int)m.cols, f16, scratch, xscale, stream, launches);
+  cudaError_t e = x_staged ? cudaSuccess : tc_convert_activations(x, tokens, (int)m.cols, f16, scratch, xscale, stream, launches);
   if (e != cudaSuccess) return e;
   float* dst = splits > 1 ? part : y;
 #define LLR_TC(D) (f16 ? launch_dt<D, true>(m, scratch, xscale, dst, (int)tokens, splits, stream, err_flag) \

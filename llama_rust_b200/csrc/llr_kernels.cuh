@@ -63,10 +63,12 @@ constexpr int64_t TC_MIN_TOKENS = 64;  // from here on AUTO prefers the bf16 tcg
 // entry points accept.  `launches` is incremented by the kernels launched.
 // `err_flag` is a device int that kernels with bounded waits set to non-zero when a wait ran out.
 // `scratch` lets the tensor-core GEMM stage 16-bit activations (matmul_wants_tc: matmul_scratch_bytes) or the integer GEMM its
-// digits (matmul_wants_i8: gemm_i8_scratch_bytes); null: other kernels run.
+// digits (matmul_wants_i8: gemm_i8_scratch_bytes); null: other kernels run.  x_staged: the launch before this one staged the same x
+// in the same scratch (matmul_stages_alike), so it is not staged again.
 cudaError_t launch_matmul(const MatView& m, const float* x, float* y, int64_t tokens,
                           cudaStream_t stream, int path, int sm_count, int* err_flag,
-                          void* scratch, uint64_t* launches);
+                          void* scratch, uint64_t* launches, bool x_staged = false);
+bool matmul_stages_alike(const MatView& a, const MatView& b, int64_t tokens, int path);
 bool matmul_wants_tc(const MatView& m, int64_t tokens, int path);
 bool matmul_wants_i8(const MatView& m, int64_t tokens, int path);
 size_t matmul_scratch_bytes(const MatView& m, int64_t tokens);  // for launch_matmul when matmul_wants_tc
@@ -102,7 +104,8 @@ cudaError_t launch_gemv_mma(const MatView& m, const float* x, float* y, int64_t 
 constexpr int64_t I8_MIN_TOKENS = 13, I8_MAX_TOKENS = 4096;
 bool gemm_i8_supported(const MatView& m, int64_t tokens);
 size_t gemm_i8_scratch_bytes(const MatView& m, int64_t tokens);
-cudaError_t launch_gemm_i8(const MatView& m, const float* x, float* y, int64_t tokens, void* scratch, cudaStream_t stream, int* err_flag, uint64_t* launches);
+cudaError_t launch_gemm_i8(const MatView& m, const float* x, float* y, int64_t tokens, void* scratch, cudaStream_t stream, int* err_flag, uint64_t* launches,
+                           bool x_staged);
 // Result delivery to the host by the kernel itself (host-pointer calls with at most 8 activation
 // rows): the reducer also stores each finished value at y + y_delta bytes, a device alias of
 // mapped pinned host memory, and the CTA that finishes last stores `ticket` into *done (mapped
@@ -225,7 +228,7 @@ cudaError_t launch_gemm_tc_grouped(const GemmGroupSpec* specs, int n_groups, boo
                                    cudaStream_t stream, int* err_flag, uint64_t* launches);
 size_t gemm_tc_scratch_bytes(const MatView& m, int64_t tokens);
 cudaError_t launch_gemm_tc(const MatView& m, const float* x, float* y, int64_t tokens, void* scratch, size_t scratch_bytes,
-                           cudaStream_t stream, int* err_flag, uint64_t* launches);
+                           cudaStream_t stream, int* err_flag, uint64_t* launches, bool x_staged = false);
 
 // Same kernels with the staging buffer in a file-scope __device__ array (no allocation).
 constexpr size_t GEMM_STATIC_SCRATCH_BYTES = 32u << 20;

@@ -145,6 +145,7 @@ struct llr_exec {
   float* dev_moe = nullptr; size_t dev_moe_cap = 0;  // workspace of the routed-expert layer
   uint8_t* dev_s = nullptr; size_t dev_s_cap = 0;  // kernel scratch (bf16 activations of the tensor-core GEMM)
   uint8_t* dev_q = nullptr; size_t dev_q_cap = 0;  // kernel scratch (digits of the integer GEMM), this executor's stream only
+  size_t dev_q_limit = SIZE_MAX;                   // LLR_DIGITS_LIMIT: what it may grow to
   // residency
   std::list<CacheEntry> cache;  // front = least recently used
   bool limit_resolved = false;
@@ -303,14 +304,16 @@ MatView view_of(const llr_matrix* m) {
 // scratch for the tensor-core GEMM; growing frees the old buffer, which synchronizes the device.
 // The integer GEMM has a buffer of its own, and does without where that is not safe or not to be had (the decode kernel then runs,
 // with the same results): on a stream of the caller's, whose work may overlap other work of this executor; under capture, since a
-// replay would outlive the buffer; when memory is short.
+// replay would outlive the buffer; when memory is short or LLR_DIGITS_LIMIT smaller than what it needs.
 cudaError_t ensure_scratch(llr_exec* e, const llr_matrix* m, size_t tokens, cudaStream_t stream, void** out) {
   *out = nullptr;
   const MatView v = view_of(m);
   if (matmul_wants_i8(v, (int64_t)tokens, e->path)) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (stream != e->stream || cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return cudaSuccess;
-    if (grow_device(&e->dev_q, &e->dev_q_cap, gemm_i8_scratch_bytes(v, (int64_t)tokens)) == cudaSuccess) *out = e->dev_q;
+    const size_t need = gemm_i8_scratch_bytes(v, (int64_t)tokens);
+    if (need > e->dev_q_limit) return cudaSuccess;
+    if (grow_device(&e->dev_q, &e->dev_q_cap, need) == cudaSuccess) *out = e->dev_q;
     else cudaGetLastError();
     return cudaSuccess;
   }
@@ -452,22 +455,16 @@ bool matmul_wants_tc(const MatView& m, int64_t tokens, int path) {
 bool matmul_wants_i8(const MatView& m, int64_t tokens, int path) {
   return (path == PATH_AUTO || path == PATH_MMA || path == PATH_TC) && !matmul_wants_tc(m, tokens, path) && gemm_i8_supported(m, tokens);
 }
-// Both products stage their activations (16-bit rows and scales, or digit records) alike: the layout hangs on rows, columns and operand
-// format alone, not on the weight rows.
-bool matmul_stages_alike(const MatView& a, const MatView& b, int64_t tokens, int path) {
-  if (a.cols != b.cols) return false;
-  if (matmul_wants_i8(a, tokens, path)) return matmul_wants_i8(b, tokens, path);
-  return matmul_wants_tc(a, tokens, path) && matmul_wants_tc(b, tokens, path) && gemm_tc_supported(a, tokens) && gemm_tc_supported(b, tokens) &&
-         (a.f16_ok == 1) == (b.f16_ok == 1);
-}
 size_t matmul_scratch_bytes(const MatView& m, int64_t tokens) {
   return bf16_chunk(m, tokens) ? ((size_t)tokens * m.cols * 2 + 255) / 256 * 256 : gemm_tc_scratch_bytes(m, tokens);
 }
 
 cudaError_t launch_matmul(const MatView& m, const float* x, float* y, int64_t tokens,
                           cudaStream_t stream, int path, int sm_count, int* err_flag,
-                          void* scratch, uint64_t* launches, bool x_staged) {
+                          void* scratch, uint64_t* launches, StagedRows* staged) {
   const bool x_aligned = ((uintptr_t)x & 15) == 0 && (m.cols % 4 == 0);
+  const StagedRows before = staged ? *staged : StagedRows{};
+  if (staged) *staged = StagedRows{};
   if (scratch && err_flag && x_aligned && ((uintptr_t)y & 15) == 0 && matmul_wants_tc(m, tokens, path) && bf16_chunk(m, tokens)) {
     const cudaError_t ce = tc_convert_activations(x, tokens, (int)m.cols, false, scratch, nullptr, stream, launches);
     if (ce != cudaSuccess) return ce;
@@ -476,9 +473,17 @@ cudaError_t launch_matmul(const MatView& m, const float* x, float* y, int64_t to
     p.tokens = (int)tokens; p.rows = (int)m.rows; p.cols = (int)m.cols; p.batch = 1; p.slices = 1;
     return launch_gemm_bf16(p, stream, err_flag, launches);
   }
-  if (scratch && err_flag && x_aligned && matmul_wants_tc(m, tokens, path) && gemm_tc_supported(m, tokens))
-    return launch_gemm_tc(m, x, y, tokens, scratch, gemm_tc_scratch_bytes(m, tokens), stream, err_flag, launches, x_staged);
-  if (scratch && err_flag && x_aligned && matmul_wants_i8(m, tokens, path)) return launch_gemm_i8(m, x, y, tokens, scratch, stream, err_flag, launches, x_staged);
+  const bool tc = scratch && err_flag && x_aligned && matmul_wants_tc(m, tokens, path) && gemm_tc_supported(m, tokens);
+  const bool i8 = scratch && err_flag && x_aligned && !tc && matmul_wants_i8(m, tokens, path);
+  if (tc || i8) {
+    // rows, columns and operand format fix the layout; the weight rows do not enter
+    const StagedRows mine{i8 ? StagedRows::DIGITS : m.f16_ok == 1 ? StagedRows::F16 : StagedRows::BF16, scratch, x, tokens, m.cols};
+    const bool there = before == mine;
+    const cudaError_t ce = tc ? launch_gemm_tc(m, x, y, tokens, scratch, gemm_tc_scratch_bytes(m, tokens), stream, err_flag, launches, there)
+                              : launch_gemm_i8(m, x, y, tokens, scratch, stream, err_flag, launches, there);
+    if (staged && ce == cudaSuccess) *staged = mine;
+    return ce;
+  }
   if (path == PATH_TC) path = PATH_AUTO;
   if ((path == PATH_AUTO || path == PATH_MMA) && x_aligned && err_flag && gemv_mma_supported(m))
     return launch_gemv_mma(m, x, y, tokens, stream, sm_count, err_flag, launches);
@@ -545,6 +550,7 @@ int llr_exec_create(int device, llr_exec** out) {
   if (const char* bf = std::getenv("LLR_GEMM_BF16")) { if (std::strcmp(bf, "0") != 0) e->bound_dev = nullptr; }  // keep bfloat16 operands
   if (const char* vh = std::getenv("LLAMA_CUDA_CACHE_VERIFY")) e->verify_hits = std::strcmp(vh, "0") != 0;
   if (const char* hd = std::getenv("LLR_HOST_DELIVERY")) e->host_delivery = std::strcmp(hd, "0") != 0;
+  if (const char* dl = std::getenv("LLR_DIGITS_LIMIT")) e->dev_q_limit = (size_t)std::strtoull(dl, nullptr, 10);
   if (ce != cudaSuccess) {
     if (err_host) cudaFreeHost(err_host);
     cudaGetLastError();
@@ -1768,15 +1774,15 @@ void session_orphan(llr_session* s) {
   s->owner = nullptr;
 }
 
-// before: the matrix of the product launched just before on the same x, or null; its staged activations are used again where they
-// still lie in the same buffer (q, k, v and gate, up read the same rows: three of a layer's seven conversions, 4 us each at 512 rows)
-cudaError_t session_matmul(llr_exec* e, const llr_matrix* m, size_t tokens, const float* x, float* y, const llr_matrix* before = nullptr) {
-  const void *const s_was = e->dev_s, *const q_was = e->dev_q;
+// rows: carried through the products of the same x that follow each other, which then stage it once (q, k, v and gate, up: three of
+// a layer's seven conversions, 4 us each at 512 rows)
+cudaError_t session_matmul(llr_exec* e, const llr_matrix* m, size_t tokens, const float* x, float* y, StagedRows* rows = nullptr) {
+  const size_t s_cap = e->dev_s_cap, q_cap = e->dev_q_cap;
   void* scratch = nullptr;
   cudaError_t ce = ensure_scratch(e, m, tokens, e->stream, &scratch);
   if (ce != cudaSuccess) return ce;
-  const bool staged = before && scratch && (scratch == s_was || scratch == q_was) && matmul_stages_alike(view_of(before), view_of(m), (int64_t)tokens, e->path);
-  return launch_matmul(view_of(m), x, y, (int64_t)tokens, e->stream, e->path, e->sm_count, e->err_flag, scratch, &e->ctr.launches, staged);
+  if (rows && (e->dev_s_cap != s_cap || e->dev_q_cap != q_cap)) *rows = StagedRows{};  // a buffer has grown: another one, though it may lie where the old one lay
+  return launch_matmul(view_of(m), x, y, (int64_t)tokens, e->stream, e->path, e->sm_count, e->err_flag, scratch, &e->ctr.launches, rows);
 }
 
 KvView session_kv(const llr_session* s) {
@@ -1898,9 +1904,10 @@ cudaError_t session_layers(llr_session* s, const int* ids_dev, size_t n, const R
     if (one_row_programs && s->qkv_prog[li]) {
       if ((ce = program_run(s->qkv_prog[li], st, e->err_flag, e->poll_limit, L)) != cudaSuccess) break;
     } else {
-      if ((ce = session_matmul(e, W.attn_q, n, s->xn, s->q)) != cudaSuccess) break;
-      if ((ce = session_matmul(e, W.attn_k, n, s->xn, s->k, W.attn_q)) != cudaSuccess) break;
-      if ((ce = session_matmul(e, W.attn_v, n, s->xn, s->v, W.attn_k)) != cudaSuccess) break;
+      StagedRows staged;
+      if ((ce = session_matmul(e, W.attn_q, n, s->xn, s->q, &staged)) != cudaSuccess) break;
+      if ((ce = session_matmul(e, W.attn_k, n, s->xn, s->k, &staged)) != cudaSuccess) break;
+      if ((ce = session_matmul(e, W.attn_v, n, s->xn, s->v, &staged)) != cudaSuccess) break;
     }
     if (n == 1) {  // a decode token: rotation and cache store happen inside the attention kernel
       if ((ce = launch_attention(s->q, kv, s->attn, s->att_scratch, rows, (int)li, s->shape, st, L, s->k, s->v)) != cudaSuccess) break;
@@ -1924,8 +1931,9 @@ cudaError_t session_layers(llr_session* s, const int* ids_dev, size_t n, const R
     if (one_row_programs && s->gateup_prog[li]) {
       if ((ce = program_run(s->gateup_prog[li], st, e->err_flag, e->poll_limit, L)) != cudaSuccess) break;
     } else {
-      if ((ce = session_matmul(e, W.ffn_gate, n, s->xn, s->gate)) != cudaSuccess) break;
-      if ((ce = session_matmul(e, W.ffn_up, n, s->xn, s->up, W.ffn_gate)) != cudaSuccess) break;
+      StagedRows staged;
+      if ((ce = session_matmul(e, W.ffn_gate, n, s->xn, s->gate, &staged)) != cudaSuccess) break;
+      if ((ce = session_matmul(e, W.ffn_up, n, s->xn, s->up, &staged)) != cudaSuccess) break;
     }
     if ((ce = launch_swiglu(s->gate, s->up, (int64_t)(n * FF), st, L)) != cudaSuccess) break;
     if ((ce = session_matmul(e, W.ffn_down, n, s->gate, s->proj)) != cudaSuccess) break;

@@ -63,12 +63,20 @@ constexpr int64_t TC_MIN_TOKENS = 64;  // from here on AUTO prefers the bf16 tcg
 // entry points accept.  `launches` is incremented by the kernels launched.
 // `err_flag` is a device int that kernels with bounded waits set to non-zero when a wait ran out.
 // `scratch` lets the tensor-core GEMM stage 16-bit activations (matmul_wants_tc: matmul_scratch_bytes) or the integer GEMM its
-// digits (matmul_wants_i8: gemm_i8_scratch_bytes); null: other kernels run.  x_staged: the launch before this one staged the same x
-// in the same scratch (matmul_stages_alike), so it is not staged again.
+// digits (matmul_wants_i8: gemm_i8_scratch_bytes); null: other kernels run.
+// `staged` (or null): what lies staged at `at`, of which rows.  A product that wants just that does not stage it again; every launch
+// leaves there what it staged itself, nothing where it staged nothing.  Whoever passes one on vouches that neither x nor the
+// buffer has been written or moved since.
+struct StagedRows {
+  enum Kind { NONE, DIGITS, F16, BF16 } kind = NONE;
+  const void* at = nullptr;
+  const float* x = nullptr;
+  int64_t tokens = 0, cols = 0;
+  bool operator==(const StagedRows& o) const { return kind == o.kind && at == o.at && x == o.x && tokens == o.tokens && cols == o.cols; }
+};
 cudaError_t launch_matmul(const MatView& m, const float* x, float* y, int64_t tokens,
                           cudaStream_t stream, int path, int sm_count, int* err_flag,
-                          void* scratch, uint64_t* launches, bool x_staged = false);
-bool matmul_stages_alike(const MatView& a, const MatView& b, int64_t tokens, int path);
+                          void* scratch, uint64_t* launches, StagedRows* staged = nullptr);
 bool matmul_wants_tc(const MatView& m, int64_t tokens, int path);
 bool matmul_wants_i8(const MatView& m, int64_t tokens, int path);
 size_t matmul_scratch_bytes(const MatView& m, int64_t tokens);  // for launch_matmul when matmul_wants_tc

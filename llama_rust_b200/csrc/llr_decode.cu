@@ -35,7 +35,7 @@ __device__ __forceinline__ int64_t kv_offset(const KvView& kv, int seq, int laye
 // one block per activation row; a row of up to 4096 values stays in registers between the two passes
 constexpr int NORM_THREADS = 1024;
 __global__ void __launch_bounds__(NORM_THREADS)
-rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ add, const float* __restrict__ w, float* __restrict__ y,
+rmsnorm_kernel(float* x, const float* add, const float* __restrict__ w, float* __restrict__ y,
                int n, float eps) {
   pdl_enter();
   __shared__ float sh[32];
@@ -87,7 +87,7 @@ rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ add, const float
 // One block per token: the cosine and sine of every pair's angle once (all heads of a token turn by the same
 // angles), then the rotation of every q and k head, then the k and v rows into the cache.
 __global__ void __launch_bounds__(256)
-rope_store_kernel(float* __restrict__ q, float* __restrict__ k, const float* __restrict__ v, KvView kv, RowMap rows, int layer,
+rope_store_kernel(float* q, float* k, const float* v, KvView kv, RowMap rows, int layer,
                   WalkShape w) {
   pdl_enter();
   __shared__ float s_cos[128], s_sin[128];  // head_dim <= 256
@@ -183,8 +183,8 @@ struct RowTiles {
 // rotated as it is loaded, and the block whose slice holds the token's position rotates the new key, writes it and
 // the new value into the cache and then reads them back like any other position: one launch less per layer.
 template <int G>
-__device__ __forceinline__ void attention_partial_row(const float* __restrict__ q, const KvView& kv, float* __restrict__ part, const RowMap& rows, int t, int layer,
-                                                      int chunk, const WalkShape& w, const float* __restrict__ k_new, const float* __restrict__ v_new) {
+__device__ __forceinline__ void attention_partial_row(const float* q, const KvView& kv, float* __restrict__ part, const RowMap& rows, int t, int layer,
+                                                      int chunk, const WalkShape& w, const float* k_new, const float* v_new) {
   extern __shared__ float sm[];  // slots[slot_words] | q[gqa][hd] | scores[gqa][chunk] or sums[P][gqa][hd]
   const int hkv = blockIdx.x, split = blockIdx.y;
   const int hd = w.head_dim, gqa = w.n_head / w.n_head_kv;
@@ -222,15 +222,15 @@ __device__ __forceinline__ void attention_partial_row(const float* __restrict__ 
 }
 template <int G>
 __global__ void __launch_bounds__(ATT_THREADS)
-attention_partial_kernel(const float* __restrict__ q, KvView kv, float* __restrict__ part, RowMap rows, int layer, int chunk,
-                         WalkShape w, const float* __restrict__ k_new, const float* __restrict__ v_new) {
+attention_partial_kernel(const float* q, KvView kv, float* __restrict__ part, RowMap rows, int layer, int chunk,
+                         WalkShape w, const float* k_new, const float* v_new) {
   pdl_enter();
   attention_partial_row<G>(q, kv, part, rows, blockIdx.z, layer, chunk, w, k_new, v_new);
 }
 // the listed rows of a batch, one per blockIdx.z
 template <int G>
 __global__ void __launch_bounds__(ATT_THREADS)
-attention_rows_kernel(const float* __restrict__ q, KvView kv, float* __restrict__ part, RowMap rows, int layer, int chunk, WalkShape w,
+attention_rows_kernel(const float* q, KvView kv, float* __restrict__ part, RowMap rows, int layer, int chunk, WalkShape w,
                       const __grid_constant__ RowTiles tiles) {
   pdl_enter();
   attention_partial_row<G>(q, kv, part, rows, tiles.begin(blockIdx.z), layer, chunk, w, nullptr, nullptr);
@@ -339,7 +339,7 @@ __device__ __forceinline__ void attend_slice_warp(const KV& src, const float* sq
 // the other: 24 rows of 24 sequences 129 us.)
 template <int GQA, int P>
 __global__ void __launch_bounds__(ATT_THREADS, 3)
-attention_tile_kernel(const float* __restrict__ q, KvView kv, float* __restrict__ part, RowMap rows, int layer, int chunk,
+attention_tile_kernel(const float* q, KvView kv, float* __restrict__ part, RowMap rows, int layer, int chunk,
                       WalkShape w, const __grid_constant__ RowTiles tiles) {
   pdl_enter();
   extern __shared__ float sm[];  // k tile [chunk][hd] | v tile [chunk][hd] | per warp: q[gqa][hd], scores[gqa][chunk]
@@ -400,7 +400,7 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], u
 
 template <int GQA, int HD, int NT, int RT>
 __global__ void __launch_bounds__(32 * GQA * RT)
-attention_tile_mma_kernel(const float* __restrict__ q, KvView kv, float* __restrict__ part, RowMap rows, int layer, WalkShape w,
+attention_tile_mma_kernel(const float* q, KvView kv, float* __restrict__ part, RowMap rows, int layer, WalkShape w,
                           int n_split, const __grid_constant__ RowTiles tiles) {
   pdl_enter();
   // strides in 32-bit words (two binary16 each); + 4 words spreads the fragment reads of eight rows over all banks
@@ -553,7 +553,7 @@ struct RowRanges {
 // slice sp's maximum into the weight exp(m_slice - m); the denominator is the shuffle-tree sum of the weighted slice
 // sums; then every lane adds its dimensions over the slices in ascending order, the weights coming by shuffle.
 __global__ void __launch_bounds__(128)
-attention_combine_kernel(const float* __restrict__ part, float* __restrict__ out, RowMap rows, int chunk, WalkShape w, int heads_per_block,
+attention_combine_kernel(const float* part, float* __restrict__ out, RowMap rows, int chunk, WalkShape w, int heads_per_block,
                          int max_records, int record_chunk, const __grid_constant__ RowRanges mma_rows) {
   pdl_enter();
   // heads_per_block 4: one warp per head (many rows: fewer, fuller blocks); 1: the four warps share a head's
@@ -601,19 +601,19 @@ attention_combine_kernel(const float* __restrict__ part, float* __restrict__ out
 }
 
 __device__ __forceinline__ float swiglu_of(float a, float b) { return __fmul_rn(__fdiv_rn(a, 1.0f + expf(-a)), b); }  // silu(gate) * up (decode.rs:11826, :2984)
-__global__ void swiglu_kernel(float* __restrict__ g, const float* __restrict__ u, int64_t n) {
+__global__ void swiglu_kernel(float* g, const float* u, int64_t n) {
   pdl_enter();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) g[i] = swiglu_of(g[i], u[i]);
 }
 // the same, four elements per thread and step (n4 = n / 4; g and u 16-byte aligned)
-__global__ void swiglu4_kernel(float4* __restrict__ g, const float4* __restrict__ u, int64_t n4) {
+__global__ void swiglu4_kernel(float4* g, const float4* u, int64_t n4) {
   pdl_enter();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
     const float4 a = g[i], b = u[i];
     g[i] = make_float4(swiglu_of(a.x, b.x), swiglu_of(a.y, b.y), swiglu_of(a.z, b.z), swiglu_of(a.w, b.w));
   }
 }
-__global__ void add_kernel(float* __restrict__ x, const float* __restrict__ y, int64_t n) {
+__global__ void add_kernel(float* x, const float* y, int64_t n) {
   pdl_enter();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     x[i] = __fadd_rn(y[i], x[i]);
@@ -622,8 +622,8 @@ __global__ void add_kernel(float* __restrict__ x, const float* __restrict__ y, i
 // one block: index of the first strict maximum (sample.rs:293: `v > best` scanning upwards, so ties go to the
 // lower index), its margin over the largest other value, and the position counter advanced for the next step
 __global__ void __launch_bounds__(1024)
-argmax_kernel(const float* __restrict__ logits, int n, int* __restrict__ out_id, float* __restrict__ out_margin,
-              int* __restrict__ pos_dev, int advance, int* __restrict__ count_dev) {
+argmax_kernel(const float* logits, int n, int* __restrict__ out_id, float* __restrict__ out_margin,
+              int* pos_dev, int advance, int* count_dev) {
   pdl_enter();
   // with count_dev: out_id[0] is the slot the next step reads its token from, and the token and its margin are also
   // appended at out_id[1 + *count_dev] / out_margin[*count_dev]: every step of a generation is then the same launch
@@ -688,7 +688,7 @@ argmax_kernel(const float* __restrict__ logits, int n, int* __restrict__ out_id,
 // maxima still wins (sample.rs:293), and applies the bookkeeping of argmax_kernel.
 constexpr int ARG_BLOCKS = 128;
 __global__ void __launch_bounds__(256)
-argmax_part_kernel(const float* __restrict__ logits, int n, float* __restrict__ pbest, int* __restrict__ pidx, float* __restrict__ psecond) {
+argmax_part_kernel(const float* logits, int n, float* __restrict__ pbest, int* __restrict__ pidx, float* __restrict__ psecond) {
   pdl_enter();
   __shared__ float sv[8], s2[8];
   __shared__ int si[8];
@@ -723,9 +723,9 @@ argmax_part_kernel(const float* __restrict__ logits, int n, float* __restrict__ 
   }
 }
 __global__ void __launch_bounds__(ARG_BLOCKS)
-argmax_merge_kernel(const float* __restrict__ pbest, const int* __restrict__ pidx, const float* __restrict__ psecond, int parts,
-                    int* __restrict__ out_id, float* __restrict__ out_margin, int* __restrict__ pos_dev, int advance,
-                    int* __restrict__ count_dev) {
+argmax_merge_kernel(const float* pbest, const int* pidx, const float* psecond, int parts,
+                    int* __restrict__ out_id, float* __restrict__ out_margin, int* pos_dev, int advance,
+                    int* count_dev) {
   pdl_enter();
   if (threadIdx.x != 0) return;  // a hundred-odd triples: one thread, ascending order
   float best = -CUDART_INF_F, second = -CUDART_INF_F;

@@ -464,7 +464,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap wmap, const Args P, int* __re
 // A record's digits lie as the MMA reads them: two panels of 128 columns, a row of 128 bytes per plane (4 t + p), 16-byte chunks
 // swizzled with the row number's low three bits.
 __global__ void __launch_bounds__(256)
-digit_records_kernel(const float* __restrict__ x, uint8_t* __restrict__ rec, int cols, int tokens, int tile, int places) {
+digit_records_kernel(const float* x, uint8_t* __restrict__ rec, int cols, int tokens, int tile, int places) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int lane = threadIdx.x & 31, place = (int)blockIdx.y * 8 + (threadIdx.x >> 5), b = blockIdx.x, blocks = gridDim.x;
@@ -493,7 +493,7 @@ digit_records_kernel(const float* __restrict__ x, uint8_t* __restrict__ rec, int
 
 // The units' floats -> y: eight units of a part in order from zero, then the parts, as the reducer of the decode kernel adds them
 __global__ void __launch_bounds__(256)
-add_units_kernel(const float* __restrict__ part, float* __restrict__ y, int64_t n, int units) {
+add_units_kernel(const float* part, float* __restrict__ y, int64_t n, int units) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {

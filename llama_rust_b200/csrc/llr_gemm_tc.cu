@@ -443,7 +443,7 @@ __device__ __forceinline__ void dequant_sub_h(uint32_t prow, uint32_t (&out)[16]
 // single product, an array in global memory for a grouped launch.
 template <int DT, int BN, bool F16>
 __device__ __forceinline__ void gemm_tc_tile(const CUtensorMap* wmap_p, const CUtensorMap* xmap_p, int rows, int ms_begin,
-                                             int ms_count, int tokens, const float* __restrict__ xscale,
+                                             int ms_count, int tokens, const float* xscale,
                                              float* __restrict__ Y, int row_tile, int tok_tile, int* __restrict__ err) {
   using L = GLay<DT, BN>;
   constexpr int NA = L::NA, NB = L::NB, NPK = L::NPK, NMMA = L::NMMA, PITCH = Pk<DT>::PITCH, RB = Pk<DT>::RB;
@@ -555,7 +555,7 @@ __device__ __forceinline__ void gemm_tc_tile(const CUtensorMap* wmap_p, const CU
     float scale[NS];
     if constexpr (F16) {
 #pragma unroll
-      for (int i = 0; i < NS; ++i) scale[i] = 32 * i + lane < left ? __ldg(xscale + tok0 + c_first + 32 * i + lane) : 0.f;
+      for (int i = 0; i < NS; ++i) scale[i] = 32 * i + lane < left ? xscale[tok0 + c_first + 32 * i + lane] : 0.f;
     }
     if (ok && !bar_wait(acc_full, 0)) { ok = false; report_error(err, 3); }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -687,7 +687,7 @@ __device__ __forceinline__ void gemm_tc_tile(const CUtensorMap* wmap_p, const CU
 template <int DT, int BN, bool F16>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int rows, int cols, int tokens,
-               const __grid_constant__ CUtensorMap xmap, const float* __restrict__ xscale, float* __restrict__ Y,
+               const __grid_constant__ CUtensorMap xmap, const float* xscale, float* __restrict__ Y,
                int* __restrict__ err) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // split-K: gridDim.z CTAs share a tile's K range; slice z writes its partial sums to Y + z * tokens * rows
@@ -697,7 +697,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int rows, int cols, int
                             Y + (size_t)blockIdx.z * (size_t)tokens * (size_t)rows, (int)blockIdx.x, (int)blockIdx.y, err);
 }
 
-__global__ void add_slices_kernel(const float* __restrict__ part, float* __restrict__ y, int64_t n, int slices) {
+__global__ void add_slices_kernel(const float* part, float* __restrict__ y, int64_t n, int slices) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < n; i += (int64_t)gridDim.x * blockDim.x * 4) {
@@ -724,7 +724,7 @@ gemm_tc_grouped_kernel(const GemmGroup* __restrict__ groups, int n_groups, int* 
                             local / row_tiles, err);
 }
 
-__global__ void to_bf16_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ o, int64_t n) {
+__global__ void to_bf16_kernel(const float* x, __nv_bfloat16* __restrict__ o, int64_t n) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < n; i += (int64_t)gridDim.x * blockDim.x * 4) {
@@ -741,7 +741,7 @@ __global__ void to_bf16_kernel(const float* __restrict__ x, __nv_bfloat16* __res
 // binary16 activations: one CTA per activation row.  The row is multiplied by the power of two that
 // puts its largest magnitude into [2^14, 2^15) (binary16 tops out at 65504), and the inverse goes
 // to inv_scale[row] for the epilogue.  A zero or non-finite row is left unscaled.
-__global__ void to_f16_rows_kernel(const float* __restrict__ x, __half* __restrict__ o, float* __restrict__ inv_scale, int cols) {
+__global__ void to_f16_rows_kernel(const float* x, __half* __restrict__ o, float* __restrict__ inv_scale, int cols) {
   __shared__ float wmax[8];
   asm volatile("griddepcontrol.wait;" ::: "memory");               // x may come from the kernel before
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the GEMM may start its weight pipeline
@@ -782,7 +782,7 @@ __global__ void to_f16_rows_kernel(const float* __restrict__ x, __half* __restri
 // (silu(g) * u was tried in here as well: with one CTA per row it took longer than the two
 // separate element-wise kernels.)
 template <bool F16>
-__global__ void expert_rows_16bit_kernel(const float* __restrict__ x, const int* __restrict__ src_row,
+__global__ void expert_rows_16bit_kernel(const float* x, const int* src_row,
                                          void* __restrict__ o, float* __restrict__ inv_scale, int cols) {
   __shared__ float wmax[8];
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -658,7 +658,7 @@ gemv_stream_hostout_kernel(const __grid_constant__ ProgEntry one, const __grid_c
 // *sel is written by an earlier kernel of the stream, so nothing is fetched before that kernel has finished.
 template <int DT>
 __global__ void __launch_bounds__(NTHREADS, 2)
-gemv_stream_select_kernel(const __grid_constant__ ProgEntry one, const CUtensorMap* __restrict__ maps, const int* __restrict__ sel,
+gemv_stream_select_kernel(const __grid_constant__ ProgEntry one, const CUtensorMap* __restrict__ maps, const int* sel,
                           int* __restrict__ err) {
   __shared__ ProgPhase phase;
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -702,7 +702,7 @@ gemv_sharded_program_kernel(const ProgEntry* __restrict__ entries, const ProgPha
 // One phase of one-token products that each pick one of several equally shaped matrices through a device table.
 __global__ void __launch_bounds__(NTHREADS, 2)
 gemv_select_program_kernel(const ProgEntry* __restrict__ entries, const ProgPhase* __restrict__ phases,
-                           const CUtensorMap* __restrict__ maps, const int* __restrict__ sel,
+                           const CUtensorMap* __restrict__ maps, const int* sel,
                            unsigned long long* __restrict__ counters, const RunArgs run, int* __restrict__ err) {
   Work wk{entries, phases, 1, nullptr, HostOut{}, maps, run.n_entries, run.tag_base, run.poll_limit, sel};
   if (blockIdx.x == 0 && threadIdx.x == 0) counters[TAG_SLOT] = run.tag_next;

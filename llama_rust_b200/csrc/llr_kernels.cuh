@@ -31,7 +31,9 @@ struct PerDevice {
 __device__ __forceinline__ void report_error(int* err, int code) { *(volatile int*)err = code; }
 
 // A launch that may be placed on the SMs while its predecessor in the stream still runs (programmatic stream serialization).  The
-// kernel waits (griddepcontrol.wait) before it touches anything but weights.
+// kernel waits (griddepcontrol.wait) before it touches anything but weights, and takes what a predecessor wrote through pointers without
+// __restrict__ and without __ldg: both promise data that nobody writes while the kernel lives, which lets a load take the
+// non-coherent path or move above the wait.
 template <class... P, class... A>
 cudaError_t launch_overlapped(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A... args) {
   cudaLaunchAttribute attr;

@@ -35,7 +35,7 @@ __device__ __forceinline__ float4 widen4(uint2 u) {
 
 // ---- embedding ------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-embed_kernel(const uint16_t* __restrict__ table, const uint16_t* __restrict__ pos_table, const int* __restrict__ ids, RowMap rows, float scale,
+embed_kernel(const uint16_t* __restrict__ table, const uint16_t* __restrict__ pos_table, const int* ids, RowMap rows, float scale,
              float* __restrict__ x, __nv_bfloat16* __restrict__ x16, int n, RotTable rot) {
   pdl_enter();
   const int t = blockIdx.x;
@@ -204,7 +204,7 @@ __device__ __forceinline__ void store_latent(const float* p, const float* w, int
   }
 }
 __global__ void __launch_bounds__(PROJ_THREADS)
-latent_store_kernel(const float* __restrict__ proj, int ld, const float* __restrict__ w, int n, float eps, LayerKv kv, RowMap rows) {
+latent_store_kernel(const float* proj, int ld, const float* __restrict__ w, int n, float eps, LayerKv kv, RowMap rows) {
   pdl_enter();
   __shared__ float red[32];
   const int t = blockIdx.x;
@@ -212,7 +212,7 @@ latent_store_kernel(const float* __restrict__ proj, int ld, const float* __restr
 }
 
 __global__ void __launch_bounds__(256)
-rows_bf16_kernel(const float* __restrict__ x, int64_t ld, int n, __nv_bfloat16* __restrict__ o) {
+rows_bf16_kernel(const float* x, int64_t ld, int n, __nv_bfloat16* __restrict__ o) {
   pdl_enter();
   const float* xr = x + (int64_t)blockIdx.x * ld;
   __nv_bfloat16* orow = o + (int64_t)blockIdx.x * n;
@@ -228,7 +228,7 @@ rows_bf16_kernel(const float* __restrict__ x, int64_t ld, int n, __nv_bfloat16* 
 // read along its rows), the four partial sums are added in order.
 template <int TT>
 __global__ void __launch_bounds__(256)
-head_product_t_kernel(const uint16_t* __restrict__ w, int heads, int rows, int cols, const float* __restrict__ x, int64_t x_ld,
+head_product_t_kernel(const uint16_t* __restrict__ w, int heads, int rows, int cols, const float* x, int64_t x_ld,
                       float* __restrict__ y, int tokens) {
   pdl_enter();
   __shared__ float part[4][TT][128];
@@ -272,8 +272,8 @@ head_product_t_kernel(const uint16_t* __restrict__ w, int heads, int rows, int c
 // y[t][h * rows + r] = sum_c W[h * rows + r][c] x[t][h * cols + c], times the head's gate: one warp per row of W
 template <int TT>
 __global__ void __launch_bounds__(256)
-head_product_kernel(const uint16_t* __restrict__ w, int heads, int rows, int cols, const float* __restrict__ x, int64_t x_ld,
-                    float* __restrict__ y, const float* __restrict__ gate, int64_t gate_ld, int tokens) {
+head_product_kernel(const uint16_t* __restrict__ w, int heads, int rows, int cols, const float* x, int64_t x_ld,
+                    float* __restrict__ y, const float* gate, int64_t gate_ld, int tokens) {
   pdl_enter();
   const int lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5), t0 = blockIdx.y * TT;
   if (row >= heads * rows) return;
@@ -378,7 +378,7 @@ struct SpanRuns {
 static_assert(PROJ_THREADS == ATT_THREADS, "the sums over a projection are formed in one order");
 template <int MAX_VALUE, int G>  // G: the most query heads of a block
 __global__ void __launch_bounds__(ATT_THREADS)
-span_partial_kernel(const float* __restrict__ q, int64_t q_ld, SpanShape sh, LayerKv kv, RowMap rows, const __grid_constant__ SpanRuns runs, int chunk,
+span_partial_kernel(const float* q, int64_t q_ld, SpanShape sh, LayerKv kv, RowMap rows, const __grid_constant__ SpanRuns runs, int chunk,
                     float* __restrict__ part, NewToken nt) {
   pdl_enter();
   __shared__ float red[2][32];
@@ -424,7 +424,7 @@ span_partial_kernel(const float* __restrict__ q, int64_t q_ld, SpanShape sh, Lay
 
 // grid (query head, row, 128 dimensions): merges a head's slices (at most 32) and the sink, applies the gate
 __global__ void __launch_bounds__(128)
-span_combine_kernel(const float* __restrict__ part, SpanShape sh, RowMap rows, const __grid_constant__ SpanRuns runs, int n_split, SpanOut so) {
+span_combine_kernel(const float* part, SpanShape sh, RowMap rows, const __grid_constant__ SpanRuns runs, int n_split, SpanOut so) {
   pdl_enter();
   const int lane = threadIdx.x & 31, h = blockIdx.x, t = runs.row(blockIdx.y);
   const int gq = sh.n_head / sh.n_kv, per = span_heads(sh), groups = (gq + per - 1) / per;
@@ -568,7 +568,7 @@ span_gather_kernel(SpanShape sh, LayerKv kv, RowMap rows, const __grid_constant_
 
 template <int ND, int NS>
 __global__ void __launch_bounds__(128 * NS)
-span_mma_kernel(const float* __restrict__ q, int64_t q_ld, SpanShape sh, const __half* __restrict__ scratch, bool shared_kv, RowMap rows,
+span_mma_kernel(const float* q, int64_t q_ld, SpanShape sh, const __half* scratch, bool shared_kv, RowMap rows,
                 const __grid_constant__ SpanBatch b, SpanOut so) {
   pdl_enter();
   const int gi = span_group(b.tiles_at, b.n, blockIdx.x), t0 = b.t0[gi], tokens = b.rows[gi];
@@ -798,7 +798,7 @@ span_mma_kernel(const float* __restrict__ q, int64_t q_ld, SpanShape sh, const _
 // ---- norm on a sublayer's output, residual add ------------------------------------------------------------------------
 constexpr int NORM_ADD_THREADS = 512, NORM_ADD_KEEP = 4;  // up to 8192 values of a row stay in registers
 __global__ void __launch_bounds__(NORM_ADD_THREADS)
-norm_add_kernel(float* __restrict__ x, const float* __restrict__ y, int slices, int64_t slice_stride, const float* __restrict__ w, float eps,
+norm_add_kernel(float* x, const float* y, int slices, int64_t slice_stride, const float* __restrict__ w, float eps,
                 __nv_bfloat16* __restrict__ x16, int n) {
   pdl_enter();
   __shared__ float sh[32];
@@ -855,7 +855,7 @@ norm_add_kernel(float* __restrict__ x, const float* __restrict__ y, int slices, 
 
 // ---- residual add, norm of the sum: what a sublayer reads ------------------------------------------------------------
 __global__ void __launch_bounds__(NORM_ADD_THREADS)
-add_norm_kernel(float* __restrict__ x, const float* __restrict__ y, int slices, int64_t slice_stride, const float* __restrict__ w, float eps,
+add_norm_kernel(float* x, const float* y, int slices, int64_t slice_stride, const float* __restrict__ w, float eps,
                 float* __restrict__ h, __nv_bfloat16* __restrict__ h16, int n) {
   pdl_enter();
   __shared__ float sh[32];
@@ -908,7 +908,7 @@ add_norm_kernel(float* __restrict__ x, const float* __restrict__ y, int slices, 
 
 // ---- gated unit ----------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-gated_unit_kernel(const float* __restrict__ gu, GluShape sh, float* __restrict__ out, __nv_bfloat16* __restrict__ out16, int tokens) {
+gated_unit_kernel(const float* gu, GluShape sh, float* __restrict__ out, __nv_bfloat16* __restrict__ out16, int tokens) {
   pdl_enter();
   const int64_t step = (int64_t)gridDim.x * blockDim.x, first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (sh.n % 4 == 0) {

@@ -159,7 +159,7 @@ bucket_kernel(const int* __restrict__ ids, const float* __restrict__ wts, const 
 
 // One token's selection in ascending expert id (the order scatter_expert_rows :10263 adds in), for the products whose
 // matrix is chosen on the device.  n_used <= 8; one thread.
-__global__ void select_sorted_kernel(const int* __restrict__ ids, const float* __restrict__ wts, int n_used, int* __restrict__ sel,
+__global__ void select_sorted_kernel(const int* ids, const float* wts, int n_used, int* __restrict__ sel,
                                      float* __restrict__ selw) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (threadIdx.x != 0) return;
@@ -176,7 +176,7 @@ __global__ void select_sorted_kernel(const int* __restrict__ ids, const float* _
 
 // out[c] = sum over the selected experts, in the order given, of y[j][c] * w[j]: product rounded, then added, from zero
 // (what scatter_combine_kernel does for a packed batch)
-__global__ void combine_one_kernel(const float* __restrict__ y, const float* __restrict__ selw, float* __restrict__ out, int n_used,
+__global__ void combine_one_kernel(const float* y, const float* selw, float* __restrict__ out, int n_used,
                                    int n_embd) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n_embd; c += gridDim.x * blockDim.x) {

@@ -110,7 +110,7 @@ __device__ __forceinline__ void in_parts(float v, __nv_bfloat16 (&p)[3]) {
 // grid (row, CONV_COLS channels); vec: four channels per thread, everything on boundaries of four
 constexpr int CONV_THREADS = 128;
 __global__ void __launch_bounds__(CONV_THREADS)
-conv_rows_kernel(const float* __restrict__ x, int64_t ld, ConvShape cv, float* __restrict__ u, __nv_bfloat16* __restrict__ u16, int block, RowMap rows, bool vec) {
+conv_rows_kernel(const float* x, int64_t ld, ConvShape cv, float* __restrict__ u, __nv_bfloat16* __restrict__ u16, int block, RowMap rows, bool vec) {
   pdl_enter();
   const int t = blockIdx.x, near = rows_before(rows, t, cv.taps - 1), pos = row_position(rows, t), at = blockIdx.y * CONV_THREADS + threadIdx.x;
   const float* tail = cv.tail.state + row_sequence(rows, t) * cv.tail.stride;
@@ -156,7 +156,7 @@ __device__ __forceinline__ float fade(float rate, float a, float bias) { return 
 // grid (row, key/value head), a thread per value where they fit a block: the head's query and key, and values and decays of the
 // heads that share them
 __global__ void __launch_bounds__(1024)
-delta_prepare_kernel(const float* __restrict__ proj, int64_t ld, const float* __restrict__ a, const float* __restrict__ b, DeltaShape d, ConvShape cv,
+delta_prepare_kernel(const float* proj, int64_t ld, const float* a, const float* b, DeltaShape d, ConvShape cv,
                      float* __restrict__ prep, int64_t prep_ld, RowMap rows) {
   pdl_enter();
   extern __shared__ float qk[];  // the head's q | k behind convolution and silu
@@ -226,7 +226,7 @@ __device__ __forceinline__ float dot4(float4 a, float4 b) { return fmaf(a.x, b.x
 
 // grid (block of rows, head), a warp per row, a lane per four key channels
 __global__ void __launch_bounds__(32 * BLOCK_ROWS)
-delta_blocks_kernel(const float* __restrict__ proj, int64_t ld, const float* __restrict__ a, const float* __restrict__ b, DeltaShape d, ConvShape cv,
+delta_blocks_kernel(const float* proj, int64_t ld, const float* a, const float* b, DeltaShape d, ConvShape cv,
                     int dp, float* __restrict__ rec, float* __restrict__ v_out, RowGroups groups, RowMap rows, int tokens) {
   pdl_enter();
   __shared__ float4 sq[BLOCK_ROWS][32], sk[BLOCK_ROWS][32], sg[BLOCK_ROWS][32];
@@ -384,7 +384,7 @@ __device__ __forceinline__ void head_out(const float* o, int vdim, const HeadOut
   }
 }
 __global__ void __launch_bounds__(256)
-head_out_kernel(const float* __restrict__ o, int heads, int vdim, HeadOut ho, int tokens) {
+head_out_kernel(const float* o, int heads, int vdim, HeadOut ho, int tokens) {
   pdl_enter();
   const int64_t i = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (i >= (int64_t)tokens * heads) return;
@@ -637,7 +637,7 @@ struct BlockLay {
 };
 template <int LPC, int R, int C, bool DELTA>
 __global__ void __launch_bounds__(256)
-block_scan_kernel(MatrixScan m, RowGroups groups, RowMap rows, int tokens, int cols, const float* __restrict__ rec, float* __restrict__ o_raw) {
+block_scan_kernel(MatrixScan m, RowGroups groups, RowMap rows, int tokens, int cols, const float* rec, float* __restrict__ o_raw) {
   pdl_enter();
   constexpr int DP = LPC * R, P = R / 2, V = 4 * C, REP = LPC / V;
   static_assert(REP >= 1, "a lane per dot product");

@@ -305,10 +305,10 @@ MatView view_of(const llr_matrix* m) {
 // The integer GEMM has a buffer of its own, and does without where that is not safe or not to be had (the decode kernel then runs,
 // with the same results): on a stream of the caller's, whose work may overlap other work of this executor; under capture, since a
 // replay would outlive the buffer; when memory is short or LLR_DIGITS_LIMIT smaller than what it needs.
-cudaError_t ensure_scratch(llr_exec* e, const llr_matrix* m, size_t tokens, cudaStream_t stream, void** out) {
+cudaError_t ensure_scratch(llr_exec* e, const llr_matrix* m, size_t tokens, int path, cudaStream_t stream, void** out) {
   *out = nullptr;
   const MatView v = view_of(m);
-  if (matmul_wants_i8(v, (int64_t)tokens, e->path)) {
+  if (matmul_wants_i8(v, (int64_t)tokens, path)) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (stream != e->stream || cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return cudaSuccess;
     const size_t need = gemm_i8_scratch_bytes(v, (int64_t)tokens);
@@ -317,7 +317,7 @@ cudaError_t ensure_scratch(llr_exec* e, const llr_matrix* m, size_t tokens, cuda
     else cudaGetLastError();
     return cudaSuccess;
   }
-  if (!matmul_wants_tc(v, (int64_t)tokens, e->path)) return cudaSuccess;
+  if (!matmul_wants_tc(v, (int64_t)tokens, path)) return cudaSuccess;
   cudaError_t ce = grow_device(&e->dev_s, &e->dev_s_cap, matmul_scratch_bytes(v, (int64_t)tokens));
   if (ce == cudaSuccess) *out = e->dev_s;
   return ce;
@@ -397,7 +397,7 @@ int run_host(llr_exec* e, const llr_matrix* m, size_t tokens, const float* x, fl
     y_alias = e->pin_y_alias;
   }
   void* scratch = nullptr;
-  if ((ce = ensure_scratch(e, m, tokens, e->stream, &scratch)) != cudaSuccess) return fail_cuda(e, ce, "kernel scratch");
+  if ((ce = ensure_scratch(e, m, tokens, e->path, e->stream, &scratch)) != cudaSuccess) return fail_cuda(e, ce, "kernel scratch");
   if ((ce = cudaMemcpyAsync(e->dev_x, src, nx * sizeof(float), cudaMemcpyHostToDevice, e->stream)) != cudaSuccess)
     return fail_cuda(e, ce, "activation upload");
   const MatView v = view_of(m);
@@ -845,7 +845,7 @@ int llr_matmul_device(llr_exec* e, const llr_matrix* m, size_t tokens, const flo
   DeviceGuard guard(e->device);
   cudaStream_t s = stream ? (cudaStream_t)stream : e->stream;
   void* scratch = nullptr;
-  cudaError_t ce = ensure_scratch(e, m, tokens, s, &scratch);
+  cudaError_t ce = ensure_scratch(e, m, tokens, e->path, s, &scratch);
   if (ce != cudaSuccess) return fail_cuda(e, ce, "kernel scratch");
   ce = launch_matmul(view_of(m), x_dev, y_dev, (int64_t)tokens, s, e->path, e->sm_count, e->err_flag,
                      scratch, &e->ctr.launches);
@@ -896,14 +896,9 @@ int expert_path(const llr_exec* e, size_t n_rows) { return e->path == PATH_AUTO 
 
 cudaError_t matmul_dev(llr_exec* e, const llr_matrix* m, size_t tokens, const float* x, float* y, int path) {
   void* scratch = nullptr;
-  const int saved = e->path;
-  e->path = path;
-  cudaError_t ce = ensure_scratch(e, m, tokens, e->stream, &scratch);
-  if (ce == cudaSuccess)
-    ce = launch_matmul(view_of(m), x, y, (int64_t)tokens, e->stream, path, e->sm_count, e->err_flag, scratch,
-                       &e->ctr.launches);
-  e->path = saved;
-  return ce;
+  const cudaError_t ce = ensure_scratch(e, m, tokens, path, e->stream, &scratch);
+  if (ce != cudaSuccess) return ce;
+  return launch_matmul(view_of(m), x, y, (int64_t)tokens, e->stream, path, e->sm_count, e->err_flag, scratch, &e->ctr.launches);
 }
 
 }  // namespace
@@ -983,17 +978,9 @@ cudaError_t moe_run_experts(llr_exec* e, const llr_moe_layer* L, const MoeShape&
   cudaError_t ce = cudaSuccess;
   if (n_rows == 0) return ce;
   if (S.any_remote && (ce = cudaMemsetAsync(B.y, 0, n_rows * n_embd * 4, e->stream)) != cudaSuccess) return ce;  // rows nobody computes here
-  {  // size the GEMM staging buffer once, for the busiest expert's widest product: growing it between
-     // launches would free and reallocate, which synchronizes the device
-    size_t busiest = 0, most = 0;
-    for (size_t ex = 0; ex < n_exp; ++ex)
-      if (S.local[ex] && (size_t)(first_row[ex + 1] - first_row[ex]) > most) { most = (size_t)(first_row[ex + 1] - first_row[ex]); busiest = ex; }
-    void* unused = nullptr;
-    if (most > 0 && ((ce = ensure_scratch(e, L->down[busiest], most, e->stream, &unused)) != cudaSuccess ||
-                     (ce = ensure_scratch(e, L->gate[busiest], most, e->stream, &unused)) != cudaSuccess))
-      return ce;
-    if (most == 0) return cudaSuccess;  // nothing routed to a resident expert
-  }
+  bool any = false;
+  for (size_t ex = 0; ex < n_exp; ++ex) any = any || (S.local[ex] && first_row[ex + 1] > first_row[ex]);
+  if (!any) return cudaSuccess;  // nothing routed to a resident expert
   // Grouped tensor-core path (automatic choice, 64 routed rows or more, formats the GEMM takes): the tiles of
   // all experts' gate and up products in one launch, silu(g)*u, all down products in one launch.
   bool grouped = e->path == PATH_AUTO && n_rows >= 64;
@@ -1009,6 +996,15 @@ cudaError_t moe_run_experts(llr_exec* e, const llr_moe_layer* L, const MoeShape&
     if (vg.f16_ok != 1 || vu.f16_ok != 1) f16a = 0;
     if (vd.f16_ok != 1) f16b = 0;
   }
+  if (!grouped)  // the products' workspaces before the first of them: growing one between launches synchronizes the device.  Every
+                 // expert is asked: fewer rows may need more (unit sums of products spread over several CTAs)
+    for (size_t ex = 0; ex < n_exp; ++ex) {
+      const size_t n = (size_t)(first_row[ex + 1] - first_row[ex]);
+      void* unused = nullptr;
+      if (n == 0 || !S.local[ex]) continue;
+      for (const llr_matrix* m : {L->gate[ex], L->up[ex], L->down[ex]})
+        if ((ce = ensure_scratch(e, m, n, expert_path(e, n), e->stream, &unused)) != cudaSuccess) return ce;
+    }
   const float* rows_f32 = d_x;  // packed f32 rows for the per-expert path
   if (!grouped && d_tok_of_row) {
     if ((ce = launch_gather_rows(d_x, d_tok_of_row, B.pack, (int)n_rows, (int)n_embd, e->stream, &e->ctr.launches)) != cudaSuccess) return ce;
@@ -1779,7 +1775,7 @@ void session_orphan(llr_session* s) {
 cudaError_t session_matmul(llr_exec* e, const llr_matrix* m, size_t tokens, const float* x, float* y, StagedRows* rows = nullptr) {
   const size_t s_cap = e->dev_s_cap, q_cap = e->dev_q_cap;
   void* scratch = nullptr;
-  cudaError_t ce = ensure_scratch(e, m, tokens, e->stream, &scratch);
+  cudaError_t ce = ensure_scratch(e, m, tokens, e->path, e->stream, &scratch);
   if (ce != cudaSuccess) return ce;
   if (rows && (e->dev_s_cap != s_cap || e->dev_q_cap != q_cap)) *rows = StagedRows{};  // a buffer has grown: another one, though it may lie where the old one lay
   return launch_matmul(view_of(m), x, y, (int64_t)tokens, e->stream, e->path, e->sm_count, e->err_flag, scratch, &e->ctr.launches, rows);

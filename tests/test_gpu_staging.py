@@ -1,5 +1,5 @@
-"""Products of the same rows that follow each other in a session (q, k, v and gate, up) share their staged activations: digit records
-up to 63 rows, 16-bit rows from 64 on.  A wrong reuse multiplies other rows than the layer's."""
+"""Workspaces of staged activations: digit records up to 63 rows, 16-bit rows from 64 on.  Products of the same rows that follow each
+other in a session (q, k, v and gate, up) share them; a wrong reuse multiplies other rows than the layer's."""
 import numpy as np
 import pytest
 
@@ -120,3 +120,27 @@ def test_16_bit_rows_shared_by_products_of_the_same_rows(n):
             assert err.max() <= 2.0 ** -6, (wide, err.max())
             s.free()
     assert launches[("attn_k", "ffn_up")] - launches[()] == 3
+
+
+def test_routed_layers_ask_for_the_workspaces_they_use(monkeypatch):
+    """Experts of 13 to 63 rows each.  In one grouped launch (the automatic choice) they use no workspace of digits, and none is
+    allocated: the device's free memory does not hang on LLR_DIGITS_LIMIT (8 MB for the gate matrices, were it grown).  On the
+    f32-faithful path they use it, and the layer's bits are those without."""
+    import torch
+    from llama_rust_b200 import Executor
+    width, ff, n = 2048, 8192, 40
+    x = np.random.default_rng(5).standard_normal((n, width)).astype(np.float32)
+    taken, out = {}, {}
+    for turn, limit in enumerate(("0", "0", "1000000000")):  # the first loads the kernels
+        monkeypatch.setenv("LLR_DIGITS_LIMIT", limit)
+        with Executor(0) as ex:
+            router = ex.synth(F32, 4, width, 70)
+            parts = [[ex.synth(Q4_K, r, c, 71 + 4 * k + i) for i in range(4)] for k, (r, c) in enumerate(((ff, width), (ff, width), (width, ff)))]
+            before = torch.cuda.mem_get_info()[0]
+            _, ids, _ = ex.moe_ffn(router, *parts, 2, True, x)
+            taken[turn] = before - torch.cuda.mem_get_info()[0]
+            assert all(13 <= c <= 63 for c in np.bincount(ids.ravel(), minlength=4))
+            ex.set_path(3)
+            out[turn] = ex.moe_ffn(router, *parts, 2, True, x)[0]
+    assert abs(taken[2] - taken[1]) < 4 << 20, taken
+    assert _same_bits(out[1], out[2])

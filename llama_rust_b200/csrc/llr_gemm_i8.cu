@@ -511,10 +511,10 @@ add_units_kernel(const float* part, float* __restrict__ y, int64_t n, int units)
   }
 }
 
-// Activation rows per tile: as few tiles as 24 rows each allow, the rows spread evenly over them
+// Activation rows per tile: as few tiles as 24 rows each allow, the rows spread evenly over them (13 at least: I8_MIN_TOKENS)
 int tile_rows(int64_t tokens) {
   const int64_t tiles = (tokens + 23) / 24, per = (tokens + tiles - 1) / tiles;
-  return per > 16 ? 24 : per > 8 ? 16 : 8;
+  return per > 16 ? 24 : 16;
 }
 // CTAs that share a tile's units.  More than one only where the row tiles leave most SMs idle: the units' floats then go through
 // memory and a second kernel.
@@ -554,8 +554,7 @@ cudaError_t launch_dt(const MatView& m, const Args& a, int tb, int slices, cudaS
   if (enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, (void*)m.w, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return cudaErrorInvalidValue;
-  return tb == 24 ? launch_tb<DT, 24>(m, wmap, a, slices, stream, err) : tb == 16 ? launch_tb<DT, 16>(m, wmap, a, slices, stream, err)
-                                                                               : launch_tb<DT, 8>(m, wmap, a, slices, stream, err);
+  return tb == 24 ? launch_tb<DT, 24>(m, wmap, a, slices, stream, err) : launch_tb<DT, 16>(m, wmap, a, slices, stream, err);
 }
 
 }  // namespace

@@ -125,12 +125,13 @@ __device__ __forceinline__ void fma2(unsigned long long& s, unsigned long long a
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s) : "l"(a), "l"(b));
 }
 template <int T> struct WideTile { static constexpr int SLOTS = T / 2 * 4 * 32; };  // 16-byte slots: (pair of rows, two columns, lane)
-template <int DT, int T, int R, bool RUNS>
-__global__ void __launch_bounds__(ROW_WARPS * 32, R * T * (DT == DT_F32 || RUNS ? 2 : 1) >= 64 ? 1 : 2)
+template <int DT, int T, int R, bool RUNS, int S>  // S: 256-column steps that a tile holds
+__global__ void __launch_bounds__(ROW_WARPS * 32, S > 1 || R * T * (DT == DT_F32 || RUNS ? 2 : 1) >= 64 ? 1 : 2)
 gemv_rows_wide_kernel(const uint8_t* __restrict__ W, int64_t row_bytes, int64_t rows, int64_t cols, const float* __restrict__ X,
                       float* __restrict__ Y, int tokens) {
-  constexpr int NP = T / 2, FILL = (NP * 64 + ROW_WARPS * 32 - 1) / (ROW_WARPS * 32);  // float4 pairs of a tile per thread
-  __shared__ __align__(16) uint4 tile[2][WideTile<T>::SLOTS];
+  constexpr int NP = T / 2, PIECES = S * NP * 64, FILL = (PIECES + ROW_WARPS * 32 - 1) / (ROW_WARPS * 32);  // float4 pairs of a tile, per thread
+  constexpr int SLOTS = WideTile<T>::SLOTS;
+  __shared__ __align__(16) uint4 tile[2][S * SLOTS];
   const int tid = threadIdx.x, lane = tid & 31;
   const int64_t row0 = (int64_t)blockIdx.x * (ROW_WARPS * R) + (tid >> 5) * R;
   const uint8_t* wr[R];
@@ -149,10 +150,10 @@ gemv_rows_wide_kernel(const uint8_t* __restrict__ W, int64_t row_bytes, int64_t 
   auto load_x = [&](int64_t c0) {  // four columns of two activation rows per piece; rows and columns beyond the end are zeros
 #pragma unroll
     for (int f = 0; f < FILL; ++f) {
-      const int piece = f * ROW_WARPS * 32 + tid, p = piece >> 6;
-      const int64_t c = c0 + 4 * (piece & 63);
+      const int piece = f * ROW_WARPS * 32 + tid, p = (piece >> 6) % NP;
+      const int64_t c = c0 + 256 * (piece / (NP * 64)) + 4 * (piece & 63);
       xa[f] = xb[f] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (piece < NP * 64 && c < cols) {
+      if (piece < PIECES && c < cols) {
         if (2 * p < tokens) xa[f] = __ldg((const float4*)(X + (int64_t)(2 * p) * cols + c));
         if (2 * p + 1 < tokens) xb[f] = __ldg((const float4*)(X + (int64_t)(2 * p + 1) * cols + c));
       }
@@ -161,50 +162,56 @@ gemv_rows_wide_kernel(const uint8_t* __restrict__ W, int64_t row_bytes, int64_t 
   auto store_x = [&](int buf) {
 #pragma unroll
     for (int f = 0; f < FILL; ++f) {
-      const int piece = f * ROW_WARPS * 32 + tid, p = piece >> 6, q = piece & 63;
-      if (piece >= NP * 64) break;
-      float4* at = (float4*)&tile[buf][(p * 4 + 2 * (q & 1)) * 32 + (q >> 1)];
+      const int piece = f * ROW_WARPS * 32 + tid, p = (piece >> 6) % NP, q = piece & 63;
+      if (piece >= PIECES) break;
+      float4* at = (float4*)&tile[buf][piece / (NP * 64) * SLOTS + (p * 4 + 2 * (q & 1)) * 32 + (q >> 1)];
       at[0] = make_float4(xa[f].x, xb[f].x, xa[f].y, xb[f].y);
       at[32] = make_float4(xa[f].z, xb[f].z, xa[f].w, xb[f].w);
     }
   };
-  Raw8<DT> raw[2][R];
-  auto load_w = [&](int64_t c, Raw8<DT> (&to)[R]) {
-    if (c < cols) {
+  Raw8<DT> raw[2][S][R];
+  auto load_w = [&](int64_t c0, Raw8<DT> (&to)[S][R]) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) fetch8<DT>(wr[r], c, to[r]);
+    for (int j = 0; j < S; ++j) {
+      const int64_t c = c0 + 256 * j + 8 * lane;
+      if (c < cols) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) fetch8<DT>(wr[r], c, to[j][r]);
+      }
     }
   };
-  load_w(8 * lane, raw[0]);
+  load_w(0, raw[0]);
   load_x(0);
   store_x(0);
   __syncthreads();
-  auto step = [&](int64_t c0, int buf, Raw8<DT> (&now)[R], Raw8<DT> (&next)[R]) {
-    load_w(c0 + 256 + 8 * lane, next);
-    load_x(c0 + 256);
-    if (c0 + 8 * lane < cols) {
+  auto step = [&](int64_t c0, int buf, Raw8<DT> (&now)[S][R], Raw8<DT> (&next)[S][R]) {
+    load_w(c0 + 256 * S, next);
+    load_x(c0 + 256 * S);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {  // four columns at a time
-        unsigned long long w2[R][4];
+    for (int j = 0; j < S; ++j)
+      if (c0 + 256 * j + 8 * lane < cols) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          float w[8];
-          widen8<DT>(now[r], w);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) w2[r][k] = pack2(w[4 * h + k], w[4 * h + k]);
-        }
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-          const ulonglong2 u = *(const ulonglong2*)&tile[buf][(p * 4 + 2 * h) * 32 + lane];
-          const ulonglong2 v = *(const ulonglong2*)&tile[buf][(p * 4 + 2 * h + 1) * 32 + lane];
+        for (int h = 0; h < 2; ++h) {  // four columns at a time
+          unsigned long long w2[R][4];
 #pragma unroll
           for (int r = 0; r < R; ++r) {
-            fma2(acc[r][p], w2[r][0], u.x); fma2(acc[r][p], w2[r][1], u.y);
-            fma2(acc[r][p], w2[r][2], v.x); fma2(acc[r][p], w2[r][3], v.y);
+            float w[8];
+            widen8<DT>(now[j][r], w);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w2[r][k] = pack2(w[4 * h + k], w[4 * h + k]);
+          }
+#pragma unroll
+          for (int p = 0; p < NP; ++p) {
+            const ulonglong2 u = *(const ulonglong2*)&tile[buf][j * SLOTS + (p * 4 + 2 * h) * 32 + lane];
+            const ulonglong2 v = *(const ulonglong2*)&tile[buf][j * SLOTS + (p * 4 + 2 * h + 1) * 32 + lane];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              fma2(acc[r][p], w2[r][0], u.x); fma2(acc[r][p], w2[r][1], u.y);
+              fma2(acc[r][p], w2[r][2], v.x); fma2(acc[r][p], w2[r][3], v.y);
+            }
           }
         }
       }
-    }
     store_x(buf ^ 1);
     __syncthreads();
   };
@@ -217,10 +224,11 @@ gemv_rows_wide_kernel(const uint8_t* __restrict__ W, int64_t row_bytes, int64_t 
         acc[r][p] = 0ull;
       }
   };
-  for (int64_t c0 = 0; c0 < cols; c0 += 512) {
+  static_assert(!RUNS || S == 1, "runs are closed between steps");
+  for (int64_t c0 = 0; c0 < cols; c0 += 512 * S) {
     step(c0, 0, raw[0], raw[1]);
     if (RUNS && cols <= 2048) close_run();
-    if (c0 + 256 < cols) step(c0 + 256, 1, raw[1], raw[0]);
+    if (c0 + 256 * S < cols) step(c0 + 256 * S, 1, raw[1], raw[0]);
     if (RUNS) close_run();
   }
 #pragma unroll
@@ -314,9 +322,9 @@ cudaError_t launch_rows(const MatView& m, const float* x, float* y, int tokens, 
   return cudaGetLastError();
 }
 
-template <int DT, int T, int R, bool RUNS = false>
+template <int DT, int T, int R, bool RUNS = false, int S = 1>
 cudaError_t launch_rows_wide(const MatView& m, const float* x, float* y, int tokens, cudaStream_t stream) {
-  gemv_rows_wide_kernel<DT, T, R, RUNS><<<(unsigned)((m.rows + ROW_WARPS * R - 1) / (ROW_WARPS * R)), ROW_WARPS * 32, 0, stream>>>(
+  gemv_rows_wide_kernel<DT, T, R, RUNS, S><<<(unsigned)((m.rows + ROW_WARPS * R - 1) / (ROW_WARPS * R)), ROW_WARPS * 32, 0, stream>>>(
       m.w, m.row_bytes, m.rows, m.cols, x, y, tokens);
   return cudaGetLastError();
 }
@@ -328,6 +336,11 @@ cudaError_t launch_rows_mt(const MatView& m, const float* x, float* y, int token
   if (tokens == 2) return launch_rows<DT, 2>(m, x, y, tokens, stream, sm_count);
   // four weight rows per warp, two where they would leave SMs without a block
   const bool few = m.rows < (int64_t)sm_count * 2 * ROW_WARPS * 4;
+  // Up to four activation rows of a matrix that has at most a block per SM: a step of 256 columns is little work, and what a CTA waits
+  // for is one trip to memory per tile; tiles of four steps make a quarter of the trips.  From 1024 columns on, where the first
+  // tile is full (2048 x 256: 4.2 us with one step, 4.8 with four).  Three rows, weights from HBM, one / four steps a tile, and a
+  // warp per weight row (the kernel above): 128 x 28672 F32 88 / 51 / 67 us, BF16 80 / 34 / 71; 1024 x 4096 F32 16.3 / 11.2 / 14.2.
+  if (tokens <= 4 && m.cols >= 1024 && m.rows <= (int64_t)sm_count * 2 * ROW_WARPS) return launch_rows_wide<DT, 4, 2, false, 4>(m, x, y, tokens, stream);
   if (tokens <= 4) return few ? launch_rows_wide<DT, 4, 2>(m, x, y, tokens, stream) : launch_rows_wide<DT, 4, 4>(m, x, y, tokens, stream);
   if (tokens <= 8) return few ? launch_rows_wide<DT, 8, 2>(m, x, y, tokens, stream) : launch_rows_wide<DT, 8, 4>(m, x, y, tokens, stream);
   return few ? launch_rows_wide<DT, 16, 2>(m, x, y, tokens, stream) : launch_rows_wide<DT, 16, 4>(m, x, y, tokens, stream);

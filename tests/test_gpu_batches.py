@@ -46,6 +46,21 @@ def test_rows_of_unpacked_formats_alone_and_in_a_batch(ex, name, rows, cols):
     m.free()
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 1024), (17, 1032), (33, 2048), (7, 2304), (40, 5000), (2368, 1096), (2369, 1096)])
+@pytest.mark.parametrize("name", ["F32", "F16", "BF16"])
+def test_few_weight_rows_in_tiles_of_many_columns(ex, name, rows, cols):
+    """Three and four activation rows against up to a block per SM of weight rows (2368 of them on 148 SMs): whole tiles of 1024 columns,
+    tiles that end in the middle of a step, one tile alone.  The bits of each row alone."""
+    from llama_rust_b200 import synth
+    ex.set_path(0)
+    m = ex.synth(ALL[name], rows, cols, 15)
+    x = synth.activations(4 * cols, 16).reshape(4, cols)
+    alone = np.concatenate([_product(ex, m, x[t:t + 1]) for t in range(4)])
+    for n in (3, 4):
+        assert _same_bits(_product(ex, m, x[:n]), alone[:n]), n
+    m.free()
+
+
 # tiles of 256 activation rows: whole ones and not, with rows that are and are not stored as vectors
 @pytest.mark.parametrize("rows,cols,tokens", [(16400, 264, 257), (16390, 128, 300), (16384, 192, 489), (16384, 64, 512)])
 def test_wide_tiles_of_bf16_products(ex, rows, cols, tokens):

@@ -487,7 +487,9 @@ cudaError_t launch_matmul(const MatView& m, const float* x, float* y, int64_t to
   if (path == PATH_TC) path = PATH_AUTO;
   if ((path == PATH_AUTO || path == PATH_MMA) && x_aligned && err_flag && gemv_mma_supported(m))
     return launch_gemv_mma(m, x, y, tokens, stream, sm_count, err_flag, launches);
-  if (path == PATH_AUTO && x_aligned && gemv_rows_supported(m))
+  // more than 32 rows of fewer than 128 columns keep less than half of a warp's lanes busy there (32000 x 64, 41 rows:
+  // 131 us, staged 124; 1 x 8, 33 rows: 31 against 21)
+  if (path == PATH_AUTO && x_aligned && gemv_rows_supported(m) && (tokens <= 32 || m.cols >= 128))
     return launch_gemv_rows(m, x, y, tokens, stream, sm_count, launches);
   if (path != PATH_GENERIC && x_aligned && gemv_staged_supported(m))
     return launch_gemv_staged(m, x, y, tokens, stream, sm_count, launches);

@@ -329,13 +329,16 @@ cudaError_t launch_rows_wide(const MatView& m, const float* x, float* y, int tok
   return cudaGetLastError();
 }
 
+// four weight rows per warp, two where they would leave SMs without a block
+bool few_rows(const MatView& m, int sm_count) { return m.rows < (int64_t)sm_count * 2 * ROW_WARPS * 4; }
+
 template <int DT>
 cudaError_t launch_rows_mt(const MatView& m, const float* x, float* y, int tokens, bool runs, cudaStream_t stream, int sm_count) {
-  if (runs) return launch_rows_wide<DT, 8, 4, true>(m, x, y, tokens, stream);
+  const bool few = few_rows(m, sm_count);
+  if (runs) return !few ? launch_rows_wide<DT, 8, 4, true>(m, x, y, tokens, stream)
+                   : tokens <= 8 ? launch_rows_wide<DT, 8, 2, true>(m, x, y, tokens, stream) : launch_rows_wide<DT, 16, 2, true>(m, x, y, tokens, stream);
   if (tokens == 1) return launch_rows<DT, 1>(m, x, y, tokens, stream, sm_count);
   if (tokens == 2) return launch_rows<DT, 2>(m, x, y, tokens, stream, sm_count);
-  // four weight rows per warp, two where they would leave SMs without a block
-  const bool few = m.rows < (int64_t)sm_count * 2 * ROW_WARPS * 4;
   // Up to four activation rows of a matrix that has at most a block per SM: a step of 256 columns is little work, and what a CTA waits
   // for is one trip to memory per tile; tiles of four steps make a quarter of the trips.  From 1024 columns on, where the first
   // tile is full (2048 x 256: 4.2 us with one step, 4.8 with four).  Three rows, weights from HBM, one / four steps a tile, and a
@@ -364,8 +367,11 @@ bool gemv_rows_supported(const MatView& m) {
 
 cudaError_t launch_gemv_rows(const MatView& m, const float* x, float* y, int64_t tokens, cudaStream_t stream, int sm_count,
                              uint64_t* launches) {
-  const bool runs = tokens > 32;
-  const int64_t pass = runs ? 8 : 16;
+  // A matrix of up to 256 columns is one run: the sums of the kernels without runs are the same.  Runs double the accumulators, so a
+  // pass has sixteen rows only where a warp has two weight rows.  33 rows, passes of eight / these / the staged kernel: 2048 x 256
+  // 30.9 / 16.5 / 28.8 us, 1024 x 4096 F32 95 / 59 / 150, 32000 x 256 F32 146 / 105 / 124.
+  const bool runs = tokens > 32 && m.cols > 256;
+  const int64_t pass = runs && !few_rows(m, sm_count) ? 8 : 16;
   for (int64_t t0 = 0; t0 < tokens; t0 += pass) {
     const int nt = (int)(tokens - t0 < pass ? tokens - t0 : pass);
     const float* xp = x + t0 * m.cols;

@@ -46,6 +46,25 @@ def test_rows_of_unpacked_formats_alone_and_in_a_batch(ex, name, rows, cols):
     m.free()
 
 
+@pytest.mark.parametrize("rows,cols", [(5, 128), (200, 256), (9500, 200), (31, 520), (130, 2056), (9500, 264)])
+@pytest.mark.parametrize("name", ["F32", "F16"])
+def test_more_than_32_rows_of_unpacked_formats(ex, name, rows, cols):
+    """Passes of sixteen and of eight rows with remainders of both kinds.  Up to 256 columns a sum is one run and has the bits of the row
+    alone; beyond, it stays within the bound of a sum of `cols` products formed in any order."""
+    from llama_rust_b200 import synth
+    ex.set_path(0)
+    m = ex.synth(ALL[name], rows, cols, 17)
+    x = synth.activations(58 * cols, 18).reshape(58, cols)
+    w = ex.dequant_rows(m).astype(np.float64)
+    exact, size = x.astype(np.float64) @ w.T, np.abs(x).astype(np.float64) @ np.abs(w).T
+    alone = np.concatenate([_product(ex, m, x[t:t + 1]) for t in range(58)]) if cols <= 256 else None
+    for n in (33, 41, 48, 58):
+        y = _product(ex, m, x[:n])
+        assert np.all(np.abs(y - exact[:n]) <= 2.0 ** -24 * (cols + 3) * size[:n]), n
+        assert alone is None or _same_bits(y, alone[:n]), n
+    m.free()
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 1024), (17, 1032), (33, 2048), (7, 2304), (40, 5000), (2368, 1096), (2369, 1096)])
 @pytest.mark.parametrize("name", ["F32", "F16", "BF16"])
 def test_few_weight_rows_in_tiles_of_many_columns(ex, name, rows, cols):

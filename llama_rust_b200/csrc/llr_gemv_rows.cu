@@ -114,8 +114,11 @@ gemv_rows_kernel(const uint8_t* __restrict__ W, int64_t row_bytes, int64_t rows,
 // fma.rn.f32x2 carries two sums.  A sum is formed as above: per lane in ascending columns, then the shuffles; a row's result
 // is the same alone and in a batch.  Bound: the FMA pipe and the shared-memory reads, which four weight rows per warp balance.
 // Measured, 32000 x 2048 BF16: 3 / 8 / 16 rows 62 / 144 / 287 -> 37 / 49 / 92 us; 4096 x 4104 F32, 7 rows 59 -> 25 us.
-// RUNS (batches of more than 32 rows): a lane's sum is closed every 512 columns (256 up to 2048 columns) and added to the row's, which keeps the rounding
-// error below that of the staged kernel, which served such batches at 8 rows per pass (14336 x 4096 F16, 100 rows: 2234 us).
+// RUNS (batches of more than 32 rows): a lane's sum is closed every 512 columns (256 up to RUN_COLS columns) and added to the row's.  The
+// staged kernel, which served such batches at 8 rows per pass (14336 x 4096 F16, 100 rows: 2234 us), rounds as runs of 256 do: relative
+// error 1.01e-7 at 2304 columns, 1.12e-7 at 4096, 1.33e-7 at 8192, 2.1e-7 at 28672.  Runs of 512 have 1.05, 1.11, 1.22, 1.7e-7 on
+// inputs of one size, and up to a tenth more than runs of 256 on inputs of very different sizes until about 6000 columns.
+constexpr int64_t RUN_COLS = 6144;
 __device__ __forceinline__ unsigned long long pack2(float a, float b) {
   unsigned long long v;
   asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
@@ -227,7 +230,7 @@ gemv_rows_wide_kernel(const uint8_t* __restrict__ W, int64_t row_bytes, int64_t 
   static_assert(!RUNS || S == 1, "runs are closed between steps");
   for (int64_t c0 = 0; c0 < cols; c0 += 512 * S) {
     step(c0, 0, raw[0], raw[1]);
-    if (RUNS && cols <= 2048) close_run();
+    if (RUNS && cols <= RUN_COLS) close_run();
     if (c0 + 256 * S < cols) step(c0 + 256 * S, 1, raw[1], raw[0]);
     if (RUNS) close_run();
   }

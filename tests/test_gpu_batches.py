@@ -65,6 +65,27 @@ def test_more_than_32_rows_of_unpacked_formats(ex, name, rows, cols):
     m.free()
 
 
+@pytest.mark.parametrize("cols", [264, 2304, 4096, 6144, 6152, 14336])
+@pytest.mark.parametrize("name", ["F32", "BF16"])
+def test_rounding_of_more_than_32_rows(ex, name, cols):
+    """40 rows, values of one size and of very different sizes: the error against 64-bit sums is no larger than that of the staged
+    kernel (path 2), which took such batches before; two hundredths for the chance of 20000 roundings that fall otherwise."""
+    import torch
+    from llama_rust_b200 import synth
+    m = ex.synth(ALL[name], 500, cols, 19)
+    w = torch.from_numpy(ex.dequant_rows(m)).cuda().double()
+    x = synth.activations(40 * cols, 20).reshape(40, cols)
+    for rows in (x, x * np.exp(3 * synth.activations(40 * cols, 21).reshape(40, cols)).astype(np.float32)):
+        exact = torch.from_numpy(rows).cuda().double() @ w.T
+        err = {}
+        for path in (0, 2):
+            ex.set_path(path)
+            err[path] = float((torch.from_numpy(_product(ex, m, rows)).cuda().double() - exact).norm())
+        assert err[0] <= 1.02 * err[2], err
+    ex.set_path(0)
+    m.free()
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 1024), (17, 1032), (33, 2048), (7, 2304), (40, 5000), (2368, 1096), (2369, 1096)])
 @pytest.mark.parametrize("name", ["F32", "F16", "BF16"])
 def test_few_weight_rows_in_tiles_of_many_columns(ex, name, rows, cols):

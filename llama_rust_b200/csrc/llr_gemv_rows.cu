@@ -1,10 +1,11 @@
-// Decode GEMV (1..8 activation rows) for the element formats F32, F16 and BF16: gemv_f32 / gemv_f16 of
-// langtax/src/quant.rs (:6191, :6144) and their gemm twins for a handful of rows.
+// Products of the element formats F32, F16 and BF16 in f32 arithmetic, any number of activation rows: gemv_f32 / gemv_f16 of
+// langtax/src/quant.rs (:6191, :6144) and their gemm twins.
 //
-// These formats need no unpacking, so the kernel is a plain stream: one warp per weight row, every lane pulls
+// These formats need no unpacking, so one or two activation rows are a plain stream: one warp per weight row, every lane pulls
 // 16-byte pieces of the row straight from HBM with streaming loads (several pieces in flight per lane, no shared
 // memory in between), multiplies them into f32 accumulators against activations that stay in L1, and the warp
-// finishes with shuffles.  Bound: HBM.  Algorithmic bytes per weight: 4 (F32), 2 (F16, BF16).
+// finishes with shuffles.  Bound: HBM.  Algorithmic bytes per weight: 4 (F32), 2 (F16, BF16).  More rows share the weights in passes of
+// eight or sixteen (gemv_rows_wide_kernel).
 // Rows must start 16-byte aligned and hold a multiple of eight columns; other shapes take the shape-agnostic kernel.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -61,7 +62,7 @@ template <int DT> __device__ __forceinline__ void widen8(const Raw8<DT>& r, floa
 }
 
 template <int DT, int MT>
-__global__ void __launch_bounds__(ROW_WARPS * 32, (DT == DT_F32 || MT > 2) ? 2 : 4)
+__global__ void __launch_bounds__(ROW_WARPS * 32, DT == DT_F32 ? 2 : 4)
 gemv_rows_kernel(const uint8_t* __restrict__ W, int64_t row_bytes, int64_t rows, int64_t cols,
                  const float* __restrict__ X, float* __restrict__ Y, int tokens) {
   const int lane = threadIdx.x & 31;
@@ -109,10 +110,10 @@ gemv_rows_kernel(const uint8_t* __restrict__ W, int64_t row_bytes, int64_t rows,
 
 // Three rows of activations and more.  The kernel above reads every activation from L1 once per weight row: with eight of them a
 // warp moves 16 bytes of activations per byte of BF16 weights, and the load path, not HBM, sets the time (32000 x 2048 BF16,
-// eight rows: 158 us for 131 MB).  Here a warp works on R weight rows, the CTA's warps share a tile of the activations in shared
+// eight rows: 144 us for 131 MB).  Here a warp works on R weight rows, the CTA's warps share a tile of the activations in shared
 // memory, and each value read from it serves R rows.  Activations of two rows lie side by side in the tile, so that one
 // fma.rn.f32x2 carries two sums.  A sum is formed as above: per lane in ascending columns, then the shuffles; a row's result
-// is the same alone and in a batch.  Bound: the FMA pipe and the shared-memory reads, which four weight rows per warp balance.
+// is the same alone and in a batch of up to 32 rows.  Bound: the FMA pipe and the shared-memory reads, which four weight rows per warp balance.
 // Measured, 32000 x 2048 BF16: 3 / 8 / 16 rows 62 / 144 / 287 -> 37 / 49 / 92 us; 4096 x 4104 F32, 7 rows 59 -> 25 us.
 // RUNS (batches of more than 32 rows): a lane's sum is closed every 512 columns (256 up to RUN_COLS columns) and added to the row's.  The
 // staged kernel, which served such batches at 8 rows per pass (14336 x 4096 F16, 100 rows: 2234 us), rounds as runs of 256 do: relative

@@ -92,7 +92,7 @@ bool gemv_staged_supported(const MatView& m);
 cudaError_t launch_gemv_staged(const MatView& m, const float* x, float* y, int64_t tokens,
                                cudaStream_t stream, int sm_count, uint64_t* launches);
 
-// Streaming decode GEMV for the element formats F32 / F16 / BF16 (tokens <= 8 per pass); see llr_gemv_rows.cu.
+// Products of the element formats F32 / F16 / BF16 in f32 arithmetic, in passes of up to sixteen rows; see llr_gemv_rows.cu.
 bool gemv_rows_supported(const MatView& m);
 cudaError_t launch_gemv_rows(const MatView& m, const float* x, float* y, int64_t tokens, cudaStream_t stream, int sm_count,
                              uint64_t* launches);
@@ -108,8 +108,10 @@ bool gemv_mma_supported(const MatView& m);
 cudaError_t launch_gemv_mma(const MatView& m, const float* x, float* y, int64_t tokens,
                             cudaStream_t stream, int sm_count, int* err_flag, uint64_t* launches);
 // The same products, bit for bit, for more activation rows and the K-quants: tcgen05 integer MMAs (llr_gemm_i8.cu).  Below
-// I8_MIN_TOKENS a pass of eight rows and a narrower one are as fast (Q4_K 14336 x 4096: 9 rows 30 us against 30, 13 rows 40
-// against 30; 4096 x 4096: 16 against 14, 21 against 14).  scratch: gemm_i8_scratch_bytes of the caller's, used until the
+// I8_MIN_TOKENS a pass of eight rows and a narrower one stay, which are the faster ones where the matrix is tall, and cost no workspace
+// (Q4_K, passes / this, 9, 11 and 13 rows: 32000 x 4096 47 / 57, 55 / 57, 66 / 57 us; 14336 x 4096 30 / 30, 34 / 30, 40 / 30;
+// 4096 x 4096 16 / 13, 19 / 13, 21 / 13; 256 x 2048 8.8 / 8.1, 9.7 / 8.3, 10.9 / 8.2).  From 13 rows on no shape was found that
+// passes serve faster.  scratch: gemm_i8_scratch_bytes of the caller's, used until the
 // launched work has finished.
 constexpr int64_t I8_MIN_TOKENS = 13, I8_MAX_TOKENS = 4096;
 bool gemm_i8_supported(const MatView& m, int64_t tokens);

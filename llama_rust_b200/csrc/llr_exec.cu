@@ -1941,16 +1941,16 @@ cudaError_t session_layers(llr_session* s, const int* ids_dev, size_t n, const R
   return ce;
 }
 
-// One forward pass of sequence 0 over `n` tokens at its device-side position; with_logits: the last token's logits, then
+// One forward pass of sequence 0 over `n` tokens at its device-side position (`first`, where the host knows it); with_logits: the last token's logits, then
 // (generate) argmax into ids[0] and the history, and the position advanced by n.
-cudaError_t session_forward(llr_session* s, const int* ids_dev, size_t n, bool with_logits, bool generate) {
+cudaError_t session_forward(llr_session* s, const int* ids_dev, size_t n, bool with_logits, bool generate, int first = -1) {
   llr_exec* e = s->owner;
   const llr_llama_config& c = s->cfg;
   const size_t E = c.n_embd;
   cudaStream_t st = e->stream;
   uint64_t* L = &e->ctr.launches;
   const float* pending = nullptr;
-  cudaError_t ce = session_layers(s, ids_dev, n, RowMap{s->pos_dev, nullptr, nullptr}, &pending);
+  cudaError_t ce = session_layers(s, ids_dev, n, RowMap{s->pos_dev, nullptr, nullptr, first}, &pending);
   if (ce != cudaSuccess) return ce;
   if (with_logits) {
     // LogitsKind::Last (decode.rs:3058-3079): the last row only
@@ -2271,7 +2271,7 @@ int llr_session_prefill(llr_session* s, const int32_t* tokens, size_t n, float* 
   cudaError_t ce = cudaMemcpyAsync(s->ids + 1, tokens, n * sizeof(int), cudaMemcpyHostToDevice, e->stream);
   for (size_t t0 = 0; t0 < n && ce == cudaSuccess; t0 += s->max_batch) {
     const size_t m = n - t0 < s->max_batch ? n - t0 : s->max_batch;
-    ce = session_forward(s, s->ids + 1 + t0, m, t0 + m == n, false);
+    ce = session_forward(s, s->ids + 1 + t0, m, t0 + m == n, false, (int)(s->position[0] + t0));
   }
   if (ce == cudaSuccess && last_logits)
     ce = cudaMemcpyAsync(last_logits, s->logits, s->cfg.n_vocab * sizeof(float), cudaMemcpyDeviceToHost, e->stream);

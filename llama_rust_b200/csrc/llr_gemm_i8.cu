@@ -239,7 +239,6 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap wmap, const Args P, int* __re
   const int row0 = (int)blockIdx.x * BM, tok0 = (int)blockIdx.y * TB;
   const int units = units_of(P.blocks), u_begin = (int)((int64_t)units * blockIdx.z / gridDim.z), u_end = (int)((int64_t)units * (blockIdx.z + 1) / gridDim.z);
 
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (tid == 0) {
     for (int s = 0; s < NA; ++s) { bar_init(&full_a[s], 8); bar_init(&empty_a[s], 2); }
     for (int s = 0; s < NB; ++s) { bar_init(&full_b[s], 1); bar_init(&empty_b[s], 2); }
@@ -257,6 +256,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap wmap, const Args P, int* __re
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  // only now: a dependent that is placed here finds its tensor memory after this block has its own, and does not wait with it for this grid
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   bool ok = true;
   auto wait = [&](uint64_t* bar, int n, int ring) {  // n-th use of a ring: its stage n % ring
     if (ok && !bar_wait(bar + n % ring, (uint32_t)((n / ring) & 1))) { ok = false; report_error(err, 3); }

@@ -444,7 +444,7 @@ __device__ __forceinline__ void dequant_sub_h(uint32_t prow, uint32_t (&out)[16]
 template <int DT, int BN, bool F16>
 __device__ __forceinline__ void gemm_tc_tile(const CUtensorMap* wmap_p, const CUtensorMap* xmap_p, int rows, int ms_begin,
                                              int ms_count, int tokens, const float* xscale,
-                                             float* __restrict__ Y, int row_tile, int tok_tile, int* __restrict__ err) {
+                                             float* __restrict__ Y, int row_tile, int tok_tile, bool dependents, int* __restrict__ err) {
   using L = GLay<DT, BN>;
   constexpr int NA = L::NA, NB = L::NB, NPK = L::NPK, NMMA = L::NMMA, PITCH = Pk<DT>::PITCH, RB = Pk<DT>::RB;
   extern __shared__ uint8_t smem_raw[];
@@ -478,6 +478,8 @@ __device__ __forceinline__ void gemm_tc_tile(const CUtensorMap* wmap_p, const CU
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  // only now: a dependent that is placed here finds its tensor memory after this block has its own, and does not wait with it for this grid
+  if (dependents) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   bool ok = true;
 
   if (warp < DQ_WARPS) {
@@ -689,12 +691,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, int rows, int cols, int tokens,
                const __grid_constant__ CUtensorMap xmap, const float* xscale, float* __restrict__ Y,
                int* __restrict__ err) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // split-K: gridDim.z CTAs share a tile's K range; slice z writes its partial sums to Y + z * tokens * rows
   // (with one slice Y is the result itself), and a second kernel adds the slices in order
   const int per = cols / MACRO / (int)gridDim.z;
   gemm_tc_tile<DT, BN, F16>(&wmap, &xmap, rows, (int)blockIdx.z * per, per, tokens, xscale,
-                            Y + (size_t)blockIdx.z * (size_t)tokens * (size_t)rows, (int)blockIdx.x, (int)blockIdx.y, err);
+                            Y + (size_t)blockIdx.z * (size_t)tokens * (size_t)rows, (int)blockIdx.x, (int)blockIdx.y, true, err);
 }
 
 __global__ void add_slices_kernel(const float* part, float* __restrict__ y, int64_t n, int slices) {
@@ -721,7 +722,7 @@ gemm_tc_grouped_kernel(const GemmGroup* __restrict__ groups, int n_groups, int* 
   const GemmGroup* G = groups + g;
   const int local = tile - G->tile_begin, row_tiles = (G->rows + BM - 1) / BM;
   gemm_tc_tile<DT, BN, F16>(&G->wmap, &G->xmap, G->rows, 0, G->cols / MACRO, G->tokens, G->xscale, G->y, local % row_tiles,
-                            local / row_tiles, err);
+                            local / row_tiles, false, err);
 }
 
 __global__ void to_bf16_kernel(const float* x, __nv_bfloat16* __restrict__ o, int64_t n) {

@@ -323,6 +323,7 @@ struct RowMap {
   const int* pos_dev;
   const int* row_pos;
   const int* row_seq;
+  int first = -1;  // position of row 0 where all rows are one run and the host knows it (it sizes launches)
 };
 // RoPE (adjacent pairs) on q and k at each row's position, then k and v into the cache.
 cudaError_t launch_rope_store(float* q, float* k, const float* v, const KvView& kv, const RowMap& rows, int tokens, int layer,
@@ -474,7 +475,14 @@ bool span_supported(const SpanShape& sh);
 // scratch holds their gathered keys; the rows of shorter groups share a launch of the f32 kernels.
 struct SpanGroup { int t0, rows, first; };
 cudaError_t launch_span_attention(const float* q, int64_t q_ld, const SpanShape& sh, const LayerKv& kv, const RowMap& rows, const SpanGroup* groups, int n_groups,
-                                  const SpanOut& out, float* scratch, size_t scratch_floats, bool tensor_cores, const NewToken* nt, cudaStream_t s, uint64_t* launches);
+                                  const SpanOut& out, float* scratch, size_t scratch_floats, bool tensor_cores, const NewToken* nt, cudaStream_t s, int* err, uint64_t* launches);
+// The groups of at least min_rows rows on tcgen05 (llr_attend_umma.cu), where span_umma_supported: a gather of their keys and values into
+// the scratch, then the attention; all groups in one launch of each as far as the scratch holds their keys.
+bool span_umma_supported(const SpanShape& sh, bool shared, const SpanOut& out);
+size_t span_umma_scratch_floats(const SpanShape& sh, int max_rows);
+int span_group_keys(const SpanShape& sh, int rows);  // most keys a group of consecutive rows sees
+cudaError_t launch_span_umma(const float* q, int64_t q_ld, const SpanShape& sh, const LayerKv& kv, const RowMap& rows, const SpanGroup* groups, int n_groups,
+                             int min_rows, const SpanOut& out, float* scratch, size_t scratch_floats, cudaStream_t s, int* err, uint64_t* launches);
 // x[t] += y[t] / rms(y[t]) * w, y given as `slices` partial sums `slice_stride` floats apart; x16 (may be null): the new x
 cudaError_t launch_norm_add(float* x, const float* y, int slices, int64_t slice_stride, const float* w, float eps, void* x16, int tokens, int n,
                             cudaStream_t s, uint64_t* launches);

@@ -220,13 +220,13 @@ struct LayeredPass {
     nt.k_norm = latent ? M.kv_norm : M.k_norm;
     nt.rot = rotation(M);
     if (!rows.row_seq) {
-      const SpanGroup all{0, N, -1};
-      ce = launch_span_attention(q, q_ld, M.span, kv, rows, &all, 1, so, D.scratch, D.scratch_floats, tc, &nt, st, lc);
+      const SpanGroup all{0, N, rows.first};
+      ce = launch_span_attention(q, q_ld, M.span, kv, rows, &all, 1, so, D.scratch, D.scratch_floats, tc, &nt, st, e->err_flag, lc);
     } else {
       std::vector<SpanGroup> ragged;
       for (size_t g = 0; g < s->batch_groups.size(); ++g)
         ragged.push_back(SpanGroup{(int)s->batch_groups[g].first, (int)s->batch_groups[g].second, (int)s->batch_first[g]});
-      ce = launch_span_attention(q, q_ld, M.span, kv, rows, ragged.data(), (int)ragged.size(), so, D.scratch, D.scratch_floats, tc, &nt, st, lc);
+      ce = launch_span_attention(q, q_ld, M.span, kv, rows, ragged.data(), (int)ragged.size(), so, D.scratch, D.scratch_floats, tc, &nt, st, e->err_flag, lc);
     }
     if (ce != cudaSuccess || !latent) return ce;
     // results out of the latent space, times the head gate

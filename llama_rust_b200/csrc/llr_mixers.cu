@@ -458,343 +458,6 @@ span_combine_kernel(const float* part, SpanShape sh, RowMap rows, const __grid_c
   }
 }
 
-// ---- prompt chunks on the tensor cores ------------------------------------------------------------------------------
-// Rows of ONE sequence at consecutive positions.  The keys and values that any of the rows sees are first gathered from
-// their pages into contiguous binary16 rows (span_gather_kernel), so that the attention kernel copies tiles with 16-byte
-// asynchronous copies and neither looks pages up nor converts.
-// A block takes one kv head and 64 (row, query head) pairs in row-major order -- all query heads of a kv head share its
-// keys, so any ratio of heads fills the tile (one latent for every head included) -- and walks the keys that any of its
-// rows sees, 64 at a time.  Queries (rescaled per pair by a power of two), keys, values and the exponentials are
-// binary16 operands; scores and sums are m16n8k16 MMAs with f32 accumulators; scale, distance bias, mask, maxima,
-// exponentials and their sums are f32.
-// Sixteen pairs belong to NS warps: each scores 64 / NS of the keys and owns 8 ND of the value dimensions.
-// The copies run one tile ahead of their use: values arrive while their keys are scored, the next keys while the values
-// are added up; where keys and values are one latent there are two buffers instead.
-constexpr int CH = 64;
-__device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
-  const __half2 h = __floats2half2_rn(lo, hi);
-  return *(const uint32_t*)&h;
-}
-__device__ __forceinline__ float sat16(float v) { return fminf(fmaxf(v, -65504.f), 65504.f); }
-__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void ldm4(uint32_t (&r)[4], const __half* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
-}
-__device__ __forceinline__ void ldm4_t(uint32_t (&r)[4], const __half* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
-}
-__device__ __forceinline__ void copy16(const __half* dst, const __half* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// Widths of the gathered rows and of the tiles, in halves; multiples of 16, so that a tile's pitch (width + 8) is an odd
-// number of 16-byte units.  Where values are the keys there is one row of the wider of the two.
-struct MmaLayout {
-  int kw, vw, kr, vr;  // score columns, value columns, gathered key row, gathered value row (0: the keys)
-  bool shared;
-  int qp, kp, vp;
-};
-inline __host__ __device__ MmaLayout mma_layout(int dk, int dv, int nd, int ns, bool shared) {
-  MmaLayout L;
-  L.kw = (dk + 15) / 16 * 16;
-  L.vw = 8 * nd * ns;
-  L.shared = shared;
-  L.kr = shared && L.vw > L.kw ? L.vw : L.kw;
-  L.vr = shared ? 0 : L.vw;
-  L.qp = L.kw + 8;
-  L.kp = L.kr + 8;
-  L.vp = shared ? L.kp : L.vw + 8;
-  return L;
-}
-inline __host__ __device__ size_t mma_smem(const MmaLayout& L, int ns) {
-  return ((size_t)64 * L.qp + (size_t)CH * L.kp * (L.shared ? 2 : 1) + (L.shared ? 0 : (size_t)CH * L.vp) + (ns > 1 ? 64 * (CH + 8) : 0)) * 2;
-}
-
-// The list of keys a group of rows sees: kept tokens before the first row's window, then every position from there to the
-// last row.  Row m of the gathered keys of kv head g starts at k16 + ((int64_t)g * n + m) * kr.
-struct GroupKeys {
-  int lo, nk, n;
-  __device__ __forceinline__ int at(int m) const { return m < nk ? m : lo + m - nk; }
-  __device__ __forceinline__ int index(int j) const { return j < nk ? j : j - lo + nk; }  // of a position in the list
-};
-__device__ __forceinline__ GroupKeys group_keys(int first, int rows, int window, int keep_first) {
-  const int lo = window > 0 ? max(0, first - window + 1) : 0, nk = min(keep_first, lo);
-  return GroupKeys{lo, nk, nk + first + rows - lo};
-}
-
-// The groups of one launch: group i has the rows [t0, t0 + rows), blocks [keys_at[i], keys_at[i + 1]) of the gather and
-// [tiles_at[i], tiles_at[i + 1]) of the attention, and its gathered rows k_off / v_off halves into the scratch.  A group alone
-// fills a few SMs (a prompt of 24 rows: eight blocks), and a ragged batch has dozens: with a launch each, 24 groups of 30 rows
-// took 16 x (5 + 30) us per layer one after the other.
-constexpr int SPAN_GROUPS = 64;
-struct SpanBatch {
-  int n;
-  int t0[SPAN_GROUPS], rows[SPAN_GROUPS], keys_at[SPAN_GROUPS + 1], tiles_at[SPAN_GROUPS + 1];
-  int64_t k_off[SPAN_GROUPS], v_off[SPAN_GROUPS];
-};
-__device__ __forceinline__ int span_group(const int* at, int n, int block) {
-  int i = 0;
-  while (i + 1 < n && block >= at[i + 1]) ++i;
-  return i;
-}
-
-// one warp per key row: grid (keys / 8 of all groups, kv head)
-__global__ void __launch_bounds__(256)
-span_gather_kernel(SpanShape sh, LayerKv kv, RowMap rows, const __grid_constant__ SpanBatch b, int kr, int vr, __half* __restrict__ scratch) {
-  pdl_enter();
-  const int gi = span_group(b.keys_at, b.n, blockIdx.x), t0 = b.t0[gi];
-  const GroupKeys gk = group_keys(row_position(rows, t0), b.rows[gi], sh.window, sh.keep_first);
-  const int m = (blockIdx.x - b.keys_at[gi]) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, head = blockIdx.y, seq = row_sequence(rows, t0);
-  if (m >= gk.n) return;
-  __half *k16 = scratch + b.k_off[gi], *v16 = scratch + b.v_off[gi];
-  auto put = [&](const float* src, int d, __half* dst, int w) {
-    for (int i = 4 * lane; i < w; i += 128) {
-      const float4 v = i < d ? *(const float4*)(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);  // d is a multiple of four
-      *(uint2*)(dst + i) = make_uint2(pack_h2(sat16(v.x), sat16(v.y)), pack_h2(sat16(v.z), sat16(v.w)));
-    }
-  };
-  const int j = gk.at(m);
-  put(kv.k + slot_of(kv, seq, j, kv.k_block, head, sh.dk), sh.dk, k16 + ((int64_t)head * gk.n + m) * kr, kr);
-  if (vr) put(kv.v + slot_of(kv, seq, j, kv.v_block, head, sh.dv), sh.dv, v16 + ((int64_t)head * gk.n + m) * vr, vr);
-}
-
-template <int ND, int NS>
-__global__ void __launch_bounds__(128 * NS)
-span_mma_kernel(const float* q, int64_t q_ld, SpanShape sh, const __half* scratch, bool shared_kv, RowMap rows,
-                const __grid_constant__ SpanBatch b, SpanOut so) {
-  pdl_enter();
-  const int gi = span_group(b.tiles_at, b.n, blockIdx.x), t0 = b.t0[gi], tokens = b.rows[gi];
-  const __half *k16 = scratch + b.k_off[gi], *v16 = scratch + b.v_off[gi];
-  constexpr int THR = 128 * NS, NT = CH / 8 / NS;  // score tiles of eight keys per warp
-  static_assert(NT % 2 == 0, "keys are loaded sixteen at a time");
-  extern __shared__ __align__(16) unsigned char raw[];
-  const MmaLayout L = mma_layout(sh.dk, sh.dv, ND, NS, shared_kv);
-  __half* sq = (__half*)raw;
-  __half* sk = sq + 64 * L.qp;                                         // keys (two buffers where they are the values)
-  __half* sv = sk + CH * L.kp;                                         // values, or the second buffer
-  __half* sp = sv + CH * L.vp;                                         // exponentials, NS > 1
-  __shared__ float s_scale[64], s_red[NS][64];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
-  const int rw = warp & 3, ns = warp >> 2;  // rows 16 rw .., key and value share ns
-  // the last rows first: in a window that is still filling they see the most keys
-  const int head = blockIdx.y, gq = sh.n_head / sh.n_kv, pairs = tokens * gq, pair0 = (b.tiles_at[gi + 1] - 1 - (int)blockIdx.x) * 64;
-  const int p_first = row_position(rows, t0);
-  const GroupKeys gk = group_keys(p_first, tokens, sh.window, sh.keep_first);
-  const int pa = p_first + pair0 / gq, pb = p_first + min(pairs - 1, pair0 + 63) / gq;  // positions of the tile's rows
-  const int lo = sh.window > 0 ? max(0, pa - sh.window + 1) : 0, nk = min(sh.keep_first, lo), n_keys = nk + pb - lo + 1;
-  k16 += (int64_t)head * gk.n * L.kr;
-  v16 += (int64_t)head * gk.n * L.vr;
-
-  // rows c * CH .. of the tile's own list; rows behind its end repeat the last one (their exponentials are zero)
-  auto stage = [&](__half* dst, const __half* src, int width, int pitch, int c) {
-    for (int p = tid >> 4; p < CH; p += THR / 16) {
-      const int m = min(c * CH + p, n_keys - 1);
-      const __half* row = src + (int64_t)gk.index(m < nk ? m : lo + m - nk) * width;
-      for (int d = 8 * (tid & 15); d < width; d += 128) copy16(dst + p * pitch + d, row + d);
-    }
-  };
-  stage(sk, k16, L.kr, L.kp, 0);
-  copy_commit();
-  // queries: a warp per pair; the power of two that brings the largest magnitude into [2^9, 2^10)
-  for (int r = warp; r < 64; r += 4 * NS) {
-    const int p = pair0 + r;
-    const bool live = p < pairs;
-    const float* src = q + (int64_t)(t0 + (live ? p / gq : 0)) * q_ld + (int64_t)(head * gq + (live ? p % gq : 0)) * sh.dk;
-    float m = 0.f;
-    if (live) for (int i = lane; i < sh.dk; i += 32) m = fmaxf(m, fabsf(src[i]));
-    m = warp_max(m);
-    const int be = (int)((__float_as_uint(m) >> 23) & 0xff);
-    const int e = (be == 0 || be == 255) ? 0 : min(126, max(-126, 136 - be));
-    const float up = __uint_as_float((uint32_t)(127 + e) << 23), down = __uint_as_float((uint32_t)(127 - e) << 23);
-    for (int i = lane; i < L.kw; i += 32) sq[r * L.qp + i] = __float2half_rn(live && i < sh.dk ? sat16(src[i] * up) : 0.f);
-    if (lane == 0) s_scale[r] = down * sh.scale;
-  }
-  __syncthreads();
-
-  constexpr float LOG2E = 1.4426950408889634f;  // scores are kept in units of ln 2: exp(x) = exp2(x log2 e)
-  const int r0 = 16 * rw + g, r1 = r0 + 8;
-  const int i0 = p_first + min(pair0 + r0, pairs - 1) / gq, i1 = p_first + min(pair0 + r1, pairs - 1) / gq;  // positions of this thread's rows
-  const int i_lo = p_first + min(pair0 + 16 * rw, pairs - 1) / gq, i_hi = p_first + min(pair0 + 16 * rw + 15, pairs - 1) / gq;  // of this warp's
-  const float* b0 = sh.bias ? sh.bias + (int64_t)(head * gq + min(pair0 + r0, pairs - 1) % gq) * sh.bias_len : nullptr;
-  const float* b1 = sh.bias ? sh.bias + (int64_t)(head * gq + min(pair0 + r1, pairs - 1) % gq) * sh.bias_len : nullptr;
-  const float far0 = b0 ? b0[sh.bias_len - 1] * LOG2E : 0.f, far1 = b1 ? b1[sh.bias_len - 1] * LOG2E : 0.f;
-  const float f0 = s_scale[r0] * LOG2E, f1 = s_scale[r1] * LOG2E;
-  float m0 = -CUDART_INF_F, m1 = -CUDART_INF_F, l0 = 0.f, l1 = 0.f;
-  if (sh.sink) {  // the sink is the first score: the maximum starts there, and one thread of a row's counts it
-    m0 = sh.sink[head * gq + min(pair0 + r0, pairs - 1) % gq] * LOG2E;
-    m1 = sh.sink[head * gq + min(pair0 + r1, pairs - 1) % gq] * LOG2E;
-    l0 = l1 = t4 == 0 && ns == 0 ? 1.f : 0.f;
-  }
-  float o[ND][4];
-#pragma unroll
-  for (int nd = 0; nd < ND; ++nd)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) o[nd][i] = 0.f;
-
-  auto row_group = [&] {  // the NS warps of sixteen pairs
-    if constexpr (NS == 1) __syncwarp();
-    else asm volatile("bar.sync %0, %1;" ::"r"(1 + rw), "r"(32 * NS) : "memory");
-  };
-  const int chunks = (n_keys + CH - 1) / CH;
-  for (int c = 0; c < chunks; ++c) {
-    __half* kt = L.shared && (c & 1) ? sv : sk;
-    __half* vt = L.shared ? kt : sv;
-    if (L.shared) {
-      if (c + 1 < chunks) { stage((c & 1) ? sk : sv, k16, L.kr, L.kp, c + 1); copy_commit(); copy_wait<1>(); }
-      else copy_wait<0>();
-    } else {
-      stage(sv, v16, L.vr, L.vp, c);
-      copy_commit();
-      copy_wait<1>();  // the keys
-    }
-    __syncthreads();
-    // ---- scores of this warp's keys
-    float s[NT][4];
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) s[nt][i] = 0.f;
-    const __half* qa = sq + (16 * rw + (lane & 15)) * L.qp + (lane >> 4) * 8;
-    const __half* kb = kt + (ns * 8 * NT + (lane & 7) + (lane >> 4) * 8) * L.kp + ((lane >> 3) & 1) * 8;
-#pragma unroll 2
-    for (int k0 = 0; k0 < L.kw; k0 += 16) {
-      uint32_t a[4];
-      ldm4(a, qa + k0);
-#pragma unroll
-      for (int nt = 0; nt < NT; nt += 2) {
-        uint32_t b[4];
-        ldm4(b, kb + nt * 8 * L.kp + k0);
-        mma_f16(s[nt], a, b[0], b[1]);
-        mma_f16(s[nt + 1], a, b[2], b[3]);
-      }
-    }
-    // this warp's keys of the chunk: positions between j_lo and j_hi (ascending list)
-    const int k_lo = c * CH + ns * 8 * NT, k_hi = k_lo + 8 * NT - 1;
-    const int j_lo = k_lo < nk ? k_lo : lo + k_lo - nk, j_hi = k_hi < nk ? k_hi : lo + k_hi - nk;
-    const bool all_seen = k_hi < n_keys && j_hi <= i_lo && (sh.window <= 0 || i_hi - j_lo < sh.window || j_hi < sh.keep_first);
-    const bool all_far = i_lo - j_hi >= sh.bias_len - 1;
-    float x0 = -CUDART_INF_F, x1 = -CUDART_INF_F;
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int m = k_lo + 8 * nt + 2 * t4 + i, j = m < nk ? m : lo + m - nk;
-        float u0 = fmaf(s[nt][i], f0, far0), u1 = fmaf(s[nt][2 + i], f1, far1);
-        if (!all_far || !all_seen) {  // warp-uniform
-          const int d0 = i0 - j, d1 = i1 - j;
-          if (b0 && !all_far) {
-            u0 = fmaf(s[nt][i], f0, __ldg(b0 + min(max(d0, 0), sh.bias_len - 1)) * LOG2E);
-            u1 = fmaf(s[nt][2 + i], f1, __ldg(b1 + min(max(d1, 0), sh.bias_len - 1)) * LOG2E);
-          }
-          const bool any = m < n_keys, kept = j < sh.keep_first || sh.window <= 0;
-          if (!(any && d0 >= 0 && (kept || d0 < sh.window))) u0 = -CUDART_INF_F;
-          if (!(any && d1 >= 0 && (kept || d1 < sh.window))) u1 = -CUDART_INF_F;
-        }
-        s[nt][i] = u0;
-        s[nt][2 + i] = u1;
-        x0 = fmaxf(x0, u0);
-        x1 = fmaxf(x1, u1);
-      }
-    x0 = fmaxf(x0, __shfl_xor_sync(~0u, x0, 1)); x0 = fmaxf(x0, __shfl_xor_sync(~0u, x0, 2));
-    x1 = fmaxf(x1, __shfl_xor_sync(~0u, x1, 1)); x1 = fmaxf(x1, __shfl_xor_sync(~0u, x1, 2));
-    if constexpr (NS > 1) {
-      if (t4 == 0) { s_red[ns][r0] = x0; s_red[ns][r1] = x1; }
-      row_group();
-#pragma unroll
-      for (int k = 0; k < NS; ++k) { x0 = fmaxf(x0, s_red[k][r0]); x1 = fmaxf(x1, s_red[k][r1]); }
-    }
-    x0 = fmaxf(x0, m0);
-    x1 = fmaxf(x1, m1);
-    const float w0 = m0 == -CUDART_INF_F ? 0.f : exp2f(m0 - x0), w1 = m1 == -CUDART_INF_F ? 0.f : exp2f(m1 - x1);
-    m0 = x0;
-    m1 = x1;
-    // a row that has seen nothing yet: every score is -inf and so is the maximum; its exponentials are zero
-    const float c0 = m0 == -CUDART_INF_F ? 0.f : m0, c1 = m1 == -CUDART_INF_F ? 0.f : m1;
-    l0 *= w0;
-    l1 *= w1;
-#pragma unroll
-    for (int nd = 0; nd < ND; ++nd) { o[nd][0] *= w0; o[nd][1] *= w0; o[nd][2] *= w1; o[nd][3] *= w1; }
-    uint32_t e0[NT], e1[NT];
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      e0[nt] = pack_h2(exp2f(s[nt][0] - c0), exp2f(s[nt][1] - c0));
-      e1[nt] = pack_h2(exp2f(s[nt][2] - c1), exp2f(s[nt][3] - c1));
-      const __half2 h0 = *(const __half2*)&e0[nt], h1 = *(const __half2*)&e1[nt];
-      l0 += __low2float(h0) + __high2float(h0);  // the sum of what the weighted sum below uses
-      l1 += __low2float(h1) + __high2float(h1);
-      if constexpr (NS > 1) {
-        *(uint32_t*)(sp + r0 * (CH + 8) + ns * 8 * NT + 8 * nt + 2 * t4) = e0[nt];
-        *(uint32_t*)(sp + r1 * (CH + 8) + ns * 8 * NT + 8 * nt + 2 * t4) = e1[nt];
-      }
-    }
-    if constexpr (NS > 1) row_group();
-    if (!L.shared) {
-      copy_wait<0>();   // the values
-      __syncthreads();  // everyone's, and every warp is done with the keys
-      if (c + 1 < chunks) { stage(sk, k16, L.kr, L.kp, c + 1); copy_commit(); }
-    }
-    // ---- weighted values: this warp's dimensions over all keys of the chunk
-    const __half* vb = vt + (lane & 15) * L.vp + ns * 8 * ND + (lane >> 4) * 8;
-#pragma unroll
-    for (int k0 = 0; k0 < CH; k0 += 16) {
-      uint32_t a[4];
-      if constexpr (NS == 1) {
-        a[0] = e0[k0 / 8]; a[1] = e1[k0 / 8]; a[2] = e0[k0 / 8 + 1]; a[3] = e1[k0 / 8 + 1];
-      } else {
-        ldm4(a, sp + (16 * rw + (lane & 15)) * (CH + 8) + k0 + (lane >> 4) * 8);
-      }
-#pragma unroll
-      for (int nd = 0; nd < ND; nd += 2) {
-        uint32_t b[4];
-        ldm4_t(b, vb + k0 * L.vp + 8 * nd);
-        mma_f16(o[nd], a, b[0], b[1]);
-        mma_f16(o[nd + 1], a, b[2], b[3]);
-      }
-    }
-    __syncthreads();  // the next copies overwrite the values
-  }
-  l0 += __shfl_xor_sync(~0u, l0, 1); l0 += __shfl_xor_sync(~0u, l0, 2);
-  l1 += __shfl_xor_sync(~0u, l1, 1); l1 += __shfl_xor_sync(~0u, l1, 2);
-  if constexpr (NS > 1) {
-    if (t4 == 0) { s_red[ns][r0] = l0; s_red[ns][r1] = l1; }
-    row_group();
-    l0 = l1 = 0.f;
-#pragma unroll
-    for (int k = 0; k < NS; ++k) { l0 += s_red[k][r0]; l1 += s_red[k][r1]; }
-  }
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const int p = pair0 + (half ? r1 : r0);
-    if (p >= pairs) continue;
-    const int t = t0 + p / gq, h = head * gq + p % gq;
-    float inv = __fdiv_rn(1.0f, half ? l1 : l0) * so.scale;
-    if (so.gate && so.head_gate) inv *= sigmoid(so.gate[(int64_t)t * so.gate_ld + h]);
-    const int64_t base = (int64_t)h * sh.dv;
-#pragma unroll
-    for (int nd = 0; nd < ND; ++nd) {
-      const int d = ns * 8 * ND + 8 * nd + 2 * t4;
-      if (d >= sh.dv) continue;
-      float2 v = make_float2(o[nd][2 * half] * inv, o[nd][2 * half + 1] * inv);
-      if (so.gate && !so.head_gate) {
-        const float2 gg = *(const float2*)(so.gate + (int64_t)t * so.gate_ld + base + d);
-        v.x *= sigmoid(gg.x);
-        v.y *= sigmoid(gg.y);
-      }
-      const int64_t at = (int64_t)t * so.ld + base + d;
-      if (so.out) *(float2*)(so.out + at) = v;
-      if (so.out16) *(__nv_bfloat162*)((__nv_bfloat16*)so.out16 + at) = __floats2bfloat162_rn(v.x, v.y);
-    }
-  }
-}
-
 // ---- norm on a sublayer's output, residual add ------------------------------------------------------------------------
 constexpr int NORM_ADD_THREADS = 512, NORM_ADD_KEEP = 4;  // up to 8192 values of a row stay in registers
 __global__ void __launch_bounds__(NORM_ADD_THREADS)
@@ -948,26 +611,6 @@ size_t span_smem(const SpanShape& sh) {
 constexpr size_t SCRATCH_FLOATS = 16u << 20;
 int span_rows_per_pass(const SpanShape& sh) { return (int)std::min<size_t>(512, std::max<size_t>(1, SCRATCH_FLOATS / span_row_floats(sh))); }
 
-// most keys a group of consecutive rows sees
-int span_group_keys(const SpanShape& sh, int rows) {
-  return sh.window > 0 ? (int)std::min<int64_t>(sh.n_ctx, (int64_t)sh.window + sh.keep_first + rows) : sh.n_ctx;
-}
-int group_key_count(const SpanShape& sh, const SpanGroup& g) {
-  if (g.first < 0) return span_group_keys(sh, g.rows);
-  const int lo = sh.window > 0 ? std::max(0, g.first - sh.window + 1) : 0;  // as group_keys
-  return std::min(sh.keep_first, lo) + g.first + g.rows - lo;
-}
-constexpr size_t MMA_SMEM_LIMIT = 222 * 1024;
-
-typedef void (*MmaKernel)(const float*, int64_t, SpanShape, const __half*, bool, RowMap, const SpanBatch, SpanOut);
-// the smallest instantiation that covers the value dimensions
-MmaKernel mma_kernel(int dv, int* nd, int* ns) {
-#define LLR_SPAN(N, S) if (dv <= 8 * N * S) { *nd = N; *ns = S; return span_mma_kernel<N, S>; }
-  LLR_SPAN(4, 1) LLR_SPAN(8, 1) LLR_SPAN(12, 1) LLR_SPAN(16, 1) LLR_SPAN(12, 2) LLR_SPAN(16, 2) LLR_SPAN(12, 4) LLR_SPAN(16, 4)
-#undef LLR_SPAN
-  return nullptr;
-}
-
 }  // namespace
 
 cudaError_t launch_embed(const void* table, const void* pos_table, const int* ids, const RowMap& rows, float scale, float* x, void* x16,
@@ -1037,36 +680,14 @@ bool span_supported(const SpanShape& sh) {
          span_smem(sh) <= 200 * 1024;
 }
 size_t span_scratch_floats(const SpanShape& sh, int max_rows) {
-  int nd = 0, ns = 0;
-  size_t gathered = 0;  // binary16 keys and values of one group
-  if (mma_kernel(sh.dv, &nd, &ns)) {
-    const MmaLayout L = mma_layout(sh.dk, sh.dv, nd, ns, false);  // not shared: the larger of the two
-    gathered = (size_t)sh.n_kv * span_group_keys(sh, max_rows) * (L.kr + L.vr) / 2 + 64;
-  }
-  return std::max((size_t)span_rows_per_pass(sh) * span_row_floats(sh), gathered);
+  return std::max((size_t)span_rows_per_pass(sh) * span_row_floats(sh), span_umma_scratch_floats(sh, max_rows));
 }
 
 cudaError_t launch_span_attention(const float* q, int64_t q_ld, const SpanShape& sh, const LayerKv& kv, const RowMap& rows, const SpanGroup* groups, int n_groups,
-                                  const SpanOut& out, float* scratch, size_t scratch_floats, bool tensor_cores, const NewToken* nt, cudaStream_t s, uint64_t* launches) {
+                                  const SpanOut& out, float* scratch, size_t scratch_floats, bool tensor_cores, const NewToken* nt, cudaStream_t s, int* err, uint64_t* launches) {
   if (!span_supported(sh)) return cudaErrorInvalidValue;
   const int gq = sh.n_head / sh.n_kv;
-  int nd = 0, ns = 0;
-  const bool shared = kv.k == kv.v;
-  MmaKernel mma = nullptr;
-  if (tensor_cores && sh.dk % 8 == 0 && sh.dv % 8 == 0 && out.ld % 2 == 0 && ((uintptr_t)out.out & 7) == 0 && ((uintptr_t)out.out16 & 3) == 0 &&
-      (!out.gate || out.head_gate || (out.gate_ld % 2 == 0 && ((uintptr_t)out.gate & 7) == 0)))
-    mma = mma_kernel(sh.dv, &nd, &ns);
-  MmaLayout L{};
-  size_t mma_bytes = 0;
-  if (mma) {
-    L = mma_layout(sh.dk, sh.dv, nd, ns, shared);
-    mma_bytes = mma_smem(L, ns);
-    if (mma_bytes > MMA_SMEM_LIMIT) mma = nullptr;
-  }
-  if (mma && mma_bytes > 40 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute((const void*)mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mma_bytes);
-    if (e != cudaSuccess) return e;
-  }
+  const bool mma = tensor_cores && span_umma_supported(sh, kv.k == kv.v, out);
   const int head_groups = (gq + span_heads(sh) - 1) / span_heads(sh), chunk = span_chunk(sh), splits = span_splits(sh), per = span_rows_per_pass(sh);
   const size_t smem = span_smem(sh);
   const int most = std::min(gq, span_heads(sh));  // query heads of a block
@@ -1074,18 +695,6 @@ cudaError_t launch_span_attention(const float* q, int64_t q_ld, const SpanShape&
   auto kern = most <= 2 ? LLR_SPAN(2) : most <= 4 ? LLR_SPAN(4) : LLR_SPAN(8);
 #undef LLR_SPAN
 
-  // groups that are long enough for the tensor cores, as many per launch as the scratch holds the gathered keys of
-  SpanBatch b{};
-  size_t used = 0;  // halves of the scratch
-  auto run_batch = [&] {
-    if (b.n == 0) return cudaSuccess;
-    if (launches) *launches += 2;
-    cudaError_t e = launch_walk(span_gather_kernel, dim3(b.keys_at[b.n], sh.n_kv), dim3(256), 0, s, sh, kv, rows, b, L.kr, L.vr, (__half*)scratch);
-    if (e == cudaSuccess) e = launch_walk(mma, dim3(b.tiles_at[b.n], sh.n_kv), dim3(128 * ns), mma_bytes, s, q, q_ld, sh, (const __half*)scratch, shared, rows, b, out);
-    b.n = 0;
-    used = 0;
-    return e;
-  };
   // the rows of the others, as many runs and rows per launch as the lists and the scratch hold
   SpanRuns runs{};
   bool configured = smem <= 48 * 1024;
@@ -1104,21 +713,7 @@ cudaError_t launch_span_attention(const float* q, int64_t q_ld, const SpanShape&
     return e;
   };
   cudaError_t e = cudaSuccess;
-  for (int g = 0; g < n_groups && e == cudaSuccess; ++g) {
-    if (!mma || groups[g].rows < BF16_TC_MIN_TOKENS) continue;
-    const int keys = group_key_count(sh, groups[g]);
-    const size_t need = (size_t)sh.n_kv * keys * (L.kr + L.vr);
-    if (b.n == SPAN_GROUPS || (b.n > 0 && used + need > 2 * scratch_floats)) e = run_batch();
-    const int i = b.n++;
-    b.t0[i] = groups[g].t0;
-    b.rows[i] = groups[g].rows;
-    b.k_off[i] = (int64_t)used;
-    b.v_off[i] = b.k_off[i] + (shared ? 0 : (int64_t)sh.n_kv * keys * L.kr);
-    b.keys_at[i + 1] = b.keys_at[i] + (keys + 7) / 8;
-    b.tiles_at[i + 1] = b.tiles_at[i] + (int)(((int64_t)groups[g].rows * gq + 63) / 64);
-    used += need;
-  }
-  if (e == cudaSuccess) e = run_batch();
+  if (mma) e = launch_span_umma(q, q_ld, sh, kv, rows, groups, n_groups, BF16_TC_MIN_TOKENS, out, scratch, scratch_floats, s, err, launches);
   for (int g = 0; g < n_groups && e == cudaSuccess; ++g) {
     if (mma && groups[g].rows >= BF16_TC_MIN_TOKENS) continue;
     for (int r = 0; r < groups[g].rows && e == cudaSuccess;) {

@@ -696,7 +696,7 @@ size_t span_umma_scratch_floats(const SpanShape& sh, int max_rows) {
 
 bool span_umma_supported(const SpanShape& sh, bool shared, const SpanOut& out) {
   return sh.n_kv > 0 && sh.n_head % sh.n_kv == 0 && sh.dk % 8 == 0 && sh.dv % 8 == 0 && (!shared || (sh.dk == sh.dv && sh.dk <= 512)) && variant(sh.dk, sh.dv).kernel &&
-         (int64_t)sh.n_kv * sh.n_ctx < (1 << 24) && out.ld % 2 == 0 && ((uintptr_t)out.out & 7) == 0 && ((uintptr_t)out.out16 & 3) == 0 &&
+         (int64_t)sh.n_kv * sh.n_ctx < (1 << 30) && out.ld % 2 == 0 && ((uintptr_t)out.out & 7) == 0 && ((uintptr_t)out.out16 & 3) == 0 &&
          (!out.gate || out.head_gate || (out.gate_ld % 2 == 0 && ((uintptr_t)out.gate & 7) == 0));
 }
 

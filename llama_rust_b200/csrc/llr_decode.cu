@@ -379,167 +379,7 @@ attention_tile_kernel(const float* q, KvView kv, float* __restrict__ part, RowMa
   }
 }
 
-// ---- prompt chunks of one sequence on the tensor cores -----------------------------------------------------------
-// Same partial records as the tiled kernel above, for rows of ONE sequence at consecutive positions
-// (llr_session_prefill).  A block holds 16 RT rows and one kv head and walks the slices blockIdx.y, blockIdx.y +
-// gridDim.y, ... of CH = 8 NT positions; a warp takes one query head of the group and sixteen of the rows.  Queries, keys, values and the
-// exponentials are rounded to binary16 when they are staged in shared memory (values transposed, so that two
-// consecutive positions of a dimension share a word); scores and weighted sums are m16n8k16 MMAs with f32
-// accumulation, maxima, exponentials and their sums are f32.  This is the attention of the 16-bit tensor-core path:
-// the automatic path uses it from 64 rows on, next to the 16-bit chunk GEMM and with the same kind of tolerance; the
-// f32-faithful path never does.
-__device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
-  const __half2 h = __floats2half2_rn(lo, hi);
-  return *(const uint32_t*)&h;
-}
-__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-template <int GQA, int HD, int NT, int RT>
-__global__ void __launch_bounds__(32 * GQA * RT)
-attention_tile_mma_kernel(const float* q, KvView kv, float* __restrict__ part, RowMap rows, int layer, WalkShape w,
-                          int n_split, const __grid_constant__ RowTiles tiles) {
-  pdl_enter();
-  // strides in 32-bit words (two binary16 each); + 4 words spreads the fragment reads of eight rows over all banks
-  constexpr int CH = 8 * NT, KW = HD / 2 + 4, VW = CH / 2 + 4, QW = HD / 2 + 4, PW = CH / 2 + 4, NW = GQA * RT, NTHR = 32 * NW;
-  extern __shared__ uint32_t smw[];  // k [CH][KW] | v transposed [HD][VW] | per warp: q [16][QW] | per warp: exponentials [16][PW]
-  uint32_t* kt = smw;
-  uint32_t* vt = kt + CH * KW;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-  uint32_t* qw = vt + HD * VW + warp * 16 * QW;
-  uint32_t* pw = vt + HD * VW + NW * 16 * QW + warp * 16 * PW;
-  const int hkv = blockIdx.x, head = warp % GQA;  // a warp: one query head of the group, sixteen of the block's 16 RT rows
-  // the last rows first: they attend to the most positions, and the short blocks of the first rows then fill the tail
-  const int b_begin = tiles.begin((int)gridDim.z - 1 - (int)blockIdx.z), b_end = tiles.end((int)gridDim.z - 1 - (int)blockIdx.z), b_rows = b_end - b_begin;
-  const int last_pos = row_position(rows, b_begin) + b_rows - 1;  // of the block: the slices it walks
-  if ((int)blockIdx.y * CH > last_pos) return;
-  const int t_begin = b_begin + 16 * (warp / GQA), n_rows = max(0, min(b_end - t_begin, 16));
-  const int p0 = row_position(rows, b_begin) + 16 * (warp / GQA);  // row r of the warp stands at position p0 + r
-  const int sid = row_sequence(rows, b_begin);
-  constexpr int vec = HD / 4;
-  for (int idx = lane; idx < 16 * vec; idx += 32) {  // this warp's head of the group's rows; rows past the end are zero
-    const int r = idx / vec, c = idx % vec;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (r < n_rows) v = ((const float4*)(q + ((int64_t)(t_begin + r) * w.n_head + hkv * GQA + head) * HD))[c];
-    *(uint2*)(qw + r * QW + 2 * c) = make_uint2(pack_h2(v.x, v.y), pack_h2(v.z, v.w));
-  }
-  const float scale = 1.0f / sqrtf((float)HD);
-  // The slices a block walks are merged as they come (running maximum, rescaled sums): one record per row, head and
-  // blockIdx.y, at slice index blockIdx.y, instead of one per slice.
-  float run_m0 = -CUDART_INF_F, run_m1 = -CUDART_INF_F, run_l0 = 0.f, run_l1 = 0.f;
-  float o[HD / 8][4];
-#pragma unroll
-  for (int nd = 0; nd < HD / 8; ++nd)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) o[nd][i] = 0.f;
-  for (int split = blockIdx.y; split * CH <= last_pos; split += (int)gridDim.y) {
-    const int s0 = split * CH;
-    // ---- stage the slice: positions no row of the group attends to are zero (their exponentials are zero as well)
-    for (int idx = threadIdx.x; idx < CH * vec; idx += NTHR) {
-      const int p = idx % CH, c = idx / CH;  // consecutive threads take consecutive positions: the transposed stores of v spread over the banks
-      float4 kk = make_float4(0.f, 0.f, 0.f, 0.f), vv = kk;
-      if (s0 + p <= last_pos) {
-        const int64_t off = kv_offset(kv, sid, layer, hkv, s0 + p, w.n_head_kv, HD);
-        kk = ((const float4*)(kv.k + off))[c];
-        vv = ((const float4*)(kv.v + off))[c];
-      }
-      *(uint2*)(kt + p * KW + 2 * c) = make_uint2(pack_h2(kk.x, kk.y), pack_h2(kk.z, kk.w));
-      __half* vh = (__half*)vt;
-      vh[(4 * c + 0) * (2 * VW) + p] = __float2half_rn(vv.x);
-      vh[(4 * c + 1) * (2 * VW) + p] = __float2half_rn(vv.y);
-      vh[(4 * c + 2) * (2 * VW) + p] = __float2half_rn(vv.z);
-      vh[(4 * c + 3) * (2 * VW) + p] = __float2half_rn(vv.w);
-    }
-    __syncthreads();
-    if (p0 + n_rows - 1 >= s0) {  // warp-uniform: some row of this warp attends to the slice
-    // ---- scores: rows g and g + 8 of the group against the slice's positions 8 nt + 2t, + 1
-    float sc[NT][4];
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) sc[nt][i] = 0.f;
-#pragma unroll
-    for (int k0 = 0; k0 < HD / 2; k0 += 8) {  // in words: 16 dimensions per step
-      const uint32_t a[4] = {qw[g * QW + k0 + t], qw[(g + 8) * QW + k0 + t], qw[g * QW + k0 + t + 4], qw[(g + 8) * QW + k0 + t + 4]};
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        const uint32_t* kr = kt + (8 * nt + g) * KW + k0 + t;
-        mma_f16(sc[nt], a, kr[0], kr[4]);
-      }
-    }
-    // ---- scale, causal mask, maximum, exponentials (rounded to binary16, as the MMA below reads them) and their sum
-    const int lim0 = p0 + g - s0, lim1 = p0 + g + 8 - s0;  // last slice column rows g / g + 8 attend to
-    float m0 = -CUDART_INF_F, m1 = -CUDART_INF_F;
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int col = 8 * nt + 2 * t + j;
-        sc[nt][j] = (g < n_rows && col <= lim0) ? __fmul_rn(sc[nt][j], scale) : -CUDART_INF_F;
-        sc[nt][2 + j] = (g + 8 < n_rows && col <= lim1) ? __fmul_rn(sc[nt][2 + j], scale) : -CUDART_INF_F;
-        m0 = fmaxf(m0, sc[nt][j]);
-        m1 = fmaxf(m1, sc[nt][2 + j]);
-      }
-    m0 = fmaxf(m0, __shfl_xor_sync(~0u, m0, 1)); m0 = fmaxf(m0, __shfl_xor_sync(~0u, m0, 2));
-    m1 = fmaxf(m1, __shfl_xor_sync(~0u, m1, 1)); m1 = fmaxf(m1, __shfl_xor_sync(~0u, m1, 2));
-    // what the earlier slices left is rescaled to the new maximum (a row that has attended to nothing yet keeps zeros)
-    m0 = fmaxf(m0, run_m0);
-    m1 = fmaxf(m1, run_m1);
-    const float a0 = run_m0 == -CUDART_INF_F ? 0.f : expf(run_m0 - m0), a1 = run_m1 == -CUDART_INF_F ? 0.f : expf(run_m1 - m1);
-    run_m0 = m0;
-    run_m1 = m1;
-#pragma unroll
-    for (int nd = 0; nd < HD / 8; ++nd) { o[nd][0] *= a0; o[nd][1] *= a0; o[nd][2] *= a1; o[nd][3] *= a1; }
-    float l0 = 0.f, l1 = 0.f;
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      float e[4];
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        e[j] = sc[nt][j] == -CUDART_INF_F ? 0.f : expf(sc[nt][j] - m0);
-        e[2 + j] = sc[nt][2 + j] == -CUDART_INF_F ? 0.f : expf(sc[nt][2 + j] - m1);
-      }
-      const __half2 h0 = __floats2half2_rn(e[0], e[1]), h1 = __floats2half2_rn(e[2], e[3]);
-      l0 += __low2float(h0) + __high2float(h0);  // the sum of what the weighted sum below uses
-      l1 += __low2float(h1) + __high2float(h1);
-      pw[g * PW + 4 * nt + t] = *(const uint32_t*)&h0;
-      pw[(g + 8) * PW + 4 * nt + t] = *(const uint32_t*)&h1;
-    }
-    l0 += __shfl_xor_sync(~0u, l0, 1); l0 += __shfl_xor_sync(~0u, l0, 2);
-    l1 += __shfl_xor_sync(~0u, l1, 1); l1 += __shfl_xor_sync(~0u, l1, 2);
-    run_l0 = fmaf(run_l0, a0, l0);
-    run_l1 = fmaf(run_l1, a1, l1);
-    __syncwarp();
-    // ---- weighted value rows: dimensions 8 nd + 2t, + 1 of rows g and g + 8, added to the rescaled sums
-#pragma unroll
-    for (int k0 = 0; k0 < CH / 2; k0 += 8) {  // in words: 16 positions per step
-      const uint32_t a[4] = {pw[g * PW + k0 + t], pw[(g + 8) * PW + k0 + t], pw[g * PW + k0 + t + 4], pw[(g + 8) * PW + k0 + t + 4]};
-#pragma unroll
-      for (int nd = 0; nd < HD / 8; ++nd) {
-        const uint32_t* vr = vt + (8 * nd + g) * VW + k0 + t;
-        mma_f16(o[nd], a, vr[0], vr[4]);
-      }
-    }
-    }
-    __syncthreads();  // every warp is done with the slice before the next one is staged
-  }
-  // ---- one record per row: HD sums, the maximum, the sum of exponentials.  A row whose position lies before this
-  // block's first slice has none, and the merge does not look for one: it reads min(slices of the row, gridDim.y) records.
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const int r = g + 8 * half;
-    if (r >= n_rows || p0 + r < (int)blockIdx.y * CH) continue;
-    float* out = part + ((((int64_t)(t_begin + r) * w.n_head_kv + hkv) * n_split + blockIdx.y) * GQA + head) * (HD + 2);
-#pragma unroll
-    for (int nd = 0; nd < HD / 8; ++nd) *(float2*)(out + 8 * nd + 2 * t) = make_float2(o[nd][2 * half], o[nd][2 * half + 1]);
-    if (t == 0) { out[HD] = half ? run_m1 : run_m0; out[HD + 1] = half ? run_l1 : run_l0; }
-  }
-}
-
-// Rows whose records the tensor-core kernel left: at most eight groups of 64 rows and more in a batch of 512.
+// Rows that the tensor-core kernel has finished: at most eight groups of 64 rows and more in a batch of 512.
 struct RowRanges {
   int n, lo[8], hi[8];
   __device__ __forceinline__ bool has(int t) const {
@@ -554,8 +394,9 @@ struct RowRanges {
 // sums; then every lane adds its dimensions over the slices in ascending order, the weights coming by shuffle.
 __global__ void __launch_bounds__(128)
 attention_combine_kernel(const float* part, float* __restrict__ out, RowMap rows, int chunk, WalkShape w, int heads_per_block,
-                         int max_records, int record_chunk, const __grid_constant__ RowRanges mma_rows) {
+                         const __grid_constant__ RowRanges finished) {
   pdl_enter();
+  if (finished.has((int)blockIdx.y)) return;
   // heads_per_block 4: one warp per head (many rows: fewer, fuller blocks); 1: the four warps share a head's
   // dimensions (a decode step has few blocks to fill the device with)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -565,11 +406,7 @@ attention_combine_kernel(const float* part, float* __restrict__ out, RowMap rows
   const int hd = w.head_dim, gqa = w.n_head / w.n_head_kv;
   const int hkv = hq / gqa, g = hq % gqa;
   const int seq = row_position(rows, t) + 1;
-  // chunk: positions per slice of the f32 kernels, which fixes the room a row's records take.  The tensor-core kernel
-  // walks slices of record_chunk positions of its own and leaves one record per walked run of slices, at the first
-  // max_records indices.
-  if (!mma_rows.has(t)) { max_records = 32; record_chunk = chunk; }
-  const int n_split = (w.n_ctx + chunk - 1) / chunk, used = min(min(n_split, (seq + record_chunk - 1) / record_chunk), max_records);
+  const int n_split = (w.n_ctx + chunk - 1) / chunk, used = min(n_split, (seq + chunk - 1) / chunk);
   const float* base = part + ((int64_t)t * w.n_head_kv + hkv) * n_split * gqa * (hd + 2) + g * (hd + 2);
   const int64_t stride = (int64_t)gqa * (hd + 2);
   const float ms = lane < used ? base[lane * stride + hd] : -CUDART_INF_F;
@@ -772,8 +609,18 @@ cudaError_t launch_rope_store(float* q, float* k, const float* v, const KvView& 
   return launch_walk(rope_store_kernel, dim3(tokens), dim3(256), 0, s, q, k, v, kv, rows, layer, w);
 }
 
-size_t attention_scratch_floats(int tokens, const WalkShape& w) {
-  return (size_t)tokens * w.n_head_kv * attention_splits(w) * (w.n_head / w.n_head_kv) * (w.head_dim + 2);
+// the walk's attention as the tensor-core kernel knows it: no window, no bias
+static SpanShape span_shape(const WalkShape& w) {
+  SpanShape sh{};
+  sh.n_head = w.n_head; sh.n_kv = w.n_head_kv; sh.dk = sh.dv = w.head_dim; sh.n_ctx = w.n_ctx;
+  sh.scale = 1.0f / sqrtf((float)w.head_dim);
+  return sh;
+}
+
+size_t attention_scratch_floats(int tokens, size_t positions, const WalkShape& w) {
+  SpanShape sh = span_shape(w);
+  sh.n_ctx = (int)std::min<size_t>(w.n_ctx, positions);
+  return std::max((size_t)tokens * w.n_head_kv * attention_splits(w) * (w.n_head / w.n_head_kv) * (w.head_dim + 2), span_umma_scratch_floats(sh, tokens));
 }
 
 // The per-row kernels for the heads per group of a shape (the smallest of 1, 2, 4, 8 that holds them) and their shared memory,
@@ -817,11 +664,12 @@ cudaError_t launch_attention(const float* q, const KvView& kv, float* out, float
   if (launches) *launches += 2;
   e = launch_walk(row.partial, dim3(w.n_head_kv, splits, 1), dim3(ATT_THREADS), row.smem, s, q, kv, scratch, rows, layer, chunk, w, k_new, v_new);
   if (e != cudaSuccess) return e;
-  return launch_walk(attention_combine_kernel, dim3(w.n_head, 1), dim3(128), 0, s, (const float*)scratch, out, rows, chunk, w, 1, splits, chunk, RowRanges{});
+  return launch_walk(attention_combine_kernel, dim3(w.n_head, 1), dim3(128), 0, s, (const float*)scratch, out, rows, chunk, w, 1, RowRanges{});
 }
 
 cudaError_t launch_attention_groups(const float* q, const KvView& kv, float* out, float* scratch, const RowMap& rows, int tokens, int layer, const WalkShape& w,
-                                    const AttentionGroup* groups, int n_groups, bool tensor_cores, cudaStream_t s, uint64_t* launches) {
+                                    const AttentionGroup* groups, int n_groups, bool tensor_cores, size_t scratch_floats, cudaStream_t s, int* err,
+                                    uint64_t* launches) {
   if (tokens <= 0) return cudaSuccess;
   if (tokens > MAX_TILES) return cudaErrorInvalidValue;
   const int gqa = w.n_head_kv > 0 ? w.n_head / w.n_head_kv : 0;
@@ -830,7 +678,7 @@ cudaError_t launch_attention_groups(const float* q, const KvView& kv, float* out
   if (e != cudaSuccess) return e;
   const int splits = attention_splits(w);
   const int max_chunk = attention_chunk(w);
-  const AttentionGroup all{0, tokens};
+  const AttentionGroup all{0, tokens, rows.first};
   if (!groups) { groups = &all; n_groups = 1; }
   // prompt chunks: rows of a group share the slice's keys and values through a shared-memory tile
   const size_t tile_smem = (2 * (size_t)max_chunk * w.head_dim + (ATT_THREADS / 32) * ((size_t)gqa * w.head_dim + (size_t)gqa * max_chunk)) * sizeof(float);
@@ -841,40 +689,33 @@ cudaError_t launch_attention_groups(const float* q, const KvView& kv, float* out
 #undef LLR_TILE
   if (max_chunk > ATT_TILE_CHUNK || tile_smem > 200 * 1024) tile = nullptr;
   // groups long enough, when the caller allows 16-bit operands: tensor cores
-  void (*mma)(const float*, KvView, float*, RowMap, int, WalkShape, int, const RowTiles) = nullptr;
-  size_t mma_smem = 0;
-  int mma_rt = 1;
-  // its slices are its own (64 positions; 32 when the context is short): the records it leaves do not depend on max_chunk
-  const int mma_chunk = w.n_ctx > 1024 ? 64 : 32;
-  if (tensor_cores && (w.head_dim == 64 || w.head_dim == 128)) {
-#define LLR_MMA(G, H, N) if (gqa == G && w.head_dim == H && mma_chunk == 8 * N) mma = attention_tile_mma_kernel<G, H, N, (G <= 4 ? 4 : 2)>;
-    LLR_MMA(1, 64, 4) LLR_MMA(2, 64, 4) LLR_MMA(4, 64, 4) LLR_MMA(8, 64, 4) LLR_MMA(1, 64, 8) LLR_MMA(2, 64, 8) LLR_MMA(4, 64, 8) LLR_MMA(8, 64, 8)
-    LLR_MMA(1, 128, 4) LLR_MMA(2, 128, 4) LLR_MMA(4, 128, 4) LLR_MMA(8, 128, 4) LLR_MMA(1, 128, 8) LLR_MMA(2, 128, 8) LLR_MMA(4, 128, 8) LLR_MMA(8, 128, 8)
-#undef LLR_MMA
-    mma_rt = gqa <= 4 ? 4 : 2;  // sixteen-row tiles per block
-    mma_smem = ((size_t)mma_chunk * (w.head_dim / 2 + 4) + (size_t)w.head_dim * (mma_chunk / 2 + 4) +
-                (size_t)gqa * mma_rt * 16 * (w.head_dim / 2 + 4 + mma_chunk / 2 + 4)) * sizeof(uint32_t);
-    if (mma_smem > 200 * 1024) mma = nullptr;
-  }
+  const SpanShape span = span_shape(w);
+  const SpanOut to_out{out, nullptr, (int64_t)w.n_head * w.head_dim, nullptr, 0, false, 1.0f};
+  const bool mma = tensor_cores && (w.head_dim == 64 || w.head_dim == 128) && (gqa & (gqa - 1)) == 0 && span_umma_supported(span, false, to_out);
   // Every group goes to one of three kernels, one launch each: binary16 MMAs (64 rows and more), the tiled f32 kernel (four rows
   // and more: below that a block of eight warps would have work for one to three), the f32 kernel of a block per row.
-  RowTiles big{}, tiled{}, single{};
-  RowRanges mma_rows{};
+  RowTiles tiled{}, single{};
+  RowRanges finished{};
+  SpanGroup big[8];
+  int left = 0;
   for (int g = 0; g < n_groups; ++g) {
     const int first = groups[g].first, n = groups[g].rows;
-    const bool on_mma = mma && n >= 64 && mma_rows.n < 8;
-    RowTiles& to = on_mma ? big : tile && n >= 4 ? tiled : single;
-    const int per = on_mma ? 16 * mma_rt : tile && n >= 4 ? ATT_ROWS : 1;
+    if (mma && n >= 64 && finished.n < 8) {
+      big[finished.n] = SpanGroup{first, n, groups[g].position};
+      finished.lo[finished.n] = first;
+      finished.hi[finished.n++] = first + n;
+      continue;
+    }
+    RowTiles& to = tile && n >= 4 ? tiled : single;
+    const int per = tile && n >= 4 ? ATT_ROWS : 1;
     for (int r = 0; r < n; r += per) to.run[to.n++] = (uint32_t)std::min(per, n - r) << 16 | (uint32_t)(first + r);
-    if (on_mma) { mma_rows.lo[mma_rows.n] = first; mma_rows.hi[mma_rows.n++] = first + n; }
+    left += n;
   }
-  int max_records = splits;
-  if (big.n) {
-    if (launches) ++*launches;
-    max_records = std::min(std::min((w.n_ctx + mma_chunk - 1) / mma_chunk, splits), 4);
-    if (mma_smem > 48 * 1024 && (e = cudaFuncSetAttribute((const void*)mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mma_smem)) != cudaSuccess) return e;
-    e = launch_walk(mma, dim3(w.n_head_kv, max_records, big.n), dim3(32 * gqa * mma_rt), mma_smem, s, q, kv, scratch, rows, layer, w, splits, big);
-    if (e != cudaSuccess) return e;
+  if (finished.n) {
+    const int64_t page = (int64_t)kv.n_layer * w.n_head_kv * kv.block_tokens * w.head_dim, at = (int64_t)layer * w.n_head_kv * kv.block_tokens * w.head_dim;
+    const LayerKv pages{kv.k + at, kv.v + at, kv.table, kv.block_tokens, kv.max_blocks, page, page};
+    e = launch_span_umma(q, (int64_t)w.n_head * w.head_dim, span, pages, rows, big, finished.n, 1, to_out, scratch, scratch_floats, s, err, launches);
+    if (e != cudaSuccess || left == 0) return e;
   }
   if (tiled.n) {
     if (launches) ++*launches;
@@ -889,7 +730,7 @@ cudaError_t launch_attention_groups(const float* q, const KvView& kv, float* out
   }
   if (launches) ++*launches;
   return launch_walk(attention_combine_kernel, dim3(tokens >= 16 ? (w.n_head + 3) / 4 : w.n_head, tokens), dim3(128), 0, s, (const float*)scratch, out, rows,
-                     max_chunk, w, tokens >= 16 ? 4 : 1, max_records, mma_chunk, mma_rows);
+                     max_chunk, w, tokens >= 16 ? 4 : 1, finished);
 }
 
 cudaError_t launch_swiglu(float* g, const float* u, int64_t n, cudaStream_t s, uint64_t* launches) {

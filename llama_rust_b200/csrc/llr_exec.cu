@@ -1711,7 +1711,7 @@ struct llr_session {
   float *x = nullptr, *xn = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *attn = nullptr, *proj = nullptr,
         *gate = nullptr, *up = nullptr, *logits = nullptr, *cache_k = nullptr, *cache_v = nullptr, *att_scratch = nullptr,
         *margins = nullptr, *last_x = nullptr, *arg_part = nullptr;
-  size_t logits_rows = 1;
+  size_t logits_rows = 1, att_floats = 0;
   int *ids = nullptr, *pos_dev = nullptr;  // ids[0]: the token the next step reads; ids[1..]: prompt chunk or generated tokens
   size_t ids_cap = 0;
   int* count_dev = nullptr;  // tokens generated by the current llr_session_decode call
@@ -1914,9 +1914,10 @@ cudaError_t session_layers(llr_session* s, const int* ids_dev, size_t n, const R
       // the automatic path takes the tensor cores for chunks of 64 rows and more of one sequence, as it does for the products
       const bool tc = e->path == PATH_AUTO;
       std::vector<AttentionGroup> groups;
-      for (const auto& gr : s->batch_groups) groups.push_back(AttentionGroup{(int)gr.first, (int)gr.second});
+      for (size_t g = 0; g < s->batch_groups.size(); ++g)
+        groups.push_back(AttentionGroup{(int)s->batch_groups[g].first, (int)s->batch_groups[g].second, (int)s->batch_first[g]});
       if ((ce = launch_attention_groups(s->q, kv, s->attn, s->att_scratch, rows, (int)n, (int)li, s->shape, rows.row_seq ? groups.data() : nullptr,
-                                        rows.row_seq ? (int)groups.size() : 0, tc, st, L)) != cudaSuccess)
+                                        rows.row_seq ? (int)groups.size() : 0, tc, s->att_floats, st, e->err_flag, L)) != cudaSuccess)
         break;
     }
     if ((ce = session_matmul(e, W.attn_output, n, s->attn, s->proj)) != cudaSuccess) break;
@@ -2057,7 +2058,8 @@ int session_create(llr_exec* e, const llr_llama_model* m, size_t n_seq, size_t k
   alloc(&s->logits, s->logits_rows * V); alloc(&s->last_x, s->logits_rows * E); alloc(&s->arg_part, 512);
   const size_t pool = s->n_blocks * c.n_layer * c.n_head_kv * block_tokens * c.head_dim;
   alloc(&s->cache_k, pool); alloc(&s->cache_v, pool);
-  alloc(&s->att_scratch, attention_scratch_floats((int)B, s->shape));
+  s->att_floats = attention_scratch_floats((int)B, s->n_blocks * block_tokens, s->shape);
+  alloc(&s->att_scratch, s->att_floats);
   ialloc(&s->pos_dev, 1); ialloc(&s->count_dev, 1);
   ialloc(&s->table_dev, n_seq * s->max_blocks); ialloc(&s->row_pos, B); ialloc(&s->row_seq, B); ialloc(&s->last_rows, s->logits_rows);
   if (ce == cudaSuccess) ce = cudaMemset(s->pos_dev, 0, sizeof(int));

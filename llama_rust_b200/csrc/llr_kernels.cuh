@@ -329,17 +329,19 @@ struct RowMap {
 cudaError_t launch_rope_store(float* q, float* k, const float* v, const KvView& kv, const RowMap& rows, int tokens, int layer,
                               const WalkShape& w, cudaStream_t s, uint64_t* launches);
 // out[t][hq] = softmax(q[t][hq] . K[0..pos(t)] / sqrt(hd)) V over row t's own sequence, grouped-query heads; scratch holds
-// the partial results of the position splits (attention_scratch_floats)
-size_t attention_scratch_floats(int tokens, const WalkShape& w);
+// the partial results of the position splits, or a group's keys and values as binary16 (attention_scratch_floats; positions: the most that
+// the pool holds)
+size_t attention_scratch_floats(int tokens, size_t positions, const WalkShape& w);
 // k_new / v_new: one decode token whose rotation and cache store the attention kernel does itself
 cudaError_t launch_attention(const float* q, const KvView& kv, float* out, float* scratch, const RowMap& rows, int layer,
                              const WalkShape& w, cudaStream_t s, uint64_t* launches, const float* k_new, const float* v_new);
 // The same for the rows of a batch.  groups: runs of rows of one sequence at consecutive positions that make up the batch,
 // ascending (null: all rows are one); with tensor_cores those of 64 rows and more may run as binary16 MMAs with f32
 // accumulation (the tolerance of the 16-bit chunk GEMM).
-struct AttentionGroup { int first, rows; };
+struct AttentionGroup { int first, rows, position; };  // position of the first row, -1: the device knows it
 cudaError_t launch_attention_groups(const float* q, const KvView& kv, float* out, float* scratch, const RowMap& rows, int tokens, int layer, const WalkShape& w,
-                                    const AttentionGroup* groups, int n_groups, bool tensor_cores, cudaStream_t s, uint64_t* launches);
+                                    const AttentionGroup* groups, int n_groups, bool tensor_cores, size_t scratch_floats, cudaStream_t s, int* err,
+                                    uint64_t* launches);
 cudaError_t launch_swiglu(float* g, const float* u, int64_t n, cudaStream_t s, uint64_t* launches);
 cudaError_t launch_add(float* x, const float* y, int64_t n, cudaStream_t s, uint64_t* launches);
 // first index of the strict maximum of logits[0..n) -> *out_id (device; n == 0: no argmax), and *pos_dev += advance

@@ -583,6 +583,11 @@ argmax_merge_kernel(const float* pbest, const int* pidx, const float* psecond, i
   if (pos_dev) *pos_dev += advance;
 }
 
+__global__ void __launch_bounds__(256) table_entries_kernel(int* __restrict__ table, const int* __restrict__ entries, int n) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i < n) table[(uint32_t)entries[2 * i]] = entries[2 * i + 1];
+}
+
 // positions per attention slice: 32, or a thirty-second of the context when that is longer
 int attention_chunk(const WalkShape& w) {
   const int c = (w.n_ctx + 31) / 32;
@@ -744,6 +749,13 @@ cudaError_t launch_swiglu(float* g, const float* u, int64_t n, cudaStream_t s, u
     return launch_walk(swiglu4_kernel, dim3((unsigned)b4), dim3(256), 0, s, (float4*)g, (const float4*)u, n / 4);
   }
   return launch_walk(swiglu_kernel, dim3((unsigned)blocks), dim3(256), 0, s, g, u, n);
+}
+
+cudaError_t launch_table_entries(int* table, const int* entries, int n, cudaStream_t s, uint64_t* launches) {
+  if (n <= 0) return cudaSuccess;
+  if (launches) ++*launches;
+  table_entries_kernel<<<(n + 255) / 256, 256, 0, s>>>(table, entries, n);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_add(float* x, const float* y, int64_t n, cudaStream_t s, uint64_t* launches) {

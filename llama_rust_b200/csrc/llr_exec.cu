@@ -146,6 +146,9 @@ struct llr_exec {
   uint8_t* dev_s = nullptr; size_t dev_s_cap = 0;  // kernel scratch (bf16 activations of the tensor-core GEMM)
   uint8_t* dev_q = nullptr; size_t dev_q_cap = 0;  // kernel scratch (digits of the integer GEMM), this executor's stream only
   size_t dev_q_limit = SIZE_MAX;                   // LLR_DIGITS_LIMIT: what it may grow to
+  // logits on their way to pageable memory: two pieces of pinned memory that take turns (deliver_rows)
+  char* pin_out = nullptr;
+  cudaEvent_t out_event[2] = {nullptr, nullptr};
   // residency
   std::list<CacheEntry> cache;  // front = least recently used
   bool limit_resolved = false;
@@ -582,6 +585,8 @@ int llr_exec_destroy(llr_exec* e) {
     m->dev = nullptr;
     m->owner = nullptr;
   }
+  if (e->pin_out) cudaFreeHost(e->pin_out);
+  for (cudaEvent_t v : e->out_event) if (v) cudaEventDestroy(v);
   if (e->pin_x) cudaFreeHost(e->pin_x);
   if (e->pin_y) cudaFreeHost(e->pin_y);
   if (e->dev_x) cudaFree(e->dev_x);
@@ -1668,7 +1673,7 @@ struct LayeredDecoder {
   float2* angles = nullptr;
   cudaStream_t side = nullptr;  // of the second of two mixers
   cudaEvent_t fork = nullptr, join = nullptr;
-  int* group_first = nullptr;  // first row of each group of the batch in flight, and their end
+  const int* group_first = nullptr;  // device: first row of each group of the batch in flight, and their end
   ~LayeredDecoder() {
     for (Layer& L : layers) {
       for (Mixer& M : L.mixers) {
@@ -1682,7 +1687,7 @@ struct LayeredDecoder {
     }
     float* p[] = {proj, lat_q, lat_o, att, gu, act, y, scratch, state, prep, records, low};
     for (float* q : p) if (q) cudaFree(q);
-    void* v[] = {x16, a16, b16, freq_dev, angles, group_first};
+    void* v[] = {x16, a16, b16, freq_dev, angles};
     for (void* q : v) if (q) cudaFree(q);
     if (fork) cudaEventDestroy(fork);
     if (join) cudaEventDestroy(join);
@@ -1715,7 +1720,12 @@ struct llr_session {
   int *ids = nullptr, *pos_dev = nullptr;  // ids[0]: the token the next step reads; ids[1..]: prompt chunk or generated tokens
   size_t ids_cap = 0;
   int* count_dev = nullptr;  // tokens generated by the current llr_session_decode call
-  int *table_dev = nullptr, *row_pos = nullptr, *row_seq = nullptr, *last_rows = nullptr;
+  int *table_dev = nullptr, *last_rows = nullptr;
+  // A batch's ids, positions, sequences, last rows, groups and new table entries: one block, one copy from pinned memory.  Behind it in
+  // pinned memory the winners that come back, and sequence 0's position.
+  int *batch_dev = nullptr, *batch_host = nullptr;
+  size_t batch_words = 0;
+  bool batch_in_flight = false;  // a batch has failed since its upload was enqueued
   // decode steps (one row): the independent products of a layer as one launch each -- {q, k, v} and {gate, up}
   std::vector<llr::Program*> qkv_prog, gateup_prog;
   // routed layers, one token: the chosen experts' {gate, up} products as one launch and their down products as another
@@ -1752,8 +1762,9 @@ void session_release(llr_session* s) {
   float* bufs[] = {s->out_norm, s->x, s->xn, s->q, s->k, s->v, s->attn, s->proj, s->gate, s->up, s->logits,
                    s->cache_k, s->cache_v, s->att_scratch, s->margins, s->last_x, s->arg_part};
   for (float* p : bufs) if (p) cudaFree(p);
-  int* ibufs[] = {s->ids, s->pos_dev, s->count_dev, s->table_dev, s->row_pos, s->row_seq, s->last_rows};
+  int* ibufs[] = {s->ids, s->pos_dev, s->count_dev, s->table_dev, s->batch_dev, s->last_rows};
   for (int* p : ibufs) if (p) cudaFree(p);
+  if (s->batch_host) cudaFreeHost(s->batch_host);
   if (s->step_graph) cudaGraphExecDestroy(s->step_graph);
   if (s->moe_tables) cudaFree(s->moe_tables);
   if (s->moe_sel) cudaFree(s->moe_sel);
@@ -1787,8 +1798,46 @@ KvView session_kv(const llr_session* s) {
   return KvView{s->cache_k, s->cache_v, s->table_dev, (int)s->block_tokens, (int)s->max_blocks, (int)s->cfg.n_layer};
 }
 
-// Blocks for positions [0, upto) of a sequence; new table entries go to the device on the executor's stream.
-int session_reserve(llr_session* s, size_t seq, size_t upto) {
+// Results of the work enqueued before to the caller's memory, which then holds them (the stream is waited for).  The driver's copy to
+// pageable memory that nobody has touched yet takes a page fault per 4 KB while the device waits (4 MB: 1.2 ms), so large pageable buffers
+// have their pages brought in while the device still works, and the bytes pass through two pinned pieces, one filled while the other is emptied.
+cudaError_t deliver_rows(llr_exec* e, void* dst, const void* src, size_t bytes) {
+  constexpr size_t PIECE = 1 << 20;
+  cudaError_t ce;
+  void* alias = nullptr;
+  if (bytes < 256 * 1024 || pinned_alias(dst, &alias)) {
+    if ((ce = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, e->stream)) != cudaSuccess) return ce;
+    return cudaStreamSynchronize(e->stream);
+  }
+  if (!e->pin_out) {
+    for (cudaEvent_t& v : e->out_event)
+      if (!v && (ce = cudaEventCreateWithFlags(&v, cudaEventDisableTiming)) != cudaSuccess) return ce;
+    if ((ce = cudaMallocHost((void**)&e->pin_out, 2 * PIECE)) != cudaSuccess) return ce;
+  }
+  const size_t n = (bytes + PIECE - 1) / PIECE;
+  auto size = [&](size_t i) { return std::min(PIECE, bytes - i * PIECE); };
+  auto fetch = [&](size_t i) {
+    const cudaError_t c = cudaMemcpyAsync(e->pin_out + (i & 1) * PIECE, (const char*)src + i * PIECE, size(i), cudaMemcpyDeviceToHost, e->stream);
+    return c == cudaSuccess ? cudaEventRecord(e->out_event[i & 1], e->stream) : c;
+  };
+  if ((ce = fetch(0)) != cudaSuccess || (n > 1 && (ce = fetch(1)) != cudaSuccess)) return ce;
+  for (size_t at = 0; at < bytes; at += 4096) {
+    volatile char* p = (volatile char*)dst + at;
+    *p = *p;
+  }
+  for (size_t i = 0; i < n; ++i) {
+    if ((ce = cudaEventSynchronize(e->out_event[i & 1])) != cudaSuccess) return ce;
+    std::memcpy((char*)dst + i * PIECE, e->pin_out + (i & 1) * PIECE, size(i));
+    if (i + 2 < n && (ce = fetch(i + 2)) != cudaSuccess) return ce;
+  }
+  return cudaStreamSynchronize(e->stream);
+}
+
+// (index, block) words of table entries that the device has yet to learn
+typedef std::vector<int> TableEntries;
+
+// Blocks for positions [0, upto) of a sequence; new table entries go to the device on the executor's stream, or to `later`.
+int session_reserve(llr_session* s, size_t seq, size_t upto, TableEntries* later = nullptr) {
   llr_exec* e = s->owner;
   const size_t need = (upto + s->block_tokens - 1) / s->block_tokens;
   std::vector<int>& mine = s->seq_blocks[seq];
@@ -1798,11 +1847,22 @@ int session_reserve(llr_session* s, size_t seq, size_t upto) {
     return fail(e, LLR_ERR_OOM, "the session's KV pool has no free block left (" + std::to_string(s->n_blocks) + " blocks of " +
                                     std::to_string(s->block_tokens) + " positions)");
   while (mine.size() < need) { mine.push_back(s->free_blocks.back()); s->free_blocks.pop_back(); }
+  if (later) {
+    for (size_t b = had; b < need; ++b) { later->push_back((int)(seq * s->max_blocks + b)); later->push_back(mine[b]); }
+    return LLR_OK;
+  }
   cudaError_t ce = cudaMemcpyAsync(s->table_dev + seq * s->max_blocks + had, mine.data() + had, (need - had) * sizeof(int),
                                    cudaMemcpyHostToDevice, e->stream);
   if (ce != cudaSuccess) return fail_cuda(e, ce, "block table upload");
   // the host vector may grow again before the copy has run: pageable copies of this size are staged by the driver at call time
   return LLR_OK;
+}
+
+cudaError_t session_batch_buffers(llr_session* s) {
+  s->batch_words = 9 * s->max_batch + 8;  // at most max_batch groups, and a new block per row and group
+  cudaError_t ce = cudaMalloc((void**)&s->batch_dev, s->batch_words * sizeof(int));
+  if (ce == cudaSuccess) ce = cudaMallocHost((void**)&s->batch_host, (s->batch_words + s->max_batch + 1) * sizeof(int));
+  return ce;
 }
 
 // Sequences and their paged pool: n_seq sequences of at most n_ctx positions over kv_blocks blocks (0: enough for all).
@@ -2061,7 +2121,8 @@ int session_create(llr_exec* e, const llr_llama_model* m, size_t n_seq, size_t k
   s->att_floats = attention_scratch_floats((int)B, s->n_blocks * block_tokens, s->shape);
   alloc(&s->att_scratch, s->att_floats);
   ialloc(&s->pos_dev, 1); ialloc(&s->count_dev, 1);
-  ialloc(&s->table_dev, n_seq * s->max_blocks); ialloc(&s->row_pos, B); ialloc(&s->row_seq, B); ialloc(&s->last_rows, s->logits_rows);
+  ialloc(&s->table_dev, n_seq * s->max_blocks); ialloc(&s->last_rows, s->logits_rows);
+  if (ce == cudaSuccess) ce = session_batch_buffers(s);
   if (ce == cudaSuccess) ce = cudaMemset(s->pos_dev, 0, sizeof(int));
   if (ce == cudaSuccess) ce = cudaMemset(s->table_dev, 0, n_seq * s->max_blocks * sizeof(int));
   if (max_expert > 0 && ce == cudaSuccess) {
@@ -2400,13 +2461,22 @@ static int session_batch(llr_session* s, size_t n_groups, const uint32_t* seq_id
   std::vector<size_t> order(n_groups);
   for (size_t g = 0; g < n_groups; ++g) order[g] = g;
   std::sort(order.begin(), order.end(), [&](size_t a, size_t b) { return seq_ids[a] < seq_ids[b]; });
-  std::vector<int> ids(total), rpos(total), rseq(total), last(n_groups), row_of(rows ? total : 0);
+  if (s->batch_in_flight) cudaStreamSynchronize(e->stream);  // the copy of a batch that failed may still read the pinned words
+  s->batch_in_flight = false;
+  int *ids = s->batch_host, *rpos = ids + total, *rseq = rpos + total, *last = rseq + total, *starts = last + n_groups;
+  std::vector<int> row_of(rows ? total : 0);
+  TableEntries entries;
   size_t r = 0;
   s->batch_groups.clear();
   s->batch_first.clear();
   for (size_t oi = 0; oi < n_groups; ++oi) {
     const size_t g = order[oi], q = seq_ids[g];
-    if ((rc = session_reserve(s, q, s->position[q] + counts[g]))) return rc;
+    if ((rc = session_reserve(s, q, s->position[q] + counts[g], &entries))) {
+      // the blocks of the groups before this one are theirs: the device learns of them now
+      for (size_t i = 0; i < entries.size(); i += 2)
+        cudaMemcpyAsync(s->table_dev + (uint32_t)entries[i], &entries[i + 1], sizeof(int), cudaMemcpyHostToDevice, e->stream);
+      return rc;
+    }
     s->batch_groups.emplace_back(r, (size_t)counts[g]);
     s->batch_first.push_back(s->position[q]);
     for (size_t i = 0; i < counts[g]; ++i, ++r) {
@@ -2415,26 +2485,24 @@ static int session_batch(llr_session* s, size_t n_groups, const uint32_t* seq_id
       rpos[r] = (int)(s->position[q] + i);
       rseq[r] = (int)q;
     }
-    last[oi] = (int)r - 1;
+    last[g] = (int)r - 1;  // in the caller's order: what is taken from the last rows comes back in it
+    starts[oi] = (int)s->batch_groups[oi].first;
   }
+  starts[n_groups] = (int)total;
+  const size_t words = (size_t)(starts + n_groups + 1 - ids);
+  std::copy(entries.begin(), entries.end(), ids + words);
   cudaStream_t st = e->stream;
   uint64_t* L = &e->ctr.launches;
   cudaError_t ce;
-  if ((ce = cudaMemcpyAsync(s->ids + 1, ids.data(), total * sizeof(int), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-      (ce = cudaMemcpyAsync(s->row_pos, rpos.data(), total * sizeof(int), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-      (ce = cudaMemcpyAsync(s->row_seq, rseq.data(), total * sizeof(int), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-      (ce = cudaMemcpyAsync(s->last_rows, last.data(), n_groups * sizeof(int), cudaMemcpyHostToDevice, st)) != cudaSuccess)
+  const int n_new = (int)(entries.size() / 2);
+  s->batch_in_flight = true;
+  if ((ce = cudaMemcpyAsync(s->batch_dev, ids, (words + entries.size()) * sizeof(int), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+      (ce = launch_table_entries(s->table_dev, s->batch_dev + words, n_new, st, L)) != cudaSuccess)
     return fail_cuda(e, ce, "batch upload");
-  if (s->dec && s->dec->state_floats > 0) {
-    std::vector<int> starts;
-    for (const auto& g : s->batch_groups) starts.push_back((int)g.first);
-    starts.push_back((int)total);
-    if ((ce = cudaMemcpyAsync(s->dec->group_first, starts.data(), starts.size() * sizeof(int), cudaMemcpyHostToDevice, st)) != cudaSuccess)
-      return fail_cuda(e, ce, "batch upload");
-  }
+  const int *dev_ids = s->batch_dev, *dev_pos = dev_ids + total, *dev_seq = dev_pos + total, *dev_last = dev_seq + total;
+  if (s->dec) s->dec->group_first = dev_last + n_groups;
   const float* pending = nullptr;
-  if ((ce = session_layers(s, s->ids + 1, total, RowMap{nullptr, s->row_pos, s->row_seq}, &pending)) != cudaSuccess)
-    return fail_cuda(e, ce, "kernel launch");
+  if ((ce = session_layers(s, dev_ids, total, RowMap{nullptr, dev_pos, dev_seq}, &pending)) != cudaSuccess) return fail_cuda(e, ce, "kernel launch");
   // each group's last row: residual add, output norm, logits (LogitsKind::Last per sequence)
   if (pending && (ce = launch_add(s->x, pending, (int64_t)(total * E), st, L)) != cudaSuccess) return fail_cuda(e, ce, "kernel launch");
   if (rows) {
@@ -2447,38 +2515,32 @@ static int session_batch(llr_session* s, size_t n_groups, const uint32_t* seq_id
           (ce = launch_gather_rows(s->x, s->last_rows, s->last_x, (int)nw, (int)E, st, L)) != cudaSuccess ||
           (ce = launch_rmsnorm(s->last_x, nullptr, s->out_norm, s->last_x, (int)nw, (int)E, c.rms_eps, st, L)) != cudaSuccess ||
           (ce = session_matmul(e, s->output, nw, s->last_x, s->logits)) != cudaSuccess ||
-          (ce = cudaMemcpyAsync(rows->logits + w0 * V, s->logits, nw * V * sizeof(float), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
-          (ce = cudaStreamSynchronize(st)) != cudaSuccess)
+          (ce = deliver_rows(e, rows->logits + w0 * V, s->logits, nw * V * sizeof(float))) != cudaSuccess)
         return fail_cuda(e, ce, "logits of the wanted rows");
     }
-  } else if ((ce = launch_gather_rows(s->x, s->last_rows, s->last_x, (int)n_groups, (int)E, st, L)) != cudaSuccess ||
+  } else if ((ce = launch_gather_rows(s->x, dev_last, s->last_x, (int)n_groups, (int)E, st, L)) != cudaSuccess ||
       (ce = launch_rmsnorm(s->last_x, nullptr, s->out_norm, s->last_x, (int)n_groups, (int)E, c.rms_eps, st, L)) != cudaSuccess ||
       (ce = session_matmul(e, s->output, n_groups, s->last_x, s->logits)) != cudaSuccess)
     return fail_cuda(e, ce, "kernel launch");
-  std::vector<int> win(n_groups);
+  int *win = s->batch_host + s->batch_words, *pos0 = win + s->max_batch;
   if (next_ids) {
     if ((ce = launch_argmax_rows(s->logits, (int)n_groups, (int)V, s->ids, nullptr, st, L)) != cudaSuccess ||
-        (ce = cudaMemcpyAsync(win.data(), s->ids, n_groups * sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
+        (ce = cudaMemcpyAsync(win, s->ids, n_groups * sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
       return fail_cuda(e, ce, "argmax");
   }
-  std::vector<float> lg(last_logits ? n_groups * V : 0);
-  if (last_logits && (ce = cudaMemcpyAsync(lg.data(), s->logits, n_groups * V * sizeof(float), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
-    return fail_cuda(e, ce, "logits download");
-  if ((ce = cudaStreamSynchronize(st)) != cudaSuccess) return fail_cuda(e, ce, "batch");
+  if ((ce = last_logits ? deliver_rows(e, last_logits, s->logits, n_groups * V * sizeof(float)) : cudaStreamSynchronize(st)) != cudaSuccess)
+    return fail_cuda(e, ce, "batch");
+  s->batch_in_flight = false;
   if (take_device_error(e) != 0) return fail(e, LLR_ERR_CUDA, "a device-side wait ran out of iterations");
-  for (size_t oi = 0; oi < n_groups; ++oi) {  // results back in the caller's group order
-    const size_t g = order[oi];
-    if (next_ids) next_ids[g] = win[oi];
-    if (last_logits) std::memcpy(last_logits + g * V, lg.data() + oi * V, V * sizeof(float));
+  for (size_t g = 0; g < n_groups; ++g) {
+    if (next_ids) next_ids[g] = win[g];
     s->position[seq_ids[g]] += counts[g];
     s->have_logits[seq_ids[g]] = 0;  // the single-sequence decode loop keeps its own logits
   }
-  // sequence 0's device-side position follows what was appended to it here
+  // sequence 0's device-side position follows what was appended to it here (the word is written again behind the next batch's wait)
   if (seen[0]) {
-    const int p0 = (int)s->position[0];
-    if ((ce = cudaMemcpyAsync(s->pos_dev, &p0, sizeof(int), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-        (ce = cudaStreamSynchronize(st)) != cudaSuccess)
-      return fail_cuda(e, ce, "position upload");
+    *pos0 = (int)s->position[0];
+    if ((ce = cudaMemcpyAsync(s->pos_dev, pos0, sizeof(int), cudaMemcpyHostToDevice, st)) != cudaSuccess) return fail_cuda(e, ce, "position upload");
   }
   return LLR_OK;
 }

@@ -343,6 +343,8 @@ cudaError_t launch_attention_groups(const float* q, const KvView& kv, float* out
                                     const AttentionGroup* groups, int n_groups, bool tensor_cores, size_t scratch_floats, cudaStream_t s, int* err,
                                     uint64_t* launches);
 cudaError_t launch_swiglu(float* g, const float* u, int64_t n, cudaStream_t s, uint64_t* launches);
+// table[entries[2 i]] = entries[2 i + 1] for i < n
+cudaError_t launch_table_entries(int* table, const int* entries, int n, cudaStream_t s, uint64_t* launches);
 cudaError_t launch_add(float* x, const float* y, int64_t n, cudaStream_t s, uint64_t* launches);
 // first index of the strict maximum of logits[0..n) -> *out_id (device; n == 0: no argmax), and *pos_dev += advance
 // With count_dev the token also goes to out_id[1 + *count_dev], its margin to out_margin[*count_dev], and the

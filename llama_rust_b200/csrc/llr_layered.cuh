@@ -639,7 +639,7 @@ int layered_create(llr_exec* e, const llr_decoder_model* m, size_t n_seq, size_t
   D->scratch_floats = scratch;
   if (lat) { alloc(&D->lat_q, B * lat); alloc(&D->lat_o, B * lat); }
   if (ff) { alloc(&D->gu, B * 2 * ff); alloc(&D->act, B * ff); }
-  if (D->state_floats) { alloc(&D->state, n_seq * D->state_floats); alloc(&D->low, B * low + 8); ialloc(&D->group_first, n_seq + 1); }
+  if (D->state_floats) { alloc(&D->state, n_seq * D->state_floats); alloc(&D->low, B * low + 8); }
   if (prep) alloc(&D->prep, B * prep);
   for (const auto& L : D->layers)
     if (L.mixers.size() == 2 && !D->side && ce == cudaSuccess) {
@@ -659,7 +659,8 @@ int layered_create(llr_exec* e, const llr_decoder_model* m, size_t n_seq, size_t
   alloc(&D->y, D->y_rows * E);
   alloc16(&D->x16, B * E); alloc16(&D->a16, B * a16); alloc16(&D->b16, B * b16);
   ialloc(&s->pos_dev, 1); ialloc(&s->count_dev, 1);
-  ialloc(&s->table_dev, n_seq * s->max_blocks); ialloc(&s->row_pos, B); ialloc(&s->row_seq, B); ialloc(&s->last_rows, s->logits_rows);
+  ialloc(&s->table_dev, n_seq * s->max_blocks); ialloc(&s->last_rows, s->logits_rows);
+  if (ce == cudaSuccess) ce = session_batch_buffers(s);
   if (ce == cudaSuccess) ce = cudaMemset(s->pos_dev, 0, sizeof(int));
   if (ce == cudaSuccess) ce = cudaMemset(s->table_dev, 0, n_seq * s->max_blocks * sizeof(int));
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);

@@ -17,7 +17,9 @@
 // them as vectors.  One warp issues the TMA loads, one the MMAs, four read the accumulators, eight where a CTA has the SM to itself.
 // Two CTAs fit an SM at BN <= 128 (96 KB of stages, 128 columns of tensor memory each), so one tile's epilogue overlaps another's
 // loads.  Wide tiles are bound by what the SMs draw from L2, so 256 activation rows share a stage's weights where that saves waves
-// (tile_shape).  A K range may be cut into slices (gridDim.z): slice s leaves its partial sums at y + s * slice_stride and the reader
+// (tile_shape).  Up to 64 activation rows the product is a stream of weights: a stage then holds 32 or 64 activation rows (the MMA
+// reads on into the weights behind them: rows of its result that nobody looks at), tiles of 32 .. 128 weight rows spread it over the SMs
+// (stream_width) and up to sixteen stages of it are under way.  16384 x 2048 gated, 32 rows: 25 -> 18 us.  A K range may be cut into slices (gridDim.z): slice s leaves its partial sums at y + s * slice_stride and the reader
 // adds them in slice order.  Every wait is bounded.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -36,14 +38,13 @@ constexpr int BM = 128;  // activation rows per MMA = UMMA M
 constexpr int BK = 64;   // columns per stage: one 128-byte swizzle row
 constexpr int SPIN = 1 << 24;
 
-// RT: tiles of BM activation rows per CTA
+// RT: tiles of BM activation rows per CTA; 0: at most 64 activation rows, stages and their number by the launch
 template <int BN, int RT> struct Lay {
   static constexpr int A_STAGE = RT * BM * 128, B_STAGE = BN * 128, STAGE = A_STAGE + B_STAGE;
-  static constexpr int NS = RT == 2 ? 3 : BN == 256 ? 4 : BN == 128 ? 3 : 4;  // 192, 192, 96, 96 KB
+  static constexpr int NS = RT == 0 ? 16 : RT == 2 ? 3 : BN == 256 ? 4 : BN == 128 ? 3 : 4;  // 192, 192, 96, 96 KB
   static constexpr int EPI = BN == 256 ? 8 : 4, W_TMA = EPI, W_MMA = EPI + 1, THREADS = (EPI + 2) * 32;  // epilogue warps first
-  static constexpr int BAR = NS * STAGE;
-  static constexpr int TOTAL = 1024 /*alignment*/ + NS * STAGE + 256;
-  static constexpr int TMEM_COLS = RT * BN;
+  static constexpr int TOTAL = 1024 /*alignment*/ + NS * STAGE + 512;
+  static constexpr int TMEM_COLS = RT == 0 ? BN : RT * BN;
 };
 
 __device__ __forceinline__ uint32_t s32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -67,10 +68,8 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(pred));
   return pred != 0;
 }
-// K-major operand tile of 128-byte swizzled rows: eight-row groups 1024 bytes apart (as in llr_gemm_tc.cu)
-__device__ __forceinline__ uint64_t tile_desc(uint32_t saddr) {
-  return ((uint64_t)(saddr >> 4) & 0x3fffu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
+// Operand tiles are K-major 128-byte swizzled rows, eight-row groups 1024 bytes apart: the high word of their descriptors is always this
+constexpr uint32_t DESC_HI = 64u | (1u << 14) | (2u << 29);
 // kind::f16: f32 accumulator, both operands bfloat16, M = 128, N = bn
 __device__ __forceinline__ uint32_t mma_desc(int bn) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
@@ -83,6 +82,7 @@ struct Args {
   int64_t y_ld, gate_ld, slice_stride;
   int tokens, rows, nk, xk;  // nk: 64-column steps of the whole K range
   int batch, slices, bn;
+  int a_rows, stages;  // activation rows of a stage, stages (RT 0)
   GluShape glu;
 };
 
@@ -98,21 +98,29 @@ __device__ __forceinline__ void load32(uint32_t taddr, uint32_t (&v)[32]) {
       : "r"(taddr) : "memory");
 }
 
+__device__ __forceinline__ void load8(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr) : "memory");
+}
+
 template <int BN, int RT, bool GLU>
 __global__ void __launch_bounds__(Lay<BN, RT>::THREADS)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const Args a, int* __restrict__ err) {
   using L = Lay<BN, RT>;
-  constexpr int NS = L::NS, W_TMA = L::W_TMA, W_MMA = L::W_MMA;
+  constexpr int W_TMA = L::W_TMA, W_MMA = L::W_MMA;
+  constexpr bool STREAM = RT == 0;
+  const int NS = STREAM ? a.stages : L::NS, A_STAGE = STREAM ? a.a_rows * 128 : L::A_STAGE, STAGE = STREAM ? A_STAGE + a.bn * 128 : L::STAGE;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint64_t* full = (uint64_t*)(smem + L::BAR);
-  uint64_t* empty = full + NS;
-  uint64_t* done = empty + NS;
+  // behind the stages, and behind what the last one's MMA reads past its activation rows
+  uint64_t* full = (uint64_t*)(smem + NS * STAGE + (STREAM ? BM * 128 : 0));
+  uint64_t* empty = full + L::NS;
+  uint64_t* done = empty + L::NS;
   uint32_t* tmem_slot = (uint32_t*)(done + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int bn = a.bn, width = GLU ? bn / 2 : bn;  // results per activation row of the tile
   // token tiles run fastest: the CTAs that share weight rows run at the same time, and the weights are read from HBM once
-  const int row0 = blockIdx.y * width, tok0 = blockIdx.x * (RT * BM);
+  const int row0 = blockIdx.y * width, tok0 = blockIdx.x * ((STREAM ? 1 : RT) * BM);
   const int z = (int)blockIdx.z / a.slices, slice = (int)blockIdx.z % a.slices;
   const int per = (a.nk + a.slices - 1) / a.slices, k0 = slice * per, k1 = min(a.nk, k0 + per);  // never empty: the launcher sees to it
 
@@ -136,12 +144,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
   if (warp == W_TMA) {
     const uint32_t base = __shfl_sync(0xffffffffu, s32(smem), 0);
     auto load_w = [&](int k, int s) {
-      bar_expect(&full[s], (uint32_t)(L::A_STAGE + bn * 128));  // boxes are always complete: what lies outside the matrices is filled with zeros
+      bar_expect(&full[s], (uint32_t)(A_STAGE + bn * 128));  // boxes are always complete: what lies outside the matrices is filled with zeros
       asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                   ::"r"(base + (uint32_t)(s * L::STAGE + L::A_STAGE)), "l"(&wmap), "r"(k * BK), "r"(z * a.rows + row0), "r"(s32(&full[s])) : "memory");
+                   ::"r"(base + (uint32_t)(s * STAGE + A_STAGE)), "l"(&wmap), "r"(k * BK), "r"(z * a.rows + row0), "r"(s32(&full[s])) : "memory");
       if constexpr (GLU)
         asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                     ::"r"(base + (uint32_t)(s * L::STAGE + L::A_STAGE + width * 128)), "l"(&wmap), "r"(k * BK), "r"(a.rows + row0), "r"(s32(&full[s])) : "memory");
+                     ::"r"(base + (uint32_t)(s * STAGE + A_STAGE + width * 128)), "l"(&wmap), "r"(k * BK), "r"(a.rows + row0), "r"(s32(&full[s])) : "memory");
     };
     // the first stages' weights are on their way while the kernel before this one still runs; its results are waited for
     const int ahead = min(NS, k1 - k0);
@@ -150,90 +158,146 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
       __syncwarp();
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    const bool leader = elect_one();
+    uint32_t s = 0, lap = 0;
     for (int k = k0; k < k1; ++k) {
-      const int s = (k - k0) % NS;
-      if (ok && !bar_wait(&empty[s], (uint32_t)((((k - k0) / NS) & 1) ^ 1))) { ok = false; report_error(err, 5); }
-      if (ok && elect_one()) {
-        if (k - k0 >= ahead) load_w(k, s);
+      if (ok && !bar_wait(&empty[s], lap ^ 1)) { ok = false; report_error(err, 5); }
+      if (ok && leader) {
+        if (k - k0 >= ahead) load_w(k, (int)s);
         asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                     ::"r"(base + (uint32_t)(s * L::STAGE)), "l"(&xmap), "r"(z * a.xk + k * BK), "r"(tok0), "r"(s32(&full[s])) : "memory");
+                     ::"r"(base + s * (uint32_t)STAGE), "l"(&xmap), "r"(z * a.xk + k * BK), "r"(tok0), "r"(s32(&full[s])) : "memory");
       }
-      __syncwarp();
+      if (++s == (uint32_t)NS) { s = 0; lap ^= 1; }
     }
+    __syncwarp();
   } else if (warp == W_MMA) {
-    const uint32_t idesc = mma_desc(bn);
-    const uint32_t td = __shfl_sync(0xffffffffu, tmem, 0), base = __shfl_sync(0xffffffffu, s32(smem), 0);
+    // One thread issues, and what it needs per step is kept ready: a step of four MMAs of N = 128 takes 256 cycles, and with a division
+    // for its stage, an election and 64-bit descriptors the step took 600.
+    const uint32_t idesc = mma_desc(bn), td = __shfl_sync(0xffffffffu, tmem, 0), base = __shfl_sync(0xffffffffu, s32(smem), 0) >> 4;
+    const bool leader = elect_one();
+    uint32_t s = 0, lap = 0, lo = base;  // low words of the operands' descriptors: addresses below 2^18, in units of 16 bytes
     for (int k = k0; k < k1; ++k) {
-      const int s = (k - k0) % NS;
-      if (ok && !bar_wait(&full[s], (uint32_t)(((k - k0) / NS) & 1))) { ok = false; report_error(err, 5); }
+      if (ok && !bar_wait(&full[s], lap)) { ok = false; report_error(err, 5); }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (elect_one()) {
-        const uint64_t da = tile_desc(base + (uint32_t)(s * L::STAGE)), db = tile_desc(base + (uint32_t)(s * L::STAGE + L::A_STAGE));
+      if (leader) {
+        const uint32_t lb = lo + (uint32_t)(A_STAGE / 16), first = k > k0 ? 1u : 0u;
 #pragma unroll
-        for (int kk = 0; kk < BK / 16; ++kk) {
-          const uint32_t acc = (k > k0 || kk > 0) ? 1u : 0u;
+        for (int kk = 0; kk < BK / 16; ++kk)
 #pragma unroll
-          for (int r = 0; r < RT; ++r)
-            asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }"
-                         ::"r"(td + (uint32_t)(r * BN)), "l"(da + (uint64_t)(r * BM * 128 / 16 + 2 * kk)), "l"(db + 2 * kk), "r"(idesc), "r"(acc) : "memory");
-        }
+          for (int r = 0; r < (STREAM ? 1 : RT); ++r)
+            asm volatile("{ .reg .pred p; .reg .b64 a, b; setp.ne.b32 p, %5, 0; mov.b64 a, {%1, %3}; mov.b64 b, {%2, %3}; "
+                         "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p; }"
+                         ::"r"(td + (uint32_t)(r * BN)), "r"(lo + (uint32_t)(r * BM * 128 / 16 + 2 * kk)), "r"(lb + (uint32_t)(2 * kk)), "r"(DESC_HI), "r"(idesc),
+                           "r"(kk > 0 ? 1u : first) : "memory");
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(&empty[s])) : "memory");
       }
-      __syncwarp();
+      lo += (uint32_t)(STAGE / 16);
+      if (++s == (uint32_t)NS) { s = 0; lap ^= 1; lo = base; }
     }
-    if (elect_one())
+    if (leader)
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(done)) : "memory");
     __syncwarp();
   } else {
     asm volatile("griddepcontrol.wait;" ::: "memory");  // gates; results may still be read by an earlier kernel
     if (!bar_wait(done, 0)) { ok = false; report_error(err, 5); }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    // warps 4.. read the second tile of activation rows, or every other run of columns of the only one
-    const int r = RT == 2 ? warp >> 2 : 0, t = tok0 + BM * r + 32 * (warp & 3) + lane;
-    constexpr int C_STEP = RT == 1 ? 8 * L::EPI : 32;
     const int n_live = min(width, a.rows - row0);
-    const int64_t off = (int64_t)t * a.y_ld + (int64_t)z * a.rows + row0;
-    float* y = a.y ? a.y + slice * a.slice_stride + off : nullptr;
-    __nv_bfloat16* y16 = a.y16 ? a.y16 + off : nullptr;
-    float gate = 1.f;
-    if (a.gate && t < a.tokens) gate = 1.0f / (1.0f + expf(-a.gate[(int64_t)t * a.gate_ld + z]));
-    const bool vec = ((a.y_ld | a.rows) & 7) == 0;  // every run of eight results starts on a 16-byte boundary in either format
+    // The code of an epilogue runs once per block, cold: straight-line gated units for 32 columns took 8 us to fetch (28672 x 4096
+    // gated, 512 rows: 118 -> 107 us with eight).  Few columns per
+    // round, and a stream of weights, whose results lie in one or two warps' lanes, spreads them over all four through shared memory.
+    if constexpr (STREAM) {
+      float* turn = (float*)smem;  // every stage has been read
+      const int pitch = bn + 1;
+      float g[2] = {1.f, 1.f};  // gates of tokens lane, 32 + lane
+      if (a.gate) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+          if (32 * k + lane < a.tokens) g[k] = 1.0f / (1.0f + expf(-a.gate[(int64_t)(32 * k + lane) * a.gate_ld + z]));
+      }
+      if (32 * warp < a.a_rows) {
 #pragma unroll 1
-    for (int c0 = RT == 1 ? 32 * (warp >> 2) : 0; c0 < n_live; c0 += C_STEP) {
-      uint32_t v[32], u[32];
-      const uint32_t taddr = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(r * BN + c0);
-      load32(taddr, v);
-      if constexpr (GLU) load32(taddr + (uint32_t)width, u);
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (t < a.tokens) {
-        float f[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          if constexpr (GLU) f[j] = gated_unit(__uint_as_float(v[j]), __uint_as_float(u[j]), a.glu);
-          else f[j] = a.gate ? __uint_as_float(v[j]) * gate : __uint_as_float(v[j]);
-        }
-        if (vec) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 8)
-            if (c0 + j < n_live) {  // rows is a multiple of eight here
-              if (y) {
-                *(float4*)(y + c0 + j) = make_float4(f[j], f[j + 1], f[j + 2], f[j + 3]);
-                *(float4*)(y + c0 + j + 4) = make_float4(f[j + 4], f[j + 5], f[j + 6], f[j + 7]);
-              }
-              if (y16) {
-                __nv_bfloat162 h[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) h[u] = __floats2bfloat162_rn(f[j + 2 * u], f[j + 2 * u + 1]);
-                *(uint4*)(y16 + c0 + j) = *(const uint4*)h;
-              }
-            }
-        } else {
+        for (int c0 = 0; c0 < bn; c0 += 32) {
+          uint32_t v[32];
+          load32(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0, v);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
           for (int j = 0; j < 32; ++j)
+            if (c0 + j < bn) turn[(32 * warp + lane) * pitch + c0 + j] = __uint_as_float(v[j]);
+        }
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * L::EPI) : "memory");
+#pragma unroll 1
+      for (int t = warp; t < a.tokens; t += L::EPI) {
+        const float gate = __shfl_sync(~0u, t < 32 ? g[0] : g[1], t & 31);
+        const int64_t off = (int64_t)t * a.y_ld + (int64_t)z * a.rows + row0;
+#pragma unroll 1
+        for (int c = lane; c < n_live; c += 32) {
+          float f = turn[t * pitch + c];
+          if constexpr (GLU) f = gated_unit(f, turn[t * pitch + width + c], a.glu);
+          else f = a.gate ? f * gate : f;
+          if (a.y) a.y[slice * a.slice_stride + off + c] = f;
+          if (a.y16) a.y16[off + c] = __float2bfloat16_rn(f);
+        }
+        __syncwarp();
+      }
+    } else {
+      // warps 4.. read the second tile of activation rows, or every other run of columns of the only one
+      constexpr int W = 8;  // columns of a round
+      const int r = RT == 2 ? warp >> 2 : 0, t = tok0 + BM * r + 32 * (warp & 3) + lane;
+      constexpr int C_STEP = RT == 1 ? W * L::EPI / 4 : W;
+      const int64_t off = (int64_t)t * a.y_ld + (int64_t)z * a.rows + row0;
+      float* y = a.y ? a.y + slice * a.slice_stride + off : nullptr;
+      __nv_bfloat16* y16 = a.y16 ? a.y16 + off : nullptr;
+      float gate = 1.f;
+      if (a.gate && t < a.tokens) gate = 1.0f / (1.0f + expf(-a.gate[(int64_t)t * a.gate_ld + z]));
+      const bool vec = ((a.y_ld | a.rows) & 7) == 0;  // every run of eight results starts on a 16-byte boundary in either format
+      const uint32_t taddr = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(r * BN);
+      const int c_first = RT == 1 ? W * (warp >> 2) : 0;
+      uint32_t v[2][W], u[2][W];  // the next round's are on their way while one is worked on
+      auto fetch = [&](int c0, int k) {
+        load8(taddr + (uint32_t)c0, v[k]);
+        if constexpr (GLU) load8(taddr + (uint32_t)(width + c0), u[k]);
+      };
+      auto finish = [&](int c0, int k) {
+        if (t >= a.tokens) return;
+        float f[W];
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+          if constexpr (GLU) f[j] = gated_unit(__uint_as_float(v[k][j]), __uint_as_float(u[k][j]), a.glu);
+          else f[j] = a.gate ? __uint_as_float(v[k][j]) * gate : __uint_as_float(v[k][j]);
+        }
+        if (vec) {  // rows is a multiple of eight here
+          if (y) {
+            *(float4*)(y + c0) = make_float4(f[0], f[1], f[2], f[3]);
+            *(float4*)(y + c0 + 4) = make_float4(f[4], f[5], f[6], f[7]);
+          }
+          if (y16) {
+            __nv_bfloat162 h[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) h[u] = __floats2bfloat162_rn(f[2 * u], f[2 * u + 1]);
+            *(uint4*)(y16 + c0) = *(const uint4*)h;
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < W; ++j)
             if (c0 + j < n_live) {
               if (y) y[c0 + j] = f[j];
               if (y16) y16[c0 + j] = __float2bfloat16_rn(f[j]);
             }
+        }
+      };
+      if (c_first < n_live) fetch(c_first, 0);
+#pragma unroll 1
+      for (int c0 = c_first; c0 < n_live; c0 += 2 * C_STEP) {
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (c0 + C_STEP < n_live) fetch(c0 + C_STEP, 1);
+        finish(c0, 0);
+        __syncwarp();
+        if (c0 + C_STEP < n_live) {
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (c0 + 2 * C_STEP < n_live) fetch(c0 + 2 * C_STEP, 0);
+          finish(c0 + C_STEP, 1);
+          __syncwarp();
         }
       }
     }
@@ -257,21 +321,24 @@ bool encode_rows(CUtensorMap* map, const void* base, int64_t cols, int64_t rows,
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+constexpr int STREAM_SMEM = 1024 + 200 * 1024 + BM * 128 + 512;
+
 template <int BN, int RT, bool GLU>
 cudaError_t launch_tiles(const Bf16Product& p, const Args& a, cudaStream_t stream, int* err) {
   CUtensorMap xmap, wmap;
   const int width = GLU ? a.bn / 2 : a.bn;  // rows of one box of W
-  if (!encode_rows(&xmap, p.x16, p.x_cols, p.tokens, p.x_ld, RT * BM) || !encode_rows(&wmap, p.w, p.cols, (int64_t)p.rows * (GLU ? 2 : p.batch), p.cols, width))
+  if (!encode_rows(&xmap, p.x16, p.x_cols, p.tokens, p.x_ld, RT == 0 ? a.a_rows : RT * BM) || !encode_rows(&wmap, p.w, p.cols, (int64_t)p.rows * (GLU ? 2 : p.batch), p.cols, width))
     return cudaErrorInvalidValue;
-  constexpr int smem = Lay<BN, RT>::TOTAL;
+  const int smem = RT == 0 ? 1024 + a.stages * (a.a_rows + a.bn) * 128 + BM * 128 + 512 : Lay<BN, RT>::TOTAL;
   static PerDevice ready;
   std::atomic<int>& slot = ready.here();
   if (slot.load(std::memory_order_relaxed) == 0) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, RT, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, RT, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, RT == 0 ? STREAM_SMEM : smem);
     if (e != cudaSuccess) return e;
     slot.store(1, std::memory_order_relaxed);
   }
-  const dim3 grid((unsigned)((p.tokens + RT * BM - 1) / (RT * BM)), (unsigned)((p.rows + width - 1) / width), (unsigned)(p.batch * a.slices));
+  constexpr int TOK = RT == 0 ? BM : RT * BM;
+  const dim3 grid((unsigned)((p.tokens + TOK - 1) / TOK), (unsigned)((p.rows + width - 1) / width), (unsigned)(p.batch * a.slices));
   if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidValue;
   return launch_overlapped(gemm_bf16_kernel<BN, RT, GLU>, grid, Lay<BN, RT>::THREADS, smem, stream, xmap, wmap, a, err);
 }
@@ -282,7 +349,7 @@ int tiles_of(int tokens, int rows, int batch, int bn, int rt = 1) { return ((tok
 // gated tile are whole eight-row groups) and one or two tiles of 128 activation rows, for which the waves over the SMs cost least.
 // What a wave costs was measured at 4096 columns, 512 activation rows: 27 / 31 / 33 us with 160 / 224 / 256 weight rows, 43 / 54 /
 // 58 us with two tiles of activation rows.  The stages come from L2 at about 50 bytes a cycle and SM, which is what bounds a
-// wave; the second tile of activation rows uses a stage's weights again.  28672 x 4096: 126 -> 111 us, 16384 x 2048: 54 -> 44,
+// wave; the second tile of activation rows uses a stage's weights again.  28672 x 4096: 126 -> 111 us (107 with the short epilogue), 16384 x 2048: 54 -> 44,
 // 10240 x 4096: 64 -> 54, and with the wide tile from 120 tiles on (132 before) 8192 x 4096: 43 -> 39.
 struct Tile { int bn, rt; };
 Tile tile_shape(int tokens, int rows, int batch, int step = 16) {
@@ -294,6 +361,19 @@ Tile tile_shape(int tokens, int rows, int batch, int step = 16) {
       const int c = (tiles_of(tokens, rows, batch, bn, rt) + SMS - 1) / SMS * (rt == 1 ? 5 * bn + 1410 : 12 * bn + 1640);
       if (c < cost) { cost = c; best = {bn, rt}; }
     }
+  return best;
+}
+
+// At most 64 activation rows: the width of a tile, for which the weights an SM draws (in waves of a tile per SM, the activations of a
+// tile at half their bytes: they come from L2) are fewest.  The stages then fill an SM's shared memory, or half of it where blocks share one.
+constexpr int STREAM_TOKENS = 64;
+int stream_width(int tokens, int rows, int batch, int slices) {
+  int best = 128;
+  int64_t cost = INT64_MAX;
+  for (int bn = 128; bn >= 32; bn -= 16) {
+    const int64_t waves = ((int64_t)tiles_of(tokens, rows, batch, bn) * slices + SMS - 1) / SMS, c = waves * (bn + (tokens > 32 ? 32 : 16) + 8);
+    if (c < cost) { cost = c; best = bn; }
+  }
   return best;
 }
 
@@ -328,8 +408,15 @@ cudaError_t launch_gemm_bf16(const Bf16Product& p, cudaStream_t stream, int* err
   a.batch = p.batch; a.slices = p.slices;
   if ((a.slices - 1) * ((a.nk + a.slices - 1) / a.slices) >= a.nk) return cudaErrorInvalidValue;
   if (launches) ++*launches;
+  if (p.glu) a.glu = *p.glu;
+  if (p.tokens <= STREAM_TOKENS) {
+    a.bn = stream_width(p.tokens, p.rows * (p.glu ? 2 : 1), p.batch, p.slices);
+    a.a_rows = p.tokens > 32 ? 64 : 32;
+    const bool alone = (int64_t)tiles_of(p.tokens, p.rows * (p.glu ? 2 : 1), p.batch, a.bn) * p.slices <= SMS;
+    a.stages = std::max(4, std::min(16, (alone ? 200 : 80) * 1024 / ((a.a_rows + a.bn) * 128)));
+    return p.glu ? launch_tiles<128, 0, true>(p, a, stream, err) : launch_tiles<128, 0, false>(p, a, stream, err);
+  }
   if (p.glu) {
-    a.glu = *p.glu;
     const Tile tile = tile_shape(p.tokens, 2 * p.rows, 1, 32);
     a.bn = std::max(tile.bn, 128);
     return tile.rt == 2 ? launch_tiles<256, 2, true>(p, a, stream, err) : a.bn > 128 ? launch_tiles<256, 1, true>(p, a, stream, err)

@@ -50,6 +50,7 @@ using umma::bar_expect;
 using umma::bar_init;
 using umma::bar_wait;
 using umma::elect_one;
+using umma::DESC_HI;
 using umma::s32;
 
 __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
@@ -186,8 +187,6 @@ __host__ __device__ constexpr uint32_t mma_desc(int n, bool mn_major_b) {
   return (1u << 4) | ((mn_major_b ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(PAIRS >> 4) << 24);
 }
 
-// Shared-memory operands are 128-byte swizzled rows, groups of eight 1024 bytes apart: the high word of their descriptors is always this
-constexpr uint32_t DESC_HI = 64u | (1u << 14) | (2u << 29);
 __device__ __forceinline__ void mma_ss(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t add) {
   asm volatile("{ .reg .pred p; .reg .b64 a, b; setp.ne.b32 p, %5, 0; mov.b64 a, {%1, %3}; mov.b64 b, {%2, %3}; "
                "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p; }"

@@ -439,6 +439,34 @@ __device__ __forceinline__ void dequant_sub_h(uint32_t prow, uint32_t (&out)[16]
   }
 }
 
+// Sub-blocks SB and SB + 4 of a Q4_K row (SB < 4) as binary16: what dequant_sub_h computes, from one read of the block's header.
+// The six-bit scales of the first lie in the low bits of their bytes, those of the second in nibbles and top bits: no selection at run time.
+__device__ __forceinline__ void dequant_pair_q4k_h(uint32_t prow, int sb, uint32_t (&o0)[16], uint32_t (&o1)[16]) {
+  uint32_t hdr[4], q0[8], q1[8];
+  lds_chunks<1>(prow, hdr);
+  lds_chunks<2>(prow + 16 + 32 * (sb >> 1), q0);
+  lds_chunks<2>(prow + 80 + 32 * (sb >> 1), q1);
+  const float d = h2f(hdr[0] & 0xffffu), dmin = h2f(hdr[0] >> 16);
+  const int sh = 8 * sb;
+  const uint32_t lo = hdr[1] >> sh, mid = hdr[2] >> sh, hi = hdr[3] >> sh;
+  const uint32_t sc0 = lo & 63u, mn0 = mid & 63u, sc1 = (hi & 15u) | ((lo >> 2) & 48u), mn1 = ((hi >> 4) & 15u) | ((mid >> 2) & 48u);
+  const __half2 a0 = __float2half2_rn(d * (float)sc0), n0 = __float2half2_rn(-(dmin * (float)mn0));
+  const __half2 a1 = __float2half2_rn(d * (float)sc1), n1 = __float2half2_rn(-(dmin * (float)mn1));
+  if (sb & 1) {  // warp-uniform
+    const __half2 off = __float2half2_rn(64.f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) emit4h<0x00f000f0u, 0x54005400u>(q0[i], off, a0, n0, o0[2 * i], o0[2 * i + 1]);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) emit4h<0x00f000f0u, 0x54005400u>(q1[i], off, a1, n1, o1[2 * i], o1[2 * i + 1]);
+  } else {
+    const __half2 off = __float2half2_rn(1024.f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) emit4h<0x000f000fu, 0x64006400u>(q0[i], off, a0, n0, o0[2 * i], o0[2 * i + 1]);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) emit4h<0x000f000fu, 0x64006400u>(q1[i], off, a1, n1, o1[2 * i], o1[2 * i + 1]);
+  }
+}
+
 // One 128-row x BN-token tile.  The tensor maps are addressed generically: kernel parameters for a
 // single product, an array in global memory for a grouped launch.
 template <int DT, int BN, bool F16>
@@ -514,14 +542,22 @@ __device__ __forceinline__ void gemm_tc_tile(const CUtensorMap* wmap_p, const CU
     // Per macro-step a warp decodes both of its 64-column steps (g and g + 2) back to back: two
     // independent instruction streams for the scheduler, and one round of barrier waits, tensor
     // memory store completion and arrivals for two steps instead of one each.
-    static_assert(NA % 2 == 0 && NA >= 4, "a group's two steps of a macro-step use different stages");
+    static_assert(NA % 2 == 0 && NA > 4, "a group's two steps of a macro-step use different stages");
+    // One warp issues a group's steps in order, so the later one's stage is free only after the earlier one's.  Asking a barrier takes
+    // 100 ns: where decoding is short (Q4_K) both of a macro-step's are asked in one go before it, elsewhere the stage's comes behind it
+    // (77 rows of Q5_1 84.2 us that way, 85.2 asked before).
+    constexpr bool FIRST = DT == DT_Q4_K && F16;
+    int ps = 0, s0 = g;
+    int s1 = g + 2;
+    uint32_t lp = 0, l1 = 0;
     for (int ms = 0; ms < nms; ++ms) {
-      const int ps = ms % NPK;
-      if (ok && !bar_wait(&pk_full[ps], (uint32_t)((ms / NPK) & 1))) { ok = false; report_error(err, 3); }
+      if (ok && !(FIRST ? bar_wait2(&pk_full[ps], lp, &empty_a[s1], l1 ^ 1) : bar_wait(&pk_full[ps], lp))) { ok = false; report_error(err, 3); }
       const uint32_t prow = s32(sP) + ps * L::P_STAGE + r * PITCH;
       if constexpr (DT == DT_Q6_K) lead = ((ms_begin + ms) * RB) & 15;
       uint32_t o0[16], o1[16];
-      if (g == 0) {
+      if constexpr (DT == DT_Q4_K && F16) {
+        dequant_pair_q4k_h(prow, 2 * g + h, o0, o1);
+      } else if (g == 0) {
         decode(std::integral_constant<int, 0>{}, prow, o0);
         decode(std::integral_constant<int, 2>{}, prow, o1);
       } else {
@@ -530,11 +566,7 @@ __device__ __forceinline__ void gemm_tc_tile(const CUtensorMap* wmap_p, const CU
       }
       __syncwarp();
       if (lane == 0) bar_arrive(&pk_empty[ps]);  // the packed bytes are in registers now
-      const int ks0 = 4 * ms + g, ks1 = ks0 + 2, s0 = ks0 % NA, s1 = ks1 % NA;
-      if (ok && !bar_wait2(&empty_a[s0], (uint32_t)(((ks0 / NA) & 1) ^ 1), &empty_a[s1], (uint32_t)(((ks1 / NA) & 1) ^ 1))) {
-        ok = false;
-        report_error(err, 3);
-      }
+      if (!FIRST && ok && !bar_wait(&empty_a[s1], l1 ^ 1)) { ok = false; report_error(err, 3); }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       put(o0, s0);
       put(o1, s1);
@@ -542,6 +574,9 @@ __device__ __forceinline__ void gemm_tc_tile(const CUtensorMap* wmap_p, const CU
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) { bar_arrive(&full_a[s0]); bar_arrive(&full_a[s1]); }
+      if (++ps == NPK) { ps = 0; lp ^= 1; }
+      s0 = s0 + 4 >= NA ? s0 + 4 - NA : s0 + 4;
+      if ((s1 += 4) >= NA) { s1 -= NA; l1 ^= 1; }
     }
     // --------------------------------------------------------------- epilogue
     // Bound by the stores (128 bytes per warp and token) and by whatever latency stands between them: all sixteen warps take a
@@ -625,17 +660,20 @@ __device__ __forceinline__ void gemm_tc_tile(const CUtensorMap* wmap_p, const CU
     // the warp walks the ring converged (uniform registers for the addresses), one elected lane issues
     const uint32_t sb_u = __shfl_sync(0xffffffffu, s32(sB), 0);
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the activations are the conversion kernel's output
+    const bool leader = elect_one();
+    int s = 0;
+    uint32_t lap = 0;
     for (int ks = 0; ks < nk; ++ks) {
-      const int s = ks % NB;
-      if (ok && !bar_wait(&empty_b[s], (uint32_t)(((ks / NB) & 1) ^ 1))) { ok = false; report_error(err, 3); }
-      if (elect_one()) {
+      if (ok && !bar_wait(&empty_b[s], lap ^ 1)) { ok = false; report_error(err, 3); }
+      if (leader) {
         bar_expect(&full_b[s], BN * 128);
         asm volatile(
             "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
             ::"r"(sb_u + (uint32_t)(s * L::B_STAGE)), "l"(xmap_p), "r"((ms_begin * (MACRO / BK) + ks) * BK), "r"(tok0), "r"(s32(&full_b[s])) : "memory");
       }
-      __syncwarp();
+      if (++s == NB) { s = 0; lap ^= 1; }
     }
+    __syncwarp();
   } else {
     // ------------------------------------------------------------------- MMA
     // The whole warp walks the loop converged and one elected lane issues: addresses, descriptors
@@ -648,33 +686,29 @@ __device__ __forceinline__ void gemm_tc_tile(const CUtensorMap* wmap_p, const CU
       const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
       const uint32_t sb_u = __shfl_sync(0xffffffffu, s32(sB), 0);
       const uint32_t td = tmem_u + (uint32_t)(mw * BN);
+      const bool leader = elect_one();
+      int sa = mw, sb = mw;          // stages of this warp's next step, and their laps around the rings
+      uint32_t la = 0, lb = 0;
       for (int ks = mw; ks < nk; ks += NMMA) {  // nk is a multiple of 4
-        const int sa = ks % NA, sb = ks % NB;
-        if (ok && !bar_wait2(&full_a[sa], (uint32_t)((ks / NA) & 1), &full_b[sb], (uint32_t)((ks / NB) & 1))) {
+        if (ok && !bar_wait2(&full_a[sa], la, &full_b[sb], lb)) {
           ok = false;
           report_error(err, 3);
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (elect_one()) {
-          const uint32_t ta = tmem_u + (uint32_t)(NMMA * BN + sa * L::A_COLS);
-          const uint64_t db = smem_desc_u(sb_u + (uint32_t)(sb * L::B_STAGE));
+        if (leader) {
+          const uint32_t ta = tmem_u + (uint32_t)(NMMA * BN + sa * L::A_COLS), db = (sb_u + (uint32_t)(sb * L::B_STAGE)) >> 4;
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) {
-            // 16 values along K: eight 32-bit columns of A; 32 bytes inside B's swizzled row = 2 x 16-byte units
-            if (kk == 0 && ks == mw)
-              asm volatile("{ .reg .pred p; setp.ne.b32 p, 0, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }"
-                           ::"r"(td), "r"(ta), "l"(db), "r"(idesc) : "memory");
-            else
-              asm volatile("{ .reg .pred p; setp.eq.b32 p, 0, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }"
-                           ::"r"(td), "r"(ta + 8 * kk), "l"(db + 2 * kk), "r"(idesc) : "memory");
-          }
+          for (int kk = 0; kk < BK / 16; ++kk)  // 16 values along K: eight 32-bit columns of A; 32 bytes inside B's swizzled row = 2 x 16-byte units
+            asm volatile("{ .reg .pred p; .reg .b64 b; setp.ne.b32 p, %5, 0; mov.b64 b, {%2, %3}; tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p; }"
+                         ::"r"(td), "r"(ta + (uint32_t)(8 * kk)), "r"(db + (uint32_t)(2 * kk)), "r"(DESC_HI), "r"(idesc), "r"(kk > 0 || ks > mw ? 1u : 0u) : "memory");
           // free both stages once the MMAs that read them have completed
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(&empty_a[sa])) : "memory");
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(&empty_b[sb])) : "memory");
         }
-        __syncwarp();
+        if ((sa += NMMA) >= NA) { sa -= NA; la ^= 1; }
+        if ((sb += NMMA) >= NB) { sb -= NB; lb ^= 1; }
       }
-      if (elect_one())
+      if (leader)
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(acc_full)) : "memory");
       __syncwarp();
     }

@@ -74,6 +74,8 @@ __device__ __forceinline__ uint64_t smem_desc_u(uint32_t saddr) {
   return addr | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
 
+constexpr uint32_t DESC_HI = 64u | (1u << 14) | (2u << 29);  // its high word; the low word of addresses below 2^18 without leading offset: address / 16
+
 __device__ __forceinline__ float h2f(uint32_t h) { return __half2float(__ushort_as_half((unsigned short)h)); }
 // Shared memory is addressed through 32-bit shared-window addresses and explicit ld/st.shared:
 // the tile base is aligned by integer arithmetic, which would otherwise turn every access

@@ -396,7 +396,6 @@ __global__ void __launch_bounds__(128)
 attention_combine_kernel(const float* part, float* __restrict__ out, RowMap rows, int chunk, WalkShape w, int heads_per_block,
                          const __grid_constant__ RowRanges finished) {
   pdl_enter();
-  if (finished.has((int)blockIdx.y)) return;
   // heads_per_block 4: one warp per head (many rows: fewer, fuller blocks); 1: the four warps share a head's
   // dimensions (a decode step has few blocks to fill the device with)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -406,6 +405,7 @@ attention_combine_kernel(const float* part, float* __restrict__ out, RowMap rows
   const int hd = w.head_dim, gqa = w.n_head / w.n_head_kv;
   const int hkv = hq / gqa, g = hq % gqa;
   const int seq = row_position(rows, t) + 1;
+  if (finished.has(t)) return;  // behind the load: the list's first look into the constant bank takes as long
   const int n_split = (w.n_ctx + chunk - 1) / chunk, used = min(n_split, (seq + chunk - 1) / chunk);
   const float* base = part + ((int64_t)t * w.n_head_kv + hkv) * n_split * gqa * (hd + 2) + g * (hd + 2);
   const int64_t stride = (int64_t)gqa * (hd + 2);

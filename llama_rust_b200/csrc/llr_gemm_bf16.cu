@@ -41,9 +41,10 @@ constexpr int SPIN = 1 << 24;
 // RT: tiles of BM activation rows per CTA; 0: at most 64 activation rows, stages and their number by the launch
 template <int BN, int RT> struct Lay {
   static constexpr int A_STAGE = RT * BM * 128, B_STAGE = BN * 128, STAGE = A_STAGE + B_STAGE;
-  static constexpr int NS = RT == 0 ? 16 : RT == 2 ? 3 : BN == 256 ? 4 : BN == 128 ? 3 : 4;  // 192, 192, 96, 96 KB
-  static constexpr int EPI = BN == 256 ? 8 : 4, W_TMA = EPI, W_MMA = EPI + 1, THREADS = (EPI + 2) * 32;  // epilogue warps first
-  static constexpr int TOTAL = 1024 /*alignment*/ + NS * STAGE + 512;
+  static constexpr int NS = RT == 0 ? 16 : RT == 2 ? 8 : BN == 256 ? 4 : BN == 128 ? 3 : 4;  // 192, 96, 96 KB
+  static constexpr int NB = 4;  // two tiles of activation rows: stages of weights, beside a ring of at most NS single tiles
+  static constexpr int EPI = BN < 256 ? 4 : RT == 2 ? 16 : 8, W_TMA = EPI, W_MMA = EPI + 1, THREADS = (EPI + 2 + (RT == 2)) * 32;  // epilogue warps first
+  static constexpr int TOTAL = RT == 2 ? 232448 : 1024 /*alignment*/ + NS * STAGE + 512;
   static constexpr int TMEM_COLS = RT == 0 ? BN : RT * BN;
 };
 
@@ -59,6 +60,18 @@ __device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t parity) {
     uint32_t ok;
     asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
                  : "=r"(ok) : "r"(s32(b)), "r"(parity) : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+// both barriers asked in one go
+__device__ __forceinline__ bool bar_wait2(uint64_t* a, uint32_t pa, uint64_t* b, uint32_t pb) {
+  for (int spins = 0; spins < SPIN; ++spins) {
+    uint32_t ok;
+    asm volatile(
+        "{ .reg .pred p, q; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4; "
+        "and.pred p, p, q; selp.u32 %0, 1, 0, p; }"
+        : "=r"(ok) : "r"(s32(a)), "r"(pa), "r"(s32(b)), "r"(pb) : "memory");
     if (ok) return true;
   }
   return false;
@@ -103,19 +116,28 @@ __device__ __forceinline__ void load8(uint32_t taddr, uint32_t (&v)[8]) {
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr) : "memory");
 }
 
+// operands by the low words of their descriptors
+__device__ __forceinline__ void mma(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t add) {
+  asm volatile("{ .reg .pred p; .reg .b64 a, b; setp.ne.b32 p, %5, 0; mov.b64 a, {%1, %3}; mov.b64 b, {%2, %3}; "
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p; }"
+               ::"r"(d), "r"(a), "r"(b), "r"(DESC_HI), "r"(idesc), "r"(add) : "memory");
+}
+
 template <int BN, int RT, bool GLU>
 __global__ void __launch_bounds__(Lay<BN, RT>::THREADS)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const Args a, int* __restrict__ err) {
   using L = Lay<BN, RT>;
   constexpr int W_TMA = L::W_TMA, W_MMA = L::W_MMA;
-  constexpr bool STREAM = RT == 0;
-  const int NS = STREAM ? a.stages : L::NS, A_STAGE = STREAM ? a.a_rows * 128 : L::A_STAGE, STAGE = STREAM ? A_STAGE + a.bn * 128 : L::STAGE;
+  constexpr bool STREAM = RT == 0, PAIR = RT == 2;
+  const int NS = STREAM || PAIR ? a.stages : L::NS, A_STAGE = STREAM ? a.a_rows * 128 : L::A_STAGE, STAGE = STREAM ? A_STAGE + a.bn * 128 : L::STAGE;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   // behind the stages, and behind what the last one's MMA reads past its activation rows
-  uint64_t* full = (uint64_t*)(smem + NS * STAGE + (STREAM ? BM * 128 : 0));
+  uint64_t* full = (uint64_t*)(smem + (PAIR ? NS * BM * 128 + L::NB * a.bn * 128 : NS * STAGE + (STREAM ? BM * 128 : 0)));
   uint64_t* empty = full + L::NS;
-  uint64_t* done = empty + L::NS;
+  uint64_t* full_b = empty + L::NS;  // PAIR: of the weights' ring
+  uint64_t* empty_b = full_b + L::NB;
+  uint64_t* done = empty_b + L::NB;
   uint32_t* tmem_slot = (uint32_t*)(done + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int bn = a.bn, width = GLU ? bn / 2 : bn;  // results per activation row of the tile
@@ -126,7 +148,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < NS; ++s) { bar_init(&full[s], 1); bar_init(&empty[s], 1); }
-    bar_init(done, 1);
+    if (PAIR)
+      for (int s = 0; s < L::NB; ++s) { bar_init(&full_b[s], 1); bar_init(&empty_b[s], 2); }
+    bar_init(done, PAIR ? 2 : 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == W_MMA) {
@@ -141,7 +165,69 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   bool ok = true;
 
-  if (warp == W_TMA) {
+  if (PAIR && warp == W_TMA) {
+    // Two rings: weights four steps deep, tiles of 128 activation rows three to four.  Stages of both tiles and the weights together were three
+    // (64 KB each), and a place that is free only once all eight MMAs of a step are done came back late: steps of 0.62 us instead of 0.47.
+    const uint32_t base = __shfl_sync(0xffffffffu, s32(smem), 0), base_b = base + (uint32_t)(NS * BM * 128);
+    auto load_w = [&](int k, int s) {
+      bar_expect(&full_b[s], (uint32_t)(bn * 128));  // boxes are always complete: what lies outside the matrices is filled with zeros
+      asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                   ::"r"(base_b + (uint32_t)(s * bn * 128)), "l"(&wmap), "r"(k * BK), "r"(z * a.rows + row0), "r"(s32(&full_b[s])) : "memory");
+      if constexpr (GLU)
+        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                     ::"r"(base_b + (uint32_t)(s * bn * 128 + width * 128)), "l"(&wmap), "r"(k * BK), "r"(a.rows + row0), "r"(s32(&full_b[s])) : "memory");
+    };
+    const bool leader = elect_one();
+    const int ahead = min(L::NB, k1 - k0);
+    if (leader)
+      for (int s = 0; s < ahead; ++s) load_w(k0 + s, s);
+    __syncwarp();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    uint32_t s = 0, lap = 0, sb = 0, lb = 0;
+    for (int k = k0; k < k1; ++k) {
+      if (k - k0 >= ahead) {
+        if (ok && !bar_wait(&empty_b[sb], lb ^ 1)) { ok = false; report_error(err, 5); }
+        if (ok && leader) load_w(k, (int)sb);
+      }
+      if (++sb == (uint32_t)L::NB) { sb = 0; lb ^= 1; }
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        if (ok && !bar_wait(&empty[s], lap ^ 1)) { ok = false; report_error(err, 5); }
+        if (ok && leader) {
+          bar_expect(&full[s], BM * 128);
+          asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                       ::"r"(base + s * (uint32_t)(BM * 128)), "l"(&xmap), "r"(z * a.xk + k * BK), "r"(tok0 + BM * r), "r"(s32(&full[s])) : "memory");
+        }
+        if (++s == (uint32_t)NS) { s = 0; lap ^= 1; }
+      }
+    }
+    __syncwarp();
+  } else if (PAIR && (warp == W_MMA || warp == W_MMA + 1)) {
+    // A warp per tile of activation rows: asking a barrier takes 100 ns, and the tensor pipe holds no more than a few MMAs ready, so that one
+    // thread that asks for weights and two tiles in turn leaves it idle in between (steps of 0.65 us instead of 0.47).
+    const int r = warp - W_MMA;
+    const uint32_t idesc = mma_desc(bn), td = __shfl_sync(0xffffffffu, tmem, 0) + (uint32_t)(r * BN), base = __shfl_sync(0xffffffffu, s32(smem), 0) >> 4;
+    const uint32_t base_b = base + (uint32_t)(NS * BM * 128 / 16);
+    const bool leader = elect_one();
+    int s = r, sb = 0;
+    uint32_t lap = 0, lb = 0;
+    for (int k = k0; k < k1; ++k) {
+      if (ok && !bar_wait2(&full_b[sb], lb, &full[s], lap)) { ok = false; report_error(err, 5); }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (leader) {
+        const uint32_t la = base + (uint32_t)(s * (BM * 128 / 16)), lw = base_b + (uint32_t)(sb * (bn * 128 / 16)), first = k > k0 ? 1u : 0u;
+#pragma unroll
+        for (int kk = 0; kk < BK / 16; ++kk) mma(td, la + (uint32_t)(2 * kk), lw + (uint32_t)(2 * kk), idesc, kk > 0 ? 1u : first);
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(&empty[s])) : "memory");
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(&empty_b[sb])) : "memory");
+      }
+      if ((s += 2) >= NS) { s -= NS; lap ^= 1; }
+      if (++sb == L::NB) { sb = 0; lb ^= 1; }
+    }
+    if (leader)
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(done)) : "memory");
+    __syncwarp();
+  } else if (warp == W_TMA) {
     const uint32_t base = __shfl_sync(0xffffffffu, s32(smem), 0);
     auto load_w = [&](int k, int s) {
       bar_expect(&full[s], (uint32_t)(A_STAGE + bn * 128));  // boxes are always complete: what lies outside the matrices is filled with zeros
@@ -182,13 +268,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
       if (leader) {
         const uint32_t lb = lo + (uint32_t)(A_STAGE / 16), first = k > k0 ? 1u : 0u;
 #pragma unroll
-        for (int kk = 0; kk < BK / 16; ++kk)
-#pragma unroll
-          for (int r = 0; r < (STREAM ? 1 : RT); ++r)
-            asm volatile("{ .reg .pred p; .reg .b64 a, b; setp.ne.b32 p, %5, 0; mov.b64 a, {%1, %3}; mov.b64 b, {%2, %3}; "
-                         "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p; }"
-                         ::"r"(td + (uint32_t)(r * BN)), "r"(lo + (uint32_t)(r * BM * 128 / 16 + 2 * kk)), "r"(lb + (uint32_t)(2 * kk)), "r"(DESC_HI), "r"(idesc),
-                           "r"(kk > 0 ? 1u : first) : "memory");
+        for (int kk = 0; kk < BK / 16; ++kk) mma(td, lo + (uint32_t)(2 * kk), lb + (uint32_t)(2 * kk), idesc, kk > 0 ? 1u : first);
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(&empty[s])) : "memory");
       }
       lo += (uint32_t)(STAGE / 16);
@@ -241,10 +321,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
         __syncwarp();
       }
     } else {
-      // warps 4.. read the second tile of activation rows, or every other run of columns of the only one
+      // warps 4.. read the second tile of activation rows, the next four or eight every other run of columns
       constexpr int W = 8;  // columns of a round
-      const int r = RT == 2 ? warp >> 2 : 0, t = tok0 + BM * r + 32 * (warp & 3) + lane;
-      constexpr int C_STEP = RT == 1 ? W * L::EPI / 4 : W;
+      const int r = PAIR ? (warp >> 2) & 1 : 0, t = tok0 + BM * r + 32 * (warp & 3) + lane;
+      constexpr int C_STEP = W * L::EPI / (4 * RT);
       const int64_t off = (int64_t)t * a.y_ld + (int64_t)z * a.rows + row0;
       float* y = a.y ? a.y + slice * a.slice_stride + off : nullptr;
       __nv_bfloat16* y16 = a.y16 ? a.y16 + off : nullptr;
@@ -252,7 +332,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
       if (a.gate && t < a.tokens) gate = 1.0f / (1.0f + expf(-a.gate[(int64_t)t * a.gate_ld + z]));
       const bool vec = ((a.y_ld | a.rows) & 7) == 0;  // every run of eight results starts on a 16-byte boundary in either format
       const uint32_t taddr = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(r * BN);
-      const int c_first = RT == 1 ? W * (warp >> 2) : 0;
+      const int c_first = W * (warp / (4 * RT));
       uint32_t v[2][W], u[2][W];  // the next round's are on their way while one is worked on
       auto fetch = [&](int c0, int k) {
         load8(taddr + (uint32_t)c0, v[k]);
@@ -327,13 +407,13 @@ template <int BN, int RT, bool GLU>
 cudaError_t launch_tiles(const Bf16Product& p, const Args& a, cudaStream_t stream, int* err) {
   CUtensorMap xmap, wmap;
   const int width = GLU ? a.bn / 2 : a.bn;  // rows of one box of W
-  if (!encode_rows(&xmap, p.x16, p.x_cols, p.tokens, p.x_ld, RT == 0 ? a.a_rows : RT * BM) || !encode_rows(&wmap, p.w, p.cols, (int64_t)p.rows * (GLU ? 2 : p.batch), p.cols, width))
+  if (!encode_rows(&xmap, p.x16, p.x_cols, p.tokens, p.x_ld, RT == 0 ? a.a_rows : BM) || !encode_rows(&wmap, p.w, p.cols, (int64_t)p.rows * (GLU ? 2 : p.batch), p.cols, width))
     return cudaErrorInvalidValue;
-  const int smem = RT == 0 ? 1024 + a.stages * (a.a_rows + a.bn) * 128 + BM * 128 + 512 : Lay<BN, RT>::TOTAL;
+  const int smem = RT == 0 ? 1024 + a.stages * (a.a_rows + a.bn) * 128 + BM * 128 + 512 : RT == 2 ? 1024 + (a.stages * BM + Lay<BN, RT>::NB * a.bn) * 128 + 512 : Lay<BN, RT>::TOTAL;
   static PerDevice ready;
   std::atomic<int>& slot = ready.here();
   if (slot.load(std::memory_order_relaxed) == 0) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, RT, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, RT == 0 ? STREAM_SMEM : smem);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, RT, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, RT == 0 ? STREAM_SMEM : Lay<BN, RT>::TOTAL);
     if (e != cudaSuccess) return e;
     slot.store(1, std::memory_order_relaxed);
   }
@@ -348,8 +428,8 @@ int tiles_of(int tokens, int rows, int batch, int bn, int rt = 1) { return ((tok
 // Shape of a tile.  Few tiles: 128 or 64 weight rows.  Many: 160 .. 256 weight rows (a multiple of `step`, so that both halves of a
 // gated tile are whole eight-row groups) and one or two tiles of 128 activation rows, for which the waves over the SMs cost least.
 // What a wave costs was measured at 4096 columns, 512 activation rows: 27 / 31 / 33 us with 160 / 224 / 256 weight rows, 43 / 54 /
-// 58 us with two tiles of activation rows.  The stages come from L2 at about 50 bytes a cycle and SM, which is what bounds a
-// wave; the second tile of activation rows uses a stage's weights again.  28672 x 4096: 126 -> 111 us (107 with the short epilogue), 16384 x 2048: 54 -> 44,
+// 58 us with two tiles of activation rows (50 at 224 since those have two rings, an issuing thread each and sixteen warps for results).  The stages come from L2 at about 50 bytes a cycle and SM, which is what bounds a
+// wave; the second tile of activation rows uses a stage's weights again.  28672 x 4096: 126 -> 111 us (107 with the short epilogue, 101 with two rings), 16384 x 2048: 54 -> 44,
 // 10240 x 4096: 64 -> 54, and with the wide tile from 120 tiles on (132 before) 8192 x 4096: 43 -> 39.
 struct Tile { int bn, rt; };
 Tile tile_shape(int tokens, int rows, int batch, int step = 16) {
@@ -416,14 +496,17 @@ cudaError_t launch_gemm_bf16(const Bf16Product& p, cudaStream_t stream, int* err
     a.stages = std::max(4, std::min(16, (alone ? 200 : 80) * 1024 / ((a.a_rows + a.bn) * 128)));
     return p.glu ? launch_tiles<128, 0, true>(p, a, stream, err) : launch_tiles<128, 0, false>(p, a, stream, err);
   }
+  auto pair_stages = [](int bn) { return std::min(8, (Lay<256, 2>::TOTAL - 1024 - 512 - Lay<256, 2>::NB * bn * 128) / (BM * 128)); };
   if (p.glu) {
     const Tile tile = tile_shape(p.tokens, 2 * p.rows, 1, 32);
     a.bn = std::max(tile.bn, 128);
+    a.stages = pair_stages(a.bn);
     return tile.rt == 2 ? launch_tiles<256, 2, true>(p, a, stream, err) : a.bn > 128 ? launch_tiles<256, 1, true>(p, a, stream, err)
                                                                                      : launch_tiles<128, 1, true>(p, a, stream, err);
   }
   const Tile tile = tile_shape(p.tokens, p.rows, p.batch);
   a.bn = tile.bn;
+  a.stages = pair_stages(a.bn);
   if (tile.rt == 2) return launch_tiles<256, 2, false>(p, a, stream, err);
   if (a.bn > 128) return launch_tiles<256, 1, false>(p, a, stream, err);
   return a.bn == 128 ? launch_tiles<128, 1, false>(p, a, stream, err) : launch_tiles<64, 1, false>(p, a, stream, err);

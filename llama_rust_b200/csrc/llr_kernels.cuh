@@ -370,7 +370,7 @@ __device__ __forceinline__ float gated_unit(float a, float b, const GluShape& g)
   if (g.unit == UNIT_GELU) return __fmul_rn(gelu_tanh(a), b);
   a = fminf(a, g.limit);
   b = fminf(fmaxf(b, -g.limit), g.limit);
-  return __fmul_rn(__fmul_rn(a, __fdiv_rn(1.0f, 1.0f + expf(-__fmul_rn(g.alpha, a)))), __fadd_rn(b, g.shift));
+  return __fmul_rn(__fmul_rn(a, __frcp_rn(1.0f + expf(-__fmul_rn(g.alpha, a)))), __fadd_rn(b, g.shift));
 }
 #endif
 // ---- products with bfloat16 weights for many rows (llr_gemm_bf16.cu): tcgen05, bfloat16 activations, f32 accumulation ----

@@ -805,10 +805,13 @@ block_scan_kernel(MatrixScan m, RowGroups groups, RowMap rows, int tokens, int c
 
 // ---- gated linear recurrence per channel ------------------------------------------------------------------------------------
 // grid (GS_COLS channels, group of rows).  GS_TILE rows at a time: all threads take the rows' decays and inputs, GS_COLS of them
-// run along the rows, all write the results.
-constexpr int GS_TILE = 128, GS_COLS = 16, GS_LANES = 16, GS_PER = GS_TILE / GS_LANES;  // GS_LANES threads per channel
+// run along the rows, all write the results.  LANES threads per channel: sixteen for prompts; one, and blocks of 128 channels, for groups
+// of up to sixteen rows, where 4096 blocks of 256 threads had one row's work for sixteen of them each (32 sequences x 2048
+// channels: 25 us).
+template <int GS_COLS, int GS_LANES, int GS_TILE>
 __global__ void __launch_bounds__(GS_COLS * GS_LANES)
 gated_scan_kernel(GatedScan p, RowGroups groups, RowMap rows, int tokens) {
+  constexpr int GS_PER = GS_TILE / GS_LANES;
   pdl_enter();
   __shared__ float2 ab[GS_TILE][GS_COLS];
   const Group g = group_of(groups, rows, tokens, blockIdx.y);
@@ -1006,9 +1009,9 @@ cudaError_t launch_matrix_scan(const MatrixScan& m, const HeadOut& out, float* r
 cudaError_t launch_gated_scan(const GatedScan& g, const RowGroups& groups, const RowMap& rows, int tokens, cudaStream_t s, uint64_t* launches) {
   if (tokens <= 0) return cudaSuccess;
   if (launches) ++*launches;
-  const dim3 grid((g.width + GS_COLS - 1) / GS_COLS, groups.n);
-  if (groups.longest <= SCAN_SHORT) return launch_walk(gated_scan_kernel, grid, dim3(GS_COLS * GS_LANES), 0, s, g, groups, rows, tokens);
-  gated_scan_kernel<<<grid, GS_COLS * GS_LANES, 0, s>>>(g, groups, rows, tokens);  // not placed early, as above
+  static_assert(SCAN_SHORT <= 16, "a tile of the short form");
+  if (groups.longest <= SCAN_SHORT) return launch_walk(gated_scan_kernel<128, 1, 16>, dim3((g.width + 127) / 128, groups.n), dim3(128), 0, s, g, groups, rows, tokens);
+  gated_scan_kernel<16, 16, 128><<<dim3((g.width + 15) / 16, groups.n), 256, 0, s>>>(g, groups, rows, tokens);  // not placed early, as above
   return cudaGetLastError();
 }
 

@@ -85,15 +85,26 @@ rmsnorm_kernel(float* x, const float* add, const float* __restrict__ w, float* _
 }
 
 // One block per token: the cosine and sine of every pair's angle once (all heads of a token turn by the same
-// angles), then the rotation of every q and k head, then the k and v rows into the cache.
+// angles), then the rotation of every q and k head, q in place, k and v into the cache (store_kv, decode.rs:12059: the row's sequence, paged).
+// Bound: memory latency.  The page is looked up once, values are on their way while the angles are worked out, and four pairs are fetched
+// before the first is stored (a pair at a time, and the cache filled from the rotated rows: 512 rows of 32 + 8 heads 15 us).
 __global__ void __launch_bounds__(256)
-rope_store_kernel(float* q, float* k, const float* v, KvView kv, RowMap rows, int layer,
+rope_store_kernel(float* q, const float* k, const float* v, KvView kv, RowMap rows, int layer,
                   WalkShape w) {
   pdl_enter();
   __shared__ float s_cos[128], s_sin[128];  // head_dim <= 256
+  constexpr int U = 4;
   const int t = blockIdx.x;
   const int pos = row_position(rows, t);
-  const int hd = w.head_dim, half = hd / 2;
+  const int hd = w.head_dim, half = hd / 2, n_kv = w.n_head_kv * half, n = w.n_head * half + n_kv;  // pairs
+  const int64_t slot = kv_slot(kv, row_sequence(rows, t), layer, 0, pos, w.n_head_kv);  // heads lie block_tokens slots apart
+  auto cached = [&](float* pool, int h, int p) { return (float2*)(pool + (slot + (int64_t)h * kv.block_tokens) * hd + 2 * p); };
+  const float2 *qrow = (const float2*)(q + (int64_t)t * w.n_head * hd), *krow = (const float2*)(k + (int64_t)t * w.n_head_kv * hd),
+               *vrow = (const float2*)(v + (int64_t)t * w.n_head_kv * hd);
+  float2 vv[U];
+#pragma unroll
+  for (int j = 0; j < U; ++j)
+    if ((int)threadIdx.x + 256 * j < n_kv) vv[j] = vrow[threadIdx.x + 256 * j];
   const float theta_scale = w.theta_scale;  // base^(-2/n_rot), computed once on the host in f32 as the reference does
   for (int p = threadIdx.x; p < half; p += blockDim.x) {
     float theta = (float)(pos <= 65535 ? pos : 65535);
@@ -102,24 +113,30 @@ rope_store_kernel(float* q, float* k, const float* v, KvView kv, RowMap rows, in
     s_sin[p] = sinf(theta);
   }
   __syncthreads();
-  float* qrow = q + (int64_t)t * w.n_head * hd;
-  float* krow = k + (int64_t)t * w.n_head_kv * hd;
-  for (int idx = threadIdx.x; idx < (w.n_head + w.n_head_kv) * half; idx += blockDim.x) {
-    const int h = idx / half, p = idx % half;
-    float* vec = h < w.n_head ? qrow + h * hd : krow + (h - w.n_head) * hd;
-    const float c = s_cos[p], s = s_sin[p];
-    const float2 ab = *(const float2*)(vec + 2 * p);
-    *(float2*)(vec + 2 * p) = make_float2(__fsub_rn(__fmul_rn(ab.x, c), __fmul_rn(ab.y, s)), __fadd_rn(__fmul_rn(ab.x, s), __fmul_rn(ab.y, c)));
+#pragma unroll
+  for (int j = 0; j < U; ++j) {
+    const int i = threadIdx.x + 256 * j;
+    if (i < n_kv) *cached(kv.v, i / half, i % half) = vv[j];
   }
-  __syncthreads();  // the rotated keys are read back below by other threads of the block
-  // store_kv (decode.rs:12059) into the row's sequence, paged
-  const int sid = row_sequence(rows, t);
-  const float* vrow = v + (int64_t)t * w.n_head_kv * hd;
-  for (int idx = threadIdx.x; idx < w.n_head_kv * hd; idx += blockDim.x) {
-    const int hk = idx / hd, i = idx % hd;
-    const int64_t off = kv_offset(kv, sid, layer, hk, pos, w.n_head_kv, hd);
-    kv.k[off + i] = krow[idx];
-    kv.v[off + i] = vrow[idx];
+  for (int i = threadIdx.x + 256 * U; i < n_kv; i += 256) *cached(kv.v, i / half, i % half) = vrow[i];
+  const int nq = n - n_kv;
+  for (int i0 = threadIdx.x; i0 < n; i0 += 256 * U) {
+    float2 ab[U];
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+      const int i = i0 + 256 * j;
+      if (i < n) ab[j] = i < nq ? qrow[i] : krow[i - nq];
+    }
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+      const int i = i0 + 256 * j;
+      if (i >= n) continue;
+      const int h = i / half, p = i % half;
+      const float c = s_cos[p], s = s_sin[p];
+      const float2 r = make_float2(__fsub_rn(__fmul_rn(ab[j].x, c), __fmul_rn(ab[j].y, s)), __fadd_rn(__fmul_rn(ab[j].x, s), __fmul_rn(ab[j].y, c)));
+      if (i < nq) ((float2*)(q + (int64_t)t * w.n_head * hd))[i] = r;
+      else *cached(kv.k, h - w.n_head, p) = r;
+    }
   }
 }
 

@@ -129,20 +129,54 @@ __device__ __forceinline__ float rotated(const F& f, int i, int d, const float2*
   const float2 a = cs[c < half ? c : c - half];
   return c < half ? fmaf(v, a.x, -__fmul_rn(f(i + half), a.y)) : fmaf(v, a.x, __fmul_rn(f(i - half), a.y));
 }
-// The same for `heads` whole heads, a warp per head; put(i, v) takes value i
+// The same for `heads` whole heads, a warp per head; put(i, v) takes value i.  The values of two heads and two pairs per lane are fetched before
+// the first is put: stores that the compiler cannot tell from the next loads' source would make every pair wait for memory by itself.
 template <typename F, typename P>
 __device__ __forceinline__ void rotate_all(const F& f, const P& put, int heads, int d, const float2* cs, int dims) {
-  const int half = dims / 2, lane = threadIdx.x & 31;
-  for (int h = threadIdx.x >> 5; h < heads; h += blockDim.x >> 5) {
-    const int i0 = h * d;
-#pragma unroll 2
-    for (int c = lane; c < half; c += 32) {  // a pair is read and written by one thread
-      const float u = f(i0 + c), v = f(i0 + c + half);
-      const float2 a = cs[c];
-      put(i0 + c, fmaf(u, a.x, -__fmul_rn(v, a.y)));
-      put(i0 + c + half, fmaf(v, a.x, __fmul_rn(u, a.y)));
+  const int half = dims / 2, lane = threadIdx.x & 31, step = blockDim.x >> 5;
+  for (int h = threadIdx.x >> 5; h < heads; h += 2 * step) {
+    for (int c0 = lane; c0 < half; c0 += 64) {  // a pair is read and written by one thread
+      float u[2][2], v[2][2];
+      float2 a[2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        if (c0 + 32 * j < half) {
+          const int c = c0 + 32 * j;
+          a[j] = cs[c];
+#pragma unroll
+          for (int k = 0; k < 2; ++k)
+            if (h + k * step < heads) {
+              u[k][j] = f((h + k * step) * d + c);
+              v[k][j] = f((h + k * step) * d + c + half);
+            }
+        }
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        if (c0 + 32 * j < half) {
+          const int c = c0 + 32 * j;
+#pragma unroll
+          for (int k = 0; k < 2; ++k)
+            if (h + k * step < heads) {
+              const int i0 = (h + k * step) * d;
+              put(i0 + c, fmaf(u[k][j], a[j].x, -__fmul_rn(v[k][j], a[j].y)));
+              put(i0 + c + half, fmaf(v[k][j], a[j].x, __fmul_rn(u[k][j], a[j].y)));
+            }
+        }
     }
-    for (int c = dims + lane; c < d; c += 32) put(i0 + c, f(i0 + c));
+    for (int k = 0; k < 2 && h + k * step < heads; ++k)
+      for (int c = dims + lane; c < d; c += 32) put((h + k * step) * d + c, f((h + k * step) * d + c));
+  }
+}
+// put(i, f(i)) for i < n, four values in flight; each is read and written by one thread
+template <typename F, typename P>
+__device__ __forceinline__ void move_all(const F& f, const P& put, int n) {
+  for (int i0 = threadIdx.x; i0 < n; i0 += 4 * PROJ_THREADS) {
+    float u[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) u[j] = i0 + j * PROJ_THREADS < n ? f(i0 + j * PROJ_THREADS) : 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i0 + j * PROJ_THREADS < n) put(i0 + j * PROJ_THREADS, u[j]);
   }
 }
 __device__ __forceinline__ void rotate_heads(const RotHeads& h, int64_t ld, int t) {
@@ -163,11 +197,11 @@ qkv_store_kernel(float* proj, int ld, const float* __restrict__ bias, const floa
   __shared__ float red[2][32];
   const int t = blockIdx.x, nk = sh.n_kv * sh.dk, nv = sh.n_kv * sh.dv;
   float* p = proj + (int64_t)t * ld;
-  const QkvRow r = qkv_row(p, ld, bias, q_norm, k_norm, sh, red);
+  // the page and the place in it once, looked up before the sums are waited for; heads lie block_tokens vectors apart
   const int pos = row_position(rows, t), seq = row_sequence(rows, t);
-  // the page and the place in it once; heads lie block_tokens vectors apart
   float* k0 = kv.k + slot_of(kv, seq, pos, kv.k_block, 0, sh.dk);
   float* v0 = kv.v + slot_of(kv, seq, pos, kv.v_block, 0, sh.dv);
+  const QkvRow r = qkv_row(p, ld, bias, q_norm, k_norm, sh, red);
   if (also.heads > 0) rotate_heads(also, ld, t);
   const float2* cs = rot.dims > 0 ? rot.cs + (int64_t)t * rot.ld : nullptr;
   const auto qf = [&](int i) { return r.q(i); };
@@ -176,20 +210,13 @@ qkv_store_kernel(float* proj, int ld, const float* __restrict__ bias, const floa
   if (cs) {
     rotate_all(kf, [&](int i, float v) { *k_at(i) = v; }, sh.n_kv, sh.dk, cs, rot.dims);
   } else {
-    for (int i = threadIdx.x; i < nk; i += PROJ_THREADS) *k_at(i) = r.k(i);
+    move_all(kf, [&](int i, float v) { *k_at(i) = v; }, nk);
   }
-  for (int i = threadIdx.x; i < nv; i += PROJ_THREADS) v0[(int64_t)(i / sh.dv) * kv.block_tokens * sh.dv + i % sh.dv] = r.v(i);
+  move_all([&](int i) { return r.v(i); }, [&](int i, float v) { v0[(int64_t)(i / sh.dv) * kv.block_tokens * sh.dv + i % sh.dv] = v; }, nv);
   if (cs) {
     rotate_all(qf, [&](int i, float v) { p[i] = v; }, sh.n_head, sh.dk, cs, rot.dims);
   } else if (bias || q_norm) {
-    for (int i0 = threadIdx.x; i0 < r.nq; i0 += 4 * PROJ_THREADS) {  // four values in flight; each is read and written by one thread
-      float u[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) u[j] = i0 + j * PROJ_THREADS < r.nq ? r.q(i0 + j * PROJ_THREADS) : 0.f;
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (i0 + j * PROJ_THREADS < r.nq) p[i0 + j * PROJ_THREADS] = u[j];
-    }
+    move_all(qf, [&](int i, float v) { p[i] = v; }, r.nq);
   }
 }
 

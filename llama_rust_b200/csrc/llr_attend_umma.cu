@@ -16,9 +16,10 @@
 //   values of at most 128 dimensions, NK = 128: four warps take the even steps, four the odd ones, either four with sums and references
 //     of their own that meet at the end; while one set waits for the tensor cores the other has the exponentials (eight warps a step, half
 //     of its keys each, took 2.0 us a step instead of 1.2: the registers then hold too little)
-//   more, NK = 64: eight warps a step, half of its keys each.  A block has 256 value dimensions and blocks of the other parts form the scores again: 1.5 times the operations of one pass with a latent of 512, whose sums would leave no column for
-//     scores.  The first 256 columns of the queries are operands in tensor memory, which leaves a ring of two and a half steps (with all
-//     of them in shared memory the ring held a step and a half, and a step took 2.9 us, most of it waiting for copies).
+//   more, NK = 64: eight warps a step, half of its keys each.  A block has 256 value dimensions and blocks of the other parts form the
+//     scores again: 1.5 times the operations of one pass with a latent of 512, whose sums would leave no column for scores.  The first
+//     256 columns of the queries are operands in tensor memory, which leaves a ring of two and a half steps (with all of them in shared
+//     memory the ring held a step and a half, and a step took 2.9 us, most of it waiting for copies).
 // Keys and values come through a ring of chunk pairs, 2 x [NK keys][64 dimensions], one pair of barriers each (a chunk alone is four
 // MMAs of 45 to 64 cycles: waiting for its barrier and freeing it took 460); where values are the keys, a block reads the pairs of its own
 // dimensions last and keeps them until the sums have used them.

@@ -19,8 +19,9 @@
 // loads.  Wide tiles are bound by what the SMs draw from L2, so 256 activation rows share a stage's weights where that saves waves
 // (tile_shape).  Up to 64 activation rows the product is a stream of weights: a stage then holds 32 or 64 activation rows (the MMA
 // reads on into the weights behind them: rows of its result that nobody looks at), tiles of 32 .. 128 weight rows spread it over the SMs
-// (stream_width) and up to sixteen stages of it are under way.  16384 x 2048 gated, 32 rows: 25 -> 18 us.  A K range may be cut into slices (gridDim.z): slice s leaves its partial sums at y + s * slice_stride and the reader
-// adds them in slice order.  Every wait is bounded.
+// (stream_width) and up to sixteen stages of it are under way.  16384 x 2048 gated, 32 rows: 25 -> 18 us.  A K range may be cut into
+// slices (gridDim.z): slice s leaves its partial sums at y + s * slice_stride and the reader adds them in slice order.  Every wait is
+// bounded.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -428,8 +429,9 @@ int tiles_of(int tokens, int rows, int batch, int bn, int rt = 1) { return ((tok
 // Shape of a tile.  Few tiles: 128 or 64 weight rows.  Many: 160 .. 256 weight rows (a multiple of `step`, so that both halves of a
 // gated tile are whole eight-row groups) and one or two tiles of 128 activation rows, for which the waves over the SMs cost least.
 // What a wave costs was measured at 4096 columns, 512 activation rows: 27 / 31 / 33 us with 160 / 224 / 256 weight rows, 43 / 54 /
-// 58 us with two tiles of activation rows (50 at 224 since those have two rings, an issuing thread each and sixteen warps for results).  The stages come from L2 at about 50 bytes a cycle and SM, which is what bounds a
-// wave; the second tile of activation rows uses a stage's weights again.  28672 x 4096: 126 -> 111 us (107 with the short epilogue, 101 with two rings), 16384 x 2048: 54 -> 44,
+// 58 us with two tiles of activation rows (50 at 224 since those have two rings, an issuing thread each and sixteen warps for
+// results).  The stages come from L2 at about 50 bytes a cycle and SM, which is what bounds a wave; the second tile of activation rows
+// uses a stage's weights again.  28672 x 4096: 126 -> 111 us (107 with the short epilogue, 101 with two rings), 16384 x 2048: 54 -> 44,
 // 10240 x 4096: 64 -> 54, and with the wide tile from 120 tiles on (132 before) 8192 x 4096: 43 -> 39.
 struct Tile { int bn, rt; };
 Tile tile_shape(int tokens, int rows, int batch, int step = 16) {

@@ -37,6 +37,7 @@
 #include <math_constants.h>
 
 #include <algorithm>
+#include <cfloat>
 
 #include "llr_attend.cuh"
 #include "llr_kernels.cuh"
@@ -58,7 +59,6 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
   const __half2 h = __floats2half2_rn(lo, hi);
   return *(const uint32_t*)&h;
 }
-__device__ __forceinline__ float sat16(float v) { return fminf(fmaxf(v, -65504.f), 65504.f); }
 __device__ __forceinline__ float exp2_ftz(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -95,8 +95,11 @@ __device__ __forceinline__ int span_group(const int* at, int n, int block) {
 
 constexpr int MAX_NK = 128;  // keys of a step
 
-// One warp per key row: grid (keys / 8 of all groups, kv head).  Where the host knew only a bound of a group's keys, the rows that
-// a tile may read behind the last key are zeros: whatever memory holds there must not meet a weight of zero.
+// One warp per key row: grid (keys / 8 of all groups, kv head).  What is not a number must reach the rows that see it and no others, but a
+// masked weight of zero times an infinity is not zero.  So where a value is not finite as binary16 the row's KEY says so: scores that do
+// not see it are masked by selection, those that do make their whole row not a number.  A latent is both operands at once and is bounded
+// instead, NaN included.  Where the host knew only a bound of a group's keys, the rows that a tile may read behind the last key are
+// zeros: whatever memory holds there must not meet a weight of zero.
 __global__ void __launch_bounds__(256)
 span_gather_kernel(SpanShape sh, LayerKv kv, RowMap rows, const __grid_constant__ SpanBatch b, __half* __restrict__ k16, __half* __restrict__ v16) {
   pdl_enter();
@@ -105,17 +108,34 @@ span_gather_kernel(SpanShape sh, LayerKv kv, RowMap rows, const __grid_constant_
   const int m = (blockIdx.x - b.keys_at[gi]) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, head = blockIdx.y, seq = row_sequence(rows, t0);
   if (m >= min(b.keys[gi], gk.n + MAX_NK)) return;
   const int64_t row = (int64_t)b.row0[gi] + (int64_t)head * b.keys[gi] + m;
-  const bool live = m < gk.n;
+  const bool live = m < gk.n, latent = v16 == nullptr;
   const int j = live ? gk.at(m) : 0;
   const int64_t page = live ? kv.table[(int64_t)seq * kv.max_blocks + j / kv.block_tokens] : 0, in_page = (int64_t)head * kv.block_tokens + j % kv.block_tokens;
-  auto put = [&](const float* src, int d, __half* dst) {
-    for (int i = 4 * lane; i < d; i += 128) {
-      const float4 v = live ? *(const float4*)(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);  // d is a multiple of eight
-      *(uint2*)(dst + i) = make_uint2(pack_h2(sat16(v.x), sat16(v.y)), pack_h2(sat16(v.z), sat16(v.w)));
-    }
+  const float* ks = kv.k + page * kv.k_block + in_page * sh.dk;
+  auto fetch = [&](const float* src, int i, int d) {  // d is a multiple of eight
+    return live && i < d ? *(const float4*)(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
   };
-  put(kv.k + page * kv.k_block + in_page * sh.dk, sh.dk, k16 + row * sh.dk);
-  if (v16) put(kv.v + page * kv.v_block + in_page * sh.dv, sh.dv, v16 + row * sh.dv);
+  auto operand = [&](float x) { return latent || (sh.saturate && fabsf(x) <= FLT_MAX) ? fminf(fmaxf(x, -65504.f), 65504.f) : x; };
+  auto words = [&](float4 x) { return make_uint2(pack_h2(operand(x.x), operand(x.y)), pack_h2(operand(x.z), operand(x.w))); };
+  bool special = false;
+  auto finite = [&](uint32_t w) {
+    const bool not_finite = (w & 0x7c00u) == 0x7c00u || (w & 0x7c000000u) == 0x7c000000u;
+    special |= not_finite;
+    return not_finite ? 0u : w;
+  };
+  const float4 first = fetch(ks, 4 * lane, sh.dk);  // on its way beside the values
+  if (!latent) {
+    const float* vs = kv.v + page * kv.v_block + in_page * sh.dv;
+    for (int i = 4 * lane; i < sh.dv; i += 128) {
+      const uint2 w = words(fetch(vs, i, sh.dv));
+      *(uint2*)(v16 + row * sh.dv + i) = make_uint2(finite(w.x), finite(w.y));
+    }
+    special = __any_sync(~0u, special);
+  }
+  for (int i = 4 * lane; i < sh.dk; i += 128) {
+    const uint2 w = words(i < 128 ? first : fetch(ks, i, sh.dk));
+    *(uint2*)(k16 + row * sh.dk + i) = special ? make_uint2(0x7fff7fffu, 0x7fff7fffu) : w;
+  }
 }
 
 constexpr int PAIRS = 128;
@@ -365,7 +385,8 @@ span_umma_kernel(const float* q, int64_t q_ld, SpanShape sh, Shape ms, const __g
     const int wg = warp >> 2, set = ALT ? wg : 0, half = ALT ? 0 : wg, row = 32 * (warp & 3) + lane, p = pair0 + row, pc = min(p, pairs - 1);
     const uint32_t t_lane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
     auto all_warps = [] { asm volatile("bar.sync 1, %0;" ::"n"(L::SOFT * 32) : "memory"); };
-    // ---- queries: eight lanes per pair; the power of two that brings the largest magnitude into [2^9, 2^10)
+    // ---- queries: eight lanes per pair; the power of two that brings the largest magnitude into [2^9, 2^10).  One that is not finite stays so:
+    // it meets its own row only
     {
       constexpr int OWN = PAIRS / L::SOFT;  // pairs of a warp
       const bool quads = ((uintptr_t)q & 15) == 0 && (q_ld & 3) == 0;
@@ -414,7 +435,7 @@ span_umma_kernel(const float* q, int64_t q_ld, SpanShape sh, Shape ms, const __g
 #pragma unroll
         for (int c = 0; c < 2 * KC; ++c)  // 16-byte pieces of a 128-byte row lie where their number XOR the row says
           *(uint2*)(smem + tile_of(c >> 1) + r * 128 + (((4 * (c & 1) + ((lane & 7) >> 1)) ^ (r & 7)) << 4) + 8 * (lane & 1)) =
-              make_uint2(pack_h2(sat16(v[c].x * up), sat16(v[c].y * up)), pack_h2(sat16(v[c].z * up), sat16(v[c].w * up)));
+              make_uint2(pack_h2(v[c].x * up, v[c].y * up), pack_h2(v[c].z * up, v[c].w * up));
         if ((lane & 7) == 0) red[r] = down * sh.scale;
       }
     }

@@ -48,3 +48,86 @@ def test_tiles(tmp_path, name):
         got = s.forward([(0, toks[:200]), (1, toks[:1]), (2, toks[:33])], [list(range(200)), [0], list(range(33))])
         assert nm.error(got, np.concatenate([want[:200], want[:1], want[:33]])).max() <= nm.TOLERANCE[nm.AUTO]
         s.free()
+
+
+def _llama(ex, n_ctx, n_seq=1, heads=4, kv_heads=2, head_dim=64, vocab=300, edit=None, **session):
+    """A small Llama session with F32 weights: what differs between the paths is attention alone.  edit(weights) changes them by name."""
+    import llama_walk as lw
+    from helpers import ALL
+    from llama_rust_b200 import Session
+    cfg = dict(n_layer=2, n_embd=heads * head_dim, n_head=heads, n_head_kv=kv_heads, head_dim=head_dim, n_ff=256, n_vocab=vocab)
+    rng = np.random.default_rng(72)
+    w = {n: (rng.standard_normal((r, c)) / np.sqrt(c)).astype(np.float32) for n, _, r, c in lw.tensor_list(cfg)}
+    w["embd"] = rng.standard_normal((vocab, cfg["n_embd"])).astype(np.float32)
+    if edit:
+        edit(w)
+    up = {n: ex.upload(ALL["F32"], a.shape[0], a.shape[1], np.ascontiguousarray(a).view(np.uint8).ravel()) for n, a in w.items()}
+    names = ("attn_q", "attn_k", "attn_v", "attn_output", "ffn_gate", "ffn_up", "ffn_down")
+    layers = [{n: up[f"blk.{i}.{n}.weight"] for n in names} for i in range(2)]
+    return Session(ex, dict(cfg, n_ctx=n_ctx), up["embd"], layers, output=up["output.weight"], n_seq=n_seq, **session)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_llama_rows_that_are_not_numbers(bad):
+    """A token whose activations are not numbers makes its own row and every later one of its sequence not a number, and nothing else: not
+    the rows before it, whose tiles hold its keys and values masked, nor the sequences that lie beside it in the gathered keys."""
+    from llama_rust_b200 import Executor
+    toks = [(7 * np.arange(n) + 3 * n) % 299 for n in (70, 150, 90)]  # never token 299
+    toks[1][100] = 299
+
+    def edit(w):
+        w["embd"][299, 5] = bad
+    with Executor(0) as ex:
+        got = {}
+        for path in (0, 3):
+            ex.set_path(path)
+            toks[1][100] = 299 if path == 0 else 298  # f32: another token's numbers there
+            s = _llama(ex, 200, 3, edit=edit)
+            got[path] = s.batch_rows([(q, t.tolist()) for q, t in enumerate(toks)], list(range(310)))
+            s.free()
+    finite = np.isfinite(got[0])
+    clean = np.ones(310, bool)
+    clean[70 + 100:70 + 150] = False
+    assert finite[clean].all() and not finite[~clean].any()
+    assert np.abs(got[0] - got[3])[clean].max() <= 1e-3 * np.abs(got[3]).max()
+
+
+def test_llama_values_beyond_binary16_are_not_bounded():
+    """Values of 1e6: the f32 path gives numbers, 16-bit operands infinities.  Anything else that is finite would be a wrong answer."""
+    from llama_rust_b200 import Executor
+    toks = (7 * np.arange(130)) % 299
+
+    def edit(w):
+        w["blk.0.attn_v.weight"] *= 1e6
+    with Executor(0) as ex:
+        s = _llama(ex, 200, edit=edit)
+        ex.set_path(3)
+        f32 = s.batch_rows([(0, toks.tolist())], [129])
+        assert np.isfinite(f32).all()
+        s.reset()
+        ex.set_path(0)
+        assert not np.isfinite(s.batch_rows([(0, toks.tolist())], [129])).any()
+        s.free()
+
+
+def test_layered_rows_that_are_not_numbers(tmp_path):
+    """One layer with a window: the rows that see the broken token, no more and no less; the others have the numbers they have without it."""
+    from llama_rust_b200 import Executor, models
+    cfg = nm.config(64, 90, [nm.attention(4, 2, 72, 40, 40, 3, 24)], 0)
+    w = nm.weights(cfg, 17, 10, nm.SHARP[nm.AUTO])
+    toks = [t % 89 for t in nm.tokens(320, cfg, 23)]
+    toks[200] = 89
+    want = plain.forward(cfg, w, toks)
+    w["embed"] = w["embed"].copy()
+    w["embed"][89] = np.nan
+    sees = (np.arange(320) >= 200) & (np.arange(320) < 240)
+    with Executor(0) as ex:
+        s = models.load(ex, nm.write(tmp_path / "m", cfg, w), n_seq=2)
+        got = s.forward([(0, toks), (1, toks[:150])], [list(range(320)), list(range(150))])
+        got, beside = got[:320], got[320:]
+        # the embedding is the output matrix too: its broken row is one logit of every row
+        got, beside, want = got[:, :89], beside[:, :89], want[:, :89]
+        assert np.array_equal(~np.isfinite(got).any(1), sees), np.nonzero(~np.isfinite(got).any(1) != sees)[0]
+        assert nm.error(got[~sees], want[~sees]).max() <= nm.TOLERANCE[nm.AUTO]
+        assert nm.error(beside, want[:150]).max() <= nm.TOLERANCE[nm.AUTO]
+        s.free()

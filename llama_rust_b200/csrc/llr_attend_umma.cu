@@ -672,7 +672,7 @@ struct Variant {
   int nk, smem, threads;
 };
 // Steps of 128 keys where the values fit 128 columns of tensor memory, of 64 otherwise; the queries' chunks are rounded up to an
-// instance's.  Heads of more than 768 columns leave no room for a ring.
+// instance's.
 Variant variant(int dk, int dv) {
   const int kc = (dk + 63) / 64;
 #define LLR_V(K, N) return Variant{span_umma_kernel<K, N>, N, Lay<K, N>::TOTAL, Lay<K, N>::THREADS};
@@ -715,8 +715,17 @@ size_t span_umma_scratch_floats(const SpanShape& sh, int max_rows) {
   return (size_t)sh.n_kv * span_group_keys(sh, max_rows) * (sh.dk + sh.dv) / 2 + 64;
 }
 
+// Heads that have 16-bit operands: those of which 64 queries, 64 keys and 64 values fit 222 KB as binary16, keys padded to 16 columns and values
+// to the widths below (beside up to 128 of them; more leave room for a tile of exponentials), and latents up to 512.  Wider heads have f32
+// operands whatever the number of rows, although the kernel here could hold some of them: nobody who uses them asked for fewer bits.
+static bool sixteen_bit_heads(int dk, int dv, bool shared) {
+  if (dv > 512) return false;
+  const int kw = (dk + 15) / 16 * 16, vw = dv <= 128 ? (dv + 31) / 32 * 32 : dv <= 192 ? 192 : dv <= 256 ? 256 : dv <= 384 ? 384 : 512;
+  return shared ? dk == dv : 2 * kw + vw <= (dv <= 128 ? 1752 : 1680);
+}
+
 bool span_umma_supported(const SpanShape& sh, bool shared, const SpanOut& out) {
-  return sh.n_kv > 0 && sh.n_head % sh.n_kv == 0 && sh.dk % 8 == 0 && sh.dv % 8 == 0 && (!shared || (sh.dk == sh.dv && sh.dk <= 512)) && variant(sh.dk, sh.dv).kernel &&
+  return sh.n_kv > 0 && sh.n_head % sh.n_kv == 0 && sh.dk % 8 == 0 && sh.dv % 8 == 0 && sixteen_bit_heads(sh.dk, sh.dv, shared) && variant(sh.dk, sh.dv).kernel &&
          (int64_t)sh.n_kv * sh.n_ctx < (1 << 30) && out.ld % 2 == 0 && ((uintptr_t)out.out & 7) == 0 && ((uintptr_t)out.out16 & 3) == 0 &&
          (!out.gate || out.head_gate || (out.gate_ld % 2 == 0 && ((uintptr_t)out.gate & 7) == 0));
 }

@@ -131,3 +131,19 @@ def test_layered_rows_that_are_not_numbers(tmp_path):
         assert nm.error(got[~sees], want[~sees]).max() <= nm.TOLERANCE[nm.AUTO]
         assert nm.error(beside, want[:150]).max() <= nm.TOLERANCE[nm.AUTO]
         s.free()
+
+
+# Heads beyond what 16-bit operands are for: more than 512 value dimensions, long keys beside long values.  Values of a million say which
+# operands a prompt has: binary16 ends at 65504.
+@pytest.mark.parametrize("dk,dv", [(64, 520), (64, 1024), (640, 512), (768, 192), (704, 264), (856, 32), (840, 64)])
+def test_wide_heads_keep_32_bits(tmp_path, dk, dv):
+    from llama_rust_b200 import Executor, models
+    cfg = nm.config(64, 90, [nm.attention(2, 1, dk, dv, 90, 2, 40)], 0)
+    w = nm.weights(cfg, 17, 10, nm.SHARP[nm.AUTO])
+    w["l0.mix.v"], w["l0.mix.v.b"] = w["l0.mix.v"] * 2.0 ** 20, w["l0.mix.v.b"] * 2.0 ** 20
+    toks = nm.tokens(140, cfg, 23)
+    want = plain.forward(cfg, w, toks)
+    with Executor(0) as ex:
+        s = models.load(ex, nm.write(tmp_path / "m", cfg, w))
+        assert nm.error(s.forward([(0, toks)], [list(range(140))]), want).max() <= nm.TOLERANCE[nm.AUTO]
+        s.free()

@@ -157,7 +157,7 @@ template <int KC, int NK> struct Lay {
   // last slots of the ring, through which the queries pass: as binary16 on their way to tensor memory, or (short ones) as f32
   static constexpr bool RAW = KC <= 2;
   static constexpr int TMP = RAW ? KC * PAIRS * 256 / SLOT : QT * PAIRS * 128 / SLOT, AT_TMP = Q + (NS - TMP) * SLOT;
-  static_assert(Q_COL + 32 * QT <= 512 && (2 * NS + 7) * 8 + 8 <= 512 && Q + NS * SLOT >= 2 * SOFT * 32 * OUT_PITCH + 2048 && TMP < NS, "");
+  static_assert(Q_COL + 32 * QT <= 512 && (2 * NS + 7) * 8 + 8 <= 512 && Q + NS * SLOT >= 2 * SOFT * 32 * OUT_PITCH + 2048 && TMP <= NS, "");
 };
 
 struct Shape {
@@ -672,7 +672,7 @@ struct Variant {
   int nk, smem, threads;
 };
 // Steps of 128 keys where the values fit 128 columns of tensor memory, of 64 otherwise; the queries' chunks are rounded up to an
-// instance's.
+// instance's.  The longest keys that have 16-bit operands leave a ring of four pairs, which the queries pass through before it starts.
 Variant variant(int dk, int dv) {
   const int kc = (dk + 63) / 64;
 #define LLR_V(K, N) return Variant{span_umma_kernel<K, N>, N, Lay<K, N>::TOTAL, Lay<K, N>::THREADS};
@@ -684,6 +684,7 @@ Variant variant(int dk, int dv) {
   if (kc <= 4) LLR_V(4, 64)
   if (kc <= 8) LLR_V(8, 64)
   if (kc <= 12) LLR_V(12, 64)
+  if (kc <= 14) LLR_V(14, 64)
 #undef LLR_V
   return Variant{nullptr, 0, 0, 0};
 }

@@ -18,7 +18,10 @@ SHAPES = {
     "short keys, two parts of values": nm.attention(2, 1, 64, 264, 90, 2, 40),
     "long keys and values": nm.attention(2, 2, 256, 200, 129, 2, 40),
     "keys of nine chunks": nm.attention(2, 1, 520, 64, 127, 1, 40),
-    "keys beyond the tile kernel": nm.attention(2, 1, 776, 64, 127, 1, 40),
+    "keys of thirteen chunks": nm.attention(2, 1, 776, 64, 127, 1, 40),
+    "the longest keys of 16 bits": nm.attention(3, 1, 848, 32, 127, 1, 40),
+    "long keys, values of three quarters of a part": nm.attention(2, 1, 800, 128, 127, 70, 40),
+    "keys beyond the tile kernel": nm.attention(2, 1, 856, 32, 127, 1, 40),
     "latent of one chunk": nm.latent(5, 16, 24, 64, 65),
     "latent of two chunks": nm.latent(16, 16, 24, 128, 1000),
     "latent of an odd size": nm.latent(9, 16, 24, 200, 64),

@@ -93,49 +93,43 @@ __device__ __forceinline__ int span_group(const int* at, int n, int block) {
   return i;
 }
 
-constexpr int MAX_NK = 128;  // keys of a step
-
 // One warp per key row: grid (keys / 8 of all groups, kv head).  What is not a number must reach the rows that see it and no others, but a
 // masked weight of zero times an infinity is not zero.  So where a value is not finite as binary16 the row's KEY says so: scores that do
 // not see it are masked by selection, those that do make their whole row not a number.  A latent is both operands at once and is bounded
-// instead, NaN included.  Where the host knew only a bound of a group's keys, the rows that a tile may read behind the last key are
-// zeros: whatever memory holds there must not meet a weight of zero.
+// instead, NaN included.  With that, every value that a tile reads behind its last key -- another head's, another group's, zeros
+// behind the last -- is finite and meets a weight of zero.
 __global__ void __launch_bounds__(256)
 span_gather_kernel(SpanShape sh, LayerKv kv, RowMap rows, const __grid_constant__ SpanBatch b, __half* __restrict__ k16, __half* __restrict__ v16) {
   pdl_enter();
   const int gi = span_group(b.keys_at, b.n, blockIdx.x), t0 = b.t0[gi];
   const GroupKeys gk = group_keys(row_position(rows, t0), b.rows[gi], sh.window, sh.keep_first);
   const int m = (blockIdx.x - b.keys_at[gi]) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, head = blockIdx.y, seq = row_sequence(rows, t0);
-  if (m >= min(b.keys[gi], gk.n + MAX_NK)) return;
+  if (m >= b.keys[gi]) return;
   const int64_t row = (int64_t)b.row0[gi] + (int64_t)head * b.keys[gi] + m;
-  const bool live = m < gk.n, latent = v16 == nullptr;
-  const int j = live ? gk.at(m) : 0;
-  const int64_t page = live ? kv.table[(int64_t)seq * kv.max_blocks + j / kv.block_tokens] : 0, in_page = (int64_t)head * kv.block_tokens + j % kv.block_tokens;
+  const bool latent = v16 == nullptr;
+  const int j = gk.at(m);
+  const int64_t page = kv.table[(int64_t)seq * kv.max_blocks + j / kv.block_tokens], in_page = (int64_t)head * kv.block_tokens + j % kv.block_tokens;
   const float* ks = kv.k + page * kv.k_block + in_page * sh.dk;
-  auto fetch = [&](const float* src, int i, int d) {  // d is a multiple of eight
-    return live && i < d ? *(const float4*)(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-  };
   auto operand = [&](float x) { return latent || (sh.saturate && fabsf(x) <= FLT_MAX) ? fminf(fmaxf(x, -65504.f), 65504.f) : x; };
-  auto words = [&](float4 x) { return make_uint2(pack_h2(operand(x.x), operand(x.y)), pack_h2(operand(x.z), operand(x.w))); };
+  auto words = [&](const float* src) {  // dk and dv are multiples of eight
+    const float4 x = *(const float4*)src;
+    return make_uint2(pack_h2(operand(x.x), operand(x.y)), pack_h2(operand(x.z), operand(x.w)));
+  };
+  for (int i = 4 * lane; i < sh.dk; i += 128) *(uint2*)(k16 + row * sh.dk + i) = words(ks + i);
+  if (latent) return;
   bool special = false;
   auto finite = [&](uint32_t w) {
     const bool not_finite = (w & 0x7c00u) == 0x7c00u || (w & 0x7c000000u) == 0x7c000000u;
     special |= not_finite;
     return not_finite ? 0u : w;
   };
-  const float4 first = fetch(ks, 4 * lane, sh.dk);  // on its way beside the values
-  if (!latent) {
-    const float* vs = kv.v + page * kv.v_block + in_page * sh.dv;
-    for (int i = 4 * lane; i < sh.dv; i += 128) {
-      const uint2 w = words(fetch(vs, i, sh.dv));
-      *(uint2*)(v16 + row * sh.dv + i) = make_uint2(finite(w.x), finite(w.y));
-    }
-    special = __any_sync(~0u, special);
+  const float* vs = kv.v + page * kv.v_block + in_page * sh.dv;
+  for (int i = 4 * lane; i < sh.dv; i += 128) {
+    const uint2 w = words(vs + i);
+    *(uint2*)(v16 + row * sh.dv + i) = make_uint2(finite(w.x), finite(w.y));
   }
-  for (int i = 4 * lane; i < sh.dk; i += 128) {
-    const uint2 w = words(i < 128 ? first : fetch(ks, i, sh.dk));
-    *(uint2*)(k16 + row * sh.dk + i) = special ? make_uint2(0x7fff7fffu, 0x7fff7fffu) : w;
-  }
+  if (__any_sync(~0u, special))  // the same lanes wrote the key
+    for (int i = 4 * lane; i < sh.dk; i += 128) *(uint2*)(k16 + row * sh.dk + i) = make_uint2(0x7fff7fffu, 0x7fff7fffu);
 }
 
 constexpr int PAIRS = 128;
@@ -701,16 +695,16 @@ bool encode_rows(CUtensorMap* map, const void* base, int64_t cols, int64_t rows,
 }
 
 int visible_keys(const SpanShape& sh, const SpanGroup& g) {
-  if (g.first < 0) return span_group_keys(sh, g.rows);
   const int lo = sh.window > 0 ? std::max(0, g.first - sh.window + 1) : 0;  // as group_keys
   return std::min(sh.keep_first, lo) + g.first + g.rows - lo;
 }
 
-}  // namespace
-
+// most keys a group of consecutive rows sees
 int span_group_keys(const SpanShape& sh, int rows) {
   return sh.window > 0 ? (int)std::min<int64_t>(sh.n_ctx, (int64_t)sh.window + sh.keep_first + rows) : sh.n_ctx;
 }
+
+}  // namespace
 
 size_t span_umma_scratch_floats(const SpanShape& sh, int max_rows) {
   return (size_t)sh.n_kv * span_group_keys(sh, max_rows) * (sh.dk + sh.dv) / 2 + 64;
@@ -756,7 +750,9 @@ cudaError_t launch_span_umma(const float* q, int64_t q_ld, const SpanShape& sh, 
   };
   for (int g = 0; g < n_groups && e == cudaSuccess; ++g) {
     if (groups[g].rows < min_rows) continue;
+    if (groups[g].first < 0) return cudaErrorInvalidValue;
     const int mine = visible_keys(sh, groups[g]);
+    if ((size_t)((int64_t)sh.n_kv * mine) * width > 2 * scratch_floats) return cudaErrorInvalidValue;
     if (b.n == SPAN_GROUPS || (b.n > 0 && (size_t)(keys + (int64_t)sh.n_kv * mine) * width > 2 * scratch_floats)) e = run_batch();
     const int i = b.n++;
     b.t0[i] = groups[g].t0;

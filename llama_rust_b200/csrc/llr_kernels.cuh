@@ -338,7 +338,7 @@ cudaError_t launch_attention(const float* q, const KvView& kv, float* out, float
 // The same for the rows of a batch.  groups: runs of rows of one sequence at consecutive positions that make up the batch,
 // ascending (null: all rows are one); with tensor_cores those of 64 rows and more may run as binary16 MMAs with f32
 // accumulation (the tolerance of the 16-bit chunk GEMM).
-struct AttentionGroup { int first, rows, position; };  // position of the first row, -1: the device knows it
+struct AttentionGroup { int first, rows, position; };  // position of the first row, -1: the device alone knows it (fewer than 64 rows)
 cudaError_t launch_attention_groups(const float* q, const KvView& kv, float* out, float* scratch, const RowMap& rows, int tokens, int layer, const WalkShape& w,
                                     const AttentionGroup* groups, int n_groups, bool tensor_cores, size_t scratch_floats, cudaStream_t s, int* err,
                                     uint64_t* launches);
@@ -475,7 +475,8 @@ struct SpanOut {
 };
 size_t span_scratch_floats(const SpanShape& sh, int max_rows);
 bool span_supported(const SpanShape& sh);
-// Rows [t0, t0 + rows) of a batch: one sequence at consecutive positions, from position `first` on (-1: the device knows it).
+// Rows [t0, t0 + rows) of a batch: one sequence at consecutive positions, from position `first` on (-1: the device alone knows it, which no
+// group of the tensor cores may say).
 // With tensor_cores, groups of BF16_TC_MIN_TOKENS rows and more run as binary16 MMAs, all of them in one launch as far as the
 // scratch holds their gathered keys; the rows of shorter groups share a launch of the f32 kernels.
 struct SpanGroup { int t0, rows, first; };
@@ -485,7 +486,6 @@ cudaError_t launch_span_attention(const float* q, int64_t q_ld, const SpanShape&
 // the scratch, then the attention; all groups in one launch of each as far as the scratch holds their keys.
 bool span_umma_supported(const SpanShape& sh, bool shared, const SpanOut& out);
 size_t span_umma_scratch_floats(const SpanShape& sh, int max_rows);
-int span_group_keys(const SpanShape& sh, int rows);  // most keys a group of consecutive rows sees
 cudaError_t launch_span_umma(const float* q, int64_t q_ld, const SpanShape& sh, const LayerKv& kv, const RowMap& rows, const SpanGroup* groups, int n_groups,
                              int min_rows, const SpanOut& out, float* scratch, size_t scratch_floats, cudaStream_t s, int* err, uint64_t* launches);
 // x[t] += y[t] / rms(y[t]) * w, y given as `slices` partial sums `slice_stride` floats apart; x16 (may be null): the new x

@@ -263,3 +263,38 @@ def test_llama_batch_of_every_kind_of_group(ex):
     for q, n in enumerate(lens):
         err, size = np.abs(logits[0][q] - logits[3][q]).max(), np.abs(logits[3][q]).max()
         assert err <= 1e-3 * size if n >= 64 else err <= 1e-5 * size, n
+
+
+def _llama(ex, n_ctx, n_seq, vocab=300, **session):
+    import llama_walk as lw
+    from llama_rust_b200 import Session
+    cfg = dict(n_layer=2, n_embd=256, n_head=4, n_head_kv=2, head_dim=64, n_ff=256, n_vocab=vocab, n_ctx=n_ctx)
+    rng = np.random.default_rng(72)
+    tl = lw.tensor_list(cfg)
+    mats = [ex.upload(ALL["F32"], r, c, (rng.standard_normal(r * c) / np.sqrt(c)).astype(np.float32).view(np.uint8)) for _, _, r, c in tl]
+    embd = ex.upload(ALL["F32"], vocab, 256, rng.standard_normal(vocab * 256).astype(np.float32).view(np.uint8))
+    names = ("attn_q", "attn_k", "attn_v", "attn_output", "ffn_gate", "ffn_up", "ffn_down")
+    return Session(ex, cfg, embd, [dict(zip(names, mats[7 * i:7 * i + 7])) for i in range(2)], output=mats[14], n_seq=n_seq, **session)
+
+
+def test_pool_far_smaller_than_the_context(ex):
+    """The attention scratch is sized for the positions that the pool holds: prompts that fill it, in one batch and in chunks, have the bits
+    they have beside a full pool."""
+    ex.set_path(0)
+    toks = [[(5 * i + 11 * q) % 300 for i in range(320)] for q in range(2)]
+    full, small = _llama(ex, 4096, 2), _llama(ex, 4096, 2, kv_blocks=20)
+    for lens in ([(160, 160)], [(65, 80), (95, 80)], [(0, 100), (0, 100), (0, 119)], [(64, 0), (256, 0)]):
+        got = {}
+        for s in (full, small):
+            s.reset()
+            at, out = [0, 0], []
+            for part in lens:
+                groups = [(q, toks[q][at[q]:at[q] + n]) for q, n in enumerate(part) if n]
+                out.append(s.batch_rows(groups, list(range(sum(part)))))
+                at = [a + n for a, n in zip(at, part)]
+            got[s] = np.concatenate(out)
+        assert _same_bits(got[full], got[small]), lens
+    full.reset(), small.reset()
+    assert _same_bits(full.prefill(toks[0], want_logits=True), small.prefill(toks[0], want_logits=True))
+    full.free()
+    small.free()

@@ -402,7 +402,12 @@ bool encode_rows(CUtensorMap* map, const void* base, int64_t cols, int64_t rows,
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-constexpr int STREAM_SMEM = 1024 + 200 * 1024 + BM * 128 + 512;
+// A stream's shared memory: alignment, stages, what the last stage's MMA reads past its activation rows, barriers.  Two blocks share an SM's
+// 228 KB, of which each takes a kilobyte unasked: 95 KB of stages, three at the widest (four there left one block per SM, 18432 x 4096
+// gated, 64 rows: 86 -> 74 us; one block with the full ring 82).
+constexpr int STREAM_REST = 1024 + BM * 128 + 512, STREAM_STAGES = 200 * 1024, STREAM_STAGES_OF_TWO = 228 * 1024 / 2 - 1024 - STREAM_REST;
+constexpr int STREAM_SMEM = STREAM_STAGES + STREAM_REST;
+static_assert(STREAM_STAGES_OF_TWO / ((64 + 128) * 128) >= 3, "a ring");
 
 template <int BN, int RT, bool GLU>
 cudaError_t launch_tiles(const Bf16Product& p, const Args& a, cudaStream_t stream, int* err) {
@@ -410,7 +415,7 @@ cudaError_t launch_tiles(const Bf16Product& p, const Args& a, cudaStream_t strea
   const int width = GLU ? a.bn / 2 : a.bn;  // rows of one box of W
   if (!encode_rows(&xmap, p.x16, p.x_cols, p.tokens, p.x_ld, RT == 0 ? a.a_rows : BM) || !encode_rows(&wmap, p.w, p.cols, (int64_t)p.rows * (GLU ? 2 : p.batch), p.cols, width))
     return cudaErrorInvalidValue;
-  const int smem = RT == 0 ? 1024 + a.stages * (a.a_rows + a.bn) * 128 + BM * 128 + 512 : RT == 2 ? 1024 + (a.stages * BM + Lay<BN, RT>::NB * a.bn) * 128 + 512 : Lay<BN, RT>::TOTAL;
+  const int smem = RT == 0 ? a.stages * (a.a_rows + a.bn) * 128 + STREAM_REST : RT == 2 ? 1024 + (a.stages * BM + Lay<BN, RT>::NB * a.bn) * 128 + 512 : Lay<BN, RT>::TOTAL;
   static PerDevice ready;
   std::atomic<int>& slot = ready.here();
   if (slot.load(std::memory_order_relaxed) == 0) {
@@ -453,7 +458,7 @@ int stream_width(int tokens, int rows, int batch, int slices) {
   int best = 128;
   int64_t cost = INT64_MAX;
   for (int bn = 128; bn >= 32; bn -= 16) {
-    const int64_t waves = ((int64_t)tiles_of(tokens, rows, batch, bn) * slices + SMS - 1) / SMS, c = waves * (bn + (tokens > 32 ? 32 : 16) + 8);
+    const int64_t waves = ((int64_t)tiles_of(tokens, rows, batch, bn) * slices + SMS - 1) / SMS, c = waves * (bn + (tokens > 32 ? 32 : 16));
     if (c < cost) { cost = c; best = bn; }
   }
   return best;
@@ -495,7 +500,7 @@ cudaError_t launch_gemm_bf16(const Bf16Product& p, cudaStream_t stream, int* err
     a.bn = stream_width(p.tokens, p.rows * (p.glu ? 2 : 1), p.batch, p.slices);
     a.a_rows = p.tokens > 32 ? 64 : 32;
     const bool alone = (int64_t)tiles_of(p.tokens, p.rows * (p.glu ? 2 : 1), p.batch, a.bn) * p.slices <= SMS;
-    a.stages = std::max(4, std::min(16, (alone ? 200 : 80) * 1024 / ((a.a_rows + a.bn) * 128)));
+    a.stages = std::min(16, (alone ? STREAM_STAGES : STREAM_STAGES_OF_TWO) / ((a.a_rows + a.bn) * 128));
     return p.glu ? launch_tiles<128, 0, true>(p, a, stream, err) : launch_tiles<128, 0, false>(p, a, stream, err);
   }
   auto pair_stages = [](int bn) { return std::min(8, (Lay<256, 2>::TOTAL - 1024 - 512 - Lay<256, 2>::NB * bn * 128) / (BM * 128)); };

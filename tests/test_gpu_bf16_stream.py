@@ -23,3 +23,20 @@ def test_few_rows(tmp_path, width, ff):
             got = s.forward([(0, toks[:n])], [list(range(n))])
             assert nm.error(got, want[:n]).max() <= nm.TOLERANCE[nm.AUTO], n
         s.free()
+
+
+# More tiles than SMs: gated products whose widest tiles leave rings of three stages, two blocks to an SM (33 rows and more).
+@pytest.mark.parametrize("layer,ff", [(nm.attention(2, 1, 24, 24, 50, 3, 24), 16640)])
+def test_few_rows_of_many_tiles(tmp_path, layer, ff):
+    from llama_rust_b200 import Executor, models
+    cfg = nm.config(264, 90, [layer], ff)
+    w = nm.weights(cfg, 29, 10, nm.SHARP[nm.AUTO])
+    toks = nm.tokens(65, cfg, 31)
+    want = plain.forward(cfg, w, toks)
+    with Executor(0) as ex:
+        s = models.load(ex, nm.write(tmp_path / "m", cfg, w))
+        for n in (16, 32, 33, 64, 65):
+            s.reset()
+            got = s.forward([(0, toks[:n])], [list(range(n))])
+            assert nm.error(got, want[:n]).max() <= nm.TOLERANCE[nm.AUTO], n
+        s.free()

@@ -496,7 +496,10 @@ cudaError_t launch_gemm_bf16(const Bf16Product& p, cudaStream_t stream, int* err
   if ((a.slices - 1) * ((a.nk + a.slices - 1) / a.slices) >= a.nk) return cudaErrorInvalidValue;
   if (launches) ++*launches;
   if (p.glu) a.glu = *p.glu;
-  if (p.tokens <= STREAM_TOKENS) {
+  // Plain results of 33 to 64 rows leave the stream at one and a half tiles of 128 weight rows per SM: what the tiles then write is no longer
+  // hidden behind weights (4096 columns, 64 rows, streamed and not: 24576 weight rows 56.1 / 56.5 us, 28672 62.9 / 61.7, 128256 205.6 / 196.7).
+  // Gated units, half as many, stay (128256: 206 / 203, and 1 to 8 % faster streamed everywhere below).
+  if (p.tokens <= 32 || (p.tokens <= STREAM_TOKENS && (p.glu || 2 * tiles_of(p.tokens, p.rows, p.batch, 128) <= 3 * SMS))) {
     a.bn = stream_width(p.tokens, p.rows * (p.glu ? 2 : 1), p.batch, p.slices);
     a.a_rows = p.tokens > 32 ? 64 : 32;
     const bool alone = (int64_t)tiles_of(p.tokens, p.rows * (p.glu ? 2 : 1), p.batch, a.bn) * p.slices <= SMS;

@@ -25,8 +25,9 @@ def test_few_rows(tmp_path, width, ff):
         s.free()
 
 
-# More tiles than SMs: gated products whose widest tiles leave rings of three stages, two blocks to an SM (33 rows and more).
-@pytest.mark.parametrize("layer,ff", [(nm.attention(2, 1, 24, 24, 50, 3, 24), 16640)])
+# More tiles than SMs: gated products whose widest tiles leave rings of three stages, two blocks to an SM (33 rows and more); an input
+# product of 29568 rows, which is streamed up to 32 activation rows and takes whole tiles from 33 on.
+@pytest.mark.parametrize("layer,ff", [(nm.attention(2, 1, 24, 24, 50, 3, 24), 16640), (nm.attention(32, 1, 448, 448, 50, 3, 24), 0)])
 def test_few_rows_of_many_tiles(tmp_path, layer, ff):
     from llama_rust_b200 import Executor, models
     cfg = nm.config(264, 90, [layer], ff)

@@ -1804,8 +1804,9 @@ KvView session_kv(const llr_session* s) {
 cudaError_t deliver_rows(llr_exec* e, void* dst, const void* src, size_t bytes) {
   constexpr size_t PIECE = 1 << 20;
   cudaError_t ce;
-  void* alias = nullptr;
-  if (bytes < 256 * 1024 || pinned_alias(dst, &alias)) {
+  cudaPointerAttributes to{};
+  if ((ce = cudaPointerGetAttributes(&to, dst)) != cudaSuccess) return ce;
+  if (bytes < 256 * 1024 || to.type != cudaMemoryTypeUnregistered) {  // what the driver knows it copies to, or refuses, by itself
     if ((ce = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, e->stream)) != cudaSuccess) return ce;
     return cudaStreamSynchronize(e->stream);
   }

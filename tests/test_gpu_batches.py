@@ -277,6 +277,25 @@ def _llama(ex, n_ctx, n_seq, vocab=300, **session):
     return Session(ex, cfg, embd, [dict(zip(names, mats[7 * i:7 * i + 7])) for i in range(2)], output=mats[14], n_seq=n_seq, **session)
 
 
+def test_logits_to_device_memory(ex):
+    """A device pointer is no host buffer: an error or the driver's own copy, never the host's; the session goes on."""
+    import torch
+    from llama_rust_b200.executor import lib
+    V, S = 16411, 8
+    s = _llama(ex, 16, S, vocab=V)
+    seqs, counts, toks, want = np.arange(S, dtype=np.uint32), np.ones(S, np.uint32), np.arange(S, dtype=np.int32) * 31, np.arange(S, dtype=np.uint32)
+    host = s.batch(list(enumerate(toks[:, None].tolist())), want_logits=True)[1]
+    s.reset()
+    there = torch.zeros(S, V, device="cuda")
+    for call in (lambda p: lib().llr_session_batch(s._h, S, seqs.ctypes.data, counts.ctypes.data, toks.ctypes.data, p, None),
+                 lambda p: lib().llr_session_batch_rows(s._h, S, seqs.ctypes.data, counts.ctypes.data, toks.ctypes.data, S, want.ctypes.data, p)):
+        assert call(there.data_ptr()) != 0 or _same_bits(there.cpu().numpy(), host)
+        s.reset()
+        assert _same_bits(s.batch(list(enumerate(toks[:, None].tolist())), want_logits=True)[1], host)
+        s.reset()
+    s.free()
+
+
 def test_pool_far_smaller_than_the_context(ex):
     """The attention scratch is sized for the positions that the pool holds: prompts that fill it, in one batch and in chunks, have the bits
     they have beside a full pool."""

@@ -150,3 +150,110 @@ def test_wide_heads_keep_32_bits(tmp_path, dk, dv):
         s = models.load(ex, nm.write(tmp_path / "m", cfg, w))
         assert nm.error(s.forward([(0, toks)], [list(range(140))]), want).max() <= nm.TOLERANCE[nm.AUTO]
         s.free()
+
+
+# One key that outweighs all others together.  Where it appears after a reference has been taken, sums that lie in tensor memory are rescaled
+# (steps of 128 keys: from key 256 on, each set of warps its own; of 64: from key 64 on), and rows on either side of a window's edge or of the
+# kept tokens' end differ by all of it.
+DOMINANT = {
+    "two sets of warps": (nm.attention(2, 1, 64, 64, 1000, 0, 30), (0, 127, 255, 256, 257, 300, 400)),
+    "a window of two steps": (nm.attention(6, 2, 128, 128, 256, 0, 30), (64, 130, 300)),
+    "kept tokens beyond a step": (nm.attention(4, 2, 72, 128, 40, 140, 30), (127, 139, 140, 200)),
+    "steps of 64 keys": (nm.attention(2, 1, 136, 264, 150, 70, 30), (63, 64, 69, 70, 130, 257)),
+    "latent of 128": (nm.latent(8, 16, 24, 128, 300), (100, 130, 256, 390)),
+    "latent of two parts": (nm.latent(4, 24, 24, 512, 200), (63, 64, 65, 130, 255)),
+}
+
+
+def _dominant(cfg, nats):
+    """Weights of a one-layer model whose last token's key scores about `nats` above the others', which are spread by a third of a nat."""
+    w = nm.weights(cfg, 17, 10, 0.3)
+    L, W = cfg["layers"][0], cfg["width"]
+    m, p, token = L["mixer"], "l0.mix.", cfg["vocab"] - 1
+    H, d = m["heads"], m["dim"]
+    w["embed"][:, :2] = 0  # input 0: this token; input 1: every row
+    w["pos"][:, :2] = [0, 2]
+    w["embed"][token, 0] = 4
+    heads = np.arange(H) * d
+    if L["type"] == "attention":
+        G = m["kv_heads"]
+        keys = np.arange(G) * d
+        w[p + "rel"][:] = 0
+        for t in ("q", "k", "v"):
+            w[p + t][:, :2] = 0
+        for t, at in (("q", heads), ("k", keys)):
+            w[p + t][at], w[p + t + ".b"][at] = 0, 0
+        w[p + "q.b"][heads] = 1
+        w[p + "k"][keys, 0] = 1
+        h = plain.embed(np.asarray([0, token]), w["embed"], w["pos"], cfg["embedding"]["scale"])
+        q, k = (plain.rms(h @ w[p + t].T + w[p + t + ".b"], cfg["norm"]["eps"])[i] for t, i in (("q", 0), ("k", 1)))
+        w[p + "q.norm"][heads] = 1
+        w[p + "k.norm"][keys] = nm.plain.bf16_round(nats / (m["scale"] * q[0] * k[0]))
+    else:
+        for t in ("q", "dkv"):
+            w[p + t][:, :2] = 0
+        w[p + "q"] *= 0.5
+        w[p + "q"][heads], w[p + "q"][heads, 1] = 0, 1
+        w[p + "dkv"][0] = 0
+        w[p + "dkv"][0, 0] = 1
+        w[p + "dkv.norm"][0] = 1
+        w[p + "uk"][:, 0] = 0
+        w[p + "uk"][heads] = 0
+        h = plain.embed(np.asarray([0, token]), w["embed"], w["pos"], cfg["embedding"]["scale"])
+        c = plain.latent_of(h, w, p, cfg["norm"]["eps"])[1, 0]
+        w[p + "uk"][heads, 0] = nm.plain.bf16_round(nats / (m["scale"] * (h @ w[p + "q"].T)[0, 0] * c))
+    return w
+
+
+@pytest.mark.parametrize("name", list(DOMINANT))
+def test_one_dominant_key(tmp_path, name):
+    from llama_rust_b200 import Executor, models
+    layer, places = DOMINANT[name]
+    cfg = nm.config(64, 90, [layer], 0)
+    w = _dominant(cfg, 9.0)
+    with Executor(0) as ex:
+        s = models.load(ex, nm.write(tmp_path / "m", cfg, w))
+        for at in places:
+            toks = [t % 89 for t in nm.tokens(440, cfg, 23 + at)]
+            toks[at] = 89
+            want = plain.forward(cfg, w, toks)
+            for cut in ([440], [130, 310], [16, 41, 383]):
+                s.reset()
+                done, got = 0, []
+                for n in cut:
+                    got.append(s.forward([(0, toks[done:done + n])], [list(range(n))]))
+                    done += n
+                assert nm.error(np.concatenate(got), want).max() <= nm.TOLERANCE[nm.AUTO], (at, cut)
+        s.free()
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(4, 2, 64), (4, 1, 128)])
+def test_one_dominant_key_of_a_llama_prompt(heads, kv_heads, head_dim):
+    """The same through the Llama walk: the last pair of dimensions, which turns by a twentieth of a radian over the prompt, carries the key."""
+    from llama_rust_b200 import Executor
+    E, places, n = heads * head_dim, (127, 255, 256, 300, 400), 460
+
+    def edit(w):
+        embd, wq, wk = w["embd"], w["blk.0.attn_q.weight"], w["blk.0.attn_k.weight"]
+        embd[:, :2] = [0, 1]
+        embd[299, 0] = 4
+        wq *= 0.2
+        for m in (wq, wk):
+            m[:, :2] = 0
+            m[head_dim - 2::head_dim] = 0
+            m[head_dim - 1::head_dim] = 0
+        rows = embd / np.sqrt((embd ** 2).mean(1, keepdims=True))
+        wq[head_dim - 2::head_dim, 1] = 1
+        wk[head_dim - 2::head_dim, 0] = 9.0 * np.sqrt(head_dim) / (rows[0, 1] * rows[299, 0])
+    with Executor(0) as ex:
+        s = _llama(ex, 512, 2, heads, kv_heads, head_dim, edit=edit)
+        for at in places:
+            toks = (7 * np.arange(n) + at) % 299
+            toks[at] = 299
+            got = {}
+            for path in (3, 0):
+                ex.set_path(path)
+                s.reset()
+                got[path] = s.batch_rows([(1, toks.tolist())], list(range(n)))
+            assert np.abs(got[0] - got[3]).max() <= 2e-3 * np.abs(got[3]).max(), at
+        s.free()

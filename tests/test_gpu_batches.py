@@ -277,6 +277,25 @@ def _llama(ex, n_ctx, n_seq, vocab=300, **session):
     return Session(ex, cfg, embd, [dict(zip(names, mats[7 * i:7 * i + 7])) for i in range(2)], output=mats[14], n_seq=n_seq, **session)
 
 
+def test_logits_to_pageable_memory(ex):
+    """What goes through two pinned pieces of a megabyte in turn (from 256 KB on) has the bytes of a copy to pinned memory: less than a piece,
+    a piece and a little, two whole pieces and a little, five; to addresses that are not a page's."""
+    import torch
+    from llama_rust_b200.executor import lib
+    V, S = 16411, 64  # 65644 bytes a row
+    s = _llama(ex, 16, S, vocab=V)
+    for groups in (1, 3, 4, 16, 17, 32, 47, 64):
+        seqs, counts, toks = np.arange(groups, dtype=np.uint32), np.ones(groups, np.uint32), np.arange(groups, dtype=np.int32) * 31
+        pinned = torch.full((groups * V,), float("nan")).pin_memory()
+        for shift in (0, 1, 1023):
+            room = np.full(groups * V + shift + 1, 7, np.float32)
+            for ptr in (pinned.data_ptr(), room[shift:].ctypes.data):
+                s.reset()
+                ex._check(lib().llr_session_batch(s._h, groups, seqs.ctypes.data, counts.ctypes.data, toks.ctypes.data, ptr, None))
+            assert _same_bits(room[shift:-1], pinned.numpy()) and (room[:shift] == 7).all() and room[-1] == 7, (groups, shift)
+    s.free()
+
+
 def test_logits_to_device_memory(ex):
     """A device pointer is no host buffer: an error or the driver's own copy, never the host's; the session goes on."""
     import torch
@@ -294,6 +313,30 @@ def test_logits_to_device_memory(ex):
         assert _same_bits(s.batch(list(enumerate(toks[:, None].tolist())), want_logits=True)[1], host)
         s.reset()
     s.free()
+
+
+def test_a_batch_that_runs_out_of_blocks(ex):
+    """A batch that fails in the middle of its reservations leaves the blocks of its first groups theirs: what follows finds them."""
+    from llama_rust_b200.executor import NativeCudaError
+    ex.set_path(0)
+    toks = [[(5 * i + 11 * q) % 300 for i in range(60)] for q in range(3)]
+    roomy, tight = _llama(ex, 64, 3), _llama(ex, 64, 3, kv_blocks=6)  # 16 positions a block
+    first = [(0, toks[0][:20]), (1, toks[1][:40])]  # two blocks and three
+    with pytest.raises(NativeCudaError):
+        tight.batch(first + [(2, toks[2][:40])])
+    assert [tight.seq_position(q) for q in range(3)] == [0, 0, 0]
+    for groups in (first, [(0, toks[0][20:32]), (1, toks[1][40:48])], [(0, toks[0][32:33])]):
+        assert _same_bits(tight.batch(groups, want_logits=True)[1], roomy.batch(groups, want_logits=True)[1])
+    with pytest.raises(NativeCudaError):
+        tight.batch([(1, toks[1][48:49])])
+    tight.seq_reset(0), roomy.seq_reset(0)
+    groups = [(2, toks[2][:33]), (1, toks[1][48:50])]
+    with pytest.raises(NativeCudaError):
+        tight.batch(groups + [(0, toks[0][:1])])
+    for g in (groups[1:], [(2, toks[2][:16])]):
+        assert _same_bits(tight.batch(g, want_logits=True)[1], roomy.batch(g, want_logits=True)[1])
+    roomy.free()
+    tight.free()
 
 
 def test_pool_far_smaller_than_the_context(ex):

@@ -102,9 +102,9 @@ def test_prompt_attention_on_tensor_cores_agrees_with_the_f32_kernels(orc, n_hea
     """Prompt chunks of 64 rows and more run their attention as binary16 MMAs with f32 accumulation on the automatic path.
     With F32 weights the products are the same f32 kernels on both paths, so the logits of the automatic path and of the
     f32-faithful path differ by the attention kernel alone: they must agree within the 16-bit tolerance (1e-3 of the
-    logit scale; a misplaced fragment would change them by the scale itself), for slices of 32 and of 64 positions, one
-    to eight query heads per kv head, prompts that are not a multiple of the row tile, a second chunk that starts in
-    the middle of a slice, and against the CPU walk."""
+    logit scale; a misplaced fragment would change them by the scale itself), for one to eight query heads per kv head, contexts with
+    f32 slices of 32, 64 and 128 positions beside them, prompts that are not a multiple of the row tile, a second chunk that starts in the
+    middle of a step of 128 keys, and against the CPU walk.  (Prompts beyond two steps: test_gpu_attention_tiles.py.)"""
     from llama_rust_b200 import Executor
     from helpers import F32
     cfg = dict(n_layer=2, n_embd=n_head * head_dim, n_head=n_head, n_head_kv=n_head_kv, head_dim=head_dim, n_ff=256, n_vocab=300)
@@ -122,7 +122,7 @@ def test_prompt_attention_on_tensor_cores_agrees_with_the_f32_kernels(orc, n_hea
         ex.set_path(path)
         s = _session(ex, cfg, n_ctx, mats, embd_mat)
         a = s.prefill(prompt, want_logits=True)
-        b = s.prefill(more, want_logits=True)  # positions 150..226: the chunk starts inside a slice
+        b = s.prefill(more, want_logits=True)  # positions 150..226: the chunk starts inside a step
         logits[path] = (a, b)
         s.free()
     cpu = lw.run_cpu(cfg, n_ctx, weights, embd, np.concatenate([prompt, more]), 0, want_logits=True, kinds=[F32] * len(tl), embd_kind=F32)[2]

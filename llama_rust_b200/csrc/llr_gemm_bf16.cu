@@ -14,12 +14,14 @@
 //
 // One CTA computes a tile of 128 or 256 activation rows x bn <= BN weight rows: the activation rows are the MMA's M dimension (one
 // tensor-memory lane each), so that a thread of the epilogue holds consecutive results of one activation row and stores
-// them as vectors.  One warp issues the TMA loads, one the MMAs, four read the accumulators, eight where a CTA has the SM to itself.
+// them as vectors.  One warp issues the TMA loads and one the MMAs; four read the accumulators, eight in wide tiles.  Tiles of 256 activation
+// rows have a ring per operand, a warp of MMAs for each half and sixteen for the results.
 // Two CTAs fit an SM at BN <= 128 (96 KB of stages, 128 columns of tensor memory each), so one tile's epilogue overlaps another's
 // loads.  Wide tiles are bound by what the SMs draw from L2, so 256 activation rows share a stage's weights where that saves waves
 // (tile_shape).  Up to 64 activation rows the product is a stream of weights: a stage then holds 32 or 64 activation rows (the MMA
 // reads on into the weights behind them: rows of its result that nobody looks at), tiles of 32 .. 128 weight rows spread it over the SMs
-// (stream_width) and up to sixteen stages of it are under way.  16384 x 2048 gated, 32 rows: 25 -> 18 us.  A K range may be cut into
+// (stream_width) and up to sixteen stages of it are under way; plain results of 33 rows and more against very many weight rows go by whole
+// tiles again (launch_gemm_bf16).  16384 x 2048 gated, 32 rows: 25 -> 18 us.  A K range may be cut into
 // slices (gridDim.z): slice s leaves its partial sums at y + s * slice_stride and the reader adds them in slice order.  Every wait is
 // bounded.
 #include <cuda.h>
@@ -31,13 +33,21 @@
 #include "llr_formats.cuh"
 #include "llr_kernels.cuh"
 #include "llr_tmap.cuh"
+#include "llr_umma.cuh"
 
 namespace llr {
 namespace {
 
+using umma::bar_expect;
+using umma::bar_init;
+using umma::bar_wait;
+using umma::bar_wait2;
+using umma::elect_one;
+using umma::DESC_HI;  // operand tiles are K-major 128-byte swizzled rows, eight-row groups 1024 bytes apart
+using umma::s32;
+
 constexpr int BM = 128;  // activation rows per MMA = UMMA M
 constexpr int BK = 64;   // columns per stage: one 128-byte swizzle row
-constexpr int SPIN = 1 << 24;
 
 // RT: tiles of BM activation rows per CTA; 0: at most 64 activation rows, stages and their number by the launch
 template <int BN, int RT> struct Lay {
@@ -45,45 +55,10 @@ template <int BN, int RT> struct Lay {
   static constexpr int NS = RT == 0 ? 16 : RT == 2 ? 8 : BN == 256 ? 4 : BN == 128 ? 3 : 4;  // 192, 96, 96 KB
   static constexpr int NB = 4;  // two tiles of activation rows: stages of weights, beside a ring of at most NS single tiles
   static constexpr int EPI = BN < 256 ? 4 : RT == 2 ? 16 : 8, W_TMA = EPI, W_MMA = EPI + 1, THREADS = (EPI + 2 + (RT == 2)) * 32;  // epilogue warps first
-  static constexpr int TOTAL = RT == 2 ? 232448 : 1024 /*alignment*/ + NS * STAGE + 512;
+  static constexpr int TOTAL = RT == 2 ? umma::SMEM_LIMIT : 1024 /*alignment*/ + NS * STAGE + 512;
   static constexpr int TMEM_COLS = RT == 0 ? BN : RT * BN;
 };
 
-__device__ __forceinline__ uint32_t s32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void bar_init(uint64_t* b, int n) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(s32(b)), "r"(n) : "memory");
-}
-__device__ __forceinline__ void bar_expect(uint64_t* b, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(s32(b)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t parity) {
-  for (int spins = 0; spins < SPIN; ++spins) {
-    uint32_t ok;
-    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-                 : "=r"(ok) : "r"(s32(b)), "r"(parity) : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-// both barriers asked in one go
-__device__ __forceinline__ bool bar_wait2(uint64_t* a, uint32_t pa, uint64_t* b, uint32_t pb) {
-  for (int spins = 0; spins < SPIN; ++spins) {
-    uint32_t ok;
-    asm volatile(
-        "{ .reg .pred p, q; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4; "
-        "and.pred p, p, q; selp.u32 %0, 1, 0, p; }"
-        : "=r"(ok) : "r"(s32(a)), "r"(pa), "r"(s32(b)), "r"(pb) : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-__device__ __forceinline__ bool elect_one() {
-  uint32_t pred;
-  asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(pred));
-  return pred != 0;
-}
-// Operand tiles are K-major 128-byte swizzled rows, eight-row groups 1024 bytes apart: the high word of their descriptors is always this
-constexpr uint32_t DESC_HI = 64u | (1u << 14) | (2u << 29);
 // kind::f16: f32 accumulator, both operands bfloat16, M = 128, N = bn
 __device__ __forceinline__ uint32_t mma_desc(int bn) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);

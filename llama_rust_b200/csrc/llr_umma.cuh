@@ -1,5 +1,5 @@
-// What the kernels that feed dequantized tiles to tcgen05.mma share (llr_gemm_tc.cu, llr_gemm_i8.cu): mbarrier wrappers with
-// bounded waits, shared-memory descriptors, the packed-byte ring's geometry and the Q6_K code unpacking.
+// What the kernels on tcgen05.mma share: mbarrier wrappers with bounded waits and shared-memory descriptors; for those that feed it
+// dequantized tiles (llr_gemm_tc.cu, llr_gemm_i8.cu) the packed-byte ring's geometry and the Q6_K code unpacking.
 #pragma once
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>

@@ -544,8 +544,10 @@ __device__ __forceinline__ void gemm_tc_tile(const CUtensorMap* wmap_p, const CU
     // memory store completion and arrivals for two steps instead of one each.
     static_assert(NA % 2 == 0 && NA > 4, "a group's two steps of a macro-step use different stages");
     // One warp issues a group's steps in order, so the later one's stage is free only after the earlier one's.  Asking a barrier takes
-    // 100 ns: where decoding is short (Q4_K) both of a macro-step's are asked in one go before it, elsewhere the stage's comes behind it
-    // (77 rows of Q5_1 84.2 us that way, 85.2 asked before).
+    // 100 ns: where decoding is short (Q4_K) both of a macro-step's are asked in one go before it, elsewhere the stage's comes behind it.
+    // Six products of 77 rows of Q5_1: 82.2 us that way, 83.8 asked before.  At 512 rows x 4096 x 14336 the order hardly matters
+    // (behind / before, us: Q4_0 61.5 / 61.0, Q4_1 62.4 / 61.9, Q5_0 63.4 / 62.9, Q5_1 63.7 / 63.2, Q8_0 63.6 / 63.5, Q5_K 64.6 / 64.6,
+    // Q6_K 66.6 / 66.1, Q4_K 62.6 / 62.1).
     constexpr bool FIRST = DT == DT_Q4_K && F16;
     int ps = 0, s0 = g;
     int s1 = g + 2;

@@ -6,7 +6,7 @@
 // row-major order -- all query heads of a kv head share its keys, so any ratio of heads fills the tile -- and walks the keys
 // that any of its rows sees, NK at a time:
 //   scores   S = Q K^T      tcgen05.mma, Q and K from shared memory (K-major), f32 accumulators in tensor memory, two buffers
-//   weights  P = 2^(S - m)  one pair per lane of tensor memory; binary16 back into tensor memory
+//   weights  P = 2^(S - m)  one pair per lane of tensor memory; binary16 back into tensor memory (SPLIT: and the rest)
 //   sums     O += P V       tcgen05.mma, P from tensor memory, V from shared memory as it lies (dimensions run fastest: MN-major)
 // Queries (rescaled per pair by a power of two), keys, values and the exponentials are binary16 operands; scores and sums are f32;
 // scale, distance bias, mask, maxima, exponentials and their sums are f32.
@@ -29,9 +29,12 @@
 // scores' operand traffic in shared memory.  The code is kept short (scores are masked and biased by rolled loops over 32 of them, in
 // place): a launch finds the instruction caches cold, and straight-line code then runs at eight instructions in 50 ns.  Unrolled,
 // steps with masks or biases took 5 to 9 us instead of one, and a pass over the results 12.
-// Error against 64 bits, 512 rows, 4 heads of 128 over one, scores spread by 1 / 2 / 3 nats: 3.43 / 4.94 / 5.75e-4; what rounding the
-// operands alone costs is 3.1 / 4.8 / 5.7e-4.  Weights are rounded once per reference, of which there are two; slices with a reference each
-// (mma.sync, four runs of 32 keys) rounded more of the large ones to 1: 3.39 / 4.90 / 5.72e-4.
+// Weights rounded to binary16 are a third of the error where scores are spread by a nat.  A reference per slice (four runs of 32 keys on
+// mma.sync) rounded more of the large ones to 1; with two references for all keys the Llama walk was further from 64 bits (512 rows, 4 heads of 128
+// over one, scores spread by 1 / 2 / 3 nats: 3.39 / 4.90 / 5.72e-4 -> 3.43 / 4.94 / 5.75e-4).  So there (SPLIT) a weight is two binary16 numbers, it
+// and what rounding has left of it, in the 32 columns of the scores of its 32 keys, and the second product has two MMAs for one: 3.15 / 4.83 /
+// 5.69e-4, which is what rounding queries, keys and values costs; a launch of 512 rows, 32 heads of 128 26.1 -> 27.9 us.  Layered decoders, whose
+// products are bfloat16, are as far from 64 bits either way (1.573e-3, 1.574e-3).
 // Measured, one launch: 2048 pairs x 8 kv heads of 128 dimensions, 1500 keys, window 1024, biases and gates 100 -> 35 us (mma.sync, 64
 // pairs a block, before); 512 rows x 32 heads, latent of 512, window 1024 169 -> 75 us.
 #include <cuda.h>
@@ -217,7 +220,7 @@ __device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint32_t b, uint3
 }
 
 // grid (tiles of all groups x parts, kv head)
-template <int KC, int NK>
+template <int KC, int NK, bool SPLIT>
 __global__ void __launch_bounds__(Lay<KC, NK>::THREADS, 1)
 span_umma_kernel(const float* q, int64_t q_ld, SpanShape sh, Shape ms, const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                  RowMap rows, const __grid_constant__ SpanBatch b, SpanOut so, int* __restrict__ err) {
@@ -359,8 +362,11 @@ span_umma_kernel(const float* q, int64_t q_ld, SpanShape sh, Shape ms, const __g
         const uint32_t idesc = mma_desc(min(128 * run, (own_dims - 128 * i + 15) & ~15), true), o = tmem + (uint32_t)((ALT ? 128 * (j & 1) : 0) + 128 * i);
         if (leader) {
 #pragma unroll
-          for (int kk = 0; kk < NK / 16; ++kk)  // sixteen keys: two groups of eight 128-byte rows
-            mma_ts(o, p + (uint32_t)(8 * kk), lb + (uint32_t)(128 * kk), idesc, acc | (uint32_t)kk);
+          for (int kk = 0; kk < NK / 16; ++kk) {  // sixteen keys: two groups of eight 128-byte rows
+            const uint32_t pk = p + (uint32_t)(SPLIT ? 32 * (kk >> 1) + 8 * (kk & 1) : 8 * kk);
+            mma_ts(o, pk, lb + (uint32_t)(128 * kk), idesc, acc | (uint32_t)kk);
+            if constexpr (SPLIT) mma_ts(o, pk + 16, lb + (uint32_t)(128 * kk), idesc, 1u);
+          }
           for (int k = 0; k < run; ++k) commit(&empty[at + k]);
         }
         i += run;
@@ -550,17 +556,20 @@ span_umma_kernel(const float* q, int64_t q_ld, SpanShape sh, Shape ms, const __g
         }
 #pragma unroll
         for (int k = 0; k < CB; k += 32) {
-          uint32_t e[16];
+          uint32_t e[SPLIT ? 32 : 16];
           float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            e[i] = pack_h2(exp2_ftz(fmaf(s[k + 2 * i], mul, add)), exp2_ftz(fmaf(s[k + 2 * i + 1], mul, add)));
-            const __half2 e2 = *(const __half2*)&e[i];  // the sum of what the weighted sum uses
-            sum0 += __low2float(e2);
-            sum1 += __high2float(e2);
+            const float e0 = exp2_ftz(fmaf(s[k + 2 * i], mul, add)), e1 = exp2_ftz(fmaf(s[k + 2 * i + 1], mul, add));
+            e[i] = pack_h2(e0, e1);
+            const float2 r = __half22float2(*(const __half2*)&e[i]);
+            if constexpr (SPLIT) e[16 + i] = pack_h2(e0 - r.x, e1 - r.y);
+            sum0 += SPLIT ? e0 : r.x;  // the sum of what the weighted sum uses
+            sum1 += SPLIT ? e1 : r.y;
           }
           l += sum0 + sum1;
-          tst16(t_s + (uint32_t)((half * NC + c + k) / 2), e);
+          if constexpr (SPLIT) tst32(t_mine + (uint32_t)(c + k), (const float*)e);
+          else tst16(t_s + (uint32_t)((half * NC + c + k) / 2), e);
         }
       }
       tst_wait();
@@ -672,18 +681,23 @@ struct Variant {
 };
 // Steps of 128 keys where the values fit 128 columns of tensor memory, of 64 otherwise; the queries' chunks are rounded up to an
 // instance's.  The longest keys that have 16-bit operands leave a ring of four pairs, which the queries pass through before it starts.
-Variant variant(int dk, int dv) {
+Variant variant(int dk, int dv, bool split) {
   const int kc = (dk + 63) / 64;
-#define LLR_V(K, N) { static PerDevice ready; return Variant{span_umma_kernel<K, N>, N, Lay<K, N>::TOTAL, Lay<K, N>::THREADS, &ready}; }
-  if (dv <= 128) {
-    if (kc <= 1) LLR_V(1, 128)
-    if (kc <= 2) LLR_V(2, 128)
-    if (kc <= 4) LLR_V(4, 128)
+#define LLR_V(K, N, S) { static PerDevice ready; return Variant{span_umma_kernel<K, N, S>, N, Lay<K, N>::TOTAL, Lay<K, N>::THREADS, &ready}; }
+  if (split) {
+    if (dv <= 128 && kc <= 1) LLR_V(1, 128, true)
+    if (dv <= 128 && kc <= 2) LLR_V(2, 128, true)
+    return Variant{nullptr, 0, 0, 0, nullptr};
   }
-  if (kc <= 4) LLR_V(4, 64)
-  if (kc <= 8) LLR_V(8, 64)
-  if (kc <= 12) LLR_V(12, 64)
-  if (kc <= 14) LLR_V(14, 64)
+  if (dv <= 128) {
+    if (kc <= 1) LLR_V(1, 128, false)
+    if (kc <= 2) LLR_V(2, 128, false)
+    if (kc <= 4) LLR_V(4, 128, false)
+  }
+  if (kc <= 4) LLR_V(4, 64, false)
+  if (kc <= 8) LLR_V(8, 64, false)
+  if (kc <= 12) LLR_V(12, 64, false)
+  if (kc <= 14) LLR_V(14, 64, false)
 #undef LLR_V
   return Variant{nullptr, 0, 0, 0, nullptr};
 }
@@ -725,14 +739,14 @@ static bool sixteen_bit_heads(int dk, int dv, bool shared) {
 }
 
 bool span_umma_supported(const SpanShape& sh, bool shared, const SpanOut& out) {
-  return sh.n_kv > 0 && sh.n_head % sh.n_kv == 0 && sh.dk % 8 == 0 && sh.dv % 8 == 0 && sixteen_bit_heads(sh.dk, sh.dv, shared) && variant(sh.dk, sh.dv).kernel &&
+  return sh.n_kv > 0 && sh.n_head % sh.n_kv == 0 && sh.dk % 8 == 0 && sh.dv % 8 == 0 && sixteen_bit_heads(sh.dk, sh.dv, shared) && variant(sh.dk, sh.dv, sh.split_weights).kernel &&
          (int64_t)sh.n_kv * sh.n_ctx < (1 << 30) && out.ld % 2 == 0 && ((uintptr_t)out.out & 7) == 0 && ((uintptr_t)out.out16 & 3) == 0 &&
          (!out.gate || out.head_gate || (out.gate_ld % 2 == 0 && ((uintptr_t)out.gate & 7) == 0));
 }
 
 cudaError_t launch_span_umma(const float* q, int64_t q_ld, const SpanShape& sh, const LayerKv& kv, const RowMap& rows, const SpanGroup* groups, int n_groups,
                              int min_rows, const SpanOut& out, float* scratch, size_t scratch_floats, cudaStream_t s, int* err, uint64_t* launches) {
-  const Variant v = variant(sh.dk, sh.dv);
+  const Variant v = variant(sh.dk, sh.dv, sh.split_weights);
   const bool shared = kv.k == kv.v;
   const int gq = sh.n_head / sh.n_kv, width = sh.dk + (shared ? 0 : sh.dv);
   const Shape ms{(sh.dv + PART - 1) / PART, shared};

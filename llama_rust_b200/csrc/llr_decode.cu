@@ -637,6 +637,7 @@ static SpanShape span_shape(const WalkShape& w) {
   sh.n_head = w.n_head; sh.n_kv = w.n_head_kv; sh.dk = sh.dv = w.head_dim; sh.n_ctx = w.n_ctx;
   sh.scale = 1.0f / sqrtf((float)w.head_dim);
   sh.saturate = false;  // a model whose values leave binary16's range shows it in its logits
+  sh.split_weights = true;
   return sh;
 }
 

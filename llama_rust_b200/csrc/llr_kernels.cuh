@@ -414,6 +414,7 @@ struct SpanShape {
   int bias_len;
   const float* sink;  // [n_head], or null
   bool saturate = true;  // 16-bit operands: finite keys and values beyond binary16's range become its largest number, not infinities
+  bool split_weights = false;  // 16-bit operands: exponentials as two binary16 numbers each (heads of at most 128 dimensions)
 };
 // Rotation of a head's first dims values, pairs (i, i + dims / 2): row t's cosines and sines are the dims / 2 entries from
 // cs + t * ld on.  dims 0: none.

@@ -53,12 +53,12 @@ def test_tiles(tmp_path, name):
         s.free()
 
 
-def _llama(ex, n_ctx, n_seq=1, heads=4, kv_heads=2, head_dim=64, vocab=300, edit=None, **session):
+def _llama(ex, n_ctx, n_seq=1, heads=4, kv_heads=2, head_dim=64, vocab=300, edit=None, rms_eps=1e-5, **session):
     """A small Llama session with F32 weights: what differs between the paths is attention alone.  edit(weights) changes them by name."""
     import llama_walk as lw
     from helpers import ALL
     from llama_rust_b200 import Session
-    cfg = dict(n_layer=2, n_embd=heads * head_dim, n_head=heads, n_head_kv=kv_heads, head_dim=head_dim, n_ff=256, n_vocab=vocab)
+    cfg = dict(n_layer=2, n_embd=heads * head_dim, n_head=heads, n_head_kv=kv_heads, head_dim=head_dim, n_ff=256, n_vocab=vocab, rms_eps=rms_eps)
     rng = np.random.default_rng(72)
     w = {n: (rng.standard_normal((r, c)) / np.sqrt(c)).astype(np.float32) for n, _, r, c in lw.tensor_list(cfg)}
     w["embd"] = rng.standard_normal((vocab, cfg["n_embd"])).astype(np.float32)
@@ -256,4 +256,32 @@ def test_one_dominant_key_of_a_llama_prompt(heads, kv_heads, head_dim):
                 s.reset()
                 got[path] = s.batch_rows([(1, toks.tolist())], list(range(n)))
             assert np.abs(got[0] - got[3]).max() <= 2e-3 * np.abs(got[3]).max(), at
+        s.free()
+
+
+@pytest.mark.parametrize("head_dim", [64, 128])
+def test_weights_of_a_llama_prompt_are_not_rounded_to_binary16(head_dim):
+    """Values of +-64 and scores within a few sixteenths of a nat: what 16-bit queries and keys cost is an eleventh-bit rounding of those
+    (2^-11 / 16, twice), while weights rounded to eleven bits would be off by 2^-11 / sqrt(12) = 1.4e-4, and the results with them."""
+    from llama_rust_b200 import Executor
+    E, n = 2 * head_dim, 400
+
+    def edit(w):
+        w["embd"][:] = np.where(w["embd"] > 0, 1, -1)  # root mean square 1: the norm leaves them
+        rng = np.random.default_rng(5)
+        for t, size in (("q", 1 / 16), ("k", 1), ("v", 64)):
+            m = w[f"blk.0.attn_{t}.weight"]
+            m[:] = 0
+            m[np.arange(len(m)), rng.permutation(E)[np.arange(len(m)) % E]] = size
+        for name in ("blk.0.ffn_down.weight", "blk.1.attn_output.weight", "blk.1.ffn_down.weight"):
+            w[name][:] = 0
+    toks = np.random.default_rng(6).integers(0, 300, n).tolist()
+    with Executor(0) as ex:
+        s = _llama(ex, 512, 1, 2, 1, head_dim, edit=edit, rms_eps=0.0)
+        got = {}
+        for path in (3, 0):
+            ex.set_path(path)
+            s.reset()
+            got[path] = s.batch_rows([(0, toks)], list(range(100, n))).astype(np.float64)
+        assert np.linalg.norm(got[0] - got[3]) <= 4e-5 * np.linalg.norm(got[3])
         s.free()

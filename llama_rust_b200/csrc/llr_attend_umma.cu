@@ -33,7 +33,7 @@
 // mma.sync) rounded more of the large ones to 1; with two references for all keys the Llama walk was further from 64 bits (512 rows, 4 heads of 128
 // over one, scores spread by 1 / 2 / 3 nats: 3.39 / 4.90 / 5.72e-4 -> 3.43 / 4.94 / 5.75e-4).  So there (SPLIT) a weight is two binary16 numbers, it
 // and what rounding has left of it, in the 32 columns of the scores of its 32 keys, and the second product has two MMAs for one: 3.15 / 4.83 /
-// 5.69e-4, which is what rounding queries, keys and values costs; a launch of 512 rows, 32 heads of 128 26.1 -> 27.9 us.  Layered decoders, whose
+// 5.69e-4, which is what rounding queries, keys and values costs; a launch of the walk, 512 rows, 32 heads of 128 over 8, 20.9 -> 21.0 us.  Layered decoders, whose
 // products are bfloat16, are as far from 64 bits either way (1.573e-3, 1.574e-3).
 // Measured, one launch: 2048 pairs x 8 kv heads of 128 dimensions, 1500 keys, window 1024, biases and gates 100 -> 35 us (mma.sync, 64
 // pairs a block, before); 512 rows x 32 heads, latent of 512, window 1024 169 -> 75 us.

@@ -142,7 +142,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
   bool ok = true;
 
   if (PAIR && warp == W_TMA) {
-    // Two rings: weights four steps deep, tiles of 128 activation rows three to four.  Stages of both tiles and the weights together were three
+    // Two rings: weights four steps deep, tiles of 128 activation rows three or four for each half.  Stages of both tiles and the weights together were three
     // (64 KB each), and a place that is free only once all eight MMAs of a step are done came back late: steps of 0.62 us instead of 0.47.
     const uint32_t base = __shfl_sync(0xffffffffu, s32(smem), 0), base_b = base + (uint32_t)(NS * BM * 128);
     auto load_w = [&](int k, int s) {
@@ -404,6 +404,17 @@ cudaError_t launch_tiles(const Bf16Product& p, const Args& a, cudaStream_t strea
   return launch_overlapped(gemm_bf16_kernel<BN, RT, GLU>, grid, Lay<BN, RT>::THREADS, smem, stream, xmap, wmap, a, err);
 }
 
+// Two tiles of activation rows: single tiles in their ring, as many as fit beside the weights, an EVEN number.  The halves take the places in
+// turn, and a barrier says no more than the parity of its phase: a half that shared a place with the other and got ahead of it by a lap --
+// copies need not arrive in order -- would take the phase of two laps ago for its own, multiply a tile that is not there and free it twice.
+constexpr int pair_stages(int bn) { return std::min(8, (Lay<256, 2>::TOTAL - 1024 - 512 - Lay<256, 2>::NB * bn * 128) / (BM * 128)) & ~1; }
+constexpr bool even_rings() {
+  for (int bn = 160; bn <= 256; bn += 16)
+    if (pair_stages(bn) % 2 != 0 || pair_stages(bn) < 4) return false;
+  return true;
+}
+static_assert(even_rings(), "a place of the ring belongs to one half");
+
 constexpr int SMS = 148;
 int tiles_of(int tokens, int rows, int batch, int bn, int rt = 1) { return ((tokens + rt * BM - 1) / (rt * BM)) * ((rows + bn - 1) / bn) * batch; }
 // Shape of a tile.  Few tiles: 128 or 64 weight rows.  Many: 160 .. 256 weight rows (a multiple of `step`, so that both halves of a
@@ -481,7 +492,6 @@ cudaError_t launch_gemm_bf16(const Bf16Product& p, cudaStream_t stream, int* err
     a.stages = std::min(16, (alone ? STREAM_STAGES : STREAM_STAGES_OF_TWO) / ((a.a_rows + a.bn) * 128));
     return p.glu ? launch_tiles<128, 0, true>(p, a, stream, err) : launch_tiles<128, 0, false>(p, a, stream, err);
   }
-  auto pair_stages = [](int bn) { return std::min(8, (Lay<256, 2>::TOTAL - 1024 - 512 - Lay<256, 2>::NB * bn * 128) / (BM * 128)); };
   if (p.glu) {
     const Tile tile = tile_shape(p.tokens, 2 * p.rows, 1, 32);
     a.bn = std::max(tile.bn, 128);

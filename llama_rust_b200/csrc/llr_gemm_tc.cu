@@ -85,6 +85,7 @@ template <int DT, int BN> struct GLay {
   static constexpr int NPK_FIT = (SMEM_LIMIT - FIXED - P) / P_STAGE;
   static constexpr int NPK = NPK_FIT > 6 ? 6 : NPK_FIT;
   static_assert(NPK >= 2, "packed ring needs two stages");
+  static_assert(NB % NMMA == 0 && NA % NMMA == 0, "a stage belongs to one MMA warp: it waits for every phase of the stage's barriers");
   static constexpr int BAR = P + NPK * P_STAGE + 64;  // full_a, empty_a [NA]; full_b, empty_b [NB]; pk_full, pk_empty [NPK]; acc_full; tmem slot
   static constexpr int TOTAL = BAR + 1024 + 1024;
   static_assert((2 * NA + 2 * NB + 2 * NPK + 2) * 8 <= 1024, "barrier block");

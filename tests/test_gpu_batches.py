@@ -118,6 +118,28 @@ def test_wide_tiles_of_bf16_products(ex, rows, cols, tokens):
     m.free()
 
 
+@pytest.mark.parametrize("rows", [10240, 12288, 14336, 16384])  # tiles of 160, 176, 208 and 224 weight rows: rings of eight, eight, six and six
+def test_paired_tiles_give_the_same_bits_each_time(ex, rows):
+    """Two tiles of activation rows, the second almost empty (257 rows: three of them; its copies arrive first), 64 column steps."""
+    import torch
+    from llama_rust_b200 import synth
+    ex.set_path(0)
+    m = ex.synth(ALL["BF16"], rows, 4096, 5)
+    x = torch.from_numpy(synth.activations(300 * 4096, 6)).cuda()
+    for tokens in (257, 300):
+        want = torch.empty(tokens, rows, device="cuda")
+        got = torch.empty_like(want)
+        ex.matmul_device(m, tokens, x.data_ptr(), want.data_ptr())
+        ex.synchronize()
+        for _ in range(20):
+            got.fill_(float("nan"))
+            torch.cuda.synchronize()
+            ex.matmul_device(m, tokens, x.data_ptr(), got.data_ptr())
+            ex.synchronize()
+            assert torch.equal(got, want), tokens
+    m.free()
+
+
 def test_wide_tiles_of_gated_units(ex, tmp_path):
     """A feed-forward layer whose gate | up product takes tiles of 256 activation rows, against the plain model."""
     from llama_rust_b200 import models
